@@ -13,7 +13,7 @@ plain FP64 form.  One step = one Newton finite-difference triple
 
 Also reported: roofline of the contraction kernel (algorithmic FLOPs
 8 N_alpha^2 K per determinant against an in-run cuBLAS DGEMM peak, and the
-DMMA work the chosen 4M or 3M form issues), the split-BF16 form, Newton
+DMMA work the kernel issues), the split-BF16 form, Newton
 time-to-root from the reference start (plain FP64 against the hybrid: split-
 BF16 secant steps, one FP64 anchor, anchored finish), parity against the
 default-size oracle fixture, precompute time, the CPU baseline (the oracle's
@@ -447,15 +447,15 @@ def precompute_roofline(cfg, dims, pre_ms, peak64: float, peaks: dict):
             "hbm_frac": orb_bytes / t_orb / 1e9 / hbm, "hbm_peak_note": hbm_note,
             "bound": "FP64 + transcendentals (2 nw point evaluations per orbit)"}
     if t_wl > 0:
-        wl_bytes = float(NPh) * Na * n_l * 16 + 3.0 * nwa * NPh * 8
-        wl_flops = 4.0 * n_l * nwa * Na * NPh
+        wl_bytes = float(NPh) * Na * n_l * 8 + 3.0 * nwa * NPh * 8
+        wl_flops = 2.0 * n_l * nwa * Na * NPh
         out["wl_kernel"] = {
             "ms": pre_ms[1], "algorithmic_bytes": wl_bytes, "hbm_gbs": wl_bytes / t_wl / 1e9,
             "hbm_frac": wl_bytes / t_wl / 1e9 / hbm, "hbm_peak_note": hbm_note,
             "algorithmic_flops": wl_flops, "tflops": wl_flops / t_wl / 1e12,
             "fp64_frac": wl_flops / t_wl / 1e12 / peak64,
             "fp64_peak_note": "of measured: cuBLAS DGEMM in this run",
-            "bound": "FP64 tensor pipe (DMMA); output 16 B per table entry"}
+            "bound": "FP64 tensor pipe (DMMA); output 8 B per (orbit, l, N_alpha) real table entry"}
     return out
 
 
@@ -919,7 +919,9 @@ def ours(args):
     _lib.check(h, lib.kls_set_stream(h, C.c_void_p(stream.cuda_stream)))
 
     nb = 3
-    flops_per_det = 8.0 * dims.N_alpha ** 2 * dims.K
+    # one triangle of a complex symmetric product of real rows; the complex
+    # product of the reference takes 8 N_alpha^2 K
+    flops_per_det = 2.0 * dims.N_alpha * (dims.N_alpha + 1) * dims.K
     # tensor flops of the 3-product split GEMM per determinant (unpadded)
     mixed_flops_per_det = 3 * 2.0 * (2 * dims.N_alpha) ** 2 * dims.K
     d_det = torch.empty((nb, 2), dtype=torch.float64, device="cuda")
@@ -989,9 +991,10 @@ def ours(args):
     value = world * nb * args.steps / (ms * 1e-3)
     stage = stage_times(_lib.KLS_MODE_FP64)
     achieved = nb * flops_per_det / (stage[1] * 1e-3) / 1e12
-    # real DMMA flops the kernel issues (padded tiles): 4 or 3 real products
-    f64_3m = tunes["fp64"].form == _lib.KLS_F64_3M
-    issued_per_det = (6.0 if f64_3m else 8.0) * dims.N_alpha_pad ** 2 * dims.K_pad
+    # real DMMA flops the kernel issues: the 8 x 8 blocks of one triangle of
+    # T = sum_k w_k V_k^T V_k (V real, w complex: 2 real products)
+    n8 = -(-(-(-dims.N_alpha // 2) * 2) // 8)
+    issued_per_det = 4.0 * 64 * (n8 * (n8 + 1) // 2) * dims.K_pad
     issued = nb * issued_per_det / (stage[1] * 1e-3) / 1e12
 
     # ---- end to end through the C ABI with host buffers -----------------------
@@ -1168,7 +1171,7 @@ def ours(args):
         dist.destroy_process_group()
     if rank != 0:
         return 0
-    traffic, traffic_scaled = read_traffic("contract3m_kernel" if f64_3m else "contract_kernel")
+    traffic, traffic_scaled = read_traffic("contract_kernel")
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_per_step, "higher_is_better": True,
@@ -1180,18 +1183,16 @@ def ours(args):
                    "N_alpha": cfg.grid.N_alpha, "l": [cfg.grid.l_min, cfg.grid.l_max],
                    "K": dims.K, "omegas_per_step": nb, "parallelism": f"replicas x{world}",
                    "l2": "inputs larger than L2 (W table %.1f GB in HBM)" % (
-                       2 * 8 * dims.K_pad * dims.N_alpha_pad / 1e9)},
+                       8 * dims.K_pad * dims.N_alpha / 1e9)},
         "roofline": {"bound": "tensor",
-                     "kernel": ("contract3m_kernel (FP64 DMMA m8n8k4, 3 real products per "
-                                "complex one)" if f64_3m else
-                                "contract_kernel (FP64 DMMA m8n8k4, 4 real products)"),
+                     "kernel": "contract_kernel (FP64 DMMA m8n8k4, one triangle, real table)",
                      "achieved": achieved, "peak": peak64, "unit": "TFLOP/s",
                      "frac": achieved / peak64,
                      "peak_note": "of measured: cuBLAS DGEMM 8192^3 best-of-5 in this run",
                      "algorithmic_flops_per_launch": nb * flops_per_det,
-                     "algorithmic_note": "8 N_alpha^2 K per determinant (a complex MAC as 4 "
-                                         "real ones); the 3M form issues 3, so its frac can "
-                                         "exceed the DMMA pipe's",
+                     "algorithmic_note": "2 N_alpha (N_alpha + 1) K per determinant: complex "
+                                         "weights times real rows, one triangle (the "
+                                         "reference's complex product: 8 N_alpha^2 K)",
                      "dmma_issued_tflops": issued, "dmma_issued_frac": issued / peak64,
                      "traffic": traffic, "traffic_scaled": traffic_scaled, "stage_ms": {"weights": stage[0], "contract": stage[1],
                                                       "reduce": stage[2], "lu": stage[3]}},
@@ -1202,7 +1203,7 @@ def ours(args):
         "gpu_launches": int(launches),
         "clocks": clk,
         "autotune": {k: {"splits": t.splits, "default_splits": t.default_splits,
-                         "form": ({0: "FP64 4M", 1: "FP64 3M"} if k == "fp64" else
+                         "form": ({} if k == "fp64" else
                                   {1: "one CTA", 2: "CTA pair",
                                    3: "TMEM-operand CTA pair"}).get(t.form, t.form),
                          "candidates": t.candidates, "ms_per_omega": t.ms_per_omega,

@@ -57,10 +57,12 @@ extern "C" {
                                    away: ~1e-11 of max|M|) at the cost of a
                                    KLS_MODE_MIXED evaluation                  */
 
-/* ---- forms of the FP64 contraction (kls_set_f64_form) -------------------- */
-#define KLS_F64_4M           0  /* four real DMMA products per complex one     */
-#define KLS_F64_3M           1  /* three (Gauss): Re = P1 - P2,
-                                   Im = (P3 - P1) - P2 with P3 = (ar+ai)(br+bi) */
+/* ---- forms of the FP64 contraction (kls_set_f64_form) -------------------- *
+ * Two names for ways to form a complex product of complex table rows.  The
+ * table is real (W(-alpha) = conj W(alpha)), so a product takes two real ones
+ * and both names run the same kernel with the same bits.                    */
+#define KLS_F64_4M           0
+#define KLS_F64_3M           1
 
 /* ---- configuration: the [physics] [model] [grid] TOML sections ---------- *
  * Mirrors PhysicsConfig / ModelConfig / GridConfig
@@ -96,7 +98,7 @@ typedef struct kls_dims {
     int32_t NPh;        /* NR * Ne                                          */
     int32_t n_l;        /* l_max - l_min + 1                                */
     int32_t N_alpha;
-    int32_t N_alpha_pad;/* row length of the device W table                 */
+    int32_t N_alpha_pad;/* N_alpha padded to the split-BF16 table's tiles   */
     int64_t K;          /* NPh * n_l contraction length                     */
     int64_t K_pad;      /* padded rows of the device W table                */
     int32_t nwa;
@@ -163,7 +165,7 @@ int kls_precompute(kls_ctx* ctx);
 /* Build the split-BF16 copy of the W table used by KLS_MODE_MIXED.         */
 int kls_prepare_mixed(kls_ctx* ctx);
 /* Free the FP64 W table after building the split-BF16 copy (no reference
- * counterpart): a mixed-only context, 13 GB instead of 40 GB at NR=501,
+ * counterpart): a mixed-only context, 13 GB instead of 26 GB at NR=501,
  * Ne=51, N_alpha=301, l in [-100, 100], so that many default-size models fit
  * one GPU.  Afterwards KLS_MODE_FP64 calls, kls_export_W and FP64 batches
  * return KLS_ERR_STATE.                                                     */
@@ -370,9 +372,9 @@ int kls_autotune(kls_ctx* ctx, int mode, int batch, kls_tune_result* out);
  * allows); determinants stay batch-independent for a fixed count.         */
 int kls_set_splits(kls_ctx* ctx, int mode, int splits);
 /* FP64 contraction form (no reference counterpart): KLS_F64_4M (default) or
- * KLS_F64_3M; the K split count is reset to the form's default.  Both stay
- * within the FP64 parity tolerances; they differ in the last bits.  An
- * uneven batch (kls_multi_create) needs every FP64 model in the same form. */
+ * KLS_F64_3M; a change resets the K split count to the default.  Both run the
+ * same kernel.  An uneven batch (kls_multi_create) needs every FP64 model in
+ * the same form. */
 int kls_set_f64_form(kls_ctx* ctx, int form);
 
 /* ---- determinant stage form (no reference counterpart) -------------------- *

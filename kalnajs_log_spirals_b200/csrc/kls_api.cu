@@ -102,18 +102,33 @@ void dfree(void* p) {
   if (p) cudaFree(p);
 }
 
-int ensure_ws(kls_ctx* c, int n) {
-  if (n <= c->ws_omega && c->d_part) return KLS_OK;
-  int cap = std::max(n, c->ws_omega);
-  dfree(c->d_omega); dfree(c->d_wt); dfree(c->d_part); dfree(c->d_A); dfree(c->d_det);
+// the FP64 contraction's work items and partials for n omegas
+int ensure_f64(kls_ctx* c, int n) {
+  int r;
+  if ((r = kls_f64_plan(c))) return r;
+  const size_t need = kls_f64_part_elems(c, n);
+  if (need <= c->part_elems) return KLS_OK;
+  dfree(c->d_part);
+  c->d_part = nullptr;
+  c->part_elems = 0;
+  if ((r = dalloc(c, &c->d_part, need))) return r;
+  c->part_elems = need;
+  return KLS_OK;
+}
+
+// per-omega buffers for n omegas of `mode`
+int ensure_ws(kls_ctx* c, int n, int mode) {
+  int r;
+  if (mode == KLS_MODE_FP64 && (r = ensure_f64(c, n))) return r;
+  if (n <= c->ws_omega) return KLS_OK;
+  int cap = n;
+  dfree(c->d_omega); dfree(c->d_wt); dfree(c->d_A); dfree(c->d_det);
   dfree(c->d_logabs);
-  c->d_omega = nullptr; c->d_wt = nullptr; c->d_part = nullptr; c->d_A = nullptr;
+  c->d_omega = nullptr; c->d_wt = nullptr; c->d_A = nullptr;
   c->d_det = nullptr; c->d_logabs = nullptr;
   c->ws_omega = 0;
-  int r;
   if ((r = dalloc(c, &c->d_omega, (size_t)2 * cap))) return r;
   if ((r = dalloc(c, &c->d_wt, (size_t)cap * c->K_pad))) return r;
-  if ((r = dalloc(c, &c->d_part, (size_t)cap * c->splits * c->Na_pad * c->Na_pad))) return r;
   if ((r = dalloc(c, &c->d_A, (size_t)cap * c->Na * c->Na))) return r;
   if ((r = dalloc(c, &c->d_det, (size_t)cap))) return r;
   if ((r = dalloc(c, &c->d_logabs, (size_t)cap))) return r;
@@ -127,7 +142,6 @@ int run_batch(kls_ctx* c, int n, int mode, bool export_M) {
                  : mode == KLS_MODE_MIXED ? "kls det batch (split-BF16)"
                                           : "kls det batch (anchored)");
   int r;
-  const int splits = c->splits;
   if (mode != KLS_MODE_FP64 && mode != KLS_MODE_MIXED && mode != KLS_MODE_ANCHORED)
     return kls_fail(c, KLS_ERR_CONFIG, "unknown precision mode");
   const bool anchored = mode == KLS_MODE_ANCHORED;
@@ -137,16 +151,16 @@ int run_batch(kls_ctx* c, int n, int mode, bool export_M) {
   if ((r = kls_run_weights(c, n, anchored ? c->anchor_w : nullptr))) return r;
   if (c->timing) KLS_CK(c, cudaEventRecord(c->ev[1], c->stream));
   if (mode == KLS_MODE_FP64) {
-    if (!c->d_Wre) return kls_fail(c, KLS_ERR_STATE, "the FP64 table was released (kls_release_fp64)");
-    if ((r = kls_run_contract_f64(c, n, splits))) return r;
+    if (!c->d_V) return kls_fail(c, KLS_ERR_STATE, "the FP64 table was released (kls_release_fp64)");
+    if ((r = kls_run_contract_f64(c, n))) return r;
   } else {
     if (!c->mixed && (r = kls_mixed_prepare(c))) return r;
-    if ((r = kls_mixed_contract(c, n, splits))) return r;
+    if ((r = kls_mixed_contract(c, n))) return r;
   }
   if (c->timing) KLS_CK(c, cudaEventRecord(c->ev[2], c->stream));
   if (mode != KLS_MODE_FP64) {
     if ((r = kls_mixed_reduce(c, n, export_M, anchored ? c->d_anchorM : nullptr))) return r;
-  } else if ((r = kls_run_reduce(c, n, splits, export_M))) {
+  } else if ((r = kls_run_reduce(c, n, export_M))) {
     return r;
   }
   if (c->timing) KLS_CK(c, cudaEventRecord(c->ev[3], c->stream));
@@ -183,7 +197,7 @@ int det_batch_host(kls_ctx* c, const double* omega_ri, int n, int mode, double* 
     for (int i = 0; i < 2 * nb; ++i)
       if (!std::isfinite(omega_ri[2 * b + i]))
         return kls_fail(c, KLS_ERR_NONFINITE, "non-finite omega");
-    if ((r = ensure_ws(c, nb))) return r;
+    if ((r = ensure_ws(c, nb, mode))) return r;
     KLS_CK(c, cudaMemcpyAsync(c->d_omega, omega_ri + 2 * b, 2 * nb * sizeof(double),
                               cudaMemcpyHostToDevice, c->stream));
     if ((r = run_batch(c, nb, mode, false))) return r;
@@ -263,11 +277,12 @@ int kls_create(const kls_config* cfg, int device, kls_ctx** out) {
   c->Na = cfg->N_alpha;
   c->Na_pad = ((cfg->N_alpha + KLS_TILE - 1) / KLS_TILE) * KLS_TILE;
   c->nw = cfg->nw; c->nwa = cfg->nwa; c->nwai = (cfg->nw - 1) / (cfg->nwa - 1);
+  c->ldv = kls_ldv(c->Na);
   c->K = (int64_t)c->NPh * c->n_l;
   c->K_pad = ((c->K + KLS_KROW_ALIGN - 1) / KLS_KROW_ALIGN) * KLS_KROW_ALIGN;
   c->splits = kls_choose_splits(c);
 
-  size_t need = (size_t)2 * c->K_pad * c->Na_pad * sizeof(double);
+  size_t need = (size_t)c->K_pad * c->ldv * sizeof(double);
   size_t fr = 0, tot = 0;
   cudaMemGetInfo(&fr, &tot);
   if (need > fr) {
@@ -287,8 +302,7 @@ int kls_create(const kls_config* cfg, int device, kls_ctx** out) {
       (r = dalloc(c, &c->d_alpha, c->Na)) || (r = dalloc(c, &c->d_dalpha, c->Na)) ||
       (r = dalloc(c, &c->d_N, c->Na)) || (r = dalloc(c, &c->d_Gk, c->K_pad)) ||
       (r = dalloc(c, &c->d_Ok, c->K_pad)) || (r = dalloc(c, &c->d_F0l, c->K_pad)) ||
-      (r = dalloc(c, &c->d_Wre, (size_t)c->K_pad * c->Na_pad)) ||
-      (r = dalloc(c, &c->d_Wim, (size_t)c->K_pad * c->Na_pad)) ||
+      (r = dalloc(c, &c->d_V, (size_t)c->K_pad * c->ldv)) ||
       (r = dalloc(c, &c->d_M, (size_t)c->Na * c->Na))) {
     std::string m = c->err;
     kls_destroy(c);
@@ -305,7 +319,7 @@ int kls_destroy(kls_ctx* c) {
   kls_mixed_free(c);
   void* ptrs[] = {c->d_cosw, c->d_sinw, c->d_of, c->d_SRC, c->d_rc, c->d_valid, c->d_w1, c->d_ra,
                   c->d_pha, c->d_alpha, c->d_dalpha, c->d_N, c->d_Gk, c->d_Ok, c->d_F0l,
-                  c->d_Wre, c->d_Wim, c->d_omega, c->d_wt, c->d_part, c->d_A, c->d_M,
+                  c->d_V, c->d_items, c->d_tiles, c->d_omega, c->d_wt, c->d_part, c->d_A, c->d_M,
                   c->d_anchorM, c->d_det, c->d_logabs};
   for (void* p : ptrs) dfree(p);
   for (auto& ev : c->ev) if (ev) cudaEventDestroy(ev);
@@ -355,11 +369,10 @@ int kls_release_fp64(kls_ctx* c) {
   if (r) return r;
   if (!c->mixed && (r = kls_mixed_prepare(c))) return r;
   KLS_CK(c, cudaStreamSynchronize(c->stream));
-  if (c->d_Wre) {
-    cudaFree(c->d_Wre);
-    cudaFree(c->d_Wim);
-    c->d_Wre = c->d_Wim = nullptr;
-    c->device_bytes -= (int64_t)(2 * (size_t)c->K_pad * c->Na_pad * sizeof(double));
+  if (c->d_V) {
+    cudaFree(c->d_V);
+    c->d_V = nullptr;
+    c->device_bytes -= (int64_t)((size_t)c->K_pad * c->ldv * sizeof(double));
   }
   return KLS_OK;
 }
@@ -413,27 +426,31 @@ int kls_export_resonant(kls_ctx* c, double* F0l, double* Ores) {
 }
 
 int kls_export_W(kls_ctx* c, int il0, int nl, double* W) {
-  if (c->precomputed && !c->d_Wre)
+  if (c->precomputed && !c->d_V)
     return kls_fail(c, KLS_ERR_STATE, "the FP64 table was released (kls_release_fp64)");
   int r = check_ready(c);
   if (r) return r;
   if (il0 < 0 || nl < 0 || il0 + nl > c->n_l || !W)
     return kls_fail(c, KLS_ERR_CONFIG, "bad harmonic range for kls_export_W");
-  const size_t rows = c->NPh, ld = c->Na_pad;
-  std::vector<double> re(rows * ld), im(rows * ld);
+  const size_t rows = c->NPh, ld = c->ldv;
+  const int np = (c->Na + 1) / 2;
+  std::vector<double> v(rows * ld);
   for (int q = 0; q < nl; ++q) {
     size_t r0 = (size_t)(il0 + q) * rows;
-    KLS_CK(c, cudaMemcpy(re.data(), c->d_Wre + r0 * ld, rows * ld * sizeof(double),
+    KLS_CK(c, cudaMemcpy(v.data(), c->d_V + r0 * ld, rows * ld * sizeof(double),
                          cudaMemcpyDeviceToHost));
-    KLS_CK(c, cudaMemcpy(im.data(), c->d_Wim + r0 * ld, rows * ld * sizeof(double),
-                         cudaMemcpyDeviceToHost));
-    // reference layout [NPh, N_alpha, n_l], column-major, interleaved complex
+    // reference layout [NPh, N_alpha, n_l], column-major, interleaved complex;
+    // W(-alpha) = conj W(alpha)
     double* blk = W + (size_t)2 * q * rows * c->Na;
-    for (int a = 0; a < c->Na; ++a)
+    for (int a = 0; a < c->Na; ++a) {
+      const bool neg = a < c->Na - np;
+      const size_t pair = neg ? np - 1 - a : a - (c->Na - np);
       for (size_t p = 0; p < rows; ++p) {
-        blk[2 * (p + rows * a)] = re[p * ld + a];
-        blk[2 * (p + rows * a) + 1] = im[p * ld + a];
+        blk[2 * (p + rows * a)] = v[p * ld + 2 * pair];
+        const double im = v[p * ld + 2 * pair + 1];
+        blk[2 * (p + rows * a) + 1] = neg ? -im : im;
       }
+    }
   }
   return KLS_OK;
 }
@@ -469,7 +486,7 @@ int kls_det_batch_device(kls_ctx* c, const double* d_omega, int n, int mode, dou
   if (c->timing) std::fill(c->stage_ms, c->stage_ms + 4, 0.f);
   for (int b = 0; b < n; b += WS_CHUNK) {
     int nb = std::min(WS_CHUNK, n - b);
-    if ((r = ensure_ws(c, nb))) return r;
+    if ((r = ensure_ws(c, nb, mode))) return r;
     KLS_CK(c, cudaMemcpyAsync(c->d_omega, d_omega + 2 * b, 2 * nb * sizeof(double),
                               cudaMemcpyDeviceToDevice, c->stream));
     if ((r = run_batch(c, nb, mode, false))) return r;
@@ -490,7 +507,7 @@ int kls_build_M(kls_ctx* c, double wr, double wi, int mode, double* M) {
   int r = check_ready(c);
   if (r) return r;
   if (!M) return kls_fail(c, KLS_ERR_CONFIG, "M is NULL");
-  if ((r = ensure_ws(c, 1))) return r;
+  if ((r = ensure_ws(c, 1, mode))) return r;
   double om[2] = {wr, wi};
   KLS_CK(c, cudaMemcpyAsync(c->d_omega, om, sizeof om, cudaMemcpyHostToDevice, c->stream));
   if ((r = run_batch(c, 1, mode, true))) return r;
@@ -514,10 +531,10 @@ int kls_set_anchor(kls_ctx* c, double wr, double wi, double* det_ri) {
   if (r) return r;
   if (!std::isfinite(wr) || !std::isfinite(wi))
     return kls_fail(c, KLS_ERR_NONFINITE, "non-finite anchor omega");
-  if (!c->d_Wre) return kls_fail(c, KLS_ERR_STATE, "the FP64 table was released (kls_release_fp64)");
+  if (!c->d_V) return kls_fail(c, KLS_ERR_STATE, "the FP64 table was released (kls_release_fp64)");
   if (!c->mixed && (r = kls_mixed_prepare(c))) return r;
   if (!c->d_anchorM && (r = dalloc(c, &c->d_anchorM, (size_t)c->Na * c->Na))) return r;
-  if ((r = ensure_ws(c, 1))) return r;
+  if ((r = ensure_ws(c, 1, KLS_MODE_FP64))) return r;
   c->anchor_set = false;
   const double om[2] = {wr, wi};
   KLS_CK(c, cudaMemcpyAsync(c->d_omega, om, sizeof om, cudaMemcpyHostToDevice, c->stream));
@@ -885,10 +902,7 @@ void tune_store(const std::string& key, int s, int form) {
 
 int apply_splits(kls_ctx* c, int mode, int s) {
   if (mode == KLS_MODE_FP64) {
-    if (c->splits != s) {
-      c->splits = s;
-      c->ws_omega = 0;            // the next batch reallocates the partials
-    }
+    c->splits = s;                // the next batch plans its items and partials
     return KLS_OK;
   }
   return kls_mixed_set_splits(c, s);
@@ -897,7 +911,7 @@ int apply_splits(kls_ctx* c, int mode, int s) {
 // contraction time per omega (ms) at the context's current split count
 int time_contraction(kls_ctx* c, int mode, int n, double* ms) {
   int r;
-  if ((r = ensure_ws(c, n))) return r;
+  if ((r = ensure_ws(c, n, mode))) return r;
   std::vector<double> om(2 * (size_t)n);
   for (int z = 0; z < n; ++z) {
     om[2 * z] = c->cfg.m * (0.3 + 0.3 * z / std::max(1, n));
@@ -907,8 +921,7 @@ int time_contraction(kls_ctx* c, int mode, int n, double* ms) {
                             cudaMemcpyHostToDevice, c->stream));
   if ((r = kls_run_weights(c, n))) return r;
   auto once = [&]() -> int {
-    return mode == KLS_MODE_FP64 ? kls_run_contract_f64(c, n, c->splits)
-                                 : kls_mixed_contract(c, n, 0);
+    return mode == KLS_MODE_FP64 ? kls_run_contract_f64(c, n) : kls_mixed_contract(c, n);
   };
   if ((r = once())) return r;               // warm-up (and workspace growth)
   cudaEvent_t e0, e1;
@@ -939,14 +952,14 @@ int kls_autotune(kls_ctx* c, int mode, int batch, kls_tune_result* out) {
   if (mode != KLS_MODE_FP64 && mode != KLS_MODE_MIXED)
     return kls_fail(c, KLS_ERR_CONFIG, "unknown precision mode");
   if (batch < 1 || batch > WS_CHUNK) return kls_fail(c, KLS_ERR_CONFIG, "bad autotune batch");
-  if (mode == KLS_MODE_FP64 && !c->d_Wre)
+  if (mode == KLS_MODE_FP64 && !c->d_V)
     return kls_fail(c, KLS_ERR_STATE, "the FP64 table was released (kls_release_fp64)");
   if (mode == KLS_MODE_MIXED && !c->mixed && (r = kls_mixed_prepare(c))) return r;
   const bool mixed = mode == KLS_MODE_MIXED;
   const int def = mixed ? kls_mixed_default_splits(c) : kls_choose_splits(c);
   const int def_form = mixed ? kls_mixed_form_of(c) : c->f64_form;
   const int max_s = mixed ? (int)std::max<int64_t>(1, c->K_pad / 64)
-                          : (int)std::max<int64_t>(1, c->K_pad / (16 * 8));
+                          : kls_f64_max_splits(c);
   auto apply = [&](int s, int form) -> int {
     if (mixed && (r = kls_mixed_set_form(c, form))) return r;
     if (!mixed) c->f64_form = form;
@@ -968,11 +981,10 @@ int kls_autotune(kls_ctx* c, int mode, int batch, kls_tune_result* out) {
       return KLS_OK;
     }
   }
-  // each mode also chooses its kernel: one CTA, a CTA pair or the
-  // TMEM-operand pair (split-BF16), 4 or 3 real products (FP64); split
-  // candidates around each form's own default
+  // the split-BF16 mode also chooses its kernel: one CTA, a CTA pair or the
+  // TMEM-operand pair; split candidates around each form's own default
   std::vector<int> forms = mixed ? std::vector<int>{KLS_MIXED_ONE_CTA, KLS_MIXED_PAIR}
-                                 : std::vector<int>{KLS_F64_4M, KLS_F64_3M};
+                                 : std::vector<int>{c->f64_form};
   if (mixed && kls_mixed_set_form(c, KLS_MIXED_TMEM) == KLS_OK) forms.push_back(KLS_MIXED_TMEM);
   if (mixed) kls_mixed_set_form(c, def_form);
   double best_ms = INFINITY;
@@ -987,6 +999,13 @@ int kls_autotune(kls_ctx* c, int mode, int batch, kls_tune_result* out) {
       fdef = kls_choose_splits(c);
     }
     std::vector<int> cand = {std::max(1, fdef / 2), fdef, 2 * fdef, 3 * fdef};
+    // more FP64 splits only while the partials of `batch` omegas stay within 2 GiB
+    if (!mixed) {
+      if ((r = apply(fdef, form)) || (r = kls_f64_plan(c))) return r;
+      const double bytes = (double)kls_f64_part_elems(c, batch) * sizeof(double2);
+      while (cand.size() > 2 && bytes * (cand.size() - 1) > 2.0 * 1024 * 1024 * 1024)
+        cand.pop_back();
+    }
     // the TMEM-operand form's default is the number of resident CTA pairs:
     // fewer splits leave a single omega (Newton's evaluations) on part of a
     // wave, so only whole multiples of it are candidates
@@ -1032,8 +1051,7 @@ int kls_set_splits(kls_ctx* c, int mode, int splits) {
   if (r) return r;
   if (splits < 1) return kls_fail(c, KLS_ERR_CONFIG, "splits must be >= 1");
   if (mode == KLS_MODE_FP64) {
-    const int max_s = (int)std::max<int64_t>(1, c->K_pad / (16 * 8));
-    return apply_splits(c, mode, std::min(splits, max_s));
+    return apply_splits(c, mode, std::min(splits, kls_f64_max_splits(c)));
   }
   if (mode != KLS_MODE_MIXED) return kls_fail(c, KLS_ERR_CONFIG, "unknown precision mode");
   if (!c->mixed && (r = kls_mixed_prepare(c))) return r;

@@ -39,7 +39,7 @@ constexpr int WL_SE = WL_AB + 4;   // smem row stride of E [k][a]
 constexpr int WL_THREADS = 128;
 
 struct WlParams {
-  int NPh, nwa, Na, Na_pad, n_l, l_min, m;
+  int NPh, nwa, np, ldv, n_l, l_min, m;   // np alphas >= 0
   double astep;          // alpha grid step
 };
 
@@ -51,13 +51,13 @@ __global__ void __launch_bounds__(WL_THREADS)
 wl_kernel(WlParams P, const double* __restrict__ of, const int* __restrict__ valid,
           const double* __restrict__ w1g, const double* __restrict__ rag,
           const double* __restrict__ phag, const double* __restrict__ alpha,
-          double* __restrict__ Wre, double* __restrict__ Wim) {
+          double* __restrict__ V) {
   __shared__ double sC[WL_LB * WL_SC];
   __shared__ double sEr[WL_BK * WL_SE];
   __shared__ double sEi[WL_BK * WL_SE];
   // one orbit's (l block, alpha block) CTAs are consecutive in launch order,
   // so its w1 / r / theta samples are read from DRAM once and then from L2
-  const int nlb = (P.n_l + WL_LB - 1) / WL_LB, nab = P.Na_pad / WL_AB;
+  const int nlb = (P.n_l + WL_LB - 1) / WL_LB, nab = (P.np + WL_AB - 1) / WL_AB;
   const int p = (int)(blockIdx.x / (unsigned)(nlb * nab));
   const int lb = (int)((blockIdx.x / (unsigned)nab) % (unsigned)nlb);
   const int ab = (int)(blockIdx.x % (unsigned)nab);
@@ -115,15 +115,15 @@ wl_kernel(WlParams P, const double* __restrict__ of, const int* __restrict__ val
         // E: r^{-1/2} e^{-i alpha ln r}, anchor at a_first, rotate by -astep ln r
         double lr = log(rk);
         double isq = 1.0 / sqrt(rk);
-        double ta = -KLS_LD(KLS_IB(min(a_first, P.Na - 1), P.Na, KS_WL_SAMPLES),
-                            alpha[min(a_first, P.Na - 1)], 0.0) * lr;
+        double ta = -KLS_LD(KLS_IB(min(a_first, P.np - 1), P.np, KS_WL_SAMPLES),
+                            alpha[min(a_first, P.np - 1)], 0.0) * lr;
         sincos(ta, &s, &c);
         sincos(-P.astep * lr, &ss, &cs);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           double er = c * isq, ei = s * isq;
           if (!(isfinite(er) && isfinite(ei))) { er = 0.0; ei = 0.0; }
-          bool in = a_first + j < P.Na;
+          bool in = a_first + j < P.np;
           sEr[gk * WL_SE + gsub * 8 + j] = in ? er : 0.0;
           sEi[gk * WL_SE + gsub * 8 + j] = in ? ei : 0.0;
           double cn = c * cs - s * ss;
@@ -168,18 +168,21 @@ wl_kernel(WlParams P, const double* __restrict__ of, const int* __restrict__ val
   for (int i = 0; i < 4; ++i) {
     int il = lb * WL_LB + i * 8 + (lane >> 2);
     if (il >= P.n_l) continue;
-    size_t row = ((size_t)il * NPh + p) * P.Na_pad;
+    size_t row = ((size_t)il * NPh + p) * P.ldv;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       int a0 = ab * WL_AB + warp * 16 + j * 8 + 2 * (lane & 3);
-      double r0 = accR[i][j][0] / KLS_PI, r1 = accR[i][j][1] / KLS_PI;
-      double i0 = accI[i][j][0] / KLS_PI, i1 = accI[i][j][1] / KLS_PI;
-      if (a0 >= P.Na) { r0 = 0.0; i0 = 0.0; }
-      if (a0 + 1 >= P.Na) { r1 = 0.0; i1 = 0.0; }
-      KLS_UNLESS(KLS_IB((int64_t)row + a0 + 1, (int64_t)P.n_l * NPh * P.Na_pad, KS_WL_OUT),
+      // alphas a0 and a0 + 1: columns 2 a0 .. 2 a0 + 3 (zero beyond np)
+      if (2 * a0 >= P.ldv) continue;
+      KLS_UNLESS(KLS_IB((int64_t)row + 2 * a0 + 1, (int64_t)P.n_l * NPh * P.ldv, KS_WL_OUT),
                  continue)
-      *reinterpret_cast<double2*>(Wre + row + a0) = make_double2(r0, r1);
-      *reinterpret_cast<double2*>(Wim + row + a0) = make_double2(i0, i1);
+      *reinterpret_cast<double2*>(V + row + 2 * a0) =
+          make_double2(accR[i][j][0] / KLS_PI, accI[i][j][0] / KLS_PI);
+      if (2 * a0 + 2 >= P.ldv) continue;
+      KLS_UNLESS(KLS_IB((int64_t)row + 2 * a0 + 3, (int64_t)P.n_l * NPh * P.ldv, KS_WL_OUT),
+                 continue)
+      *reinterpret_cast<double2*>(V + row + 2 * a0 + 2) =
+          make_double2(accR[i][j][1] / KLS_PI, accI[i][j][1] / KLS_PI);
     }
   }
 }
@@ -261,20 +264,18 @@ int kls_run_basis(kls_ctx* c) {
   KLS_LAUNCHED(c);
   // zero the padding rows of the table (rows K..K_pad-1)
   size_t pad_rows = (size_t)(c->K_pad - c->K);
-  if (pad_rows) {
-    KLS_CK(c, cudaMemsetAsync(c->d_Wre + (size_t)c->K * c->Na_pad, 0,
-                              pad_rows * c->Na_pad * sizeof(double), c->stream));
-    KLS_CK(c, cudaMemsetAsync(c->d_Wim + (size_t)c->K * c->Na_pad, 0,
-                              pad_rows * c->Na_pad * sizeof(double), c->stream));
-  }
+  if (pad_rows)
+    KLS_CK(c, cudaMemsetAsync(c->d_V + (size_t)c->K * c->ldv, 0,
+                              pad_rows * c->ldv * sizeof(double), c->stream));
   WlParams P{};
-  P.NPh = c->NPh; P.nwa = c->nwa; P.Na = c->Na; P.Na_pad = c->Na_pad; P.n_l = c->n_l;
+  P.NPh = c->NPh; P.nwa = c->nwa; P.np = (c->Na + 1) / 2; P.ldv = c->ldv; P.n_l = c->n_l;
   P.l_min = k.l_min; P.m = k.m;
   P.astep = c->Na > 1 ? (2.0 * k.alpha_max) / (double)(c->Na - 1) : 0.0;
-  dim3 grid((unsigned)c->NPh * ((c->n_l + WL_LB - 1) / WL_LB) * (c->Na_pad / WL_AB));
+  dim3 grid((unsigned)c->NPh * ((c->n_l + WL_LB - 1) / WL_LB) * ((P.np + WL_AB - 1) / WL_AB));
   kls_pre_mark(c, 2);
+  // the alphas >= 0 are the last np of the grid
   wl_kernel<<<grid, WL_THREADS, 0, c->stream>>>(P, c->d_of, c->d_valid, c->d_w1, c->d_ra,
-                                                c->d_pha, c->d_alpha, c->d_Wre, c->d_Wim);
+                                                c->d_pha, c->d_alpha + (c->Na - P.np), c->d_V);
   KLS_LAUNCHED(c);
   kls_pre_mark(c, 3);
   return KLS_OK;

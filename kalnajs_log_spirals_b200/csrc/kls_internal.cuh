@@ -6,6 +6,7 @@
 #include <climits>
 #include <cstdint>
 #include <string>
+#include <vector>
 #include "kls.h"
 
 #define KLS_PI 3.14159265358979323846
@@ -14,6 +15,14 @@
 // multiple of KLS_TILE so that alpha tiles never need masking.
 constexpr int KLS_TILE = 64;
 constexpr int KLS_KROW_ALIGN = 64;   // K rows padded to a multiple of this
+
+// FP64 table.  The alpha grid is symmetric about 0 and
+// W_l(-alpha) = conj W_l(alpha) (the radial factor is real, the log-spiral
+// factor is conjugated), so a row k = (l, orbit) holds, for the
+// np = ceil(N_alpha / 2) alphas >= 0, the pairs V[2p] = Re W, V[2p + 1] = Im W
+// (Im = 0 at alpha = 0 when N_alpha is odd), padded with zeros to ldv, a
+// multiple of 8 columns.
+inline int kls_ldv(int N_alpha) { return ((N_alpha + 1) / 2 * 2 + 7) / 8 * 8; }
 // TMEM-operand split-BF16 form: FP32 weight variants per k pair (float4 each)
 constexpr int KLS_TM_WVAR = 2;
 
@@ -31,20 +40,20 @@ struct kls_mixed;   // split-BF16 tables (kls_mixed.cu)
 // The tables are the model context's own; the per-omega buffers belong to
 // the batch.
 struct kls_mdesc {
-  const double* Wre;          // [K_pad][Na_pad]
-  const double* Wim;
+  const double* V;            // [K_pad][ldv]
   const double* Gk;           // [K_pad]
   const double* Ok;           // [K_pad]
   const double* Nk;           // [Na]
   const double* omega;        // [batch][2]
   double2* wt;                // [batch][K_pad]
-  double2* part;              // FP64 form: [batch][splits][Na_pad][Na_pad]
+  double2* part;              // FP64 form: [batch][n_slots][64 x 64]
+  const int2* tiles;          // FP64 form: (first slot, slots) per part
   double2* A;                 // [batch][Na][Na]
   double2* det;               // [batch]
   double* logabs;             // [batch]
   double G;
-  int64_t K_pad, k_per_split;
-  int Na, Na_pad, splits, model;
+  int64_t K_pad;
+  int Na, Na_pad, ldv, n_slots;
   // mixed form
   const void* Xh;             // BF16 hi / lo, 2 Na_pad rows in 64-k blocks
   const void* Xl;
@@ -68,7 +77,8 @@ struct alignas(64) kls_tm_model {
 };
 
 // One work item of the persistent contraction: FP64 form (model, omega z,
-// 64 x 64 tile, K split); mixed form (model, first omega z, 128-row x
+// part gi << 16 | gj, split = partial slot, 16-row slabs [kb0, kb0 + nkb));
+// mixed form (model, first omega z, 128-row x
 // 64-alpha tile, K split, n_om omegas from z, k-blocks [kb0, kb0 + nkb)).
 struct kls_item {
   int model, z, tile, split;
@@ -104,16 +114,22 @@ struct kls_ctx {
   double* d_Gk = nullptr;     // [K_pad]  DJ * F0l per row k = il*NPh + p
   double* d_Ok = nullptr;     // [K_pad]  Omega_res per row
   double* d_F0l = nullptr;    // [K_pad]  F0l per row (export only)
-  double* d_Wre = nullptr;    // [K_pad][Na_pad]
-  double* d_Wim = nullptr;
+  int ldv = 0;                // row length of the FP64 table (kls_ldv)
+  double* d_V = nullptr;      // [K_pad][ldv] FP64 table
 
   // per-batch workspace (grown on demand)
   int ws_omega = 0;           // omegas the workspace holds
-  int splits = 1;             // K splits of the contraction (fixed per context)
-  int f64_form = KLS_F64_4M;  // FP64 contraction: 4 or 3 (Gauss) real products
+  int splits = 1;             // K splits of an off-diagonal part (fixed per context)
+  int f64_form = KLS_F64_4M;  // accepted name of the FP64 form (both run one kernel)
+  // work items of the FP64 contraction for plan_splits (0: none yet)
+  int plan_splits = 0, n_slots = 0;
+  std::vector<int4> items;    // (gi << 16 | gj, slot, first slab, slabs)
+  int4* d_items = nullptr;
+  int2* d_tiles = nullptr;    // (first slot, slots) per part gi (gi + 1) / 2 + gj
   double* d_omega = nullptr;  // [ws_omega][2]
   double2* d_wt = nullptr;    // [ws_omega][K_pad]
-  double2* d_part = nullptr;  // [ws_omega][splits][Na_pad][Na_pad]
+  size_t part_elems = 0;      // values d_part holds (FP64 evaluations only)
+  double2* d_part = nullptr;  // [omega][n_slots][64 x 64]
   double2* d_A = nullptr;     // [ws_omega][Na][Na]  I - M (row-major), overwritten by LU
   double2* d_M = nullptr;     // [Na][Na] optional M export (row-major beta, alpha)
   // KLS_MODE_ANCHORED: FP64 M at the anchor omega (row-major beta, alpha)
@@ -181,26 +197,28 @@ int kls_run_orbits(kls_ctx* c);
 int kls_upload_alpha(kls_ctx* c);
 int kls_run_basis(kls_ctx* c);
 int kls_run_weights(kls_ctx* c, int n, const double* anchor = nullptr);
-int kls_run_contract_f64(kls_ctx* c, int n, int splits);
-int kls_run_reduce(kls_ctx* c, int n, int splits, bool export_M);
+int kls_run_contract_f64(kls_ctx* c, int n);
+int kls_run_reduce(kls_ctx* c, int n, bool export_M);
+int kls_f64_plan(kls_ctx* c);                       // items and slots of c->splits
+size_t kls_f64_part_elems(const kls_ctx* c, int n);
 int kls_run_lu(kls_ctx* c, int n);
 int kls_choose_splits(const kls_ctx* c);
+int kls_f64_max_splits(const kls_ctx* c);
 // mixed-precision path (kls_mixed.cu)
 int kls_mixed_prepare(kls_ctx* c);
-int kls_mixed_contract(kls_ctx* c, int n, int splits);
+int kls_mixed_contract(kls_ctx* c, int n);
 int kls_mixed_reduce(kls_ctx* c, int n, bool export_M, const double2* Ma = nullptr);
 int kls_mixed_check(kls_ctx* c);     // pipeline timeout flag of the last launches
 void kls_mixed_free(kls_ctx* c);
 // uneven batch over models (kls_multi.cu drives these)
 int kls_multi_launch_f64(cudaStream_t st, const kls_mdesc* d_md, const int2* d_pairs, int n_pairs,
                          const kls_item* d_items, int n_items, int* d_counter, int grid,
-                         int64_t max_K_pad, int form);
+                         int64_t max_K_pad, int max_ldv);
 int kls_multi_launch_lu(cudaStream_t st, const kls_mdesc* d_md, const int2* d_pairs, int n_pairs,
                         int max_Na);
 int kls_multi_launch_f64_weights(cudaStream_t st, const kls_mdesc* d_md, const int2* d_pairs,
                                  int n_pairs, int64_t max_K_pad);
-int kls_multi_contract_slots(int device, int form);
-int64_t kls_f64_k_per_split(int64_t K_pad, int splits);
+int kls_multi_contract_slots(int device);
 int kls_multi_launch_mixed(cudaStream_t st, const kls_mdesc* d_md, const int2* d_pairs,
                            int n_pairs, const kls_item* d_items, const int* d_starts, int grid,
                            int64_t max_K_pad, int* d_err);

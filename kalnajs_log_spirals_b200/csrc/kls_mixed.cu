@@ -92,33 +92,52 @@ __device__ __forceinline__ void split2(double v, __nv_bfloat16& hi, __nv_bfloat1
   lo = __float2bfloat16_rn((float)(v - (double)__bfloat162float(hi)));
 }
 
-// [K_pad][Npad] FP64 planes -> X{h,l}, rows a (Re) and Npad + a (Im), in
-// 64-k blocks: element (r, k) at (k / 64) * (2 Npad * 64) + r * 64 + k % 64
-__global__ void split_table_kernel(const double* __restrict__ Wre, const double* __restrict__ Wim,
-                                   int Npad, int64_t K_pad, __nv_bfloat16* __restrict__ Xh,
-                                   __nv_bfloat16* __restrict__ Xl) {
-  (void)K_pad;
+// FP64 table V [K_pad][ldv] (pairs Re W, Im W at the alphas >= 0) -> X{h,l},
+// rows a (Re) and Npad + a (Im) of every alpha, in 64-k blocks: element (r, k)
+// at (k / 64) * (2 Npad * 64) + r * 64 + k % 64.  Alpha -a is the conjugate of
+// alpha a (the split of -x is the negated split of x); the rows of the padding
+// alphas are zero.  Grid (K_pad / 64, pairs / 16): a CTA reads 64 rows x 16
+// pairs (256-byte pieces) and writes 64 rows of X, 128 bytes each.
+__global__ void __launch_bounds__(256)
+split_table_kernel(const double* __restrict__ V, int ldv, int Na, int Npad,
+                   __nv_bfloat16* __restrict__ Xh, __nv_bfloat16* __restrict__ Xl) {
   const size_t blk = (size_t)2 * Npad * MX_BK;      // elements of one 64-k block
-  __shared__ double tr[32][33], ti[32][33];
-  const int64_t k0 = (int64_t)blockIdx.x * 32;
-  const int a0 = blockIdx.y * 32;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  for (int i = ty; i < 32; i += 8) {
-    tr[i][tx] = Wre[(size_t)(k0 + i) * Npad + a0 + tx];
-    ti[i][tx] = Wim[(size_t)(k0 + i) * Npad + a0 + tx];
+  __shared__ double t[MX_BK][33];
+  const int64_t k0 = (int64_t)blockIdx.x * MX_BK;
+  const int p0 = blockIdx.y * 16, np = (Na + 1) / 2;
+  for (int e = threadIdx.x; e < MX_BK * 32; e += 256) {
+    const int k = e >> 5, c = e & 31;
+    t[k][c] = 2 * p0 + c < ldv ? V[(size_t)(k0 + k) * ldv + 2 * p0 + c] : 0.0;
   }
   __syncthreads();
-  for (int i = ty; i < 32; i += 8) {
-    __nv_bfloat16 h, l;
-    split2(tr[tx][i], h, l);
-    const int64_t k = k0 + tx;
-    size_t o = (size_t)(k >> 6) * blk + (size_t)(a0 + i) * MX_BK + (k & 63);
-    Xh[o] = h;
-    Xl[o] = l;
-    split2(ti[tx][i], h, l);
-    o = (size_t)(k >> 6) * blk + (size_t)(Npad + a0 + i) * MX_BK + (k & 63);
-    Xh[o] = h;
-    Xl[o] = l;
+  const int k = 2 * (threadIdx.x & 31);
+  __nv_bfloat162* xh = reinterpret_cast<__nv_bfloat162*>(Xh + (size_t)blockIdx.x * blk + k);
+  __nv_bfloat162* xl = reinterpret_cast<__nv_bfloat162*>(Xl + (size_t)blockIdx.x * blk + k);
+  auto put = [&](int row, __nv_bfloat162 h, __nv_bfloat162 l) {
+    xh[row * (MX_BK / 2)] = h;
+    xl[row * (MX_BK / 2)] = l;
+  };
+  for (int c = threadIdx.x >> 5; c < 32; c += 8) {
+    const int p = p0 + (c >> 1), part = c & 1;
+    if (p >= np) continue;
+    __nv_bfloat162 h, l;
+    split2(t[k][c], h.x, l.x);
+    split2(t[k + 1][c], h.y, l.y);
+    // alpha index of pair p: centre + p (odd Na), Na / 2 + p (even)
+    const int pos = Na / 2 + p, neg = np - 1 - p;
+    put(part * Npad + pos, h, l);
+    if (pos != neg) {
+      if (part) { h = __hneg2(h); l = __hneg2(l); }
+      put(part * Npad + neg, h, l);
+    }
+  }
+  // padding alphas: the CTAs of the first pairs clear them
+  if (blockIdx.y == 0) {
+    const __nv_bfloat162 z = __float2bfloat162_rn(0.f);
+    for (int r = Na + (threadIdx.x >> 5); r < Npad; r += 8) {
+      put(r, z, z);
+      put(Npad + r, z, z);
+    }
   }
 }
 
@@ -1198,9 +1217,8 @@ int kls_mixed_prepare(kls_ctx* c) {
   c->device_bytes += (int64_t)(2 * n * sizeof(__nv_bfloat16));
   c->mixed = m;
   KLS_CK(c, cudaMemsetAsync(m->err, 0, sizeof(int), c->stream));
-  dim3 grid((unsigned)(c->K_pad / 32), c->Na_pad / 32);
-  split_table_kernel<<<grid, dim3(32, 8), 0, c->stream>>>(c->d_Wre, c->d_Wim, c->Na_pad, c->K_pad,
-                                                          m->Xh, m->Xl);
+  dim3 grid((unsigned)(c->K_pad / MX_BK), ((c->Na + 1) / 2 + 15) / 16);
+  split_table_kernel<<<grid, 256, 0, c->stream>>>(c->d_V, c->ldv, c->Na, c->Na_pad, m->Xh, m->Xl);
   KLS_LAUNCHED(c);
   // TMA descriptors over X{h,l}: box {64 k, 128 rows, 1 block}, 128B swizzle
   void* fn = nullptr;
@@ -1236,7 +1254,7 @@ int kls_mixed_prepare(kls_ctx* c) {
   return KLS_OK;
 }
 
-int kls_mixed_contract(kls_ctx* c, int n, int) {
+int kls_mixed_contract(kls_ctx* c, int n) {
   kls_mixed* m = c->mixed;
   if (m->form == KLS_MIXED_TMEM) {
     const int fault = m->fault_mode;

@@ -31,7 +31,6 @@
 
 struct kls_multi {
   int device = 0, mode = 0, batch = 0, n_models = 0;
-  int f64_form = KLS_F64_4M;        // FP64: every model's contraction form
   std::vector<kls_ctx*> ctx;
   cudaStream_t stream = nullptr;
   std::string err;
@@ -56,7 +55,7 @@ struct kls_multi {
   int max_Npad = 0;
   double schedule_ms[2] = {0, 0};   // mixed: eager-pass time of each schedule
   std::vector<int2> pairs;          // (model, omega) pairs
-  int grid = 0, max_Na = 0;
+  int grid = 0, max_Na = 0, max_ldv = 0;
   int64_t max_K_pad = 0;
 
   kls_mdesc* d_md = nullptr;
@@ -138,18 +137,13 @@ int build_items(kls_multi* m) {
     return (double)x.K_pad * x.Na_pad * x.Na_pad > (double)y.K_pad * y.Na_pad * y.Na_pad;
   });
   if (m->mode == KLS_MODE_FP64) {
+    // each context's own items (kls_f64_plan)
     for (int i : order) {
-      const kls_mdesc& d = m->md[i];
-      const int tiles = (d.Na_pad / KLS_TILE) * (d.Na_pad / KLS_TILE);
       for (int z = 0; z < m->batch; ++z)
-        for (int s = 0; s < d.splits; ++s)
-          for (int t = 0; t < tiles; ++t) {
-            int64_t kb = (int64_t)s * d.k_per_split;
-            int64_t ke = std::min(d.K_pad, kb + d.k_per_split);
-            m->items.push_back(kls_item{i, z, t, s, 1, 0, (int)std::max<int64_t>(0, ke - kb), 0});
-          }
+        for (const int4& q : m->ctx[i]->items)
+          m->items.push_back(kls_item{i, z, q.x, q.y, 1, q.z, q.w, 0});
     }
-    m->grid = std::max(1, std::min((int)m->items.size(), kls_multi_contract_slots(m->device, m->f64_form)));
+    m->grid = std::max(1, std::min((int)m->items.size(), kls_multi_contract_slots(m->device)));
     return KLS_OK;
   }
   m->list.clear();
@@ -227,7 +221,7 @@ int launch_batch(kls_multi* m) {
   const int np = (int)m->pairs.size();
   if (m->mode == KLS_MODE_FP64) {
     r = kls_multi_launch_f64(m->stream, m->d_md, m->d_pairs, np, m->d_items, (int)m->items.size(),
-                             m->d_counter, m->grid, m->max_K_pad, m->f64_form);
+                             m->d_counter, m->grid, m->max_K_pad, m->max_ldv);
   } else {
     // the mixed weights are converted from the FP64 weights of the same pass
     r = kls_multi_launch_f64_weights(m->stream, m->d_md, m->d_pairs, np, m->max_K_pad);
@@ -376,7 +370,7 @@ int kls_multi_create(kls_ctx* const* models, int n_models, int mode, int batch, 
       return mfail(nullptr, KLS_ERR_STATE, "model " + std::to_string(i) + " is not precomputed");
     if (models[i]->device != models[0]->device)
       return mfail(nullptr, KLS_ERR_CONFIG, "all models of a batch must be on one device");
-    if (mode == KLS_MODE_FP64 && !models[i]->d_Wre)
+    if (mode == KLS_MODE_FP64 && !models[i]->d_V)
       return mfail(nullptr, KLS_ERR_STATE,
                    "model " + std::to_string(i) + ": the FP64 table was released");
     if (mode == KLS_MODE_FP64 && models[i]->f64_form != models[0]->f64_form)
@@ -385,7 +379,6 @@ int kls_multi_create(kls_ctx* const* models, int n_models, int mode, int batch, 
   kls_multi* m = new kls_multi();
   m->device = models[0]->device;
   m->mode = mode;
-  m->f64_form = models[0]->f64_form;
   m->batch = batch;
   m->n_models = n_models;
   m->ctx.assign(models, models + n_models);
@@ -433,8 +426,8 @@ int kls_multi_create(kls_ctx* const* models, int n_models, int mode, int batch, 
   for (int i = 0; i < n_models; ++i) {
     kls_ctx* c = models[i];
     kls_mdesc d{};
-    d.Wre = c->d_Wre;
-    d.Wim = c->d_Wim;
+    d.V = c->d_V;
+    d.ldv = c->ldv;
     d.Gk = c->d_Gk;
     d.Ok = c->d_Ok;
     d.Nk = c->d_N;
@@ -445,14 +438,21 @@ int kls_multi_create(kls_ctx* const* models, int n_models, int mode, int batch, 
     d.K_pad = c->K_pad;
     d.Na = c->Na;
     d.Na_pad = c->Na_pad;
-    d.model = i;
     if ((r = malloc_buf(m, &d.wt, (size_t)batch * c->K_pad))) return bail(r);
     if ((r = malloc_buf(m, &d.A, (size_t)batch * c->Na * c->Na))) return bail(r);
     if (mode == KLS_MODE_FP64) {
-      d.splits = c->splits;
-      d.k_per_split = kls_f64_k_per_split(c->K_pad, c->splits);
-      if ((r = malloc_buf(m, &d.part, (size_t)batch * d.splits * c->Na_pad * c->Na_pad)))
+      if ((r = kls_f64_plan(c))) return bail(mfail(m, r, c->err));
+      d.n_slots = c->n_slots;
+      // the batch's own copy of the slot table: the context may be retuned later
+      int2* tiles = nullptr;
+      const size_t G = (size_t)(c->ldv / 8 + 7) / 8, nt = G * (G + 1) / 2;
+      if ((r = malloc_buf(m, &tiles, nt)) ||
+          (r = malloc_buf(m, &d.part, kls_f64_part_elems(c, batch))))
         return bail(r);
+      if (cudaMemcpy(tiles, c->d_tiles, nt * sizeof(int2), cudaMemcpyDeviceToDevice) != cudaSuccess)
+        return bail(mcuda(m, cudaGetLastError(), "cudaMemcpy (slot table)"));
+      d.tiles = tiles;
+      m->max_ldv = std::max(m->max_ldv, c->ldv);
     } else {
       if (!c->mixed && (r = kls_mixed_prepare(c))) return bail(mfail(m, r, c->err));
       if (m->use_tm[i]) {
