@@ -102,11 +102,23 @@ void dfree(void* p) {
   if (p) cudaFree(p);
 }
 
-// the FP64 contraction's work items and partials for n omegas
+// the FP64 contraction's work items and partials (self-similar form: F) for n omegas
 int ensure_f64(kls_ctx* c, int n) {
   int r;
-  if ((r = kls_f64_plan(c))) return r;
-  const size_t need = kls_f64_part_elems(c, n);
+  if (c->fp64_released)
+    return kls_fail(c, KLS_ERR_STATE, "the FP64 table was released (kls_release_fp64)");
+  if (!c->sim && (r = kls_f64_plan(c))) return r;
+  const size_t need = c->sim ? kls_similar_part_elems(c, n) : kls_f64_part_elems(c, n);
+  if (c->sim && kls_similar_f_bytes(c, n) > c->F_bytes) {
+    dfree(c->d_F);
+    c->d_F = nullptr;
+    c->F_bytes = 0;
+    const size_t fb = kls_similar_f_bytes(c, n);
+    char* p = nullptr;
+    if ((r = dalloc(c, &p, fb))) return r;
+    c->d_F = p;
+    c->F_bytes = fb;
+  }
   if (need <= c->part_elems) return KLS_OK;
   dfree(c->d_part);
   c->d_part = nullptr;
@@ -151,8 +163,14 @@ int run_batch(kls_ctx* c, int n, int mode, bool export_M) {
   if ((r = kls_run_weights(c, n, anchored ? c->anchor_w : nullptr))) return r;
   if (c->timing) KLS_CK(c, cudaEventRecord(c->ev[1], c->stream));
   if (mode == KLS_MODE_FP64) {
-    if (!c->d_V) return kls_fail(c, KLS_ERR_STATE, "the FP64 table was released (kls_release_fp64)");
-    if ((r = kls_run_contract_f64(c, n))) return r;
+    if (c->sim) {
+      int launched = 0;
+      KLS_CK(c, kls_similar_launch(c, c->stream, n, c->d_wt, c->d_F, c->d_part, c->d_A,
+                                   export_M ? c->d_M : nullptr, &launched));
+      c->launches += launched;
+    } else if ((r = kls_run_contract_f64(c, n))) {
+      return r;
+    }
   } else {
     if (!c->mixed && (r = kls_mixed_prepare(c))) return r;
     if ((r = kls_mixed_contract(c, n))) return r;
@@ -160,8 +178,8 @@ int run_batch(kls_ctx* c, int n, int mode, bool export_M) {
   if (c->timing) KLS_CK(c, cudaEventRecord(c->ev[2], c->stream));
   if (mode != KLS_MODE_FP64) {
     if ((r = kls_mixed_reduce(c, n, export_M, anchored ? c->d_anchorM : nullptr))) return r;
-  } else if ((r = kls_run_reduce(c, n, export_M))) {
-    return r;
+  } else if (!c->sim && (r = kls_run_reduce(c, n, export_M))) {
+    return r;                        // (the self-similar form's is part of its launch)
   }
   if (c->timing) KLS_CK(c, cudaEventRecord(c->ev[3], c->stream));
   if ((r = kls_run_lu(c, n))) return r;
@@ -280,18 +298,7 @@ int kls_create(const kls_config* cfg, int device, kls_ctx** out) {
   c->ldv = kls_ldv(c->Na);
   c->K = (int64_t)c->NPh * c->n_l;
   c->K_pad = ((c->K + KLS_KROW_ALIGN - 1) / KLS_KROW_ALIGN) * KLS_KROW_ALIGN;
-  c->splits = kls_choose_splits(c);
 
-  size_t need = (size_t)c->K_pad * c->ldv * sizeof(double);
-  size_t fr = 0, tot = 0;
-  cudaMemGetInfo(&fr, &tot);
-  if (need > fr) {
-    char buf[200];
-    snprintf(buf, sizeof buf, "W table needs %.2f GB, device has %.2f GB free", need / 1e9,
-             fr / 1e9);
-    kls_destroy(c);
-    return kls_fail(nullptr, KLS_ERR_OOM, buf);
-  }
   if ((r = dalloc(c, &c->d_cosw, c->nw)) || (r = dalloc(c, &c->d_sinw, c->nw)) ||
       (r = dalloc(c, &c->d_of, (size_t)OF_COUNT * c->NPh)) ||
       (r = dalloc(c, &c->d_SRC, c->NR)) || (r = dalloc(c, &c->d_rc, c->NR)) ||
@@ -302,7 +309,6 @@ int kls_create(const kls_config* cfg, int device, kls_ctx** out) {
       (r = dalloc(c, &c->d_alpha, c->Na)) || (r = dalloc(c, &c->d_dalpha, c->Na)) ||
       (r = dalloc(c, &c->d_N, c->Na)) || (r = dalloc(c, &c->d_Gk, c->K_pad)) ||
       (r = dalloc(c, &c->d_Ok, c->K_pad)) || (r = dalloc(c, &c->d_F0l, c->K_pad)) ||
-      (r = dalloc(c, &c->d_V, (size_t)c->K_pad * c->ldv)) ||
       (r = dalloc(c, &c->d_M, (size_t)c->Na * c->Na))) {
     std::string m = c->err;
     kls_destroy(c);
@@ -317,9 +323,10 @@ int kls_destroy(kls_ctx* c) {
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   kls_mixed_free(c);
+  kls_similar_free(c);
   void* ptrs[] = {c->d_cosw, c->d_sinw, c->d_of, c->d_SRC, c->d_rc, c->d_valid, c->d_w1, c->d_ra,
                   c->d_pha, c->d_alpha, c->d_dalpha, c->d_N, c->d_Gk, c->d_Ok, c->d_F0l,
-                  c->d_V, c->d_items, c->d_tiles, c->d_omega, c->d_wt, c->d_part, c->d_A, c->d_M,
+                  c->d_V, c->d_items, c->d_tiles, c->d_F, c->d_omega, c->d_wt, c->d_part, c->d_A, c->d_M,
                   c->d_anchorM, c->d_det, c->d_logabs};
   for (void* p : ptrs) dfree(p);
   for (auto& ev : c->ev) if (ev) cudaEventDestroy(ev);
@@ -349,6 +356,12 @@ int kls_precompute(kls_ctx* c) {
   int r;
   if ((r = kls_run_orbits(c))) return r;
   if ((r = kls_run_basis(c))) return r;
+  // the FP64 form: self-similar where the orbits are, else over the table
+  if (!c->fp64_released) {
+    if ((r = kls_similar_prepare(c))) return r;
+    if (!c->sim && (r = kls_build_table(c))) return r;
+    if (!c->precomputed) c->splits = kls_choose_splits(c);
+  }
   KLS_CK(c, cudaStreamSynchronize(c->stream));
   if (c->timing && c->pev[3]) {
     KLS_CK(c, cudaEventElapsedTime(&c->pre_ms[0], c->pev[0], c->pev[1]));
@@ -369,11 +382,9 @@ int kls_release_fp64(kls_ctx* c) {
   if (r) return r;
   if (!c->mixed && (r = kls_mixed_prepare(c))) return r;
   KLS_CK(c, cudaStreamSynchronize(c->stream));
-  if (c->d_V) {
-    cudaFree(c->d_V);
-    c->d_V = nullptr;
-    c->device_bytes -= (int64_t)((size_t)c->K_pad * c->ldv * sizeof(double));
-  }
+  kls_drop_table(c);
+  kls_similar_free(c);
+  c->fp64_released = true;
   return KLS_OK;
 }
 
@@ -426,7 +437,7 @@ int kls_export_resonant(kls_ctx* c, double* F0l, double* Ores) {
 }
 
 int kls_export_W(kls_ctx* c, int il0, int nl, double* W) {
-  if (c->precomputed && !c->d_V)
+  if (c->precomputed && c->fp64_released)
     return kls_fail(c, KLS_ERR_STATE, "the FP64 table was released (kls_release_fp64)");
   int r = check_ready(c);
   if (r) return r;
@@ -435,10 +446,24 @@ int kls_export_W(kls_ctx* c, int il0, int nl, double* W) {
   const size_t rows = c->NPh, ld = c->ldv;
   const int np = (c->Na + 1) / 2;
   std::vector<double> v(rows * ld);
+  // without the table its rows are formed for 32 harmonics at a time
+  constexpr int NB = 32;
+  double* tmp = nullptr;
+  if (!c->d_V && nl > 0)
+    KLS_CK(c, cudaMalloc(&tmp, (size_t)std::min(nl, NB) * rows * ld * sizeof(double)));
+  struct Free { double* p; ~Free() { cudaFree(p); } } guard{tmp};
   for (int q = 0; q < nl; ++q) {
-    size_t r0 = (size_t)(il0 + q) * rows;
-    KLS_CK(c, cudaMemcpy(v.data(), c->d_V + r0 * ld, rows * ld * sizeof(double),
-                         cudaMemcpyDeviceToHost));
+    const double* src = c->d_V + (size_t)(il0 + q) * rows * ld;
+    if (!c->d_V) {
+      if (q % NB == 0) {
+        if ((r = kls_run_wl(c, c->NPh, c->cfg.l_min + il0 + q, std::min(NB, nl - q), c->d_of,
+                            c->d_valid, c->d_w1, c->d_ra, c->d_pha, tmp)))
+          return r;
+        KLS_CK(c, cudaStreamSynchronize(c->stream));
+      }
+      src = tmp + (size_t)(q % NB) * rows * ld;
+    }
+    KLS_CK(c, cudaMemcpy(v.data(), src, rows * ld * sizeof(double), cudaMemcpyDeviceToHost));
     // reference layout [NPh, N_alpha, n_l], column-major, interleaved complex;
     // W(-alpha) = conj W(alpha)
     double* blk = W + (size_t)2 * q * rows * c->Na;
@@ -531,7 +556,8 @@ int kls_set_anchor(kls_ctx* c, double wr, double wi, double* det_ri) {
   if (r) return r;
   if (!std::isfinite(wr) || !std::isfinite(wi))
     return kls_fail(c, KLS_ERR_NONFINITE, "non-finite anchor omega");
-  if (!c->d_V) return kls_fail(c, KLS_ERR_STATE, "the FP64 table was released (kls_release_fp64)");
+  if (c->fp64_released)
+    return kls_fail(c, KLS_ERR_STATE, "the FP64 table was released (kls_release_fp64)");
   if (!c->mixed && (r = kls_mixed_prepare(c))) return r;
   if (!c->d_anchorM && (r = dalloc(c, &c->d_anchorM, (size_t)c->Na * c->Na))) return r;
   if ((r = ensure_ws(c, 1, KLS_MODE_FP64))) return r;
@@ -921,7 +947,13 @@ int time_contraction(kls_ctx* c, int mode, int n, double* ms) {
                             cudaMemcpyHostToDevice, c->stream));
   if ((r = kls_run_weights(c, n))) return r;
   auto once = [&]() -> int {
-    return mode == KLS_MODE_FP64 ? kls_run_contract_f64(c, n) : kls_mixed_contract(c, n);
+    if (mode != KLS_MODE_FP64) return kls_mixed_contract(c, n);
+    if (!c->sim) return kls_run_contract_f64(c, n);
+    int launched = 0;
+    KLS_CK(c, kls_similar_launch(c, c->stream, n, c->d_wt, c->d_F, c->d_part, c->d_A, nullptr,
+                                 &launched));
+    c->launches += launched;
+    return KLS_OK;
   };
   if ((r = once())) return r;               // warm-up (and workspace growth)
   cudaEvent_t e0, e1;
@@ -952,7 +984,7 @@ int kls_autotune(kls_ctx* c, int mode, int batch, kls_tune_result* out) {
   if (mode != KLS_MODE_FP64 && mode != KLS_MODE_MIXED)
     return kls_fail(c, KLS_ERR_CONFIG, "unknown precision mode");
   if (batch < 1 || batch > WS_CHUNK) return kls_fail(c, KLS_ERR_CONFIG, "bad autotune batch");
-  if (mode == KLS_MODE_FP64 && !c->d_V)
+  if (mode == KLS_MODE_FP64 && c->fp64_released)
     return kls_fail(c, KLS_ERR_STATE, "the FP64 table was released (kls_release_fp64)");
   if (mode == KLS_MODE_MIXED && !c->mixed && (r = kls_mixed_prepare(c))) return r;
   const bool mixed = mode == KLS_MODE_MIXED;
@@ -1001,8 +1033,9 @@ int kls_autotune(kls_ctx* c, int mode, int batch, kls_tune_result* out) {
     std::vector<int> cand = {std::max(1, fdef / 2), fdef, 2 * fdef, 3 * fdef};
     // more FP64 splits only while the partials of `batch` omegas stay within 2 GiB
     if (!mixed) {
-      if ((r = apply(fdef, form)) || (r = kls_f64_plan(c))) return r;
-      const double bytes = (double)kls_f64_part_elems(c, batch) * sizeof(double2);
+      if ((r = apply(fdef, form)) || (!c->sim && (r = kls_f64_plan(c)))) return r;
+      const double bytes = sizeof(double2) * (double)(c->sim ? kls_similar_part_elems(c, batch)
+                                                             : kls_f64_part_elems(c, batch));
       while (cand.size() > 2 && bytes * (cand.size() - 1) > 2.0 * 1024 * 1024 * 1024)
         cand.pop_back();
     }

@@ -21,6 +21,7 @@
 //   Omega_res = l Om1 + m Om2.
 #include "kls_internal.cuh"
 #include <cmath>
+#include <cstdio>
 
 namespace {
 
@@ -231,8 +232,9 @@ __global__ void n_kernel(int Na, int m, const double* __restrict__ alpha,
 }
 
 __global__ void rows_kernel(int NPh, int n_l, int l_min, int m, int64_t K, int64_t K_pad,
-                            const double* __restrict__ of, double* __restrict__ Gk,
-                            double* __restrict__ Ok, double* __restrict__ F0l) {
+                            const double* __restrict__ of, const int* __restrict__ valid,
+                            double* __restrict__ Gk, double* __restrict__ Ok,
+                            double* __restrict__ F0l) {
   int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= K_pad) return;
   KLS_UNLESS(KLS_IB(k, K_pad, KS_ROWS), return)
@@ -245,7 +247,8 @@ __global__ void rows_kernel(int NPh, int n_l, int l_min, int m, int64_t K, int64
   double DJ = of[(size_t)OF_DJ * NPh + p];
   double ores = l * om1 + m * om2;
   double f0l = ores * FE + m * FL;
-  Gk[k] = DJ * f0l;
+  // an orbit with non-finite samples has W = 0: no weight either
+  Gk[k] = KLS_LD(KLS_IB(p, NPh, KS_ROWS), valid[p], 0) ? DJ * f0l : 0.0 * (DJ * f0l);
   Ok[k] = ores;
   F0l[k] = f0l;
 }
@@ -260,23 +263,53 @@ int kls_run_basis(kls_ctx* c) {
                                                       c->d_N);
   KLS_LAUNCHED(c);
   rows_kernel<<<(unsigned)((c->K_pad + 255) / 256), 256, 0, c->stream>>>(
-      c->NPh, c->n_l, k.l_min, k.m, c->K, c->K_pad, c->d_of, c->d_Gk, c->d_Ok, c->d_F0l);
+      c->NPh, c->n_l, k.l_min, k.m, c->K, c->K_pad, c->d_of, c->d_valid, c->d_Gk, c->d_Ok,
+      c->d_F0l);
   KLS_LAUNCHED(c);
-  // zero the padding rows of the table (rows K..K_pad-1)
-  size_t pad_rows = (size_t)(c->K_pad - c->K);
-  if (pad_rows)
-    KLS_CK(c, cudaMemsetAsync(c->d_V + (size_t)c->K * c->ldv, 0,
-                              pad_rows * c->ldv * sizeof(double), c->stream));
+  return KLS_OK;
+}
+
+int kls_run_wl(kls_ctx* c, int n_orb, int l_min, int n_l, const double* of, const int* valid,
+               const double* w1, const double* ra, const double* pha, double* V) {
   WlParams P{};
-  P.NPh = c->NPh; P.nwa = c->nwa; P.np = (c->Na + 1) / 2; P.ldv = c->ldv; P.n_l = c->n_l;
-  P.l_min = k.l_min; P.m = k.m;
-  P.astep = c->Na > 1 ? (2.0 * k.alpha_max) / (double)(c->Na - 1) : 0.0;
-  dim3 grid((unsigned)c->NPh * ((c->n_l + WL_LB - 1) / WL_LB) * ((P.np + WL_AB - 1) / WL_AB));
+  P.NPh = n_orb; P.nwa = c->nwa; P.np = (c->Na + 1) / 2; P.ldv = c->ldv; P.n_l = n_l;
+  P.l_min = l_min; P.m = c->cfg.m;
+  P.astep = c->Na > 1 ? (2.0 * c->cfg.alpha_max) / (double)(c->Na - 1) : 0.0;
+  dim3 grid((unsigned)n_orb * ((n_l + WL_LB - 1) / WL_LB) * ((P.np + WL_AB - 1) / WL_AB));
   kls_pre_mark(c, 2);
   // the alphas >= 0 are the last np of the grid
-  wl_kernel<<<grid, WL_THREADS, 0, c->stream>>>(P, c->d_of, c->d_valid, c->d_w1, c->d_ra,
-                                                c->d_pha, c->d_alpha + (c->Na - P.np), c->d_V);
+  wl_kernel<<<grid, WL_THREADS, 0, c->stream>>>(P, of, valid, w1, ra, pha,
+                                                c->d_alpha + (c->Na - P.np), V);
   KLS_LAUNCHED(c);
   kls_pre_mark(c, 3);
   return KLS_OK;
+}
+
+int kls_build_table(kls_ctx* c) {
+  const size_t n = (size_t)c->K_pad * c->ldv;
+  const bool had = c->d_V != nullptr;
+  cudaError_t e = c->d_V ? cudaSuccess : cudaMalloc(&c->d_V, n * sizeof(double));
+  if (e != cudaSuccess) {
+    c->d_V = nullptr;
+    size_t fr = 0, tot = 0;
+    cudaMemGetInfo(&fr, &tot);
+    char buf[200];
+    snprintf(buf, sizeof buf, "W table needs %.2f GB, device has %.2f GB free",
+             n * sizeof(double) / 1e9, fr / 1e9);
+    return kls_fail(c, KLS_ERR_OOM, buf);
+  }
+  c->device_bytes += had ? 0 : (int64_t)(n * sizeof(double));
+  // zero the padding rows (K..K_pad-1)
+  if (c->K_pad > c->K)
+    KLS_CK(c, cudaMemsetAsync(c->d_V + (size_t)c->K * c->ldv, 0,
+                              (size_t)(c->K_pad - c->K) * c->ldv * sizeof(double), c->stream));
+  return kls_run_wl(c, c->NPh, c->cfg.l_min, c->n_l, c->d_of, c->d_valid, c->d_w1, c->d_ra,
+                    c->d_pha, c->d_V);
+}
+
+void kls_drop_table(kls_ctx* c) {
+  if (!c->d_V) return;
+  cudaFree(c->d_V);
+  c->d_V = nullptr;
+  c->device_bytes -= (int64_t)((size_t)c->K_pad * c->ldv * sizeof(double));
 }

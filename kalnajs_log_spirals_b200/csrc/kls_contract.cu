@@ -507,6 +507,7 @@ static int64_t split_begin(int64_t slabs, int n, int j) {
 
 // a split has at least 4 slabs
 int kls_f64_max_splits(const kls_ctx* c) {
+  if (c->sim) return kls_similar_max_splits(c);
   return (int)std::max<int64_t>(1, std::min<int64_t>(c->K_pad / (4 * CT_BK), INT_MAX / 1024));
 }
 
@@ -519,6 +520,7 @@ int kls_f64_max_splits(const kls_ctx* c) {
 // with 470 / 935 / 2071 equal items, 1.28 without a tail).  At most 4096 items
 // (268 MB of partials per omega).
 int kls_choose_splits(const kls_ctx* c) {
+  if (c->sim) return kls_similar_splits(c);
   const int n8 = c->ldv / 8, G = (n8 + 7) / 8;
   const int slots = f64_slots(c->device, false);
   const int64_t slabs = c->K_pad / CT_BK;
@@ -624,11 +626,8 @@ int kls_run_reduce(kls_ctx* c, int n, bool export_M) {
 // ---- uneven batch over models (kls_multi.cu) ------------------------------------
 int kls_multi_launch_f64(cudaStream_t st, const kls_mdesc* d_md, const int2* d_pairs, int n_pairs,
                          const kls_item* d_items, int n_items, int* d_counter, int grid,
-                         int64_t max_K_pad, int max_ldv) {
-  int wblocks = (int)std::min<int64_t>((max_K_pad + 255) / 256, 1024);
-  multi_weights_kernel<<<dim3(wblocks, n_pairs), 256, 0, st>>>(d_md, d_pairs);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return (int)e;
+                         int max_ldv) {
+  cudaError_t e;
   if ((e = cudaFuncSetAttribute(multi_contract_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)CT_SMEM)) != cudaSuccess)
     return (int)e;

@@ -16,7 +16,8 @@
 constexpr int KLS_TILE = 64;
 constexpr int KLS_KROW_ALIGN = 64;   // K rows padded to a multiple of this
 
-// FP64 table.  The alpha grid is symmetric about 0 and
+// FP64 table (models that kls_similar.cu does not cover, exports and the source
+// of the split-BF16 table).  The alpha grid is symmetric about 0 and
 // W_l(-alpha) = conj W_l(alpha) (the radial factor is real, the log-spiral
 // factor is conjugated), so a row k = (l, orbit) holds, for the
 // np = ceil(N_alpha / 2) alphas >= 0, the pairs V[2p] = Re W, V[2p + 1] = Im W
@@ -35,6 +36,7 @@ enum OrbitField {
 };
 
 struct kls_mixed;   // split-BF16 tables (kls_mixed.cu)
+struct kls_similar; // self-similar form of the FP64 path (kls_similar.cu)
 
 // One model of an uneven batch (device-resident descriptor, kls_multi.cu).
 // The tables are the model context's own; the per-omega buffers belong to
@@ -115,11 +117,14 @@ struct kls_ctx {
   double* d_Ok = nullptr;     // [K_pad]  Omega_res per row
   double* d_F0l = nullptr;    // [K_pad]  F0l per row (export only)
   int ldv = 0;                // row length of the FP64 table (kls_ldv)
-  double* d_V = nullptr;      // [K_pad][ldv] FP64 table
+  double* d_V = nullptr;      // [K_pad][ldv] FP64 table (null while nothing needs it)
+  kls_similar* sim = nullptr; // set when the orbits are self-similar
+  bool fp64_released = false; // kls_release_fp64: no FP64 evaluations any more
 
   // per-batch workspace (grown on demand)
   int ws_omega = 0;           // omegas the workspace holds
-  int splits = 1;             // K splits of an off-diagonal part (fixed per context)
+  int splits = 1;             // K splits of an off-diagonal part, or row splits of the
+                              // self-similar form's pair sum (fixed per context)
   int f64_form = KLS_F64_4M;  // accepted name of the FP64 form (both run one kernel)
   // work items of the FP64 contraction for plan_splits (0: none yet)
   int plan_splits = 0, n_slots = 0;
@@ -130,6 +135,8 @@ struct kls_ctx {
   double2* d_wt = nullptr;    // [ws_omega][K_pad]
   size_t part_elems = 0;      // values d_part holds (FP64 evaluations only)
   double2* d_part = nullptr;  // [omega][n_slots][64 x 64]
+  void* d_F = nullptr;        // self-similar form: F of a chunk of omegas
+  size_t F_bytes = 0;
   double2* d_A = nullptr;     // [ws_omega][Na][Na]  I - M (row-major), overwritten by LU
   double2* d_M = nullptr;     // [Na][Na] optional M export (row-major beta, alpha)
   // KLS_MODE_ANCHORED: FP64 M at the anchor omega (row-major beta, alpha)
@@ -196,6 +203,21 @@ __host__ __device__ inline double kls_lin(double a, double b, int n, int i) {
 int kls_run_orbits(kls_ctx* c);
 int kls_upload_alpha(kls_ctx* c);
 int kls_run_basis(kls_ctx* c);
+// W rows of n_orb orbits and n_l harmonics from l_min: V[il * n_orb + p][ldv]
+int kls_run_wl(kls_ctx* c, int n_orb, int l_min, int n_l, const double* of, const int* valid,
+               const double* w1, const double* ra, const double* pha, double* V);
+int kls_build_table(kls_ctx* c);     // the whole FP64 table into c->d_V
+void kls_drop_table(kls_ctx* c);
+// self-similar form of the FP64 path (kls_similar.cu)
+int kls_similar_prepare(kls_ctx* c);
+void kls_similar_free(kls_ctx* c);
+int kls_similar_splits(const kls_ctx* c);
+int kls_similar_max_splits(const kls_ctx* c);
+size_t kls_similar_f_bytes(const kls_ctx* c, int n);
+size_t kls_similar_part_elems(const kls_ctx* c, int n);
+int kls_similar_ctas(const kls_ctx* c);
+cudaError_t kls_similar_launch(const kls_ctx* c, cudaStream_t st, int n, const double2* wt,
+                               void* F, double2* part, double2* A, double2* M, int* launches);
 int kls_run_weights(kls_ctx* c, int n, const double* anchor = nullptr);
 int kls_run_contract_f64(kls_ctx* c, int n);
 int kls_run_reduce(kls_ctx* c, int n, bool export_M);
@@ -213,7 +235,7 @@ void kls_mixed_free(kls_ctx* c);
 // uneven batch over models (kls_multi.cu drives these)
 int kls_multi_launch_f64(cudaStream_t st, const kls_mdesc* d_md, const int2* d_pairs, int n_pairs,
                          const kls_item* d_items, int n_items, int* d_counter, int grid,
-                         int64_t max_K_pad, int max_ldv);
+                         int max_ldv);
 int kls_multi_launch_lu(cudaStream_t st, const kls_mdesc* d_md, const int2* d_pairs, int n_pairs,
                         int max_Na);
 int kls_multi_launch_f64_weights(cudaStream_t st, const kls_mdesc* d_md, const int2* d_pairs,

@@ -1216,6 +1216,11 @@ int kls_mixed_prepare(kls_ctx* c) {
   }
   c->device_bytes += (int64_t)(2 * n * sizeof(__nv_bfloat16));
   c->mixed = m;
+  int r = c->d_V ? KLS_OK : kls_build_table(c);
+  if (r) {
+    kls_mixed_free(c);
+    return r;
+  }
   KLS_CK(c, cudaMemsetAsync(m->err, 0, sizeof(int), c->stream));
   dim3 grid((unsigned)(c->K_pad / MX_BK), ((c->Na + 1) / 2 + 15) / 16);
   split_table_kernel<<<grid, 256, 0, c->stream>>>(c->d_V, c->ldv, c->Na, c->Na_pad, m->Xh, m->Xl);
@@ -1242,7 +1247,7 @@ int kls_mixed_prepare(kls_ctx* c) {
   }
   m->splits = mixed_splits(c);
   if (kls_tm_supported(c)) {
-    int r = kls_tm_create(c, m->Xh, m->Xl, &m->tm);
+    r = kls_tm_create(c, m->Xh, m->Xl, &m->tm);
     if (r) return r;
     m->form = KLS_MIXED_TMEM;
   }
@@ -1251,6 +1256,7 @@ int kls_mixed_prepare(kls_ctx* c) {
   KLS_CK(c, cudaFuncSetAttribute(mixed_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)MP_SMEM));
   KLS_CK(c, cudaStreamSynchronize(c->stream));
+  if (c->sim) kls_drop_table(c);       // nothing else reads it
   return KLS_OK;
 }
 

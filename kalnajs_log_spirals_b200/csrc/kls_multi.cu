@@ -56,6 +56,10 @@ struct kls_multi {
   double schedule_ms[2] = {0, 0};   // mixed: eager-pass time of each schedule
   std::vector<int2> pairs;          // (model, omega) pairs
   int grid = 0, max_Na = 0, max_ldv = 0;
+  void* d_F = nullptr;              // FP64: F of the self-similar models, in turn
+  int similar_ctas = 0, launches = 0;
+  std::vector<int2> pairs_tab;      // FP64: (model, omega) pairs over the table
+  int2* d_pairs_tab = nullptr;
   int64_t max_K_pad = 0;
 
   kls_mdesc* d_md = nullptr;
@@ -124,10 +128,12 @@ int build_items(kls_multi* m) {
   m->pairs.clear();
   m->pairs_tm.clear();
   m->pairs_old.clear();
+  m->pairs_tab.clear();
   for (int i = 0; i < m->n_models; ++i)
     for (int z = 0; z < m->batch; ++z) {
       m->pairs.push_back(make_int2(i, z));
       (m->use_tm[i] ? m->pairs_tm : m->pairs_old).push_back(make_int2(i, z));
+      if (!m->ctx[i]->sim) m->pairs_tab.push_back(make_int2(i, z));
     }
   if (m->mode != KLS_MODE_FP64 && !m->old) return KLS_OK;   // TMEM items: build_tm_items
   std::vector<int> order(m->n_models);
@@ -139,11 +145,12 @@ int build_items(kls_multi* m) {
   if (m->mode == KLS_MODE_FP64) {
     // each context's own items (kls_f64_plan)
     for (int i : order) {
+      if (m->ctx[i]->sim) continue;        // kls_similar_launch
       for (int z = 0; z < m->batch; ++z)
         for (const int4& q : m->ctx[i]->items)
           m->items.push_back(kls_item{i, z, q.x, q.y, 1, q.z, q.w, 0});
     }
-    m->grid = std::max(1, std::min((int)m->items.size(), kls_multi_contract_slots(m->device)));
+    m->grid = std::min((int)m->items.size(), kls_multi_contract_slots(m->device));
     return KLS_OK;
   }
   m->list.clear();
@@ -220,8 +227,18 @@ int launch_batch(kls_multi* m) {
   int r;
   const int np = (int)m->pairs.size();
   if (m->mode == KLS_MODE_FP64) {
-    r = kls_multi_launch_f64(m->stream, m->d_md, m->d_pairs, np, m->d_items, (int)m->items.size(),
-                             m->d_counter, m->grid, m->max_K_pad, m->max_ldv);
+    r = kls_multi_launch_f64_weights(m->stream, m->d_md, m->d_pairs, np, m->max_K_pad);
+    m->launches = 2;                       // weights, LU
+    if (!r && !m->items.empty()) {
+      r = kls_multi_launch_f64(m->stream, m->d_md, m->d_pairs_tab, (int)m->pairs_tab.size(),
+                               m->d_items, (int)m->items.size(), m->d_counter, m->grid,
+                               m->max_ldv);
+      m->launches += 2;
+    }
+    for (int i = 0; !r && i < m->n_models; ++i)
+      if (m->ctx[i]->sim)
+        r = (int)kls_similar_launch(m->ctx[i], m->stream, m->batch, m->md[i].wt, m->d_F,
+                                    m->md[i].part, m->md[i].A, nullptr, &m->launches);
   } else {
     // the mixed weights are converted from the FP64 weights of the same pass
     r = kls_multi_launch_f64_weights(m->stream, m->d_md, m->d_pairs, np, m->max_K_pad);
@@ -370,7 +387,7 @@ int kls_multi_create(kls_ctx* const* models, int n_models, int mode, int batch, 
       return mfail(nullptr, KLS_ERR_STATE, "model " + std::to_string(i) + " is not precomputed");
     if (models[i]->device != models[0]->device)
       return mfail(nullptr, KLS_ERR_CONFIG, "all models of a batch must be on one device");
-    if (mode == KLS_MODE_FP64 && !models[i]->d_V)
+    if (mode == KLS_MODE_FP64 && models[i]->fp64_released)
       return mfail(nullptr, KLS_ERR_STATE,
                    "model " + std::to_string(i) + ": the FP64 table was released");
     if (mode == KLS_MODE_FP64 && models[i]->f64_form != models[0]->f64_form)
@@ -423,6 +440,7 @@ int kls_multi_create(kls_ctx* const* models, int n_models, int mode, int batch, 
       else m->old = true;
     }
   }
+  size_t F_bytes = 0;
   for (int i = 0; i < n_models; ++i) {
     kls_ctx* c = models[i];
     kls_mdesc d{};
@@ -441,6 +459,15 @@ int kls_multi_create(kls_ctx* const* models, int n_models, int mode, int batch, 
     if ((r = malloc_buf(m, &d.wt, (size_t)batch * c->K_pad))) return bail(r);
     if ((r = malloc_buf(m, &d.A, (size_t)batch * c->Na * c->Na))) return bail(r);
     if (mode == KLS_MODE_FP64) {
+      if (c->sim) {
+        if ((r = malloc_buf(m, &d.part, kls_similar_part_elems(c, batch)))) return bail(r);
+        F_bytes = std::max(F_bytes, kls_similar_f_bytes(c, batch));
+        m->similar_ctas += kls_similar_ctas(c) * batch;
+        m->md[i] = d;
+        m->max_Na = std::max(m->max_Na, c->Na);
+        m->max_K_pad = std::max(m->max_K_pad, c->K_pad);
+        continue;
+      }
       if ((r = kls_f64_plan(c))) return bail(mfail(m, r, c->err));
       d.n_slots = c->n_slots;
       // the batch's own copy of the slot table: the context may be retuned later
@@ -517,16 +544,24 @@ int kls_multi_create(kls_ctx* const* models, int n_models, int mode, int batch, 
                    cudaMemcpyHostToDevice) != cudaSuccess)
       return bail(mcuda(m, cudaGetLastError(), "cudaMemcpy (TMEM-form descriptors)"));
   }
+  if (F_bytes) {
+    char* f = nullptr;
+    if ((r = malloc_buf(m, &f, F_bytes))) return bail(r);
+    m->d_F = f;
+  }
   if ((r = build_items(m))) return bail(r);
   const size_t n_it = std::max(m->items.size(), m->list.size());
   if ((r = malloc_buf(m, &m->d_md, m->md.size())) || (r = malloc_buf(m, &m->d_items, n_it)) ||
       (r = malloc_buf(m, &m->d_pairs, m->pairs.size())) ||
       (r = malloc_buf(m, &m->d_pairs_tm, m->pairs_tm.size())) ||
       (r = malloc_buf(m, &m->d_pairs_old, m->pairs_old.size())) ||
+      (r = malloc_buf(m, &m->d_pairs_tab, m->pairs_tab.size())) ||
       (r = malloc_buf(m, &m->d_starts, n_it + 1)))
     return bail(r);
   if (cudaMemcpy(m->d_md, m->md.data(), m->md.size() * sizeof(kls_mdesc), cudaMemcpyHostToDevice) ||
       cudaMemcpy(m->d_pairs, m->pairs.data(), m->pairs.size() * sizeof(int2),
+                 cudaMemcpyHostToDevice) ||
+      cudaMemcpy(m->d_pairs_tab, m->pairs_tab.data(), m->pairs_tab.size() * sizeof(int2),
                  cudaMemcpyHostToDevice) ||
       cudaMemcpy(m->d_pairs_tm, m->pairs_tm.data(), m->pairs_tm.size() * sizeof(int2),
                  cudaMemcpyHostToDevice) ||
@@ -633,16 +668,20 @@ int kls_multi_get_info(const kls_multi* m, kls_multi_info* out) {
   out->batch = m->batch;
   out->mode = m->mode;
   const bool fp64 = m->mode == KLS_MODE_FP64;
-  out->n_items = (int32_t)((fp64 || m->old ? m->items.size() : 0) + (m->tm ? m->tm_items.size() : 0));
-  out->grid = (fp64 || m->old ? m->grid : 0) + (m->tm ? 2 * (int32_t)m->tm_items.size() : 0);
+  // (a self-similar model's items are the CTAs of its pair sum)
+  out->n_items = (int32_t)((fp64 || m->old ? m->items.size() : 0) +
+                           (m->tm ? m->tm_items.size() : 0)) + m->similar_ctas;
+  out->grid = (fp64 || m->old ? m->grid : 0) + (m->tm ? 2 * (int32_t)m->tm_items.size() : 0) +
+              m->similar_ctas;
   out->graph = m->exec ? 1 : 0;
   out->replays = m->replays;
   out->last_ms = m->last_ms;
   // kernels per replay: weights (+ FP32 copy), contraction, reduction, LU
-  // FP64: weights, contraction, reduction, LU; mixed: FP64 weights, per form
+  // FP64: weights, contraction and reduction over the tables, F / pair sum /
+  // reduction per self-similar model, LU; mixed: FP64 weights, per form
   // (FP32 weights, contraction launch(es), reduction), LU
   out->launches_per_replay =
-      fp64 ? 4
+      fp64 ? m->launches
            : 2 + (m->old ? 3 : 0) +
                  (m->tm ? 2 + (m->tm_schedule == 2 ? (int32_t)m->tmd.size() : 1) : 0);
   // the one-CTA / pair forms' schedule when the batch has such models, else
