@@ -378,12 +378,11 @@ int kls_set_splits(kls_ctx* ctx, int mode, int splits);
 int kls_set_f64_form(kls_ctx* ctx, int form);
 
 /* ---- determinant stage form (no reference counterpart) -------------------- *
- * KLS_LU_CLUSTER factors each I - M(omega) on one thread-block cluster of 8
- * (or 16) CTAs with the matrix held in their shared memory (latency: one
- * matrix per cluster); KLS_LU_CTA uses one CTA per matrix through L2
- * (throughput for many matrices).  KLS_LU_AUTO (default) takes the cluster
- * form when N_alpha >= 128 and the batch fits one wave of clusters.  Both
- * forms return bitwise the same determinants.  KLS_LU_CLUSTER fails with
+ * KLS_LU_CLUSTER factors each I - M(omega) on one thread-block cluster of 1 to
+ * 16 CTAs with the matrix held in their registers (latency: one matrix per
+ * cluster, N_alpha <= 512); KLS_LU_CTA uses one CTA per matrix through L2.
+ * KLS_LU_AUTO (default) takes the cluster form wherever it fits.  Both forms
+ * return bitwise the same determinants.  KLS_LU_CLUSTER fails with
  * KLS_ERR_UNSUPPORTED when N_alpha is too large for it.                      */
 #define KLS_LU_AUTO          0
 #define KLS_LU_CTA           1

@@ -149,7 +149,7 @@ int ensure_ws(kls_ctx* c, int n, int mode) {
 }
 
 // One launch sequence for n (<= ws) omegas already in c->d_omega.
-int run_batch(kls_ctx* c, int n, int mode, bool export_M) {
+int run_batch(kls_ctx* c, int n, int mode, bool export_M, bool want_det = true) {
   KlsRange range(mode == KLS_MODE_FP64 ? "kls det batch (FP64)"
                  : mode == KLS_MODE_MIXED ? "kls det batch (split-BF16)"
                                           : "kls det batch (anchored)");
@@ -182,7 +182,7 @@ int run_batch(kls_ctx* c, int n, int mode, bool export_M) {
     return r;                        // (the self-similar form's is part of its launch)
   }
   if (c->timing) KLS_CK(c, cudaEventRecord(c->ev[3], c->stream));
-  if ((r = kls_run_lu(c, n))) return r;
+  if (want_det && (r = kls_run_lu(c, n))) return r;
   if (c->timing) KLS_CK(c, cudaEventRecord(c->ev[4], c->stream));
   return KLS_OK;
 }
@@ -535,7 +535,7 @@ int kls_build_M(kls_ctx* c, double wr, double wi, int mode, double* M) {
   if ((r = ensure_ws(c, 1, mode))) return r;
   double om[2] = {wr, wi};
   KLS_CK(c, cudaMemcpyAsync(c->d_omega, om, sizeof om, cudaMemcpyHostToDevice, c->stream));
-  if ((r = run_batch(c, 1, mode, true))) return r;
+  if ((r = run_batch(c, 1, mode, true, false))) return r;
   std::vector<double2> h((size_t)c->Na * c->Na);
   KLS_CK(c, cudaMemcpyAsync(h.data(), c->d_M, h.size() * sizeof(double2), cudaMemcpyDeviceToHost,
                             c->stream));

@@ -154,10 +154,11 @@ struct kls_ctx {
   bool gk0_poisoned = false;
   double gk0_saved = 0.0;
 
-  // determinant stage: KLS_LU_* form and the cluster size it uses (-1: not
-  // chosen yet, 0: the cluster form does not fit)
+  // determinant stage: KLS_LU_* form and the size class of the pipelined
+  // kernel (-2: not looked up yet, -1: it does not fit)
   int lu_mode = 0;
-  int lu_cluster = -1;
+  int lu_class = -2;
+  bool lu_wide = false;       // 16 CTAs per matrix fit as well
 
   // instrumentation
   int64_t launches = 0;
@@ -237,7 +238,9 @@ int kls_multi_launch_f64(cudaStream_t st, const kls_mdesc* d_md, const int2* d_p
                          const kls_item* d_items, int n_items, int* d_counter, int grid,
                          int max_ldv);
 int kls_multi_launch_lu(cudaStream_t st, const kls_mdesc* d_md, const int2* d_pairs, int n_pairs,
-                        int max_Na);
+                        int max_Na, int cls);
+int kls_lu_class(int device, int n);
+int kls_lu_classes();
 int kls_multi_launch_f64_weights(cudaStream_t st, const kls_mdesc* d_md, const int2* d_pairs,
                                  int n_pairs, int64_t max_K_pad);
 int kls_multi_contract_slots(int device);

@@ -1,22 +1,36 @@
 // det(I - M(omega)) for a batch of matrices: complex FP64 LU with partial
-// pivoting, one CTA per matrix (the reference moves M to the host and calls
-// LinearAlgebra.det -> LAPACK zgetrf, MatrixBuilder.jl:173-182).
+// pivoting (the reference moves M to the host and calls LinearAlgebra.det ->
+// LAPACK zgetrf, MatrixBuilder.jl:173-182).
 //
 // Pivot choice follows LAPACK's izamax (largest |re| + |im|, first index on
 // ties); the column is scaled by the reciprocal of the pivot as zgetf2 does.
 // The determinant is accumulated as a mantissa and a binary exponent so that
 // products of ~N_alpha pivots neither overflow nor underflow; the result is
 // returned both as a complex number and as log|det|.
+//
+// lu_pipe_kernel (N <= 512): one thread-block cluster per matrix, the matrix in
+// registers, columns passed from warp to warp; lu_det_kernel: one CTA per
+// matrix through L2, any N.  Both return the same bits.
 #include "kls_internal.cuh"
-#include <cooperative_groups.h>
+#include "kls_tcgen05.cuh"
+#include <algorithm>
 #include <cfloat>
 
 namespace {
 
 constexpr int LU_THREADS = 1024;
 
+// 1/(c + i d) = (c - i d) / (c^2 + d^2) on values scaled by a power of two (one
+// reciprocal on the factorisation's serial chain); Smith's two divisions where
+// the exponent leaves no room to scale
 __device__ __forceinline__ double2 cinv(double c, double d) {
-  // Smith's algorithm for 1/(c + i d)
+  const int ex = max(__double2hiint(c) & 0x7ff00000, __double2hiint(d) & 0x7ff00000);
+  if (ex > (64 << 20) && ex < (1982 << 20)) {
+    const double s = __hiloint2double(0x7fe00000 - ex, 0);
+    const double x = __dmul_rn(c, s), y = __dmul_rn(d, s);
+    const double t = __dmul_rn(__drcp_rn(__fma_rn(x, x, __dmul_rn(y, y))), s);
+    return make_double2(__dmul_rn(x, t), __dmul_rn(-y, t));
+  }
   if (fabs(d) <= fabs(c)) {
     double r = d / c, t = 1.0 / (c + d * r);
     return make_double2(t, -r * t);
@@ -31,6 +45,48 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(__fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y)),
                       __fma_rn(a.x, b.y, __dmul_rn(a.y, b.x)));
 }
+
+// a - l p
+__device__ __forceinline__ double2 lu_update(double2 a, double2 l, double2 p) {
+  return make_double2(__fma_rn(l.y, p.y, __fma_rn(-l.x, p.x, a.x)),
+                      __fma_rn(-l.y, p.x, __fma_rn(-l.x, p.y, a.y)));
+}
+
+// running determinant: mant * 2^expo
+struct LuDet {
+  double2 mant = make_double2(1.0, 0.0);
+  long long expo = 0;
+  bool zero = false;
+  __device__ __forceinline__ void normalise() {
+    const double mx = fmax(fabs(mant.x), fabs(mant.y));
+    if (mx != 0.0 && isfinite(mx)) {
+      const int e = ilogb(mx);
+      mant.x = scalbn(mant.x, -e);
+      mant.y = scalbn(mant.y, -e);
+      expo += e;
+    }
+  }
+  // scaling by powers of two is exact, so it is done only when it is needed
+  __device__ __forceinline__ void times(double2 u, bool swapped) {
+    if (swapped) { mant.x = -mant.x; mant.y = -mant.y; }
+    if (u.x == 0.0 && u.y == 0.0) zero = true;
+    mant = cmul(mant, u);
+    const double mx = fmax(fabs(mant.x), fabs(mant.y));
+    if (!(mx > 0x1p-100 && mx < 0x1p100)) normalise();
+  }
+  __device__ __forceinline__ void store(double2* det, double* logabs) {
+    normalise();
+    double2 d = make_double2(0.0, 0.0);
+    double la = -INFINITY;
+    if (!zero) {
+      const long long e = expo > 4000 ? 4000 : expo < -4000 ? -4000 : expo;
+      d = make_double2(scalbn(mant.x, (int)e), scalbn(mant.y, (int)e));
+      la = log(hypot(mant.x, mant.y)) + (double)expo * 0.69314718055994530942;
+    }
+    *det = d;
+    if (logabs) *logabs = la;
+  }
+};
 
 // element (i, c) of the n x n matrix A, guarded in the bounds-checked build
 #define LU_IN(i, c) KLS_IB((int64_t)(i) * n + (c), (int64_t)n * n, KS_LU)
@@ -50,9 +106,7 @@ __device__ __forceinline__ void lu_det_body(int n, double2* __restrict__ A, doub
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nwarps = blockDim.x >> 5;
 
-  double2 mant = make_double2(1.0, 0.0);
-  long long expo = 0;
-  bool zero = false;
+  LuDet acc;
 
   for (int j = 0; j < n; ++j) {
     // ---- pivot search: izamax over rows j..n-1 of column j
@@ -108,43 +162,14 @@ __device__ __forceinline__ void lu_det_body(int n, double2* __restrict__ A, doub
         KLS_UNLESS(LU_IN(i, c), continue)
         double2 p = prow[c];
         double2 a = row[c];
-        a.x = __dsub_rn(a.x, __fma_rn(l.x, p.x, -__dmul_rn(l.y, p.y)));
-        a.y = __dsub_rn(a.y, __fma_rn(l.x, p.y, __dmul_rn(l.y, p.x)));
-        row[c] = a;
+        row[c] = lu_update(a, l, p);
       }
     }
     // ---- determinant accumulation (thread 0)
-    if (tid == 0) {
-      double2 uu = s_u;
-      if (piv != j) { mant.x = -mant.x; mant.y = -mant.y; }
-      if (uu.x == 0.0 && uu.y == 0.0) zero = true;
-      mant = cmul(mant, uu);
-      double mx = fmax(fabs(mant.x), fabs(mant.y));
-      if (mx != 0.0 && isfinite(mx)) {
-        int e = ilogb(mx);
-        mant.x = scalbn(mant.x, -e);
-        mant.y = scalbn(mant.y, -e);
-        expo += e;
-      }
-    }
+    if (tid == 0) acc.times(s_u, piv != j);
     __syncthreads();
   }
-  if (tid == 0) {
-    double2 d;
-    double la;
-    if (zero) {
-      d = make_double2(0.0, 0.0);
-      la = -INFINITY;
-    } else {
-      long long e = expo;
-      if (e > 4000) e = 4000;
-      if (e < -4000) e = -4000;
-      d = make_double2(scalbn(mant.x, (int)e), scalbn(mant.y, (int)e));
-      la = log(hypot(mant.x, mant.y)) + (double)expo * 0.69314718055994530942;
-    }
-    *det_out = d;
-    if (logabs_out) *logabs_out = la;
-  }
+  if (tid == 0) acc.store(det_out, logabs_out);
 }
 
 __global__ void __launch_bounds__(LU_THREADS)
@@ -164,234 +189,442 @@ multi_lu_kernel(const kls_mdesc* __restrict__ md, const int2* __restrict__ pairs
   lu_det_body(d.Na, d.A + (size_t)pz.y * d.Na * d.Na, sh, d.det + pz.y, d.logabs + pz.y);
 }
 
-// ---- cluster form: one thread-block cluster per matrix ---------------------------
-// The matrix is distributed by columns over the C CTAs of a cluster (column g
-// in CTA g mod C, column-major in shared memory), so the whole factorisation
-// stays on chip: per step j the owner of column j searches the pivot, swaps,
-// scales its column into multipliers; after one cluster barrier every CTA
-// reads the pivot row index and the multipliers from the owner's shared
-// memory (DSMEM) and updates its own trailing columns.  Pivot rule, multiplier
-// and update arithmetic and the order of the determinant product are those of
-// lu_det_kernel, so both kernels return the same bits.
-namespace cg = cooperative_groups;
-constexpr int LUC_THREADS = 512;
+// ---- pipelined form: one thread-block cluster per matrix -----------------------
+// Bound: the chain of N columns (pivot search, reciprocal, multipliers, update
+// of the next column), not the flops.  So nothing but that chain is serial:
+//  * every column belongs to one warp and lives in its registers (lane = row mod
+//    32); no row is ever moved: each row carries its position in LAPACK's
+//    order, and an exchange swaps two positions;
+//  * the owner of column j + 1 updates it with column j's multipliers, factors
+//    it and publishes it before it updates the rest of its columns, so the
+//    warps run as a pipeline over the columns without a block or cluster
+//    barrier: a column goes to a ring in the shared memory of every CTA of the
+//    cluster and one mbarrier per slot announces it;
+//  * 8 consecutive columns are on one CTA (its warps in turn), so most hand-overs
+//    stay inside an SM.
+// A slot is written again only when every warp has used it: each warp keeps a
+// count of the columns it is done with, and the owner of every (slots / 2)-th
+// column waits for all of them.
+// Waits are bounded (LUP_LIMIT_NS); one that runs out makes the determinant NaN.
+//
+// Measured (1 matrix, B200): N = 101 312 -> 104 us, 201 557 -> 271 us, 301 1022 ->
+// 632 us against one CTA (101) or a cluster with one barrier per column; 16
+// matrices 315 -> 105, 612 -> 656, 2760 -> 1890 us.  A column's chain is about
+// 1000 cycles at 4 rows a lane and 1900 at 10 (update 215 / 385, pivot search
+// 170 / 324, reciprocal 182, multipliers 48 / 111, hand-over 300).
+constexpr int LUP_WARPS = 8, LUP_THREADS = 32 * LUP_WARPS;
+constexpr unsigned long long LUP_LIMIT_NS = 2000000000ull;
 
-__host__ __device__ inline size_t luc_smem_bytes(int n, int C) {
-  const size_t nc = (size_t)((n + C - 1) / C);
-  return (nc * n + 3 * (size_t)n) * sizeof(double2) + (size_t)n * sizeof(int);
+struct LupMeta {
+  double2 u;                  // pivot
+  int piv, pos;               // its row, and that row's position before the exchange
+};
+
+__device__ __forceinline__ void st_cluster_v2(uint32_t addr, double2 v) {
+  asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(addr), "d"(v.x), "d"(v.y)
+               : "memory");
+}
+__device__ __forceinline__ void st_cluster_v2i(uint32_t addr, int a, int b) {
+  asm volatile("st.shared::cluster.v2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
+}
+__device__ __forceinline__ void arrive_cluster(uint32_t addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ int ld_acquire_cluster(uint32_t addr) {
+  int v;
+  asm volatile("ld.acquire.cluster.shared::cluster.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release_cluster(uint32_t addr, int v) {
+  asm volatile("st.release.cluster.shared::cta.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 
-__global__ void __launch_bounds__(LUC_THREADS)
-lu_cluster_kernel(int n, const double2* __restrict__ Aall, double2* __restrict__ det_out,
-                  double* __restrict__ logabs_out) {
-  extern __shared__ __align__(16) double2 smem[];
-  __shared__ double red_v[32];
-  __shared__ int red_i[32];
-  __shared__ int s_piv;
-  cg::cluster_group cl = cg::this_cluster();
-  const int C = (int)cl.num_blocks();
-  const int rank = (int)cl.block_rank();
-  const int mat = blockIdx.x / C;
-  const int nc = (n + C - 1) / C;
-  double2* col = smem;                        // [nc][n] owned columns g = rank + C lc
-  double2* lvec = col + (size_t)nc * n;       // multipliers of the steps this CTA owns
-  double2* lbuf = lvec + n;                   // copy of the current owner's multipliers
-  double2* rec_u = lbuf + n;                  // rank 0: pivot of every step
-  int* rec_s = reinterpret_cast<int*>(rec_u + n);   // rank 0: row interchange flags
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int T = blockDim.x, nwarps = T >> 5;
-  const int my_nc = rank < n ? (n - 1 - rank) / C + 1 : 0;
-  const double2* A = Aall + (size_t)mat * n * n;
-  for (int e = tid; e < my_nc * n; e += T) {
-    const int lc = e / n, i = e % n;
-    KLS_UNLESS(KLS_IB((int64_t)i * n + rank + C * lc, (int64_t)n * n, KS_LU), continue)
-    col[(size_t)lc * n + i] = A[(size_t)i * n + rank + C * lc];
+// Bounded wait.  The waiting warp is suspended (up to 10 us a try) instead of
+// polling: seven polling warps slow the one that the others wait for (its
+// shuffles and shared-memory reads queue behind theirs).
+__device__ __forceinline__ bool lup_wait(uint32_t bar, uint32_t parity, volatile int* abort) {
+  unsigned long long t0 = 0;
+  for (uint32_t it = 0;; ++it) {
+    uint32_t ok;
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, 10000;\n"
+        "selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if (*abort) return false;
+    if ((it & 15) == 15) {
+      const unsigned long long t = kls_tc::globaltimer();
+      if (!t0) t0 = t;
+      else if (t - t0 > LUP_LIMIT_NS) {
+        *abort = 1;
+        return false;
+      }
+    }
   }
-  double2* rec_u0 = cl.map_shared_rank(rec_u, 0);
-  int* rec_s0 = cl.map_shared_rank(rec_s, 0);
-  __syncthreads();
+}
 
-  for (int j = 0; j < n; ++j) {
-    const int owner = j % C;
-    if (rank == owner) {
-      double2* cj = col + (size_t)(j / C) * n;
-      double bv = -1.0;
-      int bi = n;
-      for (int i = j + tid; i < n; i += T) {
-        const double2 v = cj[i];
-        const double m = fabs(v.x) + fabs(v.y);
-        if (m > bv) { bv = m; bi = i; }
+// element `row` (warp-uniform) of a column held as lane = row & 31, a[row >> 5]
+template <int RPL>
+__device__ __forceinline__ double2 lup_row(const double2 (&a)[RPL], int row) {
+  double2 v = a[0];
+  const int q = row >> 5;
+#pragma unroll
+  for (int r = 1; r < RPL; ++r)
+    if (q == r) v = a[r];
+  return make_double2(__shfl_sync(0xffffffffu, v.x, row & 31),
+                      __shfl_sync(0xffffffffu, v.y, row & 31));
+}
+
+__host__ __device__ inline size_t lup_smem(int n, int slots) {
+  return (size_t)slots * ((size_t)n * sizeof(double2) + sizeof(LupMeta) + sizeof(uint64_t)) + 16;
+}
+
+// RPL rows per lane, LP columns per warp
+template <int RPL, int LP>
+__device__ __forceinline__ void lup_body(int n, int slots, const double2* __restrict__ A,
+                                         double2* __restrict__ det, double* __restrict__ logabs,
+                                         unsigned char* smem) {
+  using namespace kls_tc;
+  __shared__ int prog[LUP_WARPS];             // columns each warp is done with
+  __shared__ volatile int s_abort;
+  __shared__ int s_failed;                    // rank 0: a wait ran out somewhere
+  uint32_t rank, C;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(C));
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double2* ring = reinterpret_cast<double2*>(smem);                 // [slots][n]
+  LupMeta* meta = reinterpret_cast<LupMeta*>(ring + (size_t)slots * n);
+  uint64_t* full = reinterpret_cast<uint64_t*>(meta + slots);
+  if (tid < LUP_WARPS) prog[tid] = 0;
+  if (tid == 0) { s_abort = 0; s_failed = 0; }
+  for (int s = tid; s < slots; s += LUP_THREADS) mbar_init(smem_u32(full + s), 1);
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  // global index of local column lp
+  auto col_of = [&](int lp) {
+    return (lp * (int)C + (int)rank) * LUP_WARPS + warp;
+  };
+  double2 a[LP][RPL];
+  int pos[RPL];
+#pragma unroll
+  for (int r = 0; r < RPL; ++r) {
+    const int i = lane + 32 * r;
+    pos[r] = i < n ? i : -1;
+#pragma unroll
+    for (int lp = 0; lp < LP; ++lp) {
+      const int g = col_of(lp);
+      a[lp][r] = make_double2(0.0, 0.0);
+      if (i < n && g < n) KLS_IF(LU_IN(i, g)) a[lp][r] = A[(size_t)i * n + g];
+    }
+  }
+  cluster_sync_all();                         // barriers initialised everywhere
+
+  // pivot search, multipliers and publication (slot s) of local column c = global g
+  auto factor = [&](double2 (&c)[RPL], int g, int s) {
+    // a lane's largest |re| + |im| by its upper 32 bits, and that entry's
+    // reciprocal, which runs while the warp looks for the largest of all
+    unsigned hm = 0;
+    double2 best = make_double2(1.0, 0.0);
+    unsigned at = 0;
+#pragma unroll
+    for (int r = 0; r < RPL; ++r) {
+      const double m = fabs(c[r].x) + fabs(c[r].y);
+      const unsigned h = pos[r] >= g && m == m ? (unsigned)__double2hiint(m) | 0x80000000u : 0u;
+      if (h > hm) {
+        hm = h;
+        best = c[r];
+        at = ((unsigned)pos[r] << 16) | (unsigned)(lane + 32 * r);
       }
-      for (int off = 16; off; off >>= 1) {
-        const double ov = __shfl_down_sync(0xffffffffu, bv, off);
-        const int oi = __shfl_down_sync(0xffffffffu, bi, off);
-        if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+    }
+    double2 rb = cinv(best.x, best.y);
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hm);
+    int ties = 0;
+#pragma unroll
+    for (int r = 0; r < RPL; ++r) {
+      const double m = fabs(c[r].x) + fabs(c[r].y);
+      if (pos[r] >= g && m == m && ((unsigned)__double2hiint(m) | 0x80000000u) == mh) ++ties;
+    }
+    const unsigned who = __ballot_sync(0xffffffffu, ties > 0);
+    const unsigned more = __ballot_sync(0xffffffffu, ties > 1);
+    int src = __ffs(who) - 1;
+    if (mh == 0u || more || (who & (who - 1))) {
+      // several entries with these bits: all 64 of them, then the position; no
+      // comparable entry at all: the diagonal
+      unsigned lm = 0;
+#pragma unroll
+      for (int r = 0; r < RPL; ++r) {
+        const double m = fabs(c[r].x) + fabs(c[r].y);
+        if (mh && pos[r] >= g && m == m && ((unsigned)__double2hiint(m) | 0x80000000u) == mh)
+          lm = max(lm, (unsigned)__double2loint(m));
       }
-      if (lane == 0) { red_v[warp] = bv; red_i[warp] = bi; }
-      __syncthreads();
-      if (warp == 0) {
-        bv = lane < nwarps ? red_v[lane] : -1.0;
-        bi = lane < nwarps ? red_i[lane] : n;
-        for (int off = 16; off; off >>= 1) {
-          const double ov = __shfl_down_sync(0xffffffffu, bv, off);
-          const int oi = __shfl_down_sync(0xffffffffu, bi, off);
-          if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+      lm = __reduce_max_sync(0xffffffffu, lm);
+      unsigned cand = 0xffffffffu;
+#pragma unroll
+      for (int r = 0; r < RPL; ++r) {
+        const double m = fabs(c[r].x) + fabs(c[r].y);
+        const bool in = mh ? pos[r] >= g && m == m &&
+                                 ((unsigned)__double2hiint(m) | 0x80000000u) == mh &&
+                                 (unsigned)__double2loint(m) == lm
+                           : pos[r] == g;
+        const unsigned x = ((unsigned)pos[r] << 16) | (unsigned)(lane + 32 * r);
+        if (in && x < cand) { cand = x; best = c[r]; }
+      }
+      at = __reduce_min_sync(0xffffffffu, cand);
+      src = (int)(at & 31u);
+      rb = cinv(best.x, best.y);
+    }
+    at = __shfl_sync(0xffffffffu, at, src);
+    const int piv = (int)(at & 0xffffu), q = (int)(at >> 16);
+    const double2 u = make_double2(__shfl_sync(0xffffffffu, best.x, src),
+                                   __shfl_sync(0xffffffffu, best.y, src));
+    double2 ru = make_double2(__shfl_sync(0xffffffffu, rb.x, src),
+                              __shfl_sync(0xffffffffu, rb.y, src));
+    if (u.x == 0.0 && u.y == 0.0) ru = make_double2(0.0, 0.0);
+    if (slots < n && g >= slots && g % (slots / 2) == 0) {
+      // every warp of the cluster is done with the columns whose slots the
+      // next slots / 2 columns take
+      const int need = g - slots + slots / 2;
+      for (int w = lane; w < (int)C * LUP_WARPS; w += 32) {
+        const uint32_t ad = mapa_u32(smem_u32(&prog[w % LUP_WARPS]), w / LUP_WARPS);
+        unsigned long long t0 = 0;
+        for (uint32_t it = 0; ld_acquire_cluster(ad) < need; ++it) {
+          if (s_abort) break;
+          if ((it & 63) == 63) {
+            const unsigned long long t = globaltimer();
+            if (!t0) t0 = t;
+            else if (t - t0 > LUP_LIMIT_NS) { s_abort = 1; break; }
+          }
         }
-        if (lane == 0) s_piv = (bi < n) ? bi : j;   // NaN column: keep the diagonal
       }
-      __syncthreads();
-      const int piv = s_piv;
-      if (tid == 0 && piv != j) {
-        const double2 t = cj[j];
-        cj[j] = cj[piv];
-        cj[piv] = t;
-      }
-      __syncthreads();
-      const double2 u = cj[j];
-      const bool nz = (u.x != 0.0 || u.y != 0.0);
-      const double2 ru = nz ? cinv(u.x, u.y) : make_double2(0.0, 0.0);
-      for (int i = j + 1 + tid; i < n; i += T) lvec[i] = cmul(cj[i], ru);
-      if (tid == 0) {
-        rec_u0[j] = u;
-        rec_s0[j] = piv != j;
-      }
+      __syncwarp();
     }
-    cl.sync();                                  // owner's pivot and multipliers visible
-    const int piv = *cl.map_shared_rank(&s_piv, owner);
-    const double2* ol = cl.map_shared_rank(lvec, owner);
-    for (int i = j + 1 + tid; i < n; i += T) lbuf[i] = ol[i];
-    // owned columns right of j: g = rank + C lc > j
-    const int lc0 = j >= rank ? (j - rank) / C + 1 : 0;
-    if (piv != j)
-      for (int lc = lc0 + tid; lc < my_nc; lc += T) {
-        double2* cc = col + (size_t)lc * n;
-        const double2 t = cc[j];
-        cc[j] = cc[piv];
-        cc[piv] = t;
-      }
-    __syncthreads();
-    const int nr = n - j - 1, ncols = my_nc - lc0;
-    for (int e = tid; e < nr * ncols; e += T) {
-      const int i = j + 1 + e % nr;
-      double2* cc = col + (size_t)(lc0 + e / nr) * n;
-      const double2 l = lbuf[i], p = cc[j];
-      double2 a = cc[i];
-      a.x = __dsub_rn(a.x, __fma_rn(l.x, p.x, -__dmul_rn(l.y, p.y)));
-      a.y = __dsub_rn(a.y, __fma_rn(l.x, p.y, __dmul_rn(l.y, p.x)));
-      cc[i] = a;
+    double2* slot = ring + (size_t)s * n;
+#pragma unroll
+    for (int r = 0; r < RPL; ++r) {
+      const int i = lane + 32 * r;
+      if (i < n)
+        slot[i] = pos[r] >= g && i != piv ? cmul(c[r], ru) : make_double2(0.0, 0.0);
     }
-    __syncthreads();
+    if (lane == 0) { meta[s].u = u; meta[s].piv = piv; meta[s].pos = q; }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(full + s));
+    // the other CTAs, the next one first.  One CTA at a time: the release waits
+    // for its stores, so the SM's path to the cluster never fills up with
+    // stores that the other warps' shared-memory accesses would queue behind.
+    for (uint32_t t = 1; t < C; ++t) {
+      const uint32_t to = rank + t < C ? rank + t : rank + t - C;
+      const uint32_t base = mapa_u32(smem_u32(slot), to);
+#pragma unroll
+      for (int r = 0; r < RPL; ++r)            // (this lane's own values, read back)
+        if (lane + 32 * r < n) st_cluster_v2(base + (lane + 32 * r) * 16, slot[lane + 32 * r]);
+      if (lane == 0) {
+        const uint32_t mb = mapa_u32(smem_u32(meta + s), to);
+        st_cluster_v2(mb, u);
+        st_cluster_v2i(mb + 16, piv, q);
+      }
+      __syncwarp();
+      if (lane == 0) arrive_cluster(mapa_u32(smem_u32(full + s), to));
+    }
+  };
+
+  const bool keeper = rank == 0 && warp == 0;  // multiplies the pivots up, in order
+  LuDet acc;
+  // a[0] is the warp's next column (index `next`), a[1 .. left - 1] those after it
+  int done = 0, left = 0, last = -1, next = col_of(0);
+#pragma unroll
+  for (int lp = 0; lp < LP; ++lp)
+    if (col_of(lp) < n) { last = col_of(lp); ++left; }
+  auto shift = [&]() {
+#pragma unroll
+    for (int lp = 0; lp + 1 < LP; ++lp)
+#pragma unroll
+      for (int r = 0; r < RPL; ++r) a[lp][r] = a[lp + 1][r];
+    ++done;
+    --left;
+    next = left ? col_of(done) : n;
+  };
+  if (next == 0) {
+    factor(a[0], 0, 0);
+    shift();
   }
-  cl.sync();                                    // every record landed in rank 0
-  if (rank == 0 && tid == 0) {
-    double2 mant = make_double2(1.0, 0.0);
-    long long expo = 0;
-    bool zero = false;
-    for (int j = 0; j < n; ++j) {
-      const double2 uu = rec_u[j];
-      if (rec_s[j]) { mant.x = -mant.x; mant.y = -mant.y; }
-      if (uu.x == 0.0 && uu.y == 0.0) zero = true;
-      mant = cmul(mant, uu);
-      const double mx = fmax(fabs(mant.x), fabs(mant.y));
-      if (mx != 0.0 && isfinite(mx)) {
-        const int e = ilogb(mx);
-        mant.x = scalbn(mant.x, -e);
-        mant.y = scalbn(mant.y, -e);
-        expo += e;
+  const int until = keeper ? n : last;         // columns this warp has to take in
+  int j = 0, s = 0;                            // column j is in slot s
+  uint32_t parity = 0;
+  for (; j < until; ++j) {
+    const bool ok = lup_wait(smem_u32(full + s), parity, &s_abort);
+    if (!__all_sync(0xffffffffu, ok)) break;
+    const LupMeta mt = meta[s];
+#pragma unroll
+    for (int r = 0; r < RPL; ++r) {            // the exchange of positions j and mt.pos
+      const bool here = lane + 32 * r == mt.piv;
+      pos[r] = here ? j : pos[r] == j ? mt.pos : pos[r];
+    }
+    const double2* slot = ring + (size_t)s * n;
+    if (next == j + 1) {                       // the chain: this column is wanted next
+      const double2 u = lup_row<RPL>(a[0], mt.piv);
+#pragma unroll
+      for (int r = 0; r < RPL; ++r)
+        if (lane + 32 * r < n) a[0][r] = lu_update(a[0][r], slot[lane + 32 * r], u);
+      factor(a[0], next, s + 1 < slots ? s + 1 : 0);
+      shift();
+    }
+    if (left) {
+      double2 u[LP];
+#pragma unroll
+      for (int lp = 0; lp < LP; ++lp)
+        if (lp < left) u[lp] = lup_row<RPL>(a[lp], mt.piv);
+#pragma unroll
+      for (int r = 0; r < RPL; ++r) {
+        if (lane + 32 * r >= n) continue;
+        const double2 l = slot[lane + 32 * r];
+#pragma unroll
+        for (int lp = 0; lp < LP; ++lp)
+          if (lp < left) a[lp][r] = lu_update(a[lp][r], l, u[lp]);
       }
     }
-    double2 d;
-    double la;
-    if (zero) {
-      d = make_double2(0.0, 0.0);
-      la = -INFINITY;
-    } else {
-      long long e = expo;
-      if (e > 4000) e = 4000;
-      if (e < -4000) e = -4000;
-      d = make_double2(scalbn(mant.x, (int)e), scalbn(mant.y, (int)e));
-      la = log(hypot(mant.x, mant.y)) + (double)expo * 0.69314718055994530942;
+    if (keeper) acc.times(mt.u, mt.pos != j);
+    if (slots < n) {
+      __syncwarp();
+      if (lane == 0 && (j & 3) == 3) st_release_cluster(smem_u32(&prog[warp]), j + 1);
     }
-    det_out[mat] = d;
-    if (logabs_out) logabs_out[mat] = la;
+    if (++s == slots) { s = 0; parity ^= 1u; }
   }
+  __syncwarp();
+  if (lane == 0) {
+    st_release_cluster(smem_u32(&prog[warp]), n);
+    if (j < until || s_abort) {                // a wait ran out
+      const uint32_t f = mapa_u32(smem_u32(&s_failed), 0);
+      asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(f), "r"(1) : "memory");
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();                          // nobody leaves while others write here
+  if (keeper && lane == 0) {
+    if (s_failed) acc.mant = make_double2(NAN, NAN);
+    acc.store(det, logabs);
+  }
+}
+
+template <int RPL, int LP>
+__global__ void __launch_bounds__(LUP_THREADS)
+lu_pipe_kernel(int n, int slots, int C, const double2* __restrict__ Aall,
+               double2* __restrict__ det_out, double* __restrict__ logabs_out) {
+  extern __shared__ __align__(16) unsigned char lsm[];
+  const int m = blockIdx.x / C;
+  lup_body<RPL, LP>(n, slots, Aall + (size_t)m * n * n, det_out + m,
+                        logabs_out ? logabs_out + m : nullptr, lsm);
+}
+
+// one (model, omega) pair per cluster; the ring holds `smem` bytes
+template <int RPL, int LP>
+__global__ void __launch_bounds__(LUP_THREADS)
+multi_lu_pipe_kernel(const kls_mdesc* __restrict__ md, const int2* __restrict__ pairs, int C,
+                     int max_slots) {
+  extern __shared__ __align__(16) unsigned char lsm[];
+  const int2 pz = pairs[blockIdx.x / C];
+  const kls_mdesc& d = md[pz.x];
+  lup_body<RPL, LP>(d.Na, d.Na < max_slots ? d.Na : max_slots, d.A + (size_t)pz.y * d.Na * d.Na,
+                        d.det + pz.y, d.logabs + pz.y, lsm);
+}
+
+// The size classes: rows per lane x columns per warp, CTAs per cluster.  The
+// classes with 8 CTAs take 16 where the batch fits one wave of them (N = 201:
+// 271 us against 331; 16 matrices 805 against 656).
+struct LupClass {
+  int n_max, C;
+  const void *one, *multi;
+};
+const LupClass lup_classes[] = {
+    {64, 1, (const void*)lu_pipe_kernel<2, 8>, (const void*)multi_lu_pipe_kernel<2, 8>},
+    {128, 4, (const void*)lu_pipe_kernel<4, 4>, (const void*)multi_lu_pipe_kernel<4, 4>},
+    {192, 8, (const void*)lu_pipe_kernel<6, 3>, (const void*)multi_lu_pipe_kernel<6, 3>},
+    {224, 8, (const void*)lu_pipe_kernel<7, 4>, (const void*)multi_lu_pipe_kernel<7, 4>},
+    {256, 8, (const void*)lu_pipe_kernel<8, 4>, (const void*)multi_lu_pipe_kernel<8, 4>},
+    {320, 16, (const void*)lu_pipe_kernel<10, 3>, (const void*)multi_lu_pipe_kernel<10, 3>},
+    {512, 16, (const void*)lu_pipe_kernel<16, 4>, (const void*)multi_lu_pipe_kernel<16, 4>},
+};
+constexpr int LUP_CLASSES = (int)(sizeof(lup_classes) / sizeof(lup_classes[0]));
+
+// Ring slots: one per column where 200 KB hold them (N <= 112: no slot is
+// written twice), else an even number of them, at least 16.
+int lup_slots(int n) {
+  const int s = (int)(204800 / (n * sizeof(double2) + 32));
+  return n <= s ? n : std::max(16, s & ~1);
+}
+
+cudaLaunchConfig_t lup_config(int C, int matrices, size_t smem, cudaStream_t st,
+                              cudaLaunchAttribute* at) {
+  cudaLaunchConfig_t cfg = {};
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = C;
+  at->val.clusterDim.y = 1;
+  at->val.clusterDim.z = 1;
+  cfg.gridDim = dim3(C * matrices);
+  cfg.blockDim = dim3(LUP_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+// shared-memory and cluster-size limits of a kernel (properties shared by every
+// context in the process: always the largest value of the class)
+cudaError_t lup_limits(const void* fn, int C) {
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024);
+  if (e == cudaSuccess && C >= 8)
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  return e;
 }
 
 }  // namespace
 
-// Cluster size for an n x n factorisation (0: does not fit): the smallest of
-// 8 (portable) and 16 whose column slab fits the shared memory of one CTA and
-// of which the device can co-schedule a cluster.
-static int lu_cluster_size(int device, int n) {
-  int max_smem = 0;
-  cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-  for (int C : {8, 16}) {
-    const size_t bytes = luc_smem_bytes(n, C);
-    if (bytes + 2048 > (size_t)max_smem) continue;
-    if (cudaFuncSetAttribute(lu_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)bytes) != cudaSuccess)
-      return 0;
-    if (C > 8 && cudaFuncSetAttribute(lu_cluster_kernel,
-                                      cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-                     cudaSuccess) {
-      cudaGetLastError();
-      continue;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = C;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(C);
-    cfg.blockDim = dim3(LUC_THREADS);
-    cfg.dynamicSmemBytes = bytes;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, lu_cluster_kernel, &cfg) == cudaSuccess &&
-        clusters > 0)
-      return C;
-    cudaGetLastError();
-  }
-  return 0;
+// can the device hold a cluster of C CTAs of fn?
+static bool lup_fits(const void* fn, int C, int n) {
+  cudaLaunchAttribute at;
+  cudaLaunchConfig_t cfg = lup_config(C, 1, lup_smem(n, lup_slots(n)), nullptr, &at);
+  int clusters = 0;
+  const bool ok = lup_limits(fn, C) == cudaSuccess &&
+                  cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess &&
+                  clusters > 0;
+  if (!ok) cudaGetLastError();
+  return ok;
 }
 
-static int run_lu_cluster(kls_ctx* c, int n, int C) {
-  const size_t bytes = luc_smem_bytes(c->Na, C);
-  // the limit is a property of the kernel shared by all contexts: set it for
-  // this context's N right before its launch (another context may have set
-  // a smaller one)
-  KLS_CK(c, cudaFuncSetAttribute(lu_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)bytes));
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = C;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3(n * C);
-  cfg.blockDim = dim3(LUC_THREADS);
-  cfg.dynamicSmemBytes = bytes;
-  cfg.stream = c->stream;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  KLS_CK(c, cudaLaunchKernelEx(&cfg, lu_cluster_kernel, c->Na, (const double2*)c->d_A, c->d_det,
-                               c->d_logabs));
-  KLS_LAUNCHED(c);
-  return KLS_OK;
+// Size class of an n x n factorisation on the current device, -1 where it does not fit
+static int lup_class(int device, int n) {
+  (void)device;
+  for (int k = 0; k < LUP_CLASSES; ++k) {
+    if (n > lup_classes[k].n_max) continue;
+    const LupClass& c = lup_classes[k];
+    return lup_fits(c.one, c.C, n) && lup_fits(c.multi, c.C, n) ? k : -1;
+  }
+  return -1;
 }
 
 int kls_run_lu(kls_ctx* c, int n) {
-  // latency form (a cluster per matrix) for the N_alpha of the benchmark
-  // sizes when the batch fits one wave; otherwise one CTA per matrix
   if (c->lu_mode != KLS_LU_CTA) {
-    if (c->lu_cluster < 0) c->lu_cluster = lu_cluster_size(c->device, c->Na);
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-    const bool want = c->lu_mode == KLS_LU_CLUSTER ||
-                      (c->Na >= 128 && (int64_t)n * c->lu_cluster <= sms);
-    if (want && c->lu_cluster > 0) return run_lu_cluster(c, n, c->lu_cluster);
+    if (c->lu_class == -2) {
+      c->lu_class = lup_class(c->device, c->Na);
+      c->lu_wide = c->lu_class >= 0 && lup_fits(lup_classes[c->lu_class].one, 16, c->Na);
+    }
+    if (c->lu_class >= 0) {
+      const LupClass& k = lup_classes[c->lu_class];
+      const int slots = lup_slots(c->Na);
+      int sms = 148;
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+      const int C = k.C == 8 && c->lu_wide && n * 16 <= sms ? 16 : k.C;
+      cudaLaunchAttribute at;
+      cudaLaunchConfig_t cfg = lup_config(C, n, lup_smem(c->Na, slots), c->stream, &at);
+      const double2* A = c->d_A;
+      void* args[] = {&c->Na, (void*)&slots, (void*)&C, &A, &c->d_det, &c->d_logabs};
+      KLS_CK(c, cudaLaunchKernelExC(&cfg, k.one, args));
+      KLS_LAUNCHED(c);
+      return KLS_OK;
+    }
     if (c->lu_mode == KLS_LU_CLUSTER)
       return kls_fail(c, KLS_ERR_UNSUPPORTED, "cluster LU does not fit this N_alpha");
   }
@@ -404,10 +637,28 @@ int kls_run_lu(kls_ctx* c, int n) {
   return KLS_OK;
 }
 
+// size class of a model's matrices for kls_multi_launch_lu (-1: one CTA each)
+int kls_lu_class(int device, int n) { return lup_class(device, n); }
+int kls_lu_classes() { return LUP_CLASSES; }
+
+// the pairs of one size class (class -1: lu_det_body, max_Na rows)
 int kls_multi_launch_lu(cudaStream_t st, const kls_mdesc* d_md, const int2* d_pairs, int n_pairs,
-                        int max_Na) {
-  size_t sm = 2 * (size_t)max_Na * sizeof(double2);
+                        int max_Na, int cls) {
   cudaError_t e;
+  if (cls >= 0) {
+    const LupClass& k = lup_classes[cls];
+    int slots = 0;
+    size_t smem = 0;
+    // one ring size for the class: as many slots as its largest matrix gets
+    slots = lup_slots(max_Na);
+    smem = lup_smem(max_Na, slots);
+    if ((e = lup_limits(k.multi, k.C)) != cudaSuccess) return (int)e;
+    cudaLaunchAttribute at;
+    cudaLaunchConfig_t cfg = lup_config(k.C, n_pairs, smem, st, &at);
+    void* args[] = {&d_md, &d_pairs, (void*)&k.C, &slots};
+    return (int)cudaLaunchKernelExC(&cfg, k.multi, args);
+  }
+  size_t sm = 2 * (size_t)max_Na * sizeof(double2);
   if (sm > 48 * 1024 &&
       (e = cudaFuncSetAttribute(multi_lu_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)sm)) != cudaSuccess)

@@ -29,6 +29,11 @@
 #include <numeric>
 #include <vector>
 
+// (model, omega) pairs whose matrices are of one size class of the LU
+struct LuGroup {
+  int cls, first, count, max_Na;
+};
+
 struct kls_multi {
   int device = 0, mode = 0, batch = 0, n_models = 0;
   std::vector<kls_ctx*> ctx;
@@ -60,6 +65,8 @@ struct kls_multi {
   int similar_ctas = 0, launches = 0;
   std::vector<int2> pairs_tab;      // FP64: (model, omega) pairs over the table
   int2* d_pairs_tab = nullptr;
+  std::vector<LuGroup> lu;
+  int2* d_pairs_lu = nullptr;       // the pairs, by size class of the LU
   int64_t max_K_pad = 0;
 
   kls_mdesc* d_md = nullptr;
@@ -228,7 +235,7 @@ int launch_batch(kls_multi* m) {
   const int np = (int)m->pairs.size();
   if (m->mode == KLS_MODE_FP64) {
     r = kls_multi_launch_f64_weights(m->stream, m->d_md, m->d_pairs, np, m->max_K_pad);
-    m->launches = 2;                       // weights, LU
+    m->launches = 1;                       // weights
     if (!r && !m->items.empty()) {
       r = kls_multi_launch_f64(m->stream, m->d_md, m->d_pairs_tab, (int)m->pairs_tab.size(),
                                m->d_items, (int)m->items.size(), m->d_counter, m->grid,
@@ -251,8 +258,11 @@ int launch_batch(kls_multi* m) {
                                  m->d_items, m->d_starts, m->grid, m->max_K_pad, m->d_err);
   }
   if (r) return mcuda(m, (cudaError_t)r, "uneven batch launch");
-  r = kls_multi_launch_lu(m->stream, m->d_md, m->d_pairs, np, m->max_Na);
-  if (r) return mcuda(m, (cudaError_t)r, "uneven batch LU launch");
+  for (const LuGroup& g : m->lu) {
+    r = kls_multi_launch_lu(m->stream, m->d_md, m->d_pairs_lu + g.first, g.count, g.max_Na, g.cls);
+    if (r) return mcuda(m, (cudaError_t)r, "uneven batch LU launch");
+    ++m->launches;
+  }
   return KLS_OK;
 }
 
@@ -556,8 +566,25 @@ int kls_multi_create(kls_ctx* const* models, int n_models, int mode, int batch, 
       (r = malloc_buf(m, &m->d_pairs_tm, m->pairs_tm.size())) ||
       (r = malloc_buf(m, &m->d_pairs_old, m->pairs_old.size())) ||
       (r = malloc_buf(m, &m->d_pairs_tab, m->pairs_tab.size())) ||
+      (r = malloc_buf(m, &m->d_pairs_lu, m->pairs.size())) ||
       (r = malloc_buf(m, &m->d_starts, n_it + 1)))
     return bail(r);
+  std::vector<int2> by_class;
+  std::vector<int> lu_class;
+  for (kls_ctx* c : m->ctx) lu_class.push_back(kls_lu_class(m->device, c->Na));
+  for (int cls = -1; cls < kls_lu_classes(); ++cls) {
+    LuGroup g{cls, (int)by_class.size(), 0, 0};
+    for (const int2& p : m->pairs)
+      if (lu_class[p.x] == cls) {
+        by_class.push_back(p);
+        g.max_Na = std::max(g.max_Na, m->ctx[p.x]->Na);
+        ++g.count;
+      }
+    if (g.count) m->lu.push_back(g);
+  }
+  if (cudaMemcpy(m->d_pairs_lu, by_class.data(), by_class.size() * sizeof(int2),
+                 cudaMemcpyHostToDevice))
+    return bail(mcuda(m, cudaGetLastError(), "cudaMemcpy (pairs)"));
   if (cudaMemcpy(m->d_md, m->md.data(), m->md.size() * sizeof(kls_mdesc), cudaMemcpyHostToDevice) ||
       cudaMemcpy(m->d_pairs, m->pairs.data(), m->pairs.size() * sizeof(int2),
                  cudaMemcpyHostToDevice) ||
@@ -682,7 +709,7 @@ int kls_multi_get_info(const kls_multi* m, kls_multi_info* out) {
   // (FP32 weights, contraction launch(es), reduction), LU
   out->launches_per_replay =
       fp64 ? m->launches
-           : 2 + (m->old ? 3 : 0) +
+           : 1 + (int32_t)m->lu.size() + (m->old ? 3 : 0) +
                  (m->tm ? 2 + (m->tm_schedule == 2 ? (int32_t)m->tmd.size() : 1) : 0);
   // the one-CTA / pair forms' schedule when the batch has such models, else
   // the TMEM-operand form's
