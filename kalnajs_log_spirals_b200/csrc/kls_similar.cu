@@ -27,10 +27,11 @@
 //   pair_kernel    : sum over (l, e) for the pairs of alphas
 //   pair_reduce    : sum over the row splits, * G * N(a), I - M
 //
-// Work per omega: 24 n_l Ne NR N_alpha flops in F and 28 FMA per pair and (l, e)
+// Work per omega: 12 n_l Ne NR N_alpha flops in F and 28 FMA per pair and (l, e)
 // row over N_alpha^2 / 4 pairs, against 2 N_alpha^2 n_l Ne NR for the table: at
-// NR = 501, Ne = 51, N_alpha = 301, l = +-100 3.7e10 and 6.5e9 against 9.3e11.
+// NR = 501, Ne = 51, N_alpha = 301, l = +-100 1.9e10 and 1.3e10 against 9.3e11.
 #include "kls_internal.cuh"
+#include "kls_tcgen05.cuh"
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -38,11 +39,13 @@
 struct kls_similar {
   int R = 0;                  // rows (l, e): il * Ne + ie
   int Nap = 0;                // N_alpha padded to the pair tiles
-  int NRp = 0;                // NR padded to the slabs of fourier_kernel
+  int K2p = 0;                // mirrored pairs of radii, padded to the slabs of fourier_kernel
   double* V = nullptr;        // [R][ldv] What, pairs (Re, Im) at the alphas >= 0
-  float* D = nullptr;         // [2][R][ldv] D_u, D_v
-  double* U = nullptr;        // [2][Ne][NR] u, v
-  double* Phi = nullptr;      // [NRp][2 Nap] cos, sin(d da ln Rc) / Rc
+  float2* Vf = nullptr;       // [R][ldv / 2] the same in FP32
+  float4* D = nullptr;        // [R][ldv / 2] Re D_u, Re D_v, Im D_u, Im D_v
+  double* U = nullptr;        // [3][Ne][NR] 1 / Rc, u / Rc, v / Rc
+  double* Phi = nullptr;      // [2][K2p][Nap] cos, sin(d x da dln): x from the grid's centre
+  double2* rot = nullptr;     // [Nap] cos, sin(d da ln Rc at the centre)
   int2* tiles = nullptr;      // pair tiles (I, J)
   int n_tiles = 0;
 };
@@ -197,22 +200,21 @@ __global__ void reference_kernel(int Ne, int nwa, const double* __restrict__ fit
 // |What|, first and second differences and |l What_l|: size[ie][6] (the bits of
 // a non-negative double order like the double)
 __global__ void combine_kernel(int n_l, int Ne, int ldv, int l_min, const double* __restrict__ T,
-                               double* __restrict__ V, float* __restrict__ D,
-                               unsigned long long* __restrict__ size) {
+                               double* __restrict__ V, float2* __restrict__ Vf,
+                               float4* __restrict__ D, unsigned long long* __restrict__ size) {
   const int r = blockIdx.x, il = r / Ne, ie = r % Ne;
-  const size_t R = (size_t)n_l * Ne;
   double mx[6] = {0, 0, 0, 0, 0, 0};
   const double l = fabs((double)(l_min + il));
   for (int c = threadIdx.x; c < ldv; c += blockDim.x) {
+    const size_t p = ((size_t)r * ldv + c) / 2;
     double x[5];
     for (int q = 0; q < 5; ++q) x[q] = T[((size_t)il * 5 * Ne + q * Ne + ie) * ldv + c];
     const double du = (x[1] - x[2]) * (0.5 / SIM_H), dv = (x[3] - x[4]) * (0.5 / SIM_H);
     const double d2u = (x[1] + x[2] - 2.0 * x[0]) * (1.0 / (SIM_H * SIM_H));
     const double d2v = (x[3] + x[4] - 2.0 * x[0]) * (1.0 / (SIM_H * SIM_H));
-    const size_t o = (size_t)r * ldv + c;
-    V[o] = x[0];
-    D[o] = (float)du;
-    D[R * ldv + o] = (float)dv;
+    V[(size_t)r * ldv + c] = x[0];
+    if (c & 1) { Vf[p].y = (float)x[0]; D[p].z = (float)du; D[p].w = (float)dv; }
+    else { Vf[p].x = (float)x[0]; D[p].x = (float)du; D[p].y = (float)dv; }
     const double a[6] = {fabs(x[0]), fabs(du), fabs(dv), fabs(d2u), fabs(d2v), l * fabs(x[0])};
     for (int q = 0; q < 6; ++q) mx[q] = fmax(mx[q], a[q]);
   }
@@ -224,76 +226,115 @@ __global__ void combine_kernel(int n_l, int Ne, int ldv, int l_min, const double
   }
 }
 
-// Phi[iR][2 d], [2 d + 1] = cos, sin(d da ln Rc) / Rc; zero beyond NR and N_alpha.
-// d * (da ln Rc) is split into its rounded value and the rounding, which the
-// first-order term restores.
-__global__ void phase_kernel(int NR, int NRp, int Na, int Nap, double da,
-                             const double* __restrict__ rc, double* __restrict__ Phi) {
-  const int d = blockIdx.x * blockDim.x + threadIdx.x, iR = blockIdx.y;
-  if (d >= Nap || iR >= NRp) return;
-  double s = 0.0, c = 0.0;
-  if (d < Na && iR < NR) {
-    const double th = da * log(rc[iR]), t = d * th, e = fma((double)d, th, -t);
+// The radii are uniform in ln Rc: ln Rc = mid + x h with x = 0, 1, .. (odd NR) or
+// 1/2, 3/2, .. and their negatives.  Phi[0][k][d] = cos(d x_k h da), Phi[1] = sin;
+// zero beyond the pairs and N_alpha.  d (x h da) is split into its rounded value
+// and the rounding, which the first-order term restores.
+__global__ void phase_kernel(int NR, int K2p, int Na, int Nap, double da,
+                             const double* __restrict__ rc, double* __restrict__ Phi,
+                             double2* __restrict__ rot) {
+  const int d = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
+  if (d >= Nap || k >= K2p) return;
+  const double la = log(rc[0]), lb = log(rc[NR - 1]);
+  auto phase = [&](double th, double* s, double* c) {
+    const double t = d * th, e = fma((double)d, th, -t);
     double s0, c0;
     sincos(t, &s0, &c0);
-    c = fma(-e, s0, c0) / rc[iR];
-    s = fma(e, c0, s0) / rc[iR];
+    *c = fma(-e, s0, c0);
+    *s = fma(e, c0, s0);
+  };
+  double s = 0.0, c = 0.0;
+  if (d < Na && k < (NR + 1) / 2)
+    phase(((NR & 1) ? (double)k : k + 0.5) * ((lb - la) / (double)(NR - 1)) * da, &s, &c);
+  Phi[(size_t)k * Nap + d] = c;
+  Phi[((size_t)K2p + k) * Nap + d] = s;
+  if (k == 0) {
+    phase(0.5 * (la + lb) * da, &s, &c);
+    rot[d] = make_double2(c, s);
   }
-  *reinterpret_cast<double2*>(Phi + ((size_t)iR * Nap + d) * 2) = make_double2(c, s);
+}
+
+// channel factors 1 / Rc, u / Rc, v / Rc of every orbit
+__global__ void channel_kernel(int NR, int NPh, const double* __restrict__ rc,
+                               const double* __restrict__ uv, double* __restrict__ U) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= NPh) return;
+  const double r = 1.0 / rc[p % NR];
+  U[p] = r;
+  U[NPh + p] = r * uv[p];
+  U[2 * (size_t)NPh + p] = r * uv[NPh + p];
 }
 
 // ---- F ---------------------------------------------------------------------------
-// F[r][d] = (A, B) = sum_R w(r, R) (cos, sin): 16 rows x 32 d per CTA, a warp 8
-// rows x 16 d (4 column blocks) x 3 channels x (re, im) = 24 DMMA blocks; the
-// channel weights are formed on the A fragment.  Bound: the DMMA pipe.
-constexpr int FA_R = 16, FA_D = 32, FA_K = 16, FA_STAGES = 3, FA_THREADS = 128;
-constexpr int FA_WS = 20;                 // row stride of w (16-byte values), 4 mod 8
-constexpr int FA_US = 20;                 // row stride of u, v (doubles), 4 mod 16
-constexpr int FA_PS = 2 * FA_D + 4;       // row stride of the phases, 4 mod 16
-constexpr int FA_W = 0, FA_U = 2 * FA_R * FA_WS, FA_P = FA_U + 2 * FA_R * FA_US,
-              FA_STAGE = FA_P + FA_K * FA_PS;   // offsets in doubles
+// With the mirrored radii mid +- x taken together, s = w+ + w-, t = w+ - w-,
+//   C = sum s cos(d x h da), S = sum t sin(d x h da),
+//   F(d) = A - i B,  (A, B) = (C, S) rotated by d da mid
+// takes half the products of a sum over the radii: K = NR / 2 for the cosines
+// with s and for the sines with t.  16 rows x 32 d per CTA, a warp 8 rows x 16 d:
+// 2 column blocks x (cos, sin) x 3 channels x (re, im) = 24 DMMA blocks on 12 A
+// fragments formed from the weights (18 FP64 operations a lane against 24 DMMA
+// of 8 FMA a lane).  152 registers, 3 CTAs per SM: a warp of 32 d halves those
+// operations but leaves 2 CTAs, 893 us against 817.  Bound: the FP64 pipe, which
+// the DMMA and the weights' operations share (23 TFLOP/s of DMMA).  Default
+// grid: 1370 -> 817 us per omega (before: a sum over all the radii).
+constexpr int FA_R = 16, FA_D = 32, FA_K = 8, FA_STAGES = 3, FA_THREADS = 128;
+constexpr int FA_S = 12;                  // row stride of w (16-byte values) and U (doubles)
+constexpr int FA_PS = FA_D + 4;           // row stride of the phases, 4 mod 16
+constexpr int FA_W = 0,                   // offsets in doubles: w+, w- [2][32][12] complex
+              FA_U = FA_W + 2 * 2 * FA_R * FA_S,        // [3][2][32][12]
+              FA_P = FA_U + 3 * 2 * FA_R * FA_S,        // [2][8][36]
+              FA_STAGE = FA_P + 2 * FA_K * FA_PS;
 constexpr size_t FA_SMEM = (size_t)FA_STAGES * FA_STAGE * sizeof(double);
 
 __global__ void __launch_bounds__(FA_THREADS, 3)
-fourier_kernel(int R, int Ne, int NR, int Nap, int64_t K_pad, const double2* __restrict__ wt,
-               const double* __restrict__ U, const double* __restrict__ Phi,
+fourier_kernel(int R, int Ne, int NR, int K2p, int Nap, int64_t K_pad,
+               const double2* __restrict__ wt, const double* __restrict__ U,
+               const double* __restrict__ Phi, const double2* __restrict__ rot,
                double4* __restrict__ F0, float4* __restrict__ Fc) {
   extern __shared__ __align__(16) double fsm[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int d0 = blockIdx.x * FA_D, r0 = blockIdx.y * FA_R, z = blockIdx.z;
   const double2* w = wt + (size_t)z * K_pad;
-  const int nk = (NR + FA_K - 1) / FA_K;
+  const int nk = K2p / FA_K, up = NR >> 1, dn = (NR - 1) >> 1;   // R of pair 0, either side
+  // a thread copies pair lk of row lr (weights and channel factors of both
+  // sides) and 16 bytes of the cosines and of the sines
+  const int lr = tid >> 3, lk = tid & 7, pk = tid >> 4, pc = tid & 15;
+  const bool row_in = r0 + lr < R;
+  const double2* wrow = w + (row_in ? (size_t)(r0 + lr) * NR : 0);
+  const double* urow = U + (row_in ? (size_t)((r0 + lr) % Ne) * NR : 0);
+  const size_t uch = (size_t)Ne * NR;
+  const double* prow = Phi + (size_t)pk * Nap + d0 + 2 * pc;
   auto load = [&](int s, int kt) {
     double* st = fsm + (size_t)s * FA_STAGE;
-    const int k0 = kt * FA_K;
+    const int k = kt * FA_K + lk;
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {                        // w: 16 rows x 16 values
-      const int e = tid + q * FA_THREADS, r = e >> 4, k = e & 15;
-      const bool in = r0 + r < R && k0 + k < NR;
-      cp16z(st + FA_W + 2 * (r * FA_WS + k),
-            w + (in ? (size_t)(r0 + r) * NR + k0 + k : 0), in ? 16 : 0);
+    for (int sd = 0; sd < 2; ++sd) {
+      const int iR = sd ? dn - k : up + k;
+      const bool k_in = iR >= 0 && iR < NR;
+      // (the centre of an odd grid is its own mirror: counted once)
+      const bool u_in = k_in && !(sd && up == dn && k == 0);
+      const int at = k_in ? iR : 0;
+      cp16z(st + FA_W + 2 * ((sd * FA_R + lr) * FA_S + lk), wrow + at, k_in && row_in ? 16 : 0);
+#pragma unroll
+      for (int ch = 0; ch < 3; ++ch)
+        cp8z(st + FA_U + ((ch * 2 + sd) * FA_R + lr) * FA_S + lk, urow + ch * uch + at,
+             u_in && row_in ? 8 : 0);
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {                        // u, v: 2 x 16 rows x 16
-      const int e = tid + q * FA_THREADS, ch = e >> 8, r = (e >> 4) & 15, k = e & 15;
-      const bool in = r0 + r < R && k0 + k < NR;
-      cp8z(st + FA_U + (ch * FA_R + r) * FA_US + k,
-           U + (in ? ((size_t)ch * Ne + (r0 + r) % Ne) * NR + k0 + k : 0), in ? 8 : 0);
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {                        // phases: 16 rows x 64
-      const int e = tid + q * FA_THREADS, k = e >> 5, c = e & 31;
-      cp16z(st + FA_P + k * FA_PS + 2 * c, Phi + ((size_t)(k0 + k) * Nap + d0 + c) * 2, 16);
-    }
+    for (int h = 0; h < 2; ++h)
+      cp16z(st + FA_P + (h * FA_K + pk) * FA_PS + 2 * pc,
+            prow + ((size_t)h * K2p + (size_t)kt * FA_K) * Nap, 16);
   };
-  double c[3][2][4][2];                                  // channel, (re, im), block, (cos, sin)
+  double c[3][2][2][2][2];                               // channel, (C, S), (re, im), block
 #pragma unroll
   for (int h = 0; h < 3; ++h)
 #pragma unroll
-    for (int x = 0; x < 2; ++x)
+    for (int p = 0; p < 2; ++p)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) c[h][x][j][0] = c[h][x][j][1] = 0.0;
-  const int wr = (warp & 1) * 8, wc = (warp >> 1) * 32;
+      for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) c[h][p][x][j][0] = c[h][p][x][j][1] = 0.0;
+  const int wr = (warp & 1) * 8 + g, wc = (warp >> 1) * 16;
 #pragma unroll
   for (int s = 0; s < FA_STAGES - 1; ++s) {
     if (s < nk) load(s, s);
@@ -309,35 +350,56 @@ fourier_kernel(int R, int Ne, int NR, int Nap, int64_t K_pad, const double2* __r
 #pragma unroll
     for (int kk = 0; kk < FA_K; kk += 4) {
       const int k = kk + t;
-      const double2 x = *reinterpret_cast<const double2*>(st + FA_W + 2 * ((wr + g) * FA_WS + k));
-      const double u = st[FA_U + (wr + g) * FA_US + k];
-      const double v = st[FA_U + (FA_R + wr + g) * FA_US + k];
-      const double a[3][2] = {{x.x, x.y}, {u * x.x, u * x.y}, {v * x.x, v * x.y}};
-      double b[4];
+      const double2 xp = *reinterpret_cast<const double2*>(st + FA_W + 2 * (wr * FA_S + k));
+      const double2 xm =
+          *reinterpret_cast<const double2*>(st + FA_W + 2 * ((FA_R + wr) * FA_S + k));
+      double bc[2], bs[2];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = st[FA_P + k * FA_PS + wc + 8 * j + g];
+      for (int j = 0; j < 2; ++j) {
+        bc[j] = st[FA_P + k * FA_PS + wc + 8 * j + g];
+        bs[j] = st[FA_P + (FA_K + k) * FA_PS + wc + 8 * j + g];
+      }
 #pragma unroll
-      for (int h = 0; h < 3; ++h)
+      for (int h = 0; h < 3; ++h) {
+        const double mp = st[FA_U + (2 * h * FA_R + wr) * FA_S + k];
+        const double mm = st[FA_U + ((2 * h + 1) * FA_R + wr) * FA_S + k];
+        const double px = mm * xm.x, py = mm * xm.y;
+        const double sx = fma(mp, xp.x, px), sy = fma(mp, xp.y, py);
+        const double tx = fma(mp, xp.x, -px), ty = fma(mp, xp.y, -py);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          dmma(c[h][0][j][0], c[h][0][j][1], a[h][0], b[j]);
-          dmma(c[h][1][j][0], c[h][1][j][1], a[h][1], b[j]);
+        for (int j = 0; j < 2; ++j) {
+          dmma(c[h][0][0][j][0], c[h][0][0][j][1], sx, bc[j]);
+          dmma(c[h][0][1][j][0], c[h][0][1][j][1], sy, bc[j]);
+          dmma(c[h][1][0][j][0], c[h][1][0][j][1], tx, bs[j]);
+          dmma(c[h][1][1][j][0], c[h][1][1][j][1], ty, bs[j]);
         }
+      }
     }
   }
   cp_wait<0>();
-  const int r = r0 + wr + g;
+  const int r = r0 + wr;
   if (r >= R) return;
-  const size_t row = ((size_t)z * R + r) * Nap + d0 + (wc >> 1);
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const size_t o = row + 4 * j + t;
-    F0[o] = make_double4(c[0][0][j][0], c[0][1][j][0], c[0][0][j][1], c[0][1][j][1]);
+  for (int j = 0; j < 2; ++j)
 #pragma unroll
-    for (int h = 1; h < 3; ++h)
-      Fc[2 * o + h - 1] = make_float4((float)c[h][0][j][0], (float)c[h][1][j][0],
-                                      (float)c[h][0][j][1], (float)c[h][1][j][1]);
-  }
+    for (int x = 0; x < 2; ++x) {
+      const int d = d0 + wc + 8 * j + 2 * t + x;
+      const double2 q = rot[d];
+      double a[3][4];                                    // A re, im, B re, im
+#pragma unroll
+      for (int h = 0; h < 3; ++h) {
+        const double cr = c[h][0][0][j][x], ci = c[h][0][1][j][x];
+        const double sr = c[h][1][0][j][x], si = c[h][1][1][j][x];
+        a[h][0] = q.x * cr - q.y * sr;
+        a[h][1] = q.x * ci - q.y * si;
+        a[h][2] = q.y * cr + q.x * sr;
+        a[h][3] = q.y * ci + q.x * si;
+      }
+      const size_t o = ((size_t)z * R + r) * Nap + d;
+      F0[o] = make_double4(a[0][0], a[0][1], a[0][2], a[0][3]);
+      Fc[2 * o] = make_float4((float)a[1][0], (float)a[2][0], (float)a[1][1], (float)a[2][1]);
+      Fc[2 * o + 1] = make_float4((float)a[1][2], (float)a[2][2], (float)a[1][3], (float)a[2][3]);
+    }
 }
 
 // ---- the sum over (l, e) -------------------------------------------------------------
@@ -350,15 +412,20 @@ fourier_kernel(int R, int Ne, int NR, int Nap, int64_t K_pad, const double2* __r
 // SIM_FIRST of the others, summed in FP32 over a split's rows and added to the
 // FP64 sums.
 //
-// A CTA takes a tile of 32 x 32 pairs and a range of rows; two halves of the
-// CTA alternate rows, a thread has 4 x 2 pairs (i = ti + 8 q, j = tj + 8 q' +
-// 16 h: the lanes of a quarter-warp read neighbouring d, and pairs with the
-// same q - q' share a d).  cp.async, 3 stages of 4 rows.  Bound: issue slots
-// and shared-memory reads about alike (12 FP64 + 32 FP32 FMA and 64 bytes a
-// pair).
-constexpr int PR_T = 32, PR_ROWS = 4, PR_STAGES = 3, PR_THREADS = 256;
-constexpr int PR_FA = 0, PR_FB = 1024, PR_C1 = 2048, PR_C2 = 3072,   // bytes in a row: 64 d
-              PR_WI = 4096, PR_WJ = 4608, PR_DI = 5120, PR_DJ = 5632, PR_ROW = 6144;
+// A CTA takes a tile of 32 x 32 pairs and a range of rows, either the FP64 sums
+// or the FP32 ones (both kinds share the SMs, each on its own pipe); its two
+// halves alternate rows, a thread has 4 x 4 pairs (i = ti + 8 q, j = tj + 8 p:
+// the lanes of a quarter-warp read neighbouring d, and pairs with the same q - p
+// share a d).  cp.async, 3 stages of 4 rows.  Bound: latency at 2 CTAs per SM (the
+// 4 x 4 sums fill the registers; 3 CTAs spill, 1.35 x the time): the FP64 CTAs
+// alone take 425 us and the FP32 ones 560, against 200 us each for their pipes
+// and for the shared-memory reads (22 and 26 bytes a pair and row).  Default
+// grid: 1542 -> 1030 us per omega (before: 4 x 2 pairs with both sums in one
+// thread, 64 bytes a pair, 2.03 waves).
+constexpr int PR_T = 32, PR_ROWS = 4, PR_STAGES = 3, PR_THREADS = 128;
+constexpr int PR_FA = 0, PR_FB = 1024,                 // bytes in a row: F of 64 d
+              PR_W = 2048,                             // 32 i, 32 j: What or D
+              PR_WF = 3072, PR_ROW = 3584;             // What in FP32
 constexpr size_t PR_SMEM = (size_t)PR_STAGES * PR_ROWS * PR_ROW;
 constexpr int PR_SLOT = PR_T * PR_T;        // pairs of a partial tile (double4 each)
 
@@ -367,99 +434,118 @@ __device__ __forceinline__ int pair_index(int Na, int i) {
   return i >= c0 ? i - c0 : np - 1 - i;
 }
 
-__global__ void __launch_bounds__(PR_THREADS, 1)
+__global__ void __launch_bounds__(PR_THREADS, 2)
 pair_kernel(int R, int Na, int Nap, int ldv, int splits, int n_tiles,
             const int2* __restrict__ tiles, const double* __restrict__ V,
-            const float* __restrict__ D, const double4* __restrict__ F0,
-            const float4* __restrict__ Fc, double4* __restrict__ part) {
+            const float2* __restrict__ Vf, const float4* __restrict__ D,
+            const double4* __restrict__ F0, const float4* __restrict__ Fc,
+            double4* __restrict__ part) {
   extern __shared__ __align__(16) unsigned char psm[];
   const int tid = threadIdx.x;
   const int2 tl = tiles[blockIdx.x];
-  const int split = blockIdx.y, z = blockIdx.z;
+  const bool fp64 = !(blockIdx.y & 1);                   // the kinds alternate over the SMs
+  const int split = blockIdx.y >> 1, z = blockIdx.z;
   const int rb = (int)((int64_t)R * split / splits), re = (int)((int64_t)R * (split + 1) / splits);
   const int nst = (re - rb + PR_ROWS - 1) / PR_ROWS;
   const int i0 = tl.x * PR_T, j0 = tl.y * PR_T, dlo = i0 - j0 - PR_T;   // d of window entry 0
-  const double4* f0 = F0 + (size_t)z * R * Nap;
-  const float4* fc = Fc + (size_t)z * R * Nap * 2;
+  // 32 bytes a (row, d) of either kind
+  const double2* f = fp64 ? reinterpret_cast<const double2*>(F0 + (size_t)z * R * Nap)
+                          : reinterpret_cast<const double2*>(Fc + (size_t)z * R * Nap * 2);
 
   auto load = [&](int s, int it) {
     unsigned char* st = psm + (size_t)s * PR_ROWS * PR_ROW;
 #pragma unroll
-    for (int q = 0; q < PR_ROWS; ++q) {                  // 256 values of 16 bytes: F of 64 d
-      const int r = rb + it * PR_ROWS + q, w = tid >> 2, x = tid & 3, d = dlo + w;
+    for (int q = 0; q < PR_ROWS; ++q) {                  // F of 64 d, its two halves apart
+      const int r = rb + it * PR_ROWS + q, w = tid >> 1, x = tid & 1, d = dlo + w;
       const bool in = r < re && d >= 0;
-      const size_t o = in ? (size_t)r * Nap + d : 0;
-      unsigned char* row = st + q * PR_ROW + w * 16;
-      if (x < 2) cp16z(row + (x ? PR_FB : PR_FA), reinterpret_cast<const double2*>(f0 + o) + x,
-                       in ? 16 : 0);
-      else cp16z(row + (x == 2 ? PR_C1 : PR_C2), fc + 2 * o + (x - 2), in ? 16 : 0);
+      cp16z(st + q * PR_ROW + (x ? PR_FB : PR_FA) + w * 16,
+            f + (in ? 2 * ((size_t)r * Nap + d) + x : 0), in ? 16 : 0);
     }
-    {                                                    // What: 4 rows x (32 i + 32 j)
-      const int q = tid >> 6, a = tid & 63, r = rb + it * PR_ROWS + q;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {                        // 4 rows x (32 i + 32 j)
+      const int row = 2 * q + (tid >> 6), a = tid & 63, r = rb + it * PR_ROWS + row;
       const int al = a < 32 ? i0 + a : j0 + a - 32;
       const bool in = r < re && al < Na;
-      const size_t o = in ? (size_t)r * ldv + 2 * pair_index(Na, al) : 0;
-      unsigned char* row = st + q * PR_ROW;
-      cp16z(row + (a < 32 ? PR_WI + a * 16 : PR_WJ + (a - 32) * 16), V + o, in ? 16 : 0);
-      unsigned char* dd = row + (a < 32 ? PR_DI + a * 16 : PR_DJ + (a - 32) * 16);
-      cp8z(dd, D + o, in ? 8 : 0);
-      cp8z(dd + 8, D + (in ? (size_t)R * ldv + o : 0), in ? 8 : 0);
+      const size_t o = in ? (size_t)r * (ldv >> 1) + pair_index(Na, al) : 0;
+      unsigned char* dst = st + row * PR_ROW + PR_W + a * 16;
+      if (fp64) {
+        cp16z(dst, V + 2 * o, in ? 16 : 0);
+      } else {
+        cp16z(dst, D + o, in ? 16 : 0);
+        cp8z(st + row * PR_ROW + PR_WF + a * 8, Vf + o, in ? 8 : 0);
+      }
     }
   };
 
-  const int ti = tid & 7, tj = (tid >> 3) & 7, h = (tid >> 6) & 1, half = tid >> 7;
+  const int ti = tid & 7, tj = (tid >> 3) & 7, half = tid >> 6;
   const int c0 = Na - ((Na + 1) >> 1);
-  double2 X[4][2], Y[4][2];
-  float2 x32[4][2], y32[4][2];
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      X[q][p] = Y[q][p] = make_double2(0.0, 0.0);
-      x32[q][p] = y32[q][p] = make_float2(0.f, 0.f);
-    }
   bool neg[4];                                           // alpha_i < 0: conj
 #pragma unroll
   for (int q = 0; q < 4; ++q) neg[q] = i0 + ti + 8 * q < c0;
+  double4* sh = reinterpret_cast<double4*>(psm);
+  double4* out = part + (((size_t)z * n_tiles + blockIdx.x) * 2 * splits + blockIdx.y) * PR_SLOT;
 
+  // rows it of the pipeline: body(row) for this half's rows
+  auto rows = [&](auto body) {
 #pragma unroll
-  for (int s = 0; s < PR_STAGES - 1; ++s) {
-    if (s < nst) load(s, s);
-    cp_commit();
-  }
-  for (int it = 0; it < nst; ++it) {
-    cp_wait<PR_STAGES - 2>();
+    for (int s = 0; s < PR_STAGES - 1; ++s) {
+      if (s < nst) load(s, s);
+      cp_commit();
+    }
+    for (int it = 0; it < nst; ++it) {
+      cp_wait<PR_STAGES - 2>();
+      __syncthreads();
+      const int nxt = it + PR_STAGES - 1;
+      if (nxt < nst) load(nxt % PR_STAGES, nxt);
+      cp_commit();
+#pragma unroll
+      for (int rr = 0; rr < PR_ROWS; rr += 2)
+        body(psm + ((size_t)(it % PR_STAGES) * PR_ROWS + rr + half) * PR_ROW);
+    }
+    cp_wait<0>();
     __syncthreads();
-    const int nxt = it + PR_STAGES - 1;
-    if (nxt < nst) load(nxt % PR_STAGES, nxt);
-    cp_commit();
+  };
+  // the other half's sums, then the partial: [j][i], the lanes' i contiguous
+  auto finish = [&](auto value) {
 #pragma unroll
-    for (int rr = 0; rr < PR_ROWS; rr += 2) {
-      const unsigned char* row =
-          psm + ((size_t)(it % PR_STAGES) * PR_ROWS + rr + half) * PR_ROW;
-      double2 wi[4], wj[2];
-      float4 di[4], dj[2];
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int p = 0; p < 4; ++p)
+        if (half) sh[(tj + 8 * p) * PR_T + ti + 8 * q] = value(q, p);
+    __syncthreads();
+    if (half) return;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        const int e = (tj + 8 * p) * PR_T + ti + 8 * q;
+        const double4 o = sh[e], v = value(q, p);
+        out[e] = make_double4(v.x + o.x, v.y + o.y, v.z + o.z, v.w + o.w);
+      }
+  };
+
+  if (fp64) {
+    double2 X[4][4], Y[4][4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int p = 0; p < 4; ++p) X[q][p] = Y[q][p] = make_double2(0.0, 0.0);
+    rows([&](const unsigned char* row) {
+      double2 wi[4], wj[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        wi[q] = *reinterpret_cast<const double2*>(row + PR_WI + (ti + 8 * q) * 16);
-        di[q] = *reinterpret_cast<const float4*>(row + PR_DI + (ti + 8 * q) * 16);
-        if (neg[q]) { wi[q].y = -wi[q].y; di[q].y = -di[q].y; di[q].w = -di[q].w; }
-      }
-      // alpha_j <= 0 in every pair that counts, so conj(What_j) is the stored pair
-#pragma unroll
-      for (int p = 0; p < 2; ++p) {
-        wj[p] = *reinterpret_cast<const double2*>(row + PR_WJ + (tj + 8 * p + 16 * h) * 16);
-        dj[p] = *reinterpret_cast<const float4*>(row + PR_DJ + (tj + 8 * p + 16 * h) * 16);
+        wi[q] = *reinterpret_cast<const double2*>(row + PR_W + (ti + 8 * q) * 16);
+        if (neg[q]) wi[q].y = -wi[q].y;
+        // alpha_j <= 0 in every pair that counts, so conj(What_j) is the stored pair
+        wj[q] = *reinterpret_cast<const double2*>(row + PR_W + (32 + tj + 8 * q) * 16);
       }
 #pragma unroll
-      for (int dd = -1; dd < 4; ++dd) {
-        const unsigned char* f = row + (ti - tj - 16 * h + 8 * dd + PR_T) * 16;
-        const double2 A = *reinterpret_cast<const double2*>(f + PR_FA);
-        const double2 B = *reinterpret_cast<const double2*>(f + PR_FB);
-        const float4 u = *reinterpret_cast<const float4*>(f + PR_C1);
-        const float4 v = *reinterpret_cast<const float4*>(f + PR_C2);
+      for (int dd = -3; dd < 4; ++dd) {
+        const unsigned char* fd = row + (ti - tj + 8 * dd + PR_T) * 16;
+        const double2 A = *reinterpret_cast<const double2*>(fd + PR_FA);
+        const double2 B = *reinterpret_cast<const double2*>(fd + PR_FB);
 #pragma unroll
-        for (int p = 0; p < 2; ++p) {
+        for (int p = 0; p < 4; ++p) {
           const int q = dd + p;
           if (q < 0 || q > 3) continue;
           const double pr = wi[q].x * wj[p].x - wi[q].y * wj[p].y;
@@ -468,45 +554,71 @@ pair_kernel(int R, int Na, int Nap, int ldv, int splits, int n_tiles,
           X[q][p].y = fma(B.y, pi, fma(A.y, pr, X[q][p].y));
           Y[q][p].x = fma(-B.x, pr, fma(A.x, pi, Y[q][p].x));
           Y[q][p].y = fma(-B.y, pr, fma(A.y, pi, Y[q][p].y));
-          const float ar = (float)wi[q].x, ai = (float)wi[q].y;
-          const float br = (float)wj[p].x, bi = (float)wj[p].y;
-          const float ur = di[q].x * br - di[q].y * bi + (ar * dj[p].x - ai * dj[p].y);
-          const float ui = di[q].x * bi + di[q].y * br + (ar * dj[p].y + ai * dj[p].x);
-          const float vr = di[q].z * br - di[q].w * bi + (ar * dj[p].z - ai * dj[p].w);
-          const float vi = di[q].z * bi + di[q].w * br + (ar * dj[p].w + ai * dj[p].z);
-          float2 &x = x32[q][p], &y = y32[q][p];
-          x.x += u.x * ur + u.z * ui + v.x * vr + v.z * vi;
-          x.y += u.y * ur + u.w * ui + v.y * vr + v.w * vi;
-          y.x += u.x * ui - u.z * ur + v.x * vi - v.z * vr;
-          y.y += u.y * ui - u.w * ur + v.y * vi - v.w * vr;
         }
       }
-    }
+    });
+    finish([&](int q, int p) { return make_double4(X[q][p].x, X[q][p].y, Y[q][p].x, Y[q][p].y); });
+    return;
   }
-  cp_wait<0>();
-  __syncthreads();
-  // rows of the other half, then the partial: [j][i], the lanes' i contiguous
-  double4* sh = reinterpret_cast<double4*>(psm);
-  double4* out = part + (((size_t)z * n_tiles + blockIdx.x) * splits + split) * PR_SLOT;
+  // both channels in one packed FP32 operation: (u, v) in the two halves
+  using kls_tc::f2_fma;
+  using kls_tc::f2_mul;
+  using kls_tc::f2_pack;
+  uint64_t X[4][4][2], Y[4][4][2];                       // (re, im) x (u, v)
 #pragma unroll
   for (int q = 0; q < 4; ++q)
 #pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      X[q][p].x += x32[q][p].x; X[q][p].y += x32[q][p].y;
-      Y[q][p].x += y32[q][p].x; Y[q][p].y += y32[q][p].y;
-      const int e = (tj + 8 * p + 16 * h) * PR_T + ti + 8 * q;
-      if (half) sh[e] = make_double4(X[q][p].x, X[q][p].y, Y[q][p].x, Y[q][p].y);
-    }
-  __syncthreads();
-  if (half) return;
+    for (int p = 0; p < 4; ++p) X[q][p][0] = X[q][p][1] = Y[q][p][0] = Y[q][p][1] = 0ull;
+  const uint64_t minus = 0x8000000080000000ull;
+  rows([&](const unsigned char* row) {
+    uint64_t wr[4], wi[4], ni[4], dr[4], di[4];          // i: What, -Im What, D
+    uint64_t vr[4], vi[4], nv[4], er[4], ei[4];          // j
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      const int e = (tj + 8 * p + 16 * h) * PR_T + ti + 8 * q;
-      const double4 o = sh[e];
-      out[e] = make_double4(X[q][p].x + o.x, X[q][p].y + o.y, Y[q][p].x + o.z, Y[q][p].y + o.w);
+    for (int q = 0; q < 4; ++q) {
+      const float2 w = *reinterpret_cast<const float2*>(row + PR_WF + (ti + 8 * q) * 8);
+      const ulonglong2 d = *reinterpret_cast<const ulonglong2*>(row + PR_W + (ti + 8 * q) * 16);
+      const float im = neg[q] ? -w.y : w.y;
+      wr[q] = f2_pack(w.x, w.x);
+      wi[q] = f2_pack(im, im);
+      ni[q] = wi[q] ^ minus;
+      dr[q] = d.x;
+      di[q] = neg[q] ? d.y ^ minus : d.y;
+      const float2 v = *reinterpret_cast<const float2*>(row + PR_WF + (32 + tj + 8 * q) * 8);
+      const ulonglong2 e = *reinterpret_cast<const ulonglong2*>(row + PR_W + (32 + tj + 8 * q) * 16);
+      vr[q] = f2_pack(v.x, v.x);
+      vi[q] = f2_pack(v.y, v.y);
+      nv[q] = vi[q] ^ minus;
+      er[q] = e.x;
+      ei[q] = e.y;
     }
+#pragma unroll
+    for (int dd = -3; dd < 4; ++dd) {
+      const unsigned char* fd = row + (ti - tj + 8 * dd + PR_T) * 16;
+      const ulonglong2 A = *reinterpret_cast<const ulonglong2*>(fd + PR_FA);
+      const ulonglong2 B = *reinterpret_cast<const ulonglong2*>(fd + PR_FB);
+      const uint64_t nx = B.x ^ minus, ny = B.y ^ minus;
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        const int q = dd + p;
+        if (q < 0 || q > 3) continue;
+        // Q = D_i conj(What_j) + What_i conj(D_j)
+        const uint64_t qr = f2_fma(dr[q], vr[p], f2_fma(di[q], nv[p],
+                                   f2_fma(wr[q], er[p], f2_mul(ni[q], ei[p]))));
+        const uint64_t qi = f2_fma(dr[q], vi[p], f2_fma(di[q], vr[p],
+                                   f2_fma(wr[q], ei[p], f2_mul(wi[q], er[p]))));
+        X[q][p][0] = f2_fma(A.x, qr, f2_fma(B.x, qi, X[q][p][0]));
+        X[q][p][1] = f2_fma(A.y, qr, f2_fma(B.y, qi, X[q][p][1]));
+        Y[q][p][0] = f2_fma(A.x, qi, f2_fma(nx, qr, Y[q][p][0]));
+        Y[q][p][1] = f2_fma(A.y, qi, f2_fma(ny, qr, Y[q][p][1]));
+      }
+    }
+  });
+  auto sum = [](uint64_t v) {
+    return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32));
+  };
+  finish([&](int q, int p) {
+    return make_double4(sum(X[q][p][0]), sum(X[q][p][1]), sum(Y[q][p][0]), sum(Y[q][p][1]));
+  });
 }
 
 // 64 pairs of a tile per CTA, 4 threads per pair over every 4th split, added in
@@ -613,7 +725,7 @@ size_t f_bytes(const kls_similar* s) { return (size_t)s->R * s->Nap * 64; }
 void kls_similar_free(kls_ctx* c) {
   kls_similar* s = c->sim;
   if (!s) return;
-  void* ptrs[] = {s->V, s->D, s->U, s->Phi, s->tiles};
+  void* ptrs[] = {s->V, s->Vf, s->D, s->U, s->Phi, s->rot, s->tiles};
   for (void* p : ptrs) cudaFree(p);
   delete s;
   c->sim = nullptr;
@@ -624,7 +736,7 @@ void kls_similar_free(kls_ctx* c) {
 int kls_similar_prepare(kls_ctx* c) {
   const int NR = c->NR, Ne = c->Ne, nwa = c->nwa, NPh = c->NPh;
   // fewer radii: the table's work is below this form's (2 N^2 NR against
-  // 24 N NR + 28 N^2 per row)
+  // 12 N NR + 14 N^2 per row)
   if (NR < 16 || nwa < 8) return KLS_OK;
   Scratch sc;
   double *d_probe, *d_fit, *d_rfit, *d_ref, *d_of5, *d_T;
@@ -705,7 +817,7 @@ int kls_similar_prepare(kls_ctx* c) {
   c->sim = s;
   s->R = c->n_l * Ne;
   s->Nap = (c->Na + PR_T - 1) / PR_T * PR_T;
-  s->NRp = (NR + FA_K - 1) / FA_K * FA_K;
+  s->K2p = ((NR + 1) / 2 + FA_K - 1) / FA_K * FA_K;
   const size_t fitn = (size_t)Ne * nwa, tab = (size_t)s->R * c->ldv;
   std::vector<int2> tiles;
   for (int J = 0; 2 * J * PR_T <= c->Na - 1; ++J)
@@ -722,12 +834,14 @@ int kls_similar_prepare(kls_ctx* c) {
   } while (0)
   if (!s->V) {
     SIM_CK(cudaMalloc(&s->V, tab * sizeof(double)));
+    SIM_CK(cudaMalloc(&s->Vf, tab * sizeof(float)));
     SIM_CK(cudaMalloc(&s->D, 2 * tab * sizeof(float)));
-    SIM_CK(cudaMalloc(&s->U, (size_t)2 * NPh * sizeof(double)));
-    SIM_CK(cudaMalloc(&s->Phi, (size_t)s->NRp * s->Nap * 2 * sizeof(double)));
+    SIM_CK(cudaMalloc(&s->U, (size_t)3 * NPh * sizeof(double)));
+    SIM_CK(cudaMalloc(&s->Phi, (size_t)2 * s->K2p * s->Nap * sizeof(double)));
+    SIM_CK(cudaMalloc(&s->rot, (size_t)s->Nap * sizeof(double2)));
     SIM_CK(cudaMalloc(&s->tiles, tiles.size() * sizeof(int2)));
   }
-  d_U = s->U;
+  SIM_CK(sc.get(&d_U, (size_t)2 * NPh));
   SIM_CK(sc.get(&d_fit, 7 * fitn));
   SIM_CK(sc.get(&d_rfit, rfit.size()));
   SIM_CK(sc.get(&d_iv, iv.size()));
@@ -760,12 +874,13 @@ int kls_similar_prepare(kls_ctx* c) {
   c->launches += 3;
   int r = kls_run_wl(c, (int)n5, c->cfg.l_min, c->n_l, d_of5, d_ok, rw, rr, rp, d_T);
   if (r) return bail(r);
-  combine_kernel<<<s->R, 128, 0, c->stream>>>(c->n_l, Ne, c->ldv, c->cfg.l_min, d_T, s->V, s->D,
-                                                d_mx);
+  combine_kernel<<<s->R, 128, 0, c->stream>>>(c->n_l, Ne, c->ldv, c->cfg.l_min, d_T, s->V, s->Vf,
+                                                s->D, d_mx);
   const double da = c->Na > 1 ? (2.0 * c->cfg.alpha_max) / (double)(c->Na - 1) : 0.0;
-  phase_kernel<<<dim3((s->Nap + 127) / 128, s->NRp), 128, 0, c->stream>>>(
-      NR, s->NRp, c->Na, s->Nap, da, c->d_rc, s->Phi);
-  c->launches += 2;
+  phase_kernel<<<dim3((s->Nap + 127) / 128, s->K2p), 128, 0, c->stream>>>(
+      NR, s->K2p, c->Na, s->Nap, da, c->d_rc, s->Phi, s->rot);
+  channel_kernel<<<(NPh + 127) / 128, 128, 0, c->stream>>>(NR, NPh, c->d_rc, d_U, s->U);
+  c->launches += 3;
   SIM_CK(cudaGetLastError());
   std::vector<double> mx((size_t)6 * Ne);
   std::vector<double2> mis(NPh);
@@ -802,14 +917,22 @@ int kls_similar_prepare(kls_ctx* c) {
 #undef SIM_CK
 }
 
-// Row splits of the pair sum: about two CTAs per SM for one omega, at least 8
-// rows each; fixed per context.
+// Row splits of the pair sum, fixed per context; an FP64 and an FP32 CTA per
+// tile and split, two of them on an SM at a time.  One wave while that leaves a
+// split fewer than 64 rows, else up to 6 waves (a last wave that is partly empty
+// costs less of them).
 int kls_similar_max_splits(const kls_ctx* c) { return std::max(1, c->sim->R / 8); }
 int kls_similar_splits(const kls_ctx* c) {
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-  const int want = (2 * sms + c->sim->n_tiles - 1) / c->sim->n_tiles;
-  return std::max(1, std::min(want, kls_similar_max_splits(c)));
+  const int per = 2 * c->sim->n_tiles;            // CTAs of one split
+  int s = 1;
+  for (int waves = 1; waves <= 6; ++waves) {
+    const int k = std::max(1, 2 * sms * waves / per);
+    if (waves > 1 && c->sim->R < 64 * k) break;
+    s = k;
+  }
+  return std::max(1, std::min(s, kls_similar_max_splits(c)));
 }
 
 // omegas whose F is held at once (256 MB, at least one), and its size
@@ -820,9 +943,9 @@ size_t kls_similar_f_bytes(const kls_ctx* c, int n) {
   return f_bytes(c->sim) * kls_similar_chunk(c, n);
 }
 size_t kls_similar_part_elems(const kls_ctx* c, int n) {   // double2
-  return (size_t)n * c->sim->n_tiles * c->splits * PR_SLOT * 2;
+  return (size_t)n * c->sim->n_tiles * 2 * c->splits * PR_SLOT * 2;
 }
-int kls_similar_ctas(const kls_ctx* c) { return c->sim->n_tiles * c->splits; }
+int kls_similar_ctas(const kls_ctx* c) { return 2 * c->sim->n_tiles * c->splits; }
 
 // F, pair sums and I - M of n omegas from their weights; no allocation, no
 // synchronisation (capturable)
@@ -839,18 +962,19 @@ cudaError_t kls_similar_launch(const kls_ctx* c, cudaStream_t st, int n, const d
   double4* F0 = reinterpret_cast<double4*>(F);
   float4* Fc = reinterpret_cast<float4*>(F0 + (size_t)nf * s->R * s->Nap);
   double4* p4 = reinterpret_cast<double4*>(part);
-  const size_t slots = (size_t)s->n_tiles * c->splits * PR_SLOT;
+  const size_t slots = (size_t)s->n_tiles * 2 * c->splits * PR_SLOT;
   for (int b = 0; b < n; b += nf) {
     const int m = std::min(nf, n - b);
     fourier_kernel<<<dim3(s->Nap / FA_D, (s->R + FA_R - 1) / FA_R, m), FA_THREADS, FA_SMEM, st>>>(
-        s->R, c->Ne, c->NR, s->Nap, c->K_pad, wt + (size_t)b * c->K_pad, s->U, s->Phi, F0, Fc);
-    pair_kernel<<<dim3(s->n_tiles, c->splits, m), PR_THREADS, PR_SMEM, st>>>(
-        s->R, c->Na, s->Nap, c->ldv, c->splits, s->n_tiles, s->tiles, s->V, s->D, F0, Fc,
+        s->R, c->Ne, c->NR, s->K2p, s->Nap, c->K_pad, wt + (size_t)b * c->K_pad, s->U, s->Phi,
+        s->rot, F0, Fc);
+    pair_kernel<<<dim3(s->n_tiles, 2 * c->splits, m), PR_THREADS, PR_SMEM, st>>>(
+        s->R, c->Na, s->Nap, c->ldv, c->splits, s->n_tiles, s->tiles, s->V, s->Vf, s->D, F0, Fc,
         p4 + b * slots);
     *launches += 2;
   }
   pair_reduce_kernel<<<dim3(s->n_tiles, PR_SLOT / 64, n), 256, 0, st>>>(
-      c->Na, c->splits, s->n_tiles, c->cfg.G, c->d_N, s->tiles, p4, A, M);
+      c->Na, 2 * c->splits, s->n_tiles, c->cfg.G, c->d_N, s->tiles, p4, A, M);
   *launches += 1;
   return cudaGetLastError();
 }
