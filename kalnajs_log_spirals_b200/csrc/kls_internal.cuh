@@ -103,6 +103,7 @@ struct kls_ctx {
   // omega-independent device data
   double* d_cosw = nullptr;   // [nw]
   double* d_sinw = nullptr;   // [nw]
+  double2* d_cs = nullptr;    // both in the orbit kernel's order
   double* d_of = nullptr;     // [OF_COUNT][NPh]
   double* d_SRC = nullptr;    // [NR]
   double* d_rc = nullptr;     // [NR] guiding-centre radii (host C-library pow)
@@ -201,6 +202,7 @@ __host__ __device__ inline double kls_lin(double a, double b, int n, int i) {
 }
 
 // ---- stage entry points (host side, launch on ctx->stream) ---------------
+size_t kls_orbit_table(int nw, int nwai);   // entries of d_cs
 int kls_run_orbits(kls_ctx* c);
 int kls_upload_alpha(kls_ctx* c);
 int kls_run_basis(kls_ctx* c);

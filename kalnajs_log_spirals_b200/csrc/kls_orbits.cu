@@ -7,9 +7,9 @@
 // src/KalnajsLogSpiral/Models.jl:40-169 of the reference.  One CTA per
 // orbit; the reference's sequential cumsum over nw points
 // (OrbitIntegration.jl:277-294) becomes a chunked block-wide prefix scan:
-// each thread sums a contiguous chunk, the chunk sums are scanned, and a
-// second pass re-evaluates the chunk to emit the running sums at the
-// subsample points 1:nwai:nw.
+// each thread sums a contiguous chunk and leaves the chunk's running sums at its
+// subsample points 1:nwai:nw; the chunk sums are scanned, and each thread adds
+// its offset to the samples that it left.
 //
 // This translation unit is compiled without FMA contraction (-fmad=false)
 // and keeps the reference's association order: v_r^2 = 2(E - ln x) x^2 - L^2
@@ -21,7 +21,7 @@
 
 namespace {
 
-constexpr int ORB_THREADS = 512;
+constexpr int ORB_THREADS = 256;
 
 struct OrbitParams {
   int NR, Ne, nw, nwa, nwai, Ia_last;
@@ -87,57 +87,84 @@ __device__ double df0(const OrbitParams& P, double E, double L) {
   return isfinite(r) ? r : 0.0;
 }
 
-// Radial-integrand pieces at point i of the w grid: x, svr (time) and
-// svr_phi (phase) before endpoint extrapolation.
-struct PointVals { double x, svr, svp; };
+// Radial-integrand pieces at a point of the w grid, before the endpoints'
+// extrapolation: x, sin w / v_r for the time, sin w / (v_r x) and the same over x
+// for the phase.  `unit`: a power of two near 1 / Rc.
+struct PointVals { double x, svr, svp, svpx; };
 
 __device__ __forceinline__ PointVals point_vals(double rs, double drs, double E, double L2,
-                                                bool nonradial, double cw, double sw) {
+                                                bool nonradial, double unit, double cw,
+                                                double sw) {
   PointVals v;
   v.x = rs - drs * cw;
+  // v_r^2 cancels and keeps the reference's association order; what is made of it
+  // does not: one reciprocal square root stands for its root and three divisions
   if (nonradial) {
-    // (2 (E - V(x))) * x^2 - L^2, the reference's association order
-    double vr2 = 2.0 * (E - log(v.x)) * (v.x * v.x) - L2;
-    double rvr = sqrt(fmax(0.0, vr2));
-    v.svr = sw * v.x / rvr;
-    v.svp = sw / rvr;
+    // (2 (E - V(x))) * x^2 - L^2
+    const double vr2 = 2.0 * (E - log(v.x)) * (v.x * v.x) - L2, t = v.x * unit;
+    const double q = sw * rsqrt(fmax(0.0, vr2) * (t * t));     // over x unit
+    v.svpx = q * unit;
+    v.svp = q * t;
+    v.svr = v.svp * v.x;
   } else {
     double vr2 = 2.0 * (E - log(v.x));
-    double vr = sqrt(fmax(0.0, vr2));
-    v.svr = sw / vr;
-    v.svp = 0.0;
+    v.svr = sw * rsqrt(fmax(0.0, vr2));
+    v.svp = v.svpx = 0.0;
   }
   return v;
 }
 
-template <typename T>
-__device__ T block_exclusive_scan(T val, T* sh, T* total) {
-  // sh: blockDim.x entries
-  int t = threadIdx.x;
-  sh[t] = val;
-  __syncthreads();
-  for (int off = 1; off < blockDim.x; off <<= 1) {
-    T add = (t >= off) ? sh[t - off] : T(0);
-    __syncthreads();
-    sh[t] += add;
-    __syncthreads();
+// exclusive prefix sums of (a, b) over the block's threads, and the totals: sums
+// in each warp, then every thread adds the warps before its own
+__device__ void block_scan2(double& a, double& b, double2* sh, double2& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double x = a, y = b;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const double u = __shfl_up_sync(~0u, x, off), v = __shfl_up_sync(~0u, y, off);
+    if (lane >= off) { x += u; y += v; }
   }
-  T incl = sh[t];
-  if (total) *total = sh[blockDim.x - 1];
+  if (lane == 31) sh[warp] = make_double2(x, y);
+  x = __shfl_up_sync(~0u, x, 1);
+  y = __shfl_up_sync(~0u, y, 1);
+  if (lane == 0) x = y = 0.0;
   __syncthreads();
-  return incl - val;  // exclusive
+  double px = 0.0, py = 0.0;
+  total = make_double2(0.0, 0.0);
+  for (int w = 0; w < ORB_THREADS / 32; ++w) {
+    if (w == warp) { px = total.x; py = total.y; }
+    total.x += sh[w].x;
+    total.y += sh[w].y;
+  }
+  a = px + x;
+  b = py + y;
+}
+
+// cos and sin of the w grid in the order the orbit kernel reads them: step s of
+// thread t's chunk at [s][t]
+__global__ void order_kernel(int nw, int chunk, const double* __restrict__ cosw,
+                             const double* __restrict__ sinw, double2* __restrict__ cs) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= (int64_t)(chunk + 1) * ORB_THREADS) return;
+  const int64_t i = (e % ORB_THREADS) * chunk + e / ORB_THREADS;
+  cs[e] = i < nw ? make_double2(cosw[i], sinw[i]) : make_double2(0.0, 0.0);
 }
 
 // table read, guarded in the bounds-checked build (plain t[i] otherwise)
 #define ORB_TAB(t, i) KLS_LD(KLS_IB((i), P.nw, KS_ORBIT_TABLE), t[i], 0.0)
 
-__global__ void __launch_bounds__(ORB_THREADS)
-orbit_kernel(OrbitParams P, const double* __restrict__ cosw, const double* __restrict__ sinw,
+// Bound: instruction issue (a logarithm and a reciprocal square root per point,
+// about 190 instructions, 73 of them FP64).  80 registers and 24 warps per SM: 512
+// threads at 64 registers take 16.7 ms, 256 at 64 16.4.  Default grid (25551 orbits
+// of 100001 points): 59 -> 14.9 ms; before, every point was evaluated twice, with a
+// root and three divisions, from tables that the lanes of a warp read a chunk apart.
+__global__ void __launch_bounds__(ORB_THREADS, 3)
+orbit_kernel(OrbitParams P, int chunk, const double* __restrict__ cosw, const double* __restrict__ sinw,
+             const double2* __restrict__ cs,
              const double* __restrict__ rc_tab, const double* __restrict__ SRC,
              double* __restrict__ of, int NPh, int* __restrict__ valid,
              double* __restrict__ w1o, double* __restrict__ rao, double* __restrict__ phao) {
-  __shared__ double sh_t[ORB_THREADS];
-  __shared__ double sh_p[ORB_THREADS];
+  __shared__ double2 sh_scan[ORB_THREADS / 32];
   __shared__ double sh_misc[4];
   const int p = blockIdx.x;
   const int iR = p % P.NR, ie = p / P.NR;
@@ -197,67 +224,65 @@ orbit_kernel(OrbitParams P, const double* __restrict__ cosw, const double* __res
     const bool phase_int = (fabs(1.0 - ecc) > 1e-10) && nonradial;
     const double dtc = drs * P.dw;
     // svr / svr_phi with the reference's endpoint extrapolation
-    auto vals_at = [&](int i, double& x, double& svr, double& svp) {
-      PointVals a = point_vals(rs, drs, E, L2, nonradial, ORB_TAB(cosw, i), ORB_TAB(sinw, i));
-      x = a.x; svr = a.svr; svp = a.svp;
+    // (NaN and infinity as from sin w / v_r: a product with an infinite q has x > 0)
+    const double unit = exp2(-rint(log2(Rc)));
+    auto vals_at = [&](int i, double cw, double sw, double& x, double& dt1, double& dt3) {
+      PointVals a = point_vals(rs, drs, E, L2, nonradial, unit, cw, sw);
+      x = a.x;
       if (i == 0 || i == nw - 1) {
         int i1 = (i == 0) ? 1 : nw - 2, i2 = (i == 0) ? 2 : nw - 3;
-        PointVals b = point_vals(rs, drs, E, L2, nonradial, ORB_TAB(cosw, i1), ORB_TAB(sinw, i1));
-        PointVals c = point_vals(rs, drs, E, L2, nonradial, ORB_TAB(cosw, i2), ORB_TAB(sinw, i2));
-        if (i == nw - 1 || nonradial) svr = 2.0 * b.svr - c.svr;
-        svp = 2.0 * b.svp - c.svp;
+        PointVals b = point_vals(rs, drs, E, L2, nonradial, unit, ORB_TAB(cosw, i1),
+                                 ORB_TAB(sinw, i1));
+        PointVals c = point_vals(rs, drs, E, L2, nonradial, unit, ORB_TAB(cosw, i2),
+                                 ORB_TAB(sinw, i2));
+        if (i == nw - 1 || nonradial) a.svr = 2.0 * b.svr - c.svr;
+        a.svpx = (2.0 * b.svp - c.svp) / x;
       }
+      dt1 = dtc * a.svr;
+      dt3 = dtc * a.svpx;
     };
-    const int chunk = (nw + blockDim.x - 1) / blockDim.x;
     const int i0 = tid * chunk, i1 = min(nw, i0 + chunk);
-    // pass 1: chunk sums of dt2 and dt4
+    // the chunk's running sums of dt2 and dt4, left at its subsample points
     double st = 0.0, sp = 0.0;
+    const int j0 = (i0 + nwai - 1) / nwai;
+    auto mine = [&](int j) { return j < nwa && j * nwai < i1; };
     if (i0 < i1) {
-      double x, svr, svp;
+      double x, dt1, dt3;
       double prev_t = 0.0, prev_p = 0.0;
-      if (i0 > 0) {
-        vals_at(i0 - 1, x, svr, svp);
-        prev_t = dtc * svr;
-        prev_p = dtc * svp / x;
-      }
+      if (i0 > 0) vals_at(i0 - 1, ORB_TAB(cosw, i0 - 1), ORB_TAB(sinw, i0 - 1), x, prev_t, prev_p);
+      int j = j0, next = j0 * nwai;
+      const double2* src = cs + tid;
+      double2 ahead = *src;                              // cs ends in a spare row
       for (int i = i0; i < i1; ++i) {
-        vals_at(i, x, svr, svp);
-        double dt1 = dtc * svr, dt3 = dtc * svp / x;
+        const double2 q = ahead;
+        src += ORB_THREADS;
+        ahead = *src;
+        vals_at(i, q.x, q.y, x, dt1, dt3);
         if (i > 0) { st += (prev_t + dt1) / 2; sp += (prev_p + dt3) / 2; }
         prev_t = dt1; prev_p = dt3;
-      }
-    }
-    double tot_t, tot_p;
-    double pre_t = block_exclusive_scan(st, sh_t, &tot_t);
-    double pre_p = block_exclusive_scan(sp, sh_p, &tot_p);
-    Om1 = KLS_PI / tot_t;
-    // pass 2: running sums at subsample points
-    if (i0 < i1) {
-      double x, svr, svp;
-      double prev_t = 0.0, prev_p = 0.0;
-      double rt = pre_t, rp = pre_p;
-      if (i0 > 0) {
-        vals_at(i0 - 1, x, svr, svp);
-        prev_t = dtc * svr;
-        prev_p = dtc * svp / x;
-      }
-      for (int i = i0; i < i1; ++i) {
-        vals_at(i, x, svr, svp);
-        double dt1 = dtc * svr, dt3 = dtc * svp / x;
-        if (i > 0) { rt += (prev_t + dt1) / 2; rp += (prev_p + dt3) / 2; }
-        prev_t = dt1; prev_p = dt3;
-        if (i % nwai == 0 && i <= P.Ia_last) {
-          int j = i / nwai;
-          double ph;
-          if (phase_int) ph = L * rp;
-          else ph = (j == 0) ? 0.0 : (KLS_PI / 2) * 1.0 * sg;
-          double wv = rt * Om1;
-          KLS_UNLESS(KLS_IB((int64_t)p * nwa + j, (int64_t)NPh * nwa, KS_ORBIT_SAMPLES), continue)
-          w1p[j] = wv; rap[j] = x; php[j] = ph;
-          fin = fin && isfinite(wv) && isfinite(x) && isfinite(ph);
-          if (i == P.Ia_last) sh_misc[0] = ph;
+        if (i == next && j < nwa) {
+          KLS_IF(KLS_IB((int64_t)p * nwa + j, (int64_t)NPh * nwa, KS_ORBIT_SAMPLES)) {
+            w1p[j] = st; rap[j] = x; php[j] = sp;
+          }
+          fin = fin && isfinite(x);
+          ++j;
+          next += nwai;
         }
       }
+    }
+    double2 tot;
+    block_scan2(st, sp, sh_scan, tot);
+    Om1 = KLS_PI / tot.x;
+    // the thread's own samples: the chunks before it, then the units
+    for (int j = j0; mine(j); ++j) {
+      KLS_UNLESS(KLS_IB((int64_t)p * nwa + j, (int64_t)NPh * nwa, KS_ORBIT_SAMPLES), continue)
+      const double wv = (st + w1p[j]) * Om1;
+      double ph;
+      if (phase_int) ph = L * (sp + php[j]);
+      else ph = (j == 0) ? 0.0 : (KLS_PI / 2) * 1.0 * sg;
+      w1p[j] = wv; php[j] = ph;
+      fin = fin && isfinite(wv) && isfinite(ph);
+      if (j == nwa - 1) sh_misc[0] = ph;
     }
     __syncthreads();
     Om2 = Om1 * sh_misc[0] / KLS_PI;
@@ -302,6 +327,17 @@ orbit_kernel(OrbitParams P, const double* __restrict__ cosw, const double* __res
 }
 
 }  // namespace
+
+// Points of a thread's chunk: nw over the threads; up to a multiple of the
+// subsampling where that is within 1 / 8, so that a warp's lanes leave their
+// samples in the same step (default grid: 391 -> 400 points).
+static int orbit_chunk(int nw, int nwai) {
+  const int c = (nw + ORB_THREADS - 1) / ORB_THREADS, m = (c + nwai - 1) / nwai * nwai;
+  return m - c <= c / 8 ? m : c;
+}
+size_t kls_orbit_table(int nw, int nwai) {
+  return (size_t)(orbit_chunk(nw, nwai) + 1) * ORB_THREADS;
+}
 
 int kls_run_orbits(kls_ctx* c) {
   const kls_config& k = c->cfg;
@@ -348,10 +384,15 @@ int kls_run_orbits(kls_ctx* c) {
                             c->stream));
   KLS_CK(c, cudaMemcpyAsync(c->d_SRC, src.data(), c->NR * sizeof(double), cudaMemcpyHostToDevice,
                             c->stream));
+  const int chunk = orbit_chunk(c->nw, c->nwai);
+  const int64_t ncs = (int64_t)kls_orbit_table(c->nw, c->nwai);
   kls_pre_mark(c, 0);
-  orbit_kernel<<<c->NPh, ORB_THREADS, 0, c->stream>>>(P, c->d_cosw, c->d_sinw, c->d_rc, c->d_SRC,
-                                                      c->d_of, c->NPh, c->d_valid, c->d_w1,
-                                                      c->d_ra, c->d_pha);
+  order_kernel<<<(unsigned)((ncs + 255) / 256), 256, 0, c->stream>>>(
+      c->nw, chunk, c->d_cosw, c->d_sinw, c->d_cs);
+  KLS_LAUNCHED(c);
+  orbit_kernel<<<c->NPh, ORB_THREADS, 0, c->stream>>>(P, chunk, c->d_cosw, c->d_sinw, c->d_cs, c->d_rc,
+                                                      c->d_SRC, c->d_of, c->NPh, c->d_valid,
+                                                      c->d_w1, c->d_ra, c->d_pha);
   KLS_LAUNCHED(c);
   kls_pre_mark(c, 1);
   // the host vectors must outlive the asynchronous copies
