@@ -13,11 +13,15 @@
 // update writes W and W^T in BF16.  GELU is the erf form
 // 0.5 x (1 + erf(x / sqrt 2)).  The loss is the mean squared error over the
 // batch and the outputs.
+//
+// A training step is 2 L + 1 launches for L layers: the forward layers (the first
+// gathers and converts its rows of X, the last forms the loss and its gradient),
+// a launch per layer for dW, the bias gradient and dH together, and the update.
+// The steps of an epoch are queued without a wait; the losses are read at its end.
 #include "kls_internal.cuh"
 #include <cuda_bf16.h>
 #include <algorithm>
 #include <cmath>
-#include <cstring>
 #include <random>
 #include <vector>
 
@@ -27,10 +31,20 @@ namespace {
 
 constexpr int ML_IN = 5, ML_OUT = 3;
 constexpr int ML_PAD = 16;            // input / output dims padded to 16 for the MMA
-constexpr int GT_BM = 64, GT_BN = 64, GT_BK = 32, GT_THREADS = 128;
-constexpr int GT_LDS = GT_BK + 8;     // bf16 row stride in shared memory
+constexpr int GT_THREADS = 128;
+// the small and the large tile, rows = columns, with depth and stages of the
+// cp.async pipeline; the number of row tiles of a batch follows from the small one
+constexpr int GT_S = 32, GT_SK = 64, GT_L = 64, GT_LK = 32, GT_STAGES = 4;
 
-enum Epi { EPI_STORE = 0, EPI_BIAS_GELU = 1, EPI_BIAS = 2, EPI_GELU_BWD = 3 };
+// Sums of the columns [0, N) of S [rows][ld], each in the order of the rows
+struct SumArgs {
+  int rows, N, ld;
+  const float* S;
+  float* out;
+};
+constexpr int CS_ROWS = 64, CS_COLS = 32;        // a stage of a block's sums
+
+enum Epi { EPI_STORE, EPI_GELU, EPI_OUT, EPI_MSE, EPI_GELU_BWD };
 
 struct GemmArgs {
   int M, N, K;
@@ -39,8 +53,14 @@ struct GemmArgs {
   float* C; int ldc;                   // fp32 output (may be null)
   const float* bias;                   // [N]
   const float* Zin; int ldz;           // pre-activations for EPI_GELU_BWD
-  __nv_bfloat16* H; int ldh;           // bf16 output [M][N]
-  __nv_bfloat16* Ht; int ldht;         // bf16 transposed output [N][M]
+  __nv_bfloat16* H; int ldh;           // bf16 output [M][N] (may be null)
+  __nv_bfloat16* Ht; int ldht;         // bf16 transposed output [N][ldht] (may be null)
+  // the first layer: A is row idx[m] (m without idx) of X; its transpose to Xt
+  const float* X;
+  const int* idx;
+  __nv_bfloat16* Xt;
+  const float* T;                      // EPI_MSE: targets, by idx as X
+  float* lpart;                        // EPI_MSE: sum of squares per row tile
 };
 
 __device__ __forceinline__ float gelu_f(float x) {
@@ -59,122 +79,325 @@ __device__ __forceinline__ void mma_bf16(float* d, const uint32_t* a, const uint
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-template <int EPI>
-__global__ void __launch_bounds__(GT_THREADS) gemm_bf16_kernel(GemmArgs g) {
-  __shared__ __align__(16) __nv_bfloat16 sA[GT_BM * GT_LDS];
-  __shared__ __align__(16) __nv_bfloat16 sB[GT_BN * GT_LDS];
-  const int m0 = blockIdx.y * GT_BM, n0 = blockIdx.x * GT_BN;
+__device__ __forceinline__ void ldsm4(uint32_t* r, const __nv_bfloat16* p) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(a));
+}
+// 16 bytes, of which the first `n` are read and the others zero
+__device__ __forceinline__ void cp16n(void* smem, const void* gmem, int n) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(n));
+}
+// the launches of a stream overlap their start with the end of the one before;
+// nothing is read or written before that one is done
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.launch_dependents;\ngriddepcontrol.wait;\n" ::: "memory");
+}
+
+// Column sums by a block: the block copies, CS_ROWS rows a stage, and the lanes of
+// its first warp add.
+__device__ void column_sums(const SumArgs& a, int blk, float* sm) {
+  const int c0 = blk * CS_COLS, tid = threadIdx.x;
+  auto load = [&](int s, int it) {
+#pragma unroll
+    for (int q = 0; q < CS_ROWS * CS_COLS / 4 / GT_THREADS; ++q) {
+      const int e = q * GT_THREADS + tid, r = it * CS_ROWS + e / (CS_COLS / 4);
+      const int c = e % (CS_COLS / 4) * 4;
+      const bool in = r < a.rows && c0 + c < a.ld;
+      cp16n(sm + (s * CS_ROWS + e / (CS_COLS / 4)) * CS_COLS + c,
+            in ? a.S + (size_t)r * a.ld + c0 + c : a.S, in ? 16 : 0);
+    }
+  };
+  const int n = (a.rows + CS_ROWS - 1) / CS_ROWS;
+#pragma unroll
+  for (int s = 0; s < GT_STAGES - 1; ++s) {
+    if (s < n) load(s, s);
+    asm volatile("cp.async.commit_group;\n" ::);
+  }
+  float s = 0.f;
+  for (int it = 0; it < n; ++it) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(GT_STAGES - 2));
+    __syncthreads();
+    if (it + GT_STAGES - 1 < n) load((it + GT_STAGES - 1) % GT_STAGES, it + GT_STAGES - 1);
+    asm volatile("cp.async.commit_group;\n" ::);
+    if (tid < 32) {
+      const float* x = sm + it % GT_STAGES * CS_ROWS * CS_COLS + tid;
+      const int m = min(CS_ROWS, a.rows - it * CS_ROWS);
+      if (m == CS_ROWS) {
+#pragma unroll 16
+        for (int r = 0; r < CS_ROWS; ++r) s += x[r * CS_COLS];
+      } else {
+        for (int r = 0; r < m; ++r) s += x[r * CS_COLS];
+      }
+    }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::);
+  if (tid < 32 && c0 + tid < a.N) a.out[c0 + tid] = s;
+}
+
+// 4 warps on a BT x BT tile, 2 x 2; a stage holds BK of K for both operands, rows
+// 16 bytes apart modulo 128 (ldmatrix without conflicts).  Every output adds its
+// products over K in order, in steps of 16.
+// Bound: latency - at a batch of 1024 and width 256 a GEMM has 0.13 Gflop and its
+// operands are in L2, 5 to 11 us a launch.  A training step 850 -> 78 us, the
+// forward pass of 820 rows 139 -> 42 us host to host; before: 2-byte loads, one
+// stage, 64 x 64 tiles (16 blocks for dW), a thread per bias column, the batch
+// gathered on the host and a wait per step.
+template <int BT, int BK, int EPI>
+__device__ __forceinline__ void gemm_tile(const GemmArgs& g, int blk,
+                                          __nv_bfloat16 (*sm)[2][BT * (BK + 8)], float* sloss) {
+  constexpr int LDS = BK + 8, MI = BT / 32, NJ = BT / 16, CH = BK / 8;
+  constexpr int TLD = BT + 8;          // row stride of the transposed tile
+  constexpr bool FIRST = EPI == EPI_GELU;              // (may be the layer that reads X)
+  const int nx = (g.N + BT - 1) / BT;
+  const int m0 = blk / nx * BT, n0 = blk % nx * BT;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
+  const int wm = (warp >> 1) * (BT / 2), wn = (warp & 1) * (BT / 2);
   const int gid = lane >> 2, tig = lane & 3;
-  float acc[2][4][4];
+  float acc[MI][NJ][4];
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int i = 0; i < MI; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < NJ; ++j)
 #pragma unroll
       for (int t = 0; t < 4; ++t) acc[i][j][t] = 0.f;
-
-  for (int k0 = 0; k0 < g.K; k0 += GT_BK) {
-    // stage tiles (zero outside the matrices)
-    for (int e = tid; e < GT_BM * GT_BK; e += GT_THREADS) {
-      int r = e / GT_BK, kk = e % GT_BK;
-      int gm = m0 + r, gk = k0 + kk;
-      sA[r * GT_LDS + kk] = (gm < g.M && gk < g.K) ? g.A[(size_t)gm * g.lda + gk]
-                                                   : __float2bfloat16(0.f);
-      int gn = n0 + r;
-      sB[r * GT_LDS + kk] = (gn < g.N && gk < g.K) ? g.B[(size_t)gn * g.ldb + gk]
-                                                   : __float2bfloat16(0.f);
-    }
-    __syncthreads();
+  auto load = [&](int s, int it) {
 #pragma unroll
-    for (int ks = 0; ks < GT_BK; ks += 16) {
-      uint32_t af[2][4], bfr[4][2];
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const __nv_bfloat16* p = sA + (wm + i * 16 + gid) * GT_LDS + ks + tig * 2;
-        af[i][0] = *reinterpret_cast<const uint32_t*>(p);
-        af[i][1] = *reinterpret_cast<const uint32_t*>(p + 8 * GT_LDS);
-        af[i][2] = *reinterpret_cast<const uint32_t*>(p + 8);
-        af[i][3] = *reinterpret_cast<const uint32_t*>(p + 8 * GT_LDS + 8);
+    for (int q = 0; q < BT * CH / GT_THREADS; ++q) {
+      const int e = q * GT_THREADS + tid, r = e / CH, k = e % CH * 8, gk = it * BK + k;
+      const int kb = min(max(g.K - gk, 0), 8) * 2;       // rows may end inside the 16 bytes
+      if (!(FIRST && g.X)) {
+        const int n = m0 + r < g.M ? kb : 0;
+        cp16n(&sm[s][0][r * LDS + k], n ? g.A + (size_t)(m0 + r) * g.lda + gk : g.A, n);
       }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const __nv_bfloat16* p = sB + (wn + j * 8 + gid) * GT_LDS + ks + tig * 2;
-        bfr[j][0] = *reinterpret_cast<const uint32_t*>(p);
-        bfr[j][1] = *reinterpret_cast<const uint32_t*>(p + 8);
-      }
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) mma_bf16(acc[i][j], af[i], bfr[j]);
+      const int n = n0 + r < g.N ? kb : 0;
+      cp16n(&sm[s][1][r * LDS + k], n ? g.B + (size_t)(n0 + r) * g.ldb + gk : g.B, n);
     }
-    __syncthreads();
+  };
+  const int nk = (g.K + BK - 1) / BK;
+#pragma unroll
+  for (int s = 0; s < GT_STAGES - 1; ++s) {
+    if (s < nk) load(s, s);
+    asm volatile("cp.async.commit_group;\n" ::);
   }
-  // epilogue: fragment element t at row gid (+8 for t >= 2), col 2 tig + (t & 1)
+  if (FIRST && g.X && tid < BT) {               // K = ML_PAD: one stage
+    const int r = m0 + tid;
+    const float* x = g.X + (size_t)(r < g.M ? (g.idx ? g.idx[r] : r) : 0) * ML_IN;
+    __align__(16) __nv_bfloat16 v[ML_PAD];
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+    for (int c = 0; c < ML_PAD; ++c)
+      v[c] = __float2bfloat16(c < ML_IN && r < g.M ? x[c < ML_IN ? c : 0] : 0.f);
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int c = 0; c < ML_PAD; c += 8)
+      *reinterpret_cast<uint4*>(&sm[0][0][tid * LDS + c]) = *reinterpret_cast<const uint4*>(v + c);
+    if (g.Xt && n0 == 0)
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const int r = m0 + wm + i * 16 + gid + (t >= 2 ? 8 : 0);
-        const int cidx = n0 + wn + j * 8 + 2 * tig + (t & 1);
-        if (r >= g.M || cidx >= g.N) continue;
-        float v = acc[i][j][t];
-        if (EPI == EPI_BIAS_GELU || EPI == EPI_BIAS) v += g.bias[cidx];
-        if (g.C) g.C[(size_t)r * g.ldc + cidx] = v;
-        float h = v;
-        if (EPI == EPI_BIAS_GELU) h = gelu_f(v);
-        if (EPI == EPI_GELU_BWD) h = v * gelu_d(g.Zin[(size_t)r * g.ldz + cidx]);
-        if (EPI == EPI_GELU_BWD && g.C) g.C[(size_t)r * g.ldc + cidx] = h;
-        if (g.H) g.H[(size_t)r * g.ldh + cidx] = __float2bfloat16(h);
-        if (g.Ht) g.Ht[(size_t)cidx * g.ldht + r] = __float2bfloat16(h);
-      }
-}
-
-// dY = 2 (Y - T) / (B * OUT) into fp32, bf16 and bf16^T; loss partial sums
-__global__ void mse_grad_kernel(int Bn, const float* __restrict__ Y, const float* __restrict__ T,
-                                float* __restrict__ dY, __nv_bfloat16* __restrict__ dYb,
-                                __nv_bfloat16* __restrict__ dYt, int ldt, float* __restrict__ loss) {
-  float s = 0.f;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < Bn * ML_PAD; e += gridDim.x * blockDim.x) {
-    const int r = e / ML_PAD, c = e % ML_PAD;
-    float g = 0.f;
-    if (c < ML_OUT) {
-      const float d = Y[(size_t)r * ML_PAD + c] - T[(size_t)r * ML_OUT + c];
-      s += d * d;
-      g = 2.f * d / (float)(Bn * ML_OUT);
-    }
-    dY[e] = g;
-    dYb[e] = __float2bfloat16(g);
-    dYt[(size_t)c * ldt + r] = __float2bfloat16(g);
+      for (int c = 0; c < ML_PAD; ++c) g.Xt[(size_t)c * g.ldht + r] = v[c];
   }
-  for (int off = 16; off; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-  if ((threadIdx.x & 31) == 0) atomicAdd(loss, s / (float)(Bn * ML_OUT));
+  // the epilogue's operands, fetched under the products
+  const int cl = wn + 2 * tig, rl = wm + gid;            // in the tile, + 8 j and + 16 i
+  float zin[MI][NJ][4];
+  if (EPI == EPI_GELU_BWD) {
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int r = m0 + rl + 16 * i + 8 * h, c = n0 + cl + 8 * j;
+          float2 z = make_float2(0.f, 0.f);
+          if (r < g.M && c < g.N) z = *reinterpret_cast<const float2*>(g.Zin + (size_t)r * g.ldz + c);
+          zin[i][j][2 * h] = z.x;
+          zin[i][j][2 * h + 1] = z.y;
+        }
+  }
+  const int lr = lane & 7, lq = lane >> 3;
+  for (int it = 0; it < nk; ++it) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(GT_STAGES - 2));
+    __syncthreads();
+    if (it + GT_STAGES - 1 < nk) load((it + GT_STAGES - 1) % GT_STAGES, it + GT_STAGES - 1);
+    asm volatile("cp.async.commit_group;\n" ::);
+    const __nv_bfloat16 *sA = sm[it % GT_STAGES][0], *sB = sm[it % GT_STAGES][1];
+    const int kend = min(BK, g.K - it * BK);
+#pragma unroll
+    for (int ks = 0; ks < BK; ks += 16) {
+      if (ks >= kend) break;
+      uint32_t af[MI][4], bf[NJ][2];
+#pragma unroll
+      for (int i = 0; i < MI; ++i)     // rows 0-7, 8-15 of k 0-7, then of k 8-15
+        ldsm4(af[i], sA + (wm + 16 * i + lr + 8 * (lq & 1)) * LDS + ks + 8 * (lq >> 1));
+#pragma unroll
+      for (int j = 0; j < NJ; j += 2)  // columns 8 j: k 0-7, 8-15, then columns 8 (j + 1)
+        ldsm4(bf[j], sB + (wn + 8 * j + lr + 8 * (lq >> 1)) * LDS + ks + 8 * (lq & 1));
+#pragma unroll
+      for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) mma_bf16(acc[i][j], af[i], bf[j]);
+    }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::);
+  __syncthreads();
+
+  // fragment element t at row gid (+ 8 for t >= 2), column 2 tig + (t & 1)
+  __nv_bfloat16* tr = &sm[0][0][0];
+  float loss = 0.f;
+#pragma unroll
+  for (int j = 0; j < NJ; ++j)
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = m0 + rl + 16 * i + 8 * h, c = n0 + cl + 8 * j;
+        float o[2];
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const bool in = r < g.M && c + x < g.N;
+          float v = acc[i][j][2 * h + x];
+          if (EPI == EPI_STORE) {
+            if (in) g.C[(size_t)r * g.ldc + c + x] = v;
+          } else if (EPI == EPI_GELU_BWD) {
+            v = v * gelu_d(zin[i][j][2 * h + x]);
+            if (in) g.C[(size_t)r * g.ldc + c + x] = v;
+          } else {
+            v = in ? v + g.bias[c + x] : 0.f;
+            if (EPI == EPI_OUT) {
+              if (in && c + x < ML_OUT) g.C[(size_t)r * ML_OUT + c + x] = v;
+            } else if (EPI == EPI_MSE) {
+              float d = 0.f;
+              if (in && c + x < ML_OUT)
+                d = v - g.T[(size_t)(g.idx ? g.idx[r] : r) * ML_OUT + c + x];
+              loss += d * d;
+              v = 2.f * d / (float)(g.M * ML_OUT);
+              if (in) g.C[(size_t)r * g.ldc + c + x] = v;
+            } else {
+              if (in && g.C) g.C[(size_t)r * g.ldc + c + x] = v;
+              v = gelu_f(v);
+            }
+          }
+          o[x] = v;
+        }
+        if (EPI == EPI_STORE || EPI == EPI_OUT) continue;
+        const __nv_bfloat162 b = __floats2bfloat162_rn(o[0], o[1]);
+        if (g.H && r < g.M && c < g.N)
+          *reinterpret_cast<__nv_bfloat162*>(g.H + (size_t)r * g.ldh + c) = b;
+        if (g.Ht) {
+          tr[(cl + 8 * j) * TLD + rl + 16 * i + 8 * h] = b.x;
+          tr[(cl + 8 * j + 1) * TLD + rl + 16 * i + 8 * h] = b.y;
+        }
+      }
+  if (EPI == EPI_MSE) {
+#pragma unroll
+    for (int off = 16; off; off >>= 1) loss += __shfl_xor_sync(~0u, loss, off);
+    if (lane == 0) sloss[warp] = loss;
+  }
+  if (EPI == EPI_STORE || EPI == EPI_OUT) return;
+  __syncthreads();
+  if (g.Ht)                            // 16 bytes a thread, along the rows
+    for (int e = tid; e < BT * (BT / 8); e += GT_THREADS) {
+      const int c = e / (BT / 8), r = e % (BT / 8) * 8;
+      if (n0 + c < g.N)                // (rows up to the tile's end are allocated)
+        *reinterpret_cast<uint4*>(g.Ht + (size_t)(n0 + c) * g.ldht + m0 + r) =
+            *reinterpret_cast<const uint4*>(tr + c * TLD + r);
+    }
+  if (EPI == EPI_MSE && tid == 0)
+    g.lpart[m0 / BT] = (sloss[0] + sloss[1]) + (sloss[2] + sloss[3]);
 }
 
-// column sums of dZ [B][N] -> db[N] (deterministic: one thread per column)
-__global__ void colsum_kernel(int Bn, int N, int ld, const float* __restrict__ dZ,
-                              float* __restrict__ db) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= N) return;
+// Blocks [0, nb0) compute g0 with EPI; for dW (EPI_STORE) [nb0, nb1) dH in g1, and the
+// others the bias gradient
+template <int BT, int BK, int EPI>
+__global__ void __launch_bounds__(GT_THREADS)
+gemm_kernel(const __grid_constant__ GemmArgs g0, const __grid_constant__ GemmArgs g1,
+            const __grid_constant__ SumArgs cs, int nb0, int nb1) {
+  __shared__ __align__(16) __nv_bfloat16 sm[GT_STAGES][2][BT * (BK + 8)];
+  __shared__ float sloss[4];
+  static_assert(sizeof(sm) >= GT_STAGES * CS_ROWS * CS_COLS * 4, "stages of the sums");
+  after_previous();
+  if (EPI == EPI_STORE && (int)blockIdx.x >= nb1)
+    column_sums(cs, blockIdx.x - nb1, reinterpret_cast<float*>(&sm[0][0][0]));
+  else if (EPI == EPI_STORE && (int)blockIdx.x >= nb0)
+    gemm_tile<BT, BK, EPI_GELU_BWD>(g1, blockIdx.x - nb0, sm, sloss);
+  else
+    gemm_tile<BT, BK, EPI>(g0, blockIdx.x, sm, sloss);
+}
+
+// one layer's view for the update: weights at w, bias behind them
+struct LayerArgs {
+  int dout, din, dout_pad, din_pad;
+  int64_t off;                                   // into the flat parameters
+  __nv_bfloat16 *Wb, *Wt;
+};
+constexpr int ML_MAX = 16;                       // layers
+struct UpdateArgs {
+  LayerArgs l[ML_MAX];
+};
+struct LossArgs {                                // squares per row tile -> *loss
+  int tiles;
+  const float* part;
+  float scale;
+  float* loss;
+};
+
+// by one warp
+__device__ void batch_loss(const LossArgs& u) {
   float s = 0.f;
-  for (int r = 0; r < Bn; ++r) s += dZ[(size_t)r * ld + c];
-  db[c] = s;
+  for (int t = threadIdx.x & 31; t < u.tiles; t += 32) s += u.part[t];
+#pragma unroll
+  for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(~0u, s, off);
+  if (threadIdx.x == 0) *u.loss = s * u.scale;
 }
 
-__global__ void adam_kernel(int64_t n, float* __restrict__ p, const float* __restrict__ g,
-                            float* __restrict__ m, float* __restrict__ v, float lr, float b1,
-                            float b2, float eps, float c1, float c2) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const float gi = g[i];
+// the loss without an update
+__global__ void loss_kernel(LossArgs u) {
+  after_previous();
+  batch_loss(u);
+}
+
+// Adam and the new BF16 copies: blocks (32 x 32 tile of W, layer), W^T through
+// shared memory; the block behind a layer's tiles takes its bias, and in layer 0
+// the loss
+__global__ void __launch_bounds__(256)
+adam_kernel(UpdateArgs u, LossArgs ls, float* __restrict__ p, const float* __restrict__ g,
+            float* __restrict__ m, float* __restrict__ v, float lr, float b1, float b2, float eps,
+            float c1, float c2) {
+  __shared__ __nv_bfloat16 tr[32][34];
+  const LayerArgs& a = u.l[blockIdx.y];
+  const int tx = (a.din + 31) / 32, nt = tx * ((a.dout + 31) / 32), t = blockIdx.x;
+  if (t > nt) return;
+  after_previous();
+  auto step = [&](int64_t i, float gi) {
     const float mi = b1 * m[i] + (1.f - b1) * gi;
     const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
     m[i] = mi;
     v[i] = vi;
-    p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    return p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  };
+  if (t == nt) {
+    for (int c = threadIdx.x; c < a.dout; c += blockDim.x) {
+      const int64_t i = a.off + (int64_t)a.dout * a.din + c;
+      step(i, g[i]);
+    }
+    if (blockIdx.y == 0 && threadIdx.x < 32) batch_loss(ls);
+    return;
+  }
+  const int r0 = t / tx * 32, c0 = t % tx * 32, x = threadIdx.x & 31, y = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 0; q < 32; q += 8) {
+    const int r = r0 + y + q, c = c0 + x;
+    if (r < a.dout && c < a.din) {
+      const int64_t i = a.off + (int64_t)r * a.din + c;
+      const __nv_bfloat16 b = __float2bfloat16(step(i, g[i]));
+      a.Wb[(size_t)r * a.din_pad + c] = b;
+      tr[y + q][x] = b;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 32; q += 8) {
+    const int r = r0 + x, c = c0 + y + q;
+    if (r < a.dout && c < a.din) a.Wt[(size_t)c * a.dout_pad + r] = tr[x][y + q];
   }
 }
 
@@ -192,17 +415,6 @@ __global__ void pack_weights_kernel(int rows, int cols, int rows_pad, int cols_p
   }
 }
 
-// features fp32 [B][5] -> bf16 [B][16] and its transpose [16][B]
-__global__ void pack_input_kernel(int Bn, const float* __restrict__ X, __nv_bfloat16* __restrict__ Xb,
-                                  __nv_bfloat16* __restrict__ Xt, int ldt) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < Bn * ML_PAD; e += gridDim.x * blockDim.x) {
-    const int r = e / ML_PAD, c = e % ML_PAD;
-    const __nv_bfloat16 b = __float2bfloat16(c < ML_IN ? X[(size_t)r * ML_IN + c] : 0.f);
-    Xb[e] = b;
-    Xt[(size_t)c * ldt + r] = b;
-  }
-}
-
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -216,10 +428,15 @@ struct kls_mlp {
   // activations for a batch of `cap` rows
   std::vector<float*> Z;                             // pre-activations [cap][dout_pad]
   std::vector<__nv_bfloat16*> H, Ht;                 // H[l]: input of layer l [cap][din_pad]
-  float *dZ = nullptr, *dZ2 = nullptr;               // fp32 [cap][width]
-  __nv_bfloat16 *dZb = nullptr, *dZb2 = nullptr;    // bf16 [cap][width] (ping-pong)
-  __nv_bfloat16 *dZt = nullptr;                      // bf16 [width][cap]
-  float *Xd = nullptr, *Td = nullptr, *loss = nullptr;
+  __nv_bfloat16 *dZ[2] = {nullptr, nullptr};         // bf16 [cap][width], by turns
+  __nv_bfloat16 *dZt[2] = {nullptr, nullptr};        // bf16 [width][cap]
+  float* dZf[2] = {nullptr, nullptr};                // fp32 [cap][width]
+  int ltiles = 0;                                    // row tiles of the last batch
+  float* lpart = nullptr;                            // squared errors per row tile
+  int rows = 0, steps = 0;                           // capacity of the buffers below
+  float *Xd = nullptr, *Td = nullptr, *Yd = nullptr; // rows of a call
+  int* idx = nullptr;                                // [rows] shuffled order
+  float* loss = nullptr;                             // [steps] of an epoch
   int64_t step = 0;
   cudaStream_t stream = nullptr;
   std::string err;
@@ -239,39 +456,88 @@ int mfail(kls_mlp* m, const std::string& s) {
 
 int ensure_cap(kls_mlp* m, int n) {
   if (n <= m->cap) return KLS_OK;
-  int cap = ((n + 63) / 64) * 64;
-  auto fr = [](void* p) { if (p) cudaFree(p); };
-  for (auto* z : m->Z) fr(z);
-  for (auto* h : m->H) fr(h);
-  for (auto* h : m->Ht) fr(h);
-  fr(m->dZ); fr(m->dZ2); fr(m->dZb); fr(m->dZb2); fr(m->dZt); fr(m->Xd); fr(m->Td);
+  const int cap = ((n + 63) / 64) * 64;
+  m->cap = 0;
+  auto fr = [](auto*& p) {
+    if (p) cudaFree((void*)p);
+    p = nullptr;
+  };
+  for (auto*& z : m->Z) fr(z);
+  for (auto*& h : m->H) fr(h);
+  for (auto*& h : m->Ht) fr(h);
+  for (int q = 0; q < 2; ++q) { fr(m->dZ[q]); fr(m->dZt[q]); fr(m->dZf[q]); }
+  fr(m->lpart);
   const int L = m->depth;
-  m->Z.assign(L, nullptr);
-  m->H.assign(L + 1, nullptr);
-  m->Ht.assign(L + 1, nullptr);
-  for (int l = 0; l < L; ++l) ML_CK(m, cudaMalloc(&m->Z[l], (size_t)cap * m->dout_pad[l] * 4));
-  for (int l = 0; l <= L; ++l) {
-    int w = l < L ? m->din_pad[l] : ML_PAD;
-    ML_CK(m, cudaMalloc(&m->H[l], (size_t)cap * w * 2));
-    ML_CK(m, cudaMalloc(&m->Ht[l], (size_t)cap * w * 2));
+  m->Z.assign(L, nullptr);             // layers 0 .. L - 2
+  m->H.assign(L, nullptr);             // inputs of the layers 1 .. L - 1
+  m->Ht.assign(L, nullptr);            // inputs of all layers
+  for (int l = 0; l < L; ++l) {
+    if (l < L - 1) ML_CK(m, cudaMalloc(&m->Z[l], (size_t)cap * m->dout_pad[l] * 4));
+    if (l) ML_CK(m, cudaMalloc(&m->H[l], (size_t)cap * m->din_pad[l] * 2));
+    ML_CK(m, cudaMalloc(&m->Ht[l], (size_t)cap * m->din_pad[l] * 2));
   }
-  ML_CK(m, cudaMalloc(&m->dZ, (size_t)cap * m->width * 4));
-  ML_CK(m, cudaMalloc(&m->dZ2, (size_t)cap * m->width * 4));
-  ML_CK(m, cudaMalloc(&m->dZb, (size_t)cap * m->width * 2));
-  ML_CK(m, cudaMalloc(&m->dZb2, (size_t)cap * m->width * 2));
-  ML_CK(m, cudaMalloc(&m->dZt, (size_t)cap * m->width * 2));
-  ML_CK(m, cudaMalloc(&m->Xd, (size_t)cap * ML_IN * 4));
-  ML_CK(m, cudaMalloc(&m->Td, (size_t)cap * ML_OUT * 4));
+  for (int q = 0; q < 2; ++q) {
+    ML_CK(m, cudaMalloc(&m->dZ[q], (size_t)cap * m->width * 2));
+    ML_CK(m, cudaMalloc(&m->dZt[q], (size_t)cap * m->width * 2));
+    ML_CK(m, cudaMalloc(&m->dZf[q], (size_t)cap * m->width * 4));
+  }
+  ML_CK(m, cudaMalloc(&m->lpart, (size_t)(cap / GT_S) * 4));
   m->cap = cap;
   return KLS_OK;
 }
 
-template <int EPI>
-int gemm(kls_mlp* m, const GemmArgs& g) {
-  dim3 grid((g.N + GT_BN - 1) / GT_BN, (g.M + GT_BM - 1) / GT_BM);
-  gemm_bf16_kernel<EPI><<<grid, GT_THREADS, 0, m->stream>>>(g);
-  ML_CK(m, cudaGetLastError());
+// X, T, Y and the order of n rows; losses of `steps` steps
+int ensure_rows(kls_mlp* m, int n, int steps) {
+  auto fr = [](auto*& p) {
+    if (p) cudaFree((void*)p);
+    p = nullptr;
+  };
+  if (n > m->rows) {
+    m->rows = 0;
+    fr(m->Xd); fr(m->Td); fr(m->Yd); fr(m->idx);
+    ML_CK(m, cudaMalloc(&m->Xd, (size_t)n * ML_IN * 4));
+    ML_CK(m, cudaMalloc(&m->Td, (size_t)n * ML_OUT * 4));
+    ML_CK(m, cudaMalloc(&m->Yd, (size_t)n * ML_OUT * 4));
+    ML_CK(m, cudaMalloc(&m->idx, (size_t)n * 4));
+    m->rows = n;
+  }
+  if (steps > m->steps) {
+    m->steps = 0;
+    fr(m->loss);
+    ML_CK(m, cudaMalloc(&m->loss, (size_t)steps * 4));
+    m->steps = steps;
+  }
   return KLS_OK;
+}
+
+template <typename... P, typename... A>
+int launch(kls_mlp* m, void (*kernel)(P...), dim3 grid, int threads, A... args) {
+  cudaLaunchConfig_t c = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  c.gridDim = grid;
+  c.blockDim = dim3(threads);
+  c.stream = m->stream;
+  c.attrs = at;
+  c.numAttrs = 1;
+  ML_CK(m, cudaLaunchKernelEx(&c, kernel, P(args)...));
+  return KLS_OK;
+}
+
+int tiles(const GemmArgs& g, int t) { return ((g.N + t - 1) / t) * ((g.M + t - 1) / t); }
+
+// The large tile from two of its blocks per SM on: there it reads half as much of
+// the operands per product (forward of 32768 rows, width 256, depth 4, host to host:
+// 189 against 222 us); below that the small one has the more SMs at work (a
+// training step of 1024 rows: 78 against 102 us; 8192 rows are alike, 85 us).
+template <int EPI>
+int gemm(kls_mlp* m, const GemmArgs& g, const GemmArgs& h = {}, const SumArgs& s = {}) {
+  const bool large = tiles(g, GT_L) + tiles(h, GT_L) >= 296;
+  const int t = large ? GT_L : GT_S, nb0 = tiles(g, t), nb1 = nb0 + tiles(h, t);
+  if (EPI == EPI_MSE) m->ltiles = (g.M + t - 1) / t;
+  return launch(m, large ? gemm_kernel<GT_L, GT_LK, EPI> : gemm_kernel<GT_S, GT_SK, EPI>,
+                dim3(nb1 + (s.N + CS_COLS - 1) / CS_COLS), GT_THREADS, g, h, s, nb0, nb1);
 }
 
 int pack_all(kls_mlp* m) {
@@ -284,85 +550,83 @@ int pack_all(kls_mlp* m) {
   return KLS_OK;
 }
 
-// forward over n rows already in m->Xd; output Z[L-1] [n][16]
-int forward(kls_mlp* m, int n) {
-  pack_input_kernel<<<(n * ML_PAD + 255) / 256, 256, 0, m->stream>>>(n, m->Xd, m->H[0], m->Ht[0],
-                                                                     m->cap);
-  ML_CK(m, cudaGetLastError());
+// forward over n rows of X (rows idx, or in order); train: keeps Z and the
+// transposes, and ends in the gradient of the loss; else the outputs to m->Yd
+int forward(kls_mlp* m, int n, const int* idx, bool train) {
   const int L = m->depth;
   for (int l = 0; l < L; ++l) {
     GemmArgs g{};
     g.M = n; g.N = m->dout_pad[l]; g.K = m->din_pad[l];
     g.A = m->H[l]; g.lda = m->din_pad[l];
     g.B = m->Wb[l]; g.ldb = m->din_pad[l];
-    g.C = m->Z[l]; g.ldc = m->dout_pad[l];
-    g.bias = nullptr;
+    // (the last layer's bias covers 3 outputs; the padded ones read zeros behind it)
+    g.bias = m->p + m->boff[l];
+    g.ldht = m->cap;
+    g.idx = idx;
+    if (l == 0) {
+      g.X = m->Xd;
+      g.Xt = train ? m->Ht[0] : nullptr;
+    }
     int r;
     if (l < L - 1) {
-      g.bias = m->p + m->boff[l];
       g.H = m->H[l + 1]; g.ldh = m->din_pad[l + 1];
-      g.Ht = m->Ht[l + 1]; g.ldht = m->cap;
-      r = gemm<EPI_BIAS_GELU>(m, g);
+      if (train) {
+        g.C = m->Z[l]; g.ldc = m->dout_pad[l];
+        g.Ht = m->Ht[l + 1];
+      }
+      r = gemm<EPI_GELU>(m, g);
+    } else if (train) {
+      g.T = m->Td;
+      g.C = m->dZf[0]; g.ldc = m->dout_pad[l];
+      g.H = m->dZ[0]; g.ldh = m->dout_pad[l];
+      g.Ht = m->dZt[0];
+      g.lpart = m->lpart;
+      r = gemm<EPI_MSE>(m, g);
     } else {
-      // the last layer's bias covers only the 3 real outputs; padded columns
-      // of the bias vector are zero-filled by a separate padded bias copy
-      g.bias = m->p + m->boff[l];
-      r = gemm<EPI_BIAS>(m, g);
+      g.C = m->Yd;
+      r = gemm<EPI_OUT>(m, g);
     }
     if (r) return r;
   }
   return KLS_OK;
 }
 
-// backward from dZ_last (fp32 [n][16] in m->dZ2 reinterpreted, bf16 copies ready)
+// backward from the gradient that a training forward leaves in dZ[0]
 int backward(kls_mlp* m, int n) {
   const int L = m->depth;
-  float* dZcur = m->dZ2;           // fp32 dZ of layer l, [n][dout_pad[l]]
-  __nv_bfloat16* dZbcur = m->dZb;  // its bf16 copy (the GEMM below reads one, writes the other)
-  for (int l = L - 1; l >= 0; --l) {
+  for (int l = L - 1, q = 0; l >= 0; --l, q ^= 1) {
     // dW_l [dout][din] = dZ_l^T (dout x n) * H_l (n x din): A = dZt [dout_pad][cap], B = Ht_l
-    {
-      GemmArgs g{};
-      g.M = m->dout[l]; g.N = m->din[l]; g.K = n;
-      g.A = m->dZt; g.lda = m->cap;
-      g.B = m->Ht[l]; g.ldb = m->cap;
-      g.C = m->g + m->woff[l]; g.ldc = m->din[l];
-      int r = gemm<EPI_STORE>(m, g);
-      if (r) return r;
+    GemmArgs w{};
+    w.M = m->dout[l]; w.N = m->din[l]; w.K = n;
+    w.A = m->dZt[q]; w.lda = m->cap;
+    w.B = m->Ht[l]; w.ldb = m->cap;
+    w.C = m->g + m->woff[l]; w.ldc = m->din[l];
+    // dZ_{l-1} = (dZ_l W_l) * gelu'(Z_{l-1}): A = dZ [n][dout_pad], B = Wt_l [din_pad][dout_pad]
+    GemmArgs h{};
+    if (l) {
+      h.M = n; h.N = m->din_pad[l]; h.K = m->dout_pad[l];
+      h.A = m->dZ[q]; h.lda = m->dout_pad[l];
+      h.B = m->Wt[l]; h.ldb = m->dout_pad[l];
+      h.Zin = m->Z[l - 1]; h.ldz = m->dout_pad[l - 1];
+      h.C = m->dZf[q ^ 1]; h.ldc = m->din_pad[l];
+      h.H = m->dZ[q ^ 1]; h.ldh = m->din_pad[l];
+      h.Ht = m->dZt[q ^ 1]; h.ldht = m->cap;
     }
-    colsum_kernel<<<(m->dout[l] + 127) / 128, 128, 0, m->stream>>>(n, m->dout[l], m->dout_pad[l],
-                                                                   dZcur, m->g + m->boff[l]);
-    ML_CK(m, cudaGetLastError());
-    if (l == 0) break;
-    // dZ_{l-1} = (dZ_l W_l) * gelu'(Z_{l-1}): A = dZb [n][dout_pad], B = Wt_l [din_pad][dout_pad]
-    float* dZnext = (dZcur == m->dZ) ? m->dZ2 : m->dZ;
-    __nv_bfloat16* dZbnext = (dZbcur == m->dZb) ? m->dZb2 : m->dZb;
-    GemmArgs g{};
-    g.M = n; g.N = m->din_pad[l]; g.K = m->dout_pad[l];
-    g.A = dZbcur; g.lda = m->dout_pad[l];
-    g.B = m->Wt[l]; g.ldb = m->dout_pad[l];
-    g.C = dZnext; g.ldc = m->din_pad[l];
-    g.Zin = m->Z[l - 1]; g.ldz = m->dout_pad[l - 1];
-    // dZ^T is read only by the dW GEMM that already ran, so it is rewritten
-    // in place; the bf16 dZ ping-pongs because this GEMM reads the other one
-    g.H = dZbnext; g.ldh = m->din_pad[l];
-    g.Ht = m->dZt; g.ldht = m->cap;
-    int r = gemm<EPI_GELU_BWD>(m, g);
+    const SumArgs s = {n, m->dout[l], m->dout_pad[l], m->dZf[q], m->g + m->boff[l]};
+    int r = gemm<EPI_STORE>(m, w, h, s);
     if (r) return r;
-    dZcur = dZnext;
-    dZbcur = dZbnext;
   }
   return KLS_OK;
 }
 
-// loss + gradients over rows [0, n) of Xd/Td into m->g; loss into *loss_out (device)
-int grad_batch(kls_mlp* m, int n) {
-  int r;
-  if ((r = forward(m, n))) return r;
-  mse_grad_kernel<<<std::min((n * ML_PAD + 255) / 256, 1024), 256, 0, m->stream>>>(
-      n, m->Z[m->depth - 1], m->Td, m->dZ2, m->dZb, m->dZt, m->cap, m->loss);
-  ML_CK(m, cudaGetLastError());
-  return backward(m, n);
+LossArgs loss_args(const kls_mlp* m, int n, float* loss) {
+  return {m->ltiles, m->lpart, 1.f / (float)(n * ML_OUT), loss};
+}
+
+// gradients into m->g and the loss by row tiles
+int grad_batch(kls_mlp* m, int n, const int* idx) {
+  int r = forward(m, n, idx, true);
+  return r ? r : backward(m, n);
 }
 
 }  // namespace
@@ -397,8 +661,7 @@ int kls_mlp_create(int device, int width, int depth, uint64_t seed, kls_mlp** ou
   }
   if (cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMalloc(&m->p, alloc * 4) != cudaSuccess || cudaMalloc(&m->g, alloc * 4) != cudaSuccess ||
-      cudaMalloc(&m->m, alloc * 4) != cudaSuccess || cudaMalloc(&m->v, alloc * 4) != cudaSuccess ||
-      cudaMalloc(&m->loss, 4) != cudaSuccess) {
+      cudaMalloc(&m->m, alloc * 4) != cudaSuccess || cudaMalloc(&m->v, alloc * 4) != cudaSuccess) {
     delete m;
     return kls_fail(nullptr, KLS_ERR_OOM, "kls_mlp_create: device allocation failed");
   }
@@ -432,7 +695,8 @@ int kls_mlp_destroy(kls_mlp* m) {
   for (auto* z : m->Z) fr(z);
   for (auto* x : m->H) fr(x);
   for (auto* x : m->Ht) fr(x);
-  fr(m->dZ); fr(m->dZ2); fr(m->dZb); fr(m->dZb2); fr(m->dZt); fr(m->Xd); fr(m->Td);
+  for (int q = 0; q < 2; ++q) { fr(m->dZ[q]); fr(m->dZt[q]); fr(m->dZf[q]); }
+  fr(m->lpart); fr(m->Xd); fr(m->Td); fr(m->Yd); fr(m->idx);
   cudaStreamDestroy(m->stream);
   delete m;
   return KLS_OK;
@@ -466,19 +730,16 @@ int kls_mlp_forward(kls_mlp* m, const float* X, int n, float* Y) {
   if (!m || n < 0 || (n && (!X || !Y))) return KLS_ERR_CONFIG;
   cudaSetDevice(m->device);
   const int chunk = 1 << 16;
-  std::vector<float> z((size_t)std::min(n, chunk) * ML_PAD);
   for (int s = 0; s < n; s += chunk) {
     int nb = std::min(chunk, n - s);
     int r = ensure_cap(m, nb);
-    if (r) return r;
+    if (r || (r = ensure_rows(m, nb, 0))) return r;
     ML_CK(m, cudaMemcpyAsync(m->Xd, X + (size_t)s * ML_IN, (size_t)nb * ML_IN * 4,
                              cudaMemcpyHostToDevice, m->stream));
-    if ((r = forward(m, nb))) return r;
-    ML_CK(m, cudaMemcpyAsync(z.data(), m->Z[m->depth - 1], (size_t)nb * ML_PAD * 4,
+    if ((r = forward(m, nb, nullptr, false))) return r;
+    ML_CK(m, cudaMemcpyAsync(Y + (size_t)s * ML_OUT, m->Yd, (size_t)nb * ML_OUT * 4,
                              cudaMemcpyDeviceToHost, m->stream));
     ML_CK(m, cudaStreamSynchronize(m->stream));
-    for (int i = 0; i < nb; ++i)
-      for (int c = 0; c < ML_OUT; ++c) Y[(size_t)(s + i) * ML_OUT + c] = z[(size_t)i * ML_PAD + c];
   }
   return KLS_OK;
 }
@@ -488,11 +749,11 @@ int kls_mlp_grad(kls_mlp* m, const float* X, const float* T, int n, float* grads
   if (!m || n < 1 || !X || !T) return KLS_ERR_CONFIG;
   cudaSetDevice(m->device);
   int r = ensure_cap(m, n);
-  if (r) return r;
+  if (r || (r = ensure_rows(m, n, 1))) return r;
   ML_CK(m, cudaMemcpyAsync(m->Xd, X, (size_t)n * ML_IN * 4, cudaMemcpyHostToDevice, m->stream));
   ML_CK(m, cudaMemcpyAsync(m->Td, T, (size_t)n * ML_OUT * 4, cudaMemcpyHostToDevice, m->stream));
-  ML_CK(m, cudaMemsetAsync(m->loss, 0, 4, m->stream));
-  if ((r = grad_batch(m, n))) return r;
+  if ((r = grad_batch(m, n, nullptr))) return r;
+  if ((r = launch(m, loss_kernel, dim3(1), 32, loss_args(m, n, m->loss)))) return r;
   if (grads) ML_CK(m, cudaMemcpyAsync(grads, m->g, m->nparams * 4, cudaMemcpyDeviceToHost, m->stream));
   if (loss) ML_CK(m, cudaMemcpyAsync(loss, m->loss, 4, cudaMemcpyDeviceToHost, m->stream));
   ML_CK(m, cudaStreamSynchronize(m->stream));
@@ -505,39 +766,41 @@ int kls_mlp_train(kls_mlp* m, const float* X, const float* T, int n, int epochs,
   if (!m || n < 1 || batch < 1 || epochs < 0 || !X || !T) return KLS_ERR_CONFIG;
   cudaSetDevice(m->device);
   batch = std::min(batch, n);
+  const int steps = n / batch;
   int r = ensure_cap(m, batch);
-  if (r) return r;
+  if (r || (r = ensure_rows(m, n, steps))) return r;
+  int tiles_w = 1;                                       // blocks of the update, per layer
+  for (int l = 0; l < m->depth; ++l)
+    tiles_w = std::max(tiles_w, ((m->din[l] + 31) / 32) * ((m->dout[l] + 31) / 32) + 1);
+  ML_CK(m, cudaMemcpyAsync(m->Xd, X, (size_t)n * ML_IN * 4, cudaMemcpyHostToDevice, m->stream));
+  ML_CK(m, cudaMemcpyAsync(m->Td, T, (size_t)n * ML_OUT * 4, cudaMemcpyHostToDevice, m->stream));
+  UpdateArgs u{};
+  for (int l = 0; l < m->depth; ++l)
+    u.l[l] = {m->dout[l], m->din[l], m->dout_pad[l], m->din_pad[l], m->woff[l], m->Wb[l], m->Wt[l]};
   std::vector<int> idx(n);
   for (int i = 0; i < n; ++i) idx[i] = i;
   std::mt19937_64 rng(seed);
-  std::vector<float> xb((size_t)batch * ML_IN), tb((size_t)batch * ML_OUT);
+  std::vector<float> ls(steps);
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+  if (epochs > 0) std::shuffle(idx.begin(), idx.end(), rng);
   for (int ep = 0; ep < epochs; ++ep) {
-    std::shuffle(idx.begin(), idx.end(), rng);
-    double lsum = 0.0;
-    int nb_count = 0;
-    for (int s = 0; s + batch <= n; s += batch) {
-      for (int i = 0; i < batch; ++i) {
-        std::memcpy(&xb[(size_t)i * ML_IN], X + (size_t)idx[s + i] * ML_IN, ML_IN * 4);
-        std::memcpy(&tb[(size_t)i * ML_OUT], T + (size_t)idx[s + i] * ML_OUT, ML_OUT * 4);
-      }
-      ML_CK(m, cudaMemcpyAsync(m->Xd, xb.data(), xb.size() * 4, cudaMemcpyHostToDevice, m->stream));
-      ML_CK(m, cudaMemcpyAsync(m->Td, tb.data(), tb.size() * 4, cudaMemcpyHostToDevice, m->stream));
-      ML_CK(m, cudaMemsetAsync(m->loss, 0, 4, m->stream));
-      if ((r = grad_batch(m, batch))) return r;
+    ML_CK(m, cudaMemcpyAsync(m->idx, idx.data(), (size_t)n * 4, cudaMemcpyHostToDevice, m->stream));
+    for (int s = 0; s < steps; ++s) {
+      if ((r = grad_batch(m, batch, m->idx + (size_t)s * batch))) return r;
       ++m->step;
       const float c1 = 1.f - std::pow(b1, (float)m->step), c2 = 1.f - std::pow(b2, (float)m->step);
-      adam_kernel<<<256, 256, 0, m->stream>>>(m->nparams, m->p, m->g, m->m, m->v, lr, b1, b2, eps,
-                                             c1, c2);
-      ML_CK(m, cudaGetLastError());
-      if ((r = pack_all(m))) return r;
-      float l = 0.f;
-      ML_CK(m, cudaMemcpyAsync(&l, m->loss, 4, cudaMemcpyDeviceToHost, m->stream));
-      ML_CK(m, cudaStreamSynchronize(m->stream));
-      lsum += l;
-      ++nb_count;
+      if ((r = launch(m, adam_kernel, dim3(tiles_w, m->depth), 256,
+                      u, loss_args(m, batch, m->loss + s), m->p, m->g, m->m, m->v, lr, b1, b2, eps,
+                      c1, c2)))
+        return r;
     }
-    if (loss_hist) loss_hist[ep] = nb_count ? (float)(lsum / nb_count) : 0.f;
+    if (ep + 1 < epochs) std::shuffle(idx.begin(), idx.end(), rng);
+    ML_CK(m, cudaMemcpyAsync(ls.data(), m->loss, (size_t)steps * 4, cudaMemcpyDeviceToHost,
+                             m->stream));
+    ML_CK(m, cudaStreamSynchronize(m->stream));
+    double lsum = 0.0;
+    for (float l : ls) lsum += l;
+    if (loss_hist) loss_hist[ep] = steps ? (float)(lsum / steps) : 0.f;
   }
   return KLS_OK;
 }
