@@ -262,7 +262,9 @@ typedef struct kls_hybrid_cfg {
     double  far_step;
 } kls_hybrid_cfg;
 /* evals[0..2] (may be NULL): split-BF16, plain FP64 (anchors included) and
- * anchored determinant evaluations.                                        */
+ * anchored determinant evaluations.  Where the model's orbits are self-similar
+ * (kls_precompute) an FP64 determinant costs less than either of the others and
+ * is taken in their place; the counts stay those of the steps above.        */
 int kls_newton_hybrid(kls_ctx* ctx, double Omega_p0, double gamma0, const kls_newton_cfg* nc,
                       const kls_hybrid_cfg* hc, kls_newton_result* res, int32_t* evals,
                       double* history);

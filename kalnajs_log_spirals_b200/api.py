@@ -668,7 +668,9 @@ def newton_search_hybrid(config: KalnajsConfig, precomputed: PrecomputedData,
     No reference counterpart: the result satisfies |det(I - M)| <
     config.newton.tol (NewtonSolver.jl:89) on an FP64-accurate determinant
     (the anchored form, or plain FP64 with ``final_fp64``); ``det_evals``
-    counts every evaluation and ``history`` has one row per evaluation.
+    counts every evaluation and ``history`` has one row per evaluation.  On a
+    model of self-similar orbits plain FP64 determinants, the cheaper ones
+    there, take the place of the split-BF16 and anchored ones in every step.
     """
     n = config.newton
     hc = hybrid or HybridConfig()
