@@ -159,7 +159,7 @@ struct kls_ctx {
   // kernel (-2: not looked up yet, -1: it does not fit)
   int lu_mode = 0;
   int lu_class = -2;
-  bool lu_wide = false;       // 16 CTAs per matrix fit as well
+  bool lu_wide = false;       // the class's wider form fits as well
 
   // instrumentation
   int64_t launches = 0;

@@ -207,9 +207,9 @@ multi_lu_kernel(const kls_mdesc* __restrict__ md, const int2* __restrict__ pairs
 // column waits for all of them.
 // Waits are bounded (LUP_LIMIT_NS); one that runs out makes the determinant NaN.
 //
-// Measured (1 matrix, B200): N = 101 312 -> 104 us, 201 557 -> 271 us, 301 1022 ->
-// 632 us against one CTA (101) or a cluster with one barrier per column; 16
-// matrices 315 -> 105, 612 -> 656, 2760 -> 1890 us.  A column's chain is about
+// Measured (1 matrix, B200): N = 101 312 -> 100 us, 201 557 -> 264 us, 301 1022 ->
+// 575 us against one CTA (101) or a cluster with one barrier per column; 16
+// matrices 315 -> 101, 612 -> 374, 2760 -> 1148 us.  A column's chain is about
 // 1000 cycles at 4 rows a lane and 1900 at 10 (update 215 / 385, pivot search
 // 170 / 324, reciprocal 182, multipliers 48 / 111, hand-over 300).
 constexpr int LUP_WARPS = 8, LUP_THREADS = 32 * LUP_WARPS;
@@ -530,22 +530,35 @@ multi_lu_pipe_kernel(const kls_mdesc* __restrict__ md, const int2* __restrict__ 
                         d.det + pz.y, d.logabs + pz.y, lsm);
 }
 
-// The size classes: rows per lane x columns per warp, CTAs per cluster.  The
-// classes with 8 CTAs take 16 where the batch fits one wave of them (N = 201:
-// 271 us against 331; 16 matrices 805 against 656).
+// The size classes: rows per lane x columns per warp, CTAs per cluster.  4 columns
+// a warp keep enough matrices on the device at once; a wider form (2 columns) for
+// batches that it holds in one wave.  1 matrix / 16, us:
+//   N =  64  <2,2> x 4   52 /  52   (<2,8> x 1    71 /  71)
+//   N = 101  <4,3> x 6  100 / 101   (<4,4> x 4   105 / 105, <4,2> x 8 128 / 249)
+//   N = 192  <6,4> x 6  276 / 278   (<6,3> x 8   306 / 605), <6,2> x 12 233 / 686
+//   N = 201  <7,5> x 6  372 / 374   (<7,4> x 8   333 / 656), <7,2> x 14 264 / 782
+//   N = 256  <8,4> x 8  462 / 920   (<8,5> x 7   574 / 1140), <8,2> x 16 398 / 1183
+//   N = 301 <10,4> x 10 575 / 1148  (<10,3> x 16 632 / 1887)
+//   N = 400 <13,4> x 13 1513 / 4550 (<16,4> x 16 3277 / 9852)
 struct LupClass {
   int n_max, C;
   const void *one, *multi;
+  int Cw;
+  const void* wide;
 };
+#define LUP_CLASS(n, c, rpl, lp)                                                     \
+  n, c, (const void*)lu_pipe_kernel<rpl, lp>, (const void*)multi_lu_pipe_kernel<rpl, lp>
 const LupClass lup_classes[] = {
-    {64, 1, (const void*)lu_pipe_kernel<2, 8>, (const void*)multi_lu_pipe_kernel<2, 8>},
-    {128, 4, (const void*)lu_pipe_kernel<4, 4>, (const void*)multi_lu_pipe_kernel<4, 4>},
-    {192, 8, (const void*)lu_pipe_kernel<6, 3>, (const void*)multi_lu_pipe_kernel<6, 3>},
-    {224, 8, (const void*)lu_pipe_kernel<7, 4>, (const void*)multi_lu_pipe_kernel<7, 4>},
-    {256, 8, (const void*)lu_pipe_kernel<8, 4>, (const void*)multi_lu_pipe_kernel<8, 4>},
-    {320, 16, (const void*)lu_pipe_kernel<10, 3>, (const void*)multi_lu_pipe_kernel<10, 3>},
-    {512, 16, (const void*)lu_pipe_kernel<16, 4>, (const void*)multi_lu_pipe_kernel<16, 4>},
+    {LUP_CLASS(64, 4, 2, 2), 0, nullptr},
+    {LUP_CLASS(128, 6, 4, 3), 0, nullptr},
+    {LUP_CLASS(192, 6, 6, 4), 12, (const void*)lu_pipe_kernel<6, 2>},
+    {LUP_CLASS(224, 6, 7, 5), 14, (const void*)lu_pipe_kernel<7, 2>},
+    {LUP_CLASS(256, 8, 8, 4), 16, (const void*)lu_pipe_kernel<8, 2>},
+    {LUP_CLASS(320, 10, 10, 4), 0, nullptr},
+    {LUP_CLASS(416, 13, 13, 4), 0, nullptr},
+    {LUP_CLASS(512, 16, 16, 4), 0, nullptr},
 };
+#undef LUP_CLASS
 constexpr int LUP_CLASSES = (int)(sizeof(lup_classes) / sizeof(lup_classes[0]));
 
 // Ring slots: one per column where 200 KB hold them (N <= 112: no slot is
@@ -575,7 +588,7 @@ cudaLaunchConfig_t lup_config(int C, int matrices, size_t smem, cudaStream_t st,
 // context in the process: always the largest value of the class)
 cudaError_t lup_limits(const void* fn, int C) {
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024);
-  if (e == cudaSuccess && C >= 8)
+  if (e == cudaSuccess && C > 8)
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   return e;
 }
@@ -609,19 +622,21 @@ int kls_run_lu(kls_ctx* c, int n) {
   if (c->lu_mode != KLS_LU_CTA) {
     if (c->lu_class == -2) {
       c->lu_class = lup_class(c->device, c->Na);
-      c->lu_wide = c->lu_class >= 0 && lup_fits(lup_classes[c->lu_class].one, 16, c->Na);
+      const LupClass* k = c->lu_class >= 0 ? lup_classes + c->lu_class : nullptr;
+      c->lu_wide = k && k->wide && lup_fits(k->wide, k->Cw, c->Na);
     }
     if (c->lu_class >= 0) {
       const LupClass& k = lup_classes[c->lu_class];
       const int slots = lup_slots(c->Na);
       int sms = 148;
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-      const int C = k.C == 8 && c->lu_wide && n * 16 <= sms ? 16 : k.C;
+      const bool wide = c->lu_wide && (int64_t)n * k.Cw <= sms;
+      const int C = wide ? k.Cw : k.C;
       cudaLaunchAttribute at;
       cudaLaunchConfig_t cfg = lup_config(C, n, lup_smem(c->Na, slots), c->stream, &at);
       const double2* A = c->d_A;
       void* args[] = {&c->Na, (void*)&slots, (void*)&C, &A, &c->d_det, &c->d_logabs};
-      KLS_CK(c, cudaLaunchKernelExC(&cfg, k.one, args));
+      KLS_CK(c, cudaLaunchKernelExC(&cfg, wide ? k.wide : k.one, args));
       KLS_LAUNCHED(c);
       return KLS_OK;
     }

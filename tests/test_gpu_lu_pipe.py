@@ -35,3 +35,19 @@ def test_pipelined_lu_is_bitwise_the_cta_lu(lib_path, Na):
     ref = np.linalg.det(np.eye(Na) - M)
     cond = np.linalg.cond(np.eye(Na) - M)
     assert abs(out[0][0][0] - ref) <= 2 * Na ** 2 * 2.0 ** -53 * cond * abs(ref)
+
+
+@pytest.mark.parametrize("Na", [225, 240, 416, 417])
+def test_pipelined_lu_between_classes(lib_path, Na):
+    """Further edges of the classes, at batches of 16 (the class's form) and 2 (its
+    wider one where it has one): the bits of the one-CTA LU."""
+    pc = K.precompute_all(kconfig(**BASE, N_alpha=Na))
+    rng = np.random.default_rng(Na)
+    om = 2 * rng.uniform(0.3, 0.6, 18) + 1j * rng.uniform(0.02, 0.25, 18)
+    out = []
+    for mode in (_lib.KLS_LU_CTA, _lib.KLS_LU_AUTO):
+        pc.ctx.call("kls_set_lu_mode", mode)
+        out.append(K.compute_determinant_batched(om, pc, None, batch_size=16, log_abs=True))
+    pc.close()
+    assert np.array_equal(out[1][0], out[0][0])
+    assert np.array_equal(out[1][1], out[0][1])
