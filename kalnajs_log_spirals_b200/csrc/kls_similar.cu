@@ -27,9 +27,10 @@
 //   pair_kernel    : sum over (l, e) for the pairs of alphas
 //   pair_reduce    : sum over the row splits, * G * N(a), I - M
 //
-// Work per omega: 12 n_l Ne NR N_alpha flops in F and 28 FMA per pair and (l, e)
-// row over N_alpha^2 / 4 pairs, against 2 N_alpha^2 n_l Ne NR for the table: at
-// NR = 501, Ne = 51, N_alpha = 301, l = +-100 1.9e10 and 1.3e10 against 9.3e11.
+// Work per omega: 12 n_l Ne NR N_alpha flops in F and 12 FP64 and 32 FP32 FMA per
+// pair and (l, e) row over N_alpha^2 / 4 pairs, against 2 N_alpha^2 n_l Ne NR for the
+// table: at NR = 501, Ne = 51, N_alpha = 301, l = +-100 1.9e10, 5.6e9 and 1.5e10
+// against 9.3e11.
 #include "kls_internal.cuh"
 #include "kls_tcgen05.cuh"
 #include <algorithm>
@@ -46,8 +47,9 @@ struct kls_similar {
   double* U = nullptr;        // [3][Ne][NR] 1 / Rc, u / Rc, v / Rc
   double* Phi = nullptr;      // [2][K2p][Nap] cos, sin(d x da dln): x from the grid's centre
   double2* rot = nullptr;     // [Nap] cos, sin(d da ln Rc at the centre)
-  int2* tiles = nullptr;      // pair tiles (I, J)
+  int4* tiles = nullptr;      // pair tiles: I, J, weight (16: a full one), limit of q + p
   int n_tiles = 0;
+  std::vector<int> weight;    // of the tiles
 };
 
 namespace {
@@ -419,15 +421,32 @@ fourier_kernel(int R, int Ne, int NR, int K2p, int Nap, int64_t K_pad,
 // share a d).  cp.async, 3 stages of 4 rows.  Bound: latency at 2 CTAs per SM (the
 // 4 x 4 sums fill the registers; 3 CTAs spill, 1.35 x the time): the FP64 CTAs
 // alone take 425 us and the FP32 ones 560, against 200 us each for their pipes
-// and for the shared-memory reads (22 and 26 bytes a pair and row).  Default
-// grid: 1542 -> 1030 us per omega (before: 4 x 2 pairs with both sums in one
-// thread, 64 bytes a pair, 2.03 waves).
+// and for the shared-memory reads (22 and 26 bytes a pair and row).  Tiles at the
+// edges of the triangle leave out their empty 8 x 8 blocks in code of their own
+// (PairShape) and have the fewer row splits for it.  Default grid: 1542 -> 1030 us
+// per omega (before: 4 x 2 pairs with both sums in one thread, 64 bytes a pair, 2.03
+// waves) -> 930 with the edges (run-time branches around the blocks: 1000);
+// N_alpha = 101, 1071 rows, batch of 16: 22 -> 19.
 constexpr int PR_T = 32, PR_ROWS = 4, PR_STAGES = 3, PR_THREADS = 128;
 constexpr int PR_FA = 0, PR_FB = 1024,                 // bytes in a row: F of 64 d
               PR_W = 2048,                             // 32 i, 32 j: What or D
               PR_WF = 3072, PR_ROW = 3584;             // What in FP32
 constexpr size_t PR_SMEM = (size_t)PR_STAGES * PR_ROWS * PR_ROW;
 constexpr int PR_SLOT = PR_T * PR_T;        // pairs of a partial tile (double4 each)
+
+// The 8 x 8 blocks (q, p) of a tile that hold pairs with i >= j (diagonal tiles:
+// q >= p) and i + j <= N - 1 (q + p <= lim; lim is even)
+template <bool DIAG, int LIM>
+struct PairShape {
+  static constexpr bool diag = DIAG;
+  static constexpr int lim = LIM;
+};
+
+// row splits of a tile of weight w where a whole tile has k
+__host__ __device__ __forceinline__ int tile_splits(int k, int w) {
+  const int n = (k * w + 8) >> 4;
+  return n > 0 ? n : 1;
+}
 
 __device__ __forceinline__ int pair_index(int Na, int i) {
   const int np = (Na + 1) >> 1, c0 = Na - np;
@@ -436,16 +455,17 @@ __device__ __forceinline__ int pair_index(int Na, int i) {
 
 __global__ void __launch_bounds__(PR_THREADS, 2)
 pair_kernel(int R, int Na, int Nap, int ldv, int splits, int n_tiles,
-            const int2* __restrict__ tiles, const double* __restrict__ V,
+            const int4* __restrict__ tiles, const double* __restrict__ V,
             const float2* __restrict__ Vf, const float4* __restrict__ D,
             const double4* __restrict__ F0, const float4* __restrict__ Fc,
             double4* __restrict__ part) {
   extern __shared__ __align__(16) unsigned char psm[];
   const int tid = threadIdx.x;
-  const int2 tl = tiles[blockIdx.x];
+  const int4 tl = tiles[blockIdx.x];
   const bool fp64 = !(blockIdx.y & 1);                   // the kinds alternate over the SMs
-  const int split = blockIdx.y >> 1, z = blockIdx.z;
-  const int rb = (int)((int64_t)R * split / splits), re = (int)((int64_t)R * (split + 1) / splits);
+  const int split = blockIdx.y >> 1, z = blockIdx.z, ns = tile_splits(splits, tl.z);
+  if (split >= ns) return;
+  const int rb = (int)((int64_t)R * split / ns), re = (int)((int64_t)R * (split + 1) / ns);
   const int nst = (re - rb + PR_ROWS - 1) / PR_ROWS;
   const int i0 = tl.x * PR_T, j0 = tl.y * PR_T, dlo = i0 - j0 - PR_T;   // d of window entry 0
   // 32 bytes a (row, d) of either kind
@@ -505,6 +525,21 @@ pair_kernel(int R, int Na, int Nap, int ldv, int splits, int n_tiles,
     cp_wait<0>();
     __syncthreads();
   };
+  // the body for this tile's shape
+  auto by_shape = [&](auto body) {
+    auto run = [&](auto t) { rows([&](const unsigned char* row) { body(row, t); }); };
+    if (tl.x != tl.y) {
+      if (tl.w == 6) run(PairShape<false, 6>{});
+      else if (tl.w == 4) run(PairShape<false, 4>{});
+      else if (tl.w == 2) run(PairShape<false, 2>{});
+      else run(PairShape<false, 0>{});
+    } else {
+      if (tl.w == 6) run(PairShape<true, 6>{});
+      else if (tl.w == 4) run(PairShape<true, 4>{});
+      else if (tl.w == 2) run(PairShape<true, 2>{});
+      else run(PairShape<true, 0>{});
+    }
+  };
   // the other half's sums, then the partial: [j][i], the lanes' i contiguous
   auto finish = [&](auto value) {
 #pragma unroll
@@ -530,7 +565,7 @@ pair_kernel(int R, int Na, int Nap, int ldv, int splits, int n_tiles,
     for (int q = 0; q < 4; ++q)
 #pragma unroll
       for (int p = 0; p < 4; ++p) X[q][p] = Y[q][p] = make_double2(0.0, 0.0);
-    rows([&](const unsigned char* row) {
+    auto body = [&](const unsigned char* row, auto t) {
       double2 wi[4], wj[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
@@ -541,6 +576,7 @@ pair_kernel(int R, int Na, int Nap, int ldv, int splits, int n_tiles,
       }
 #pragma unroll
       for (int dd = -3; dd < 4; ++dd) {
+        if (dd < (t.diag ? 0 : -3) || dd > t.lim || -dd > t.lim) continue;
         const unsigned char* fd = row + (ti - tj + 8 * dd + PR_T) * 16;
         const double2 A = *reinterpret_cast<const double2*>(fd + PR_FA);
         const double2 B = *reinterpret_cast<const double2*>(fd + PR_FB);
@@ -548,6 +584,7 @@ pair_kernel(int R, int Na, int Nap, int ldv, int splits, int n_tiles,
         for (int p = 0; p < 4; ++p) {
           const int q = dd + p;
           if (q < 0 || q > 3) continue;
+          if (q + p > t.lim) continue;
           const double pr = wi[q].x * wj[p].x - wi[q].y * wj[p].y;
           const double pi = wi[q].x * wj[p].y + wi[q].y * wj[p].x;
           X[q][p].x = fma(B.x, pi, fma(A.x, pr, X[q][p].x));
@@ -556,7 +593,8 @@ pair_kernel(int R, int Na, int Nap, int ldv, int splits, int n_tiles,
           Y[q][p].y = fma(-B.y, pr, fma(A.y, pi, Y[q][p].y));
         }
       }
-    });
+    };
+    by_shape(body);
     finish([&](int q, int p) { return make_double4(X[q][p].x, X[q][p].y, Y[q][p].x, Y[q][p].y); });
     return;
   }
@@ -570,7 +608,7 @@ pair_kernel(int R, int Na, int Nap, int ldv, int splits, int n_tiles,
 #pragma unroll
     for (int p = 0; p < 4; ++p) X[q][p][0] = X[q][p][1] = Y[q][p][0] = Y[q][p][1] = 0ull;
   const uint64_t minus = 0x8000000080000000ull;
-  rows([&](const unsigned char* row) {
+  auto body = [&](const unsigned char* row, auto t) {
     uint64_t wr[4], wi[4], ni[4], dr[4], di[4];          // i: What, -Im What, D
     uint64_t vr[4], vi[4], nv[4], er[4], ei[4];          // j
 #pragma unroll
@@ -593,6 +631,7 @@ pair_kernel(int R, int Na, int Nap, int ldv, int splits, int n_tiles,
     }
 #pragma unroll
     for (int dd = -3; dd < 4; ++dd) {
+      if (dd < (t.diag ? 0 : -3) || dd > t.lim || -dd > t.lim) continue;
       const unsigned char* fd = row + (ti - tj + 8 * dd + PR_T) * 16;
       const ulonglong2 A = *reinterpret_cast<const ulonglong2*>(fd + PR_FA);
       const ulonglong2 B = *reinterpret_cast<const ulonglong2*>(fd + PR_FB);
@@ -601,6 +640,7 @@ pair_kernel(int R, int Na, int Nap, int ldv, int splits, int n_tiles,
       for (int p = 0; p < 4; ++p) {
         const int q = dd + p;
         if (q < 0 || q > 3) continue;
+        if (q + p > t.lim) continue;
         // Q = D_i conj(What_j) + What_i conj(D_j)
         const uint64_t qr = f2_fma(dr[q], vr[p], f2_fma(di[q], nv[p],
                                    f2_fma(wr[q], er[p], f2_mul(ni[q], ei[p]))));
@@ -612,7 +652,8 @@ pair_kernel(int R, int Na, int Nap, int ldv, int splits, int n_tiles,
         Y[q][p][1] = f2_fma(A.y, qi, f2_fma(ny, qr, Y[q][p][1]));
       }
     }
-  });
+  };
+  by_shape(body);
   auto sum = [](uint64_t v) {
     return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32));
   };
@@ -625,16 +666,17 @@ pair_kernel(int R, int Na, int Nap, int ldv, int splits, int n_tiles,
 // order; a pair's up to 4 entries of I - M
 __global__ void __launch_bounds__(256)
 pair_reduce_kernel(int Na, int splits, int n_tiles, double G, const double* __restrict__ Nk,
-                   const int2* __restrict__ tiles, const double4* __restrict__ part,
+                   const int4* __restrict__ tiles, const double4* __restrict__ part,
                    double2* __restrict__ Aall, double2* __restrict__ Mall) {
   __shared__ double4 sm[4][64];
   const int tile = blockIdx.x, e = blockIdx.y * 64 + (threadIdx.x & 63), sg = threadIdx.x >> 6;
   const int z = blockIdx.z;
-  const int2 tl = tiles[tile];
-  const double4* src = part + ((size_t)z * n_tiles + tile) * splits * PR_SLOT + e;
+  const int4 tl = tiles[tile];
+  const double4* src = part + ((size_t)z * n_tiles + tile) * 2 * splits * PR_SLOT + e;
+  const int slots = 2 * tile_splits(splits, tl.z);
   double4 s = make_double4(0, 0, 0, 0);
 #pragma unroll 4
-  for (int k = sg; k < splits; k += 4) {
+  for (int k = sg; k < slots; k += 4) {
     const double4 v = src[(size_t)k * PR_SLOT];
     s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
   }
@@ -718,6 +760,13 @@ struct Scratch {                       // device buffers of the preparation
   }
 };
 
+// CTAs of the pair sum with k row splits of a whole tile
+int pair_ctas(const kls_similar* s, int k) {
+  int n = 0;
+  for (int w : s->weight) n += 2 * tile_splits(k, w);
+  return n;
+}
+
 size_t f_bytes(const kls_similar* s) { return (size_t)s->R * s->Nap * 64; }
 
 }  // namespace
@@ -736,7 +785,7 @@ void kls_similar_free(kls_ctx* c) {
 int kls_similar_prepare(kls_ctx* c) {
   const int NR = c->NR, Ne = c->Ne, nwa = c->nwa, NPh = c->NPh;
   // fewer radii: the table's work is below this form's (2 N^2 NR against
-  // 12 N NR + 14 N^2 per row)
+  // 12 N NR + 22 N^2 per row)
   if (NR < 16 || nwa < 8) return KLS_OK;
   Scratch sc;
   double *d_probe, *d_fit, *d_rfit, *d_ref, *d_of5, *d_T;
@@ -819,9 +868,18 @@ int kls_similar_prepare(kls_ctx* c) {
   s->Nap = (c->Na + PR_T - 1) / PR_T * PR_T;
   s->K2p = ((NR + 1) / 2 + FA_K - 1) / FA_K * FA_K;
   const size_t fitn = (size_t)Ne * nwa, tab = (size_t)s->R * c->ldv;
-  std::vector<int2> tiles;
+  std::vector<int4> tiles;
+  s->weight.clear();
   for (int J = 0; 2 * J * PR_T <= c->Na - 1; ++J)
-    for (int I = J; (I + J) * PR_T <= c->Na - 1; ++I) tiles.push_back(make_int2(I, J));
+    for (int I = J; (I + J) * PR_T <= c->Na - 1; ++I) {
+      const int lim = std::min(6, ((c->Na - 1 - (I + J) * PR_T) / 8 + 1) & ~1);
+      int blocks = 0;
+      for (int q = 0; q < 4; ++q)
+        for (int p = 0; p < 4; ++p) blocks += q + p <= lim && (I > J || q >= p);
+      // a row's operands cost about a quarter of a whole tile's time
+      s->weight.push_back(4 + (3 * blocks + 3) / 4);
+      tiles.push_back(make_int4(I, J, s->weight.back(), lim));
+    }
   s->n_tiles = (int)tiles.size();
   auto bail = [&](int r) {
     kls_similar_free(c);
@@ -839,7 +897,7 @@ int kls_similar_prepare(kls_ctx* c) {
     SIM_CK(cudaMalloc(&s->U, (size_t)3 * NPh * sizeof(double)));
     SIM_CK(cudaMalloc(&s->Phi, (size_t)2 * s->K2p * s->Nap * sizeof(double)));
     SIM_CK(cudaMalloc(&s->rot, (size_t)s->Nap * sizeof(double2)));
-    SIM_CK(cudaMalloc(&s->tiles, tiles.size() * sizeof(int2)));
+    SIM_CK(cudaMalloc(&s->tiles, tiles.size() * sizeof(int4)));
   }
   SIM_CK(sc.get(&d_U, (size_t)2 * NPh));
   SIM_CK(sc.get(&d_fit, 7 * fitn));
@@ -860,7 +918,7 @@ int kls_similar_prepare(kls_ctx* c) {
                          c->stream));
   SIM_CK(cudaMemcpyAsync(d_ok, ok.data(), ok.size() * sizeof(int), cudaMemcpyHostToDevice,
                          c->stream));
-  SIM_CK(cudaMemcpyAsync(s->tiles, tiles.data(), tiles.size() * sizeof(int2),
+  SIM_CK(cudaMemcpyAsync(s->tiles, tiles.data(), tiles.size() * sizeof(int4),
                          cudaMemcpyHostToDevice, c->stream));
   SIM_CK(cudaMemsetAsync(d_mx, 0, (size_t)6 * Ne * sizeof(unsigned long long), c->stream));
   fit_kernel<<<dim3((nwa + 127) / 128, Ne), 128, 0, c->stream>>>(
@@ -917,18 +975,19 @@ int kls_similar_prepare(kls_ctx* c) {
 #undef SIM_CK
 }
 
-// Row splits of the pair sum, fixed per context; an FP64 and an FP32 CTA per
-// tile and split, two of them on an SM at a time.  One wave while that leaves a
-// split fewer than 64 rows, else up to 6 waves (a last wave that is partly empty
-// costs less of them).
+// Row splits of a whole tile in the pair sum (the others have fewer, by weight),
+// fixed per context; an FP64 and an FP32 CTA per tile and split, two of them on an
+// SM at a time.  One wave while that leaves a split fewer than 64 rows, else up to 6
+// waves (a last wave that is partly empty costs less of them).
 int kls_similar_max_splits(const kls_ctx* c) { return std::max(1, c->sim->R / 8); }
 int kls_similar_splits(const kls_ctx* c) {
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-  const int per = 2 * c->sim->n_tiles;            // CTAs of one split
-  int s = 1;
+  int s = 1, sum = 0;
+  for (int w : c->sim->weight) sum += w;
   for (int waves = 1; waves <= 6; ++waves) {
-    const int k = std::max(1, 2 * sms * waves / per);
+    int k = std::max(1, sms * waves * 16 / sum);
+    while (k > 1 && pair_ctas(c->sim, k) > 2 * sms * waves) --k;
     if (waves > 1 && c->sim->R < 64 * k) break;
     s = k;
   }
@@ -945,7 +1004,7 @@ size_t kls_similar_f_bytes(const kls_ctx* c, int n) {
 size_t kls_similar_part_elems(const kls_ctx* c, int n) {   // double2
   return (size_t)n * c->sim->n_tiles * 2 * c->splits * PR_SLOT * 2;
 }
-int kls_similar_ctas(const kls_ctx* c) { return 2 * c->sim->n_tiles * c->splits; }
+int kls_similar_ctas(const kls_ctx* c) { return pair_ctas(c->sim, c->splits); }
 
 // F, pair sums and I - M of n omegas from their weights; no allocation, no
 // synchronisation (capturable)
@@ -974,7 +1033,7 @@ cudaError_t kls_similar_launch(const kls_ctx* c, cudaStream_t st, int n, const d
     *launches += 2;
   }
   pair_reduce_kernel<<<dim3(s->n_tiles, PR_SLOT / 64, n), 256, 0, st>>>(
-      c->Na, 2 * c->splits, s->n_tiles, c->cfg.G, c->d_N, s->tiles, p4, A, M);
+      c->Na, c->splits, s->n_tiles, c->cfg.G, c->d_N, s->tiles, p4, A, M);
   *launches += 1;
   return cudaGetLastError();
 }
