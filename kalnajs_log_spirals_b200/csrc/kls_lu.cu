@@ -563,8 +563,10 @@ constexpr int LUP_CLASSES = (int)(sizeof(lup_classes) / sizeof(lup_classes[0]));
 
 // Ring slots: one per column where 200 KB hold them (N <= 112: no slot is
 // written twice), else an even number of them, at least 16.
-int lup_slots(int n) {
-  const int s = (int)(204800 / (n * sizeof(double2) + 32));
+// Where a batch is more than one wave, half as many: the classes up to N = 128 then
+// have two CTAs on an SM (63 matrices of N = 101: 290 -> 246 us).
+int lup_slots(int n, bool half = false) {
+  const int s = (int)((half ? 102400 : 204800) / (n * sizeof(double2) + 32));
   return n <= s ? n : std::max(16, s & ~1);
 }
 
@@ -627,11 +629,11 @@ int kls_run_lu(kls_ctx* c, int n) {
     }
     if (c->lu_class >= 0) {
       const LupClass& k = lup_classes[c->lu_class];
-      const int slots = lup_slots(c->Na);
       int sms = 148;
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
       const bool wide = c->lu_wide && (int64_t)n * k.Cw <= sms;
       const int C = wide ? k.Cw : k.C;
+      const int slots = lup_slots(c->Na, (int64_t)n * C > sms);
       cudaLaunchAttribute at;
       cudaLaunchConfig_t cfg = lup_config(C, n, lup_smem(c->Na, slots), c->stream, &at);
       const double2* A = c->d_A;
