@@ -242,8 +242,22 @@ __device__ __forceinline__ void st_release_cluster(uint32_t addr, int v) {
 
 // Bounded wait.  The waiting warp is suspended (up to 10 us a try) instead of
 // polling: seven polling warps slow the one that the others wait for (its
-// shuffles and shared-memory reads queue behind theirs).
-__device__ __forceinline__ bool lup_wait(uint32_t bar, uint32_t parity, volatile int* abort) {
+// shuffles and shared-memory reads queue behind theirs).  Only the warp whose
+// column is next polls for a while, as it wakes up the sooner (N = 301 576 -> 556
+// us, 16 matrices of 201 374 -> 352).
+__device__ __forceinline__ bool lup_wait(uint32_t bar, uint32_t parity, volatile int* abort,
+                                         bool poll) {
+  for (int it = 0; poll && it < 200; ++it) {
+    uint32_t ok;
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
   unsigned long long t0 = 0;
   for (uint32_t it = 0;; ++it) {
     uint32_t ok;
@@ -454,7 +468,7 @@ __device__ __forceinline__ void lup_body(int n, int slots, const double2* __rest
   int j = 0, s = 0;                            // column j is in slot s
   uint32_t parity = 0;
   for (; j < until; ++j) {
-    const bool ok = lup_wait(smem_u32(full + s), parity, &s_abort);
+    const bool ok = lup_wait(smem_u32(full + s), parity, &s_abort, next == j + 1);
     if (!__all_sync(0xffffffffu, ok)) break;
     const LupMeta mt = meta[s];
 #pragma unroll
