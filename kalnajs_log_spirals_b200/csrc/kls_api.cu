@@ -103,6 +103,19 @@ int dalloc(kls_ctx* c, T** p, size_t count) {
   return KLS_OK;
 }
 
+// the arrays of a slab, as dalloc
+int dslab(kls_ctx* c, void** base, KlsSlab& s) {
+  const cudaError_t e = s.alloc(base);
+  if (e != cudaSuccess) {
+    char buf[160];
+    snprintf(buf, sizeof buf, "cudaMalloc of %.3f GB failed: %s", s.bytes() / 1e9,
+             cudaGetErrorString(e));
+    return kls_fail(c, KLS_ERR_OOM, buf);
+  }
+  c->device_bytes += (int64_t)s.bytes();
+  return KLS_OK;
+}
+
 void dfree(void* p) {
   if (p) cudaFree(p);
 }
@@ -139,16 +152,15 @@ int ensure_ws(kls_ctx* c, int n, int mode) {
   if (mode == KLS_MODE_FP64 && (r = ensure_f64(c, n))) return r;
   if (n <= c->ws_omega) return KLS_OK;
   int cap = n;
-  dfree(c->d_omega); dfree(c->d_wt); dfree(c->d_A); dfree(c->d_det);
-  dfree(c->d_logabs);
+  dfree(c->ws);
+  c->ws = nullptr;
   c->d_omega = nullptr; c->d_wt = nullptr; c->d_A = nullptr;
   c->d_det = nullptr; c->d_logabs = nullptr;
   c->ws_omega = 0;
-  if ((r = dalloc(c, &c->d_omega, (size_t)2 * cap))) return r;
-  if ((r = dalloc(c, &c->d_wt, (size_t)cap * c->K_pad))) return r;
-  if ((r = dalloc(c, &c->d_A, (size_t)cap * c->Na * c->Na))) return r;
-  if ((r = dalloc(c, &c->d_det, (size_t)cap))) return r;
-  if ((r = dalloc(c, &c->d_logabs, (size_t)cap))) return r;
+  KlsSlab s;
+  s.add(&c->d_omega, (size_t)2 * cap).add(&c->d_wt, (size_t)cap * c->K_pad);
+  s.add(&c->d_A, (size_t)cap * c->Na * c->Na).add(&c->d_det, cap).add(&c->d_logabs, cap);
+  if ((r = dslab(c, &c->ws, s))) return r;
   c->ws_omega = cap;
   return KLS_OK;
 }
@@ -292,8 +304,9 @@ int kls_create(const kls_config* cfg, int device, kls_ctx** out) {
   if (e != cudaSuccess || ndev == 0)
     return kls_fail(nullptr, KLS_ERR_CUDA, std::string("no CUDA device: ") + cudaGetErrorString(e));
   if (device < 0 || device >= ndev) return kls_fail(nullptr, KLS_ERR_CONFIG, "bad device index");
-  cudaDeviceProp prop;
-  if (cudaGetDeviceProperties(&prop, device) != cudaSuccess || prop.major < 10)
+  int major = 0;                       // (cudaGetDeviceProperties takes 2.5 ms)
+  if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device) != cudaSuccess ||
+      major < 10)
     return kls_fail(nullptr, KLS_ERR_UNSUPPORTED, "libkls.so is built for sm_100a (B200)");
   kls_ctx* c = new kls_ctx();
   c->cfg = *cfg;
@@ -314,18 +327,16 @@ int kls_create(const kls_config* cfg, int device, kls_ctx** out) {
   c->K = (int64_t)c->NPh * c->n_l;
   c->K_pad = ((c->K + KLS_KROW_ALIGN - 1) / KLS_KROW_ALIGN) * KLS_KROW_ALIGN;
 
-  if ((r = dalloc(c, &c->d_cosw, c->nw)) || (r = dalloc(c, &c->d_sinw, c->nw)) ||
-      (r = dalloc(c, &c->d_cs, kls_orbit_table(c->nw, c->nwai))) ||
-      (r = dalloc(c, &c->d_of, (size_t)OF_COUNT * c->NPh)) ||
-      (r = dalloc(c, &c->d_SRC, c->NR)) || (r = dalloc(c, &c->d_rc, c->NR)) ||
-      (r = dalloc(c, &c->d_valid, c->NPh)) ||
-      (r = dalloc(c, &c->d_w1, (size_t)c->NPh * c->nwa)) ||
-      (r = dalloc(c, &c->d_ra, (size_t)c->NPh * c->nwa)) ||
-      (r = dalloc(c, &c->d_pha, (size_t)c->NPh * c->nwa)) ||
-      (r = dalloc(c, &c->d_alpha, c->Na)) || (r = dalloc(c, &c->d_dalpha, c->Na)) ||
-      (r = dalloc(c, &c->d_N, c->Na)) || (r = dalloc(c, &c->d_Gk, c->K_pad)) ||
-      (r = dalloc(c, &c->d_Ok, c->K_pad)) || (r = dalloc(c, &c->d_F0l, c->K_pad)) ||
-      (r = dalloc(c, &c->d_M, (size_t)c->Na * c->Na))) {
+  const size_t ns = (size_t)c->NPh * c->nwa;
+  KlsSlab b;
+  b.add(&c->d_cosw, c->nw).add(&c->d_sinw, c->nw);
+  b.add(&c->d_cs, kls_orbit_table(c->nw, c->nwai)).add(&c->d_of, (size_t)OF_COUNT * c->NPh);
+  b.add(&c->d_SRC, c->NR).add(&c->d_rc, c->NR).add(&c->d_valid, c->NPh);
+  b.add(&c->d_w1, ns).add(&c->d_ra, ns).add(&c->d_pha, ns);
+  b.add(&c->d_alpha, c->Na).add(&c->d_dalpha, c->Na).add(&c->d_N, c->Na);
+  b.add(&c->d_Gk, c->K_pad).add(&c->d_Ok, c->K_pad).add(&c->d_F0l, c->K_pad);
+  b.add(&c->d_M, (size_t)c->Na * c->Na);
+  if ((r = dslab(c, &c->base, b))) {
     std::string m = c->err;
     kls_destroy(c);
     return kls_fail(nullptr, r, m);
@@ -340,10 +351,7 @@ int kls_destroy(kls_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   kls_mixed_free(c);
   kls_similar_free(c);
-  void* ptrs[] = {c->d_cosw, c->d_sinw, c->d_cs, c->d_of, c->d_SRC, c->d_rc, c->d_valid, c->d_w1, c->d_ra,
-                  c->d_pha, c->d_alpha, c->d_dalpha, c->d_N, c->d_Gk, c->d_Ok, c->d_F0l,
-                  c->d_V, c->d_items, c->d_tiles, c->d_F, c->d_omega, c->d_wt, c->d_part, c->d_A, c->d_M,
-                  c->d_anchorM, c->d_det, c->d_logabs};
+  void* ptrs[] = {c->base, c->ws, c->d_V, c->d_items, c->d_tiles, c->d_F, c->d_part, c->d_anchorM};
   for (void* p : ptrs) dfree(p);
   for (auto& ev : c->ev) if (ev) cudaEventDestroy(ev);
   for (auto& ev : c->pev) if (ev) cudaEventDestroy(ev);

@@ -87,6 +87,37 @@ struct kls_item {
   int n_om, kb0, nkb, pad;
 };
 
+// Several device arrays in one allocation, each on 256 bytes: above a megabyte a
+// cudaMalloc takes 0.36 ms and a cudaFree 0.3 to 1, whatever the size, and a new
+// model has some forty arrays.
+struct KlsSlab {
+  struct Part { void** p; size_t bytes; };
+  std::vector<Part> parts;
+  template <typename T>
+  KlsSlab& add(T** p, size_t n) {
+    parts.push_back({(void**)p, (n * sizeof(T) + 16 + 255) / 256 * 256});
+    return *this;
+  }
+  size_t bytes() const {
+    size_t n = 0;
+    for (const Part& x : parts) n += x.bytes;
+    return n;
+  }
+  cudaError_t alloc(void** base) {
+    const cudaError_t e = cudaMalloc(base, bytes());
+    if (e != cudaSuccess) {
+      *base = nullptr;
+      return e;
+    }
+    char* at = (char*)*base;
+    for (const Part& x : parts) {
+      *x.p = at;
+      at += x.bytes;
+    }
+    return e;
+  }
+};
+
 struct kls_ctx {
   kls_config cfg{};
   int device = 0;
@@ -101,6 +132,8 @@ struct kls_ctx {
   int64_t device_bytes = 0;
 
   // omega-independent device data
+  void* base = nullptr;       // the arrays up to d_M, one allocation
+  void* ws = nullptr;         // d_omega, d_wt, d_A, d_det, d_logabs
   double* d_cosw = nullptr;   // [nw]
   double* d_sinw = nullptr;   // [nw]
   double2* d_cs = nullptr;    // both in the orbit kernel's order

@@ -38,6 +38,7 @@
 #include <vector>
 
 struct kls_similar {
+  void* slab = nullptr;       // the arrays below
   int R = 0;                  // rows (l, e): il * Ne + ie
   int Nap = 0;                // N_alpha padded to the pair tiles
   int K2p = 0;                // mirrored pairs of radii, padded to the slabs of fourier_kernel
@@ -747,17 +748,10 @@ void jacobi(double A[SIM_PROBES][SIM_PROBES], double E[SIM_PROBES][SIM_PROBES],
       }
 }
 
-struct Scratch {                       // device buffers of the preparation
-  std::vector<void*> p;
-  ~Scratch() {
-    for (void* x : p) cudaFree(x);
-  }
-  template <typename T>
-  cudaError_t get(T** out, size_t n) {
-    cudaError_t e = cudaMalloc((void**)out, std::max<size_t>(n, 1) * sizeof(T));
-    if (e == cudaSuccess) p.push_back(*out);
-    return e;
-  }
+struct Scratch {                       // device arrays of the preparation
+  KlsSlab slab;
+  void* base = nullptr;
+  ~Scratch() { cudaFree(base); }
 };
 
 // CTAs of the pair sum with k row splits of a whole tile
@@ -774,8 +768,7 @@ size_t f_bytes(const kls_similar* s) { return (size_t)s->R * s->Nap * 64; }
 void kls_similar_free(kls_ctx* c) {
   kls_similar* s = c->sim;
   if (!s) return;
-  void* ptrs[] = {s->V, s->Vf, s->D, s->U, s->Phi, s->rot, s->tiles};
-  for (void* p : ptrs) cudaFree(p);
+  cudaFree(s->slab);
   delete s;
   c->sim = nullptr;
 }
@@ -795,7 +788,13 @@ int kls_similar_prepare(kls_ctx* c) {
   double2* d_mis;
   double* d_U = nullptr;
   const int PW = SIM_PROBES + 2;
-  KLS_CK(c, sc.get(&d_probe, (size_t)NPh * PW));
+  const size_t fitn = (size_t)Ne * nwa, n5 = (size_t)5 * Ne;
+  const size_t tab = (size_t)c->n_l * Ne * c->ldv;
+  sc.slab.add(&d_probe, (size_t)NPh * PW).add(&d_U, (size_t)2 * NPh).add(&d_fit, 7 * fitn);
+  sc.slab.add(&d_rfit, (size_t)3 * Ne).add(&d_iv, Ne).add(&d_ref, 3 * n5 * nwa);
+  sc.slab.add(&d_of5, (size_t)OF_COUNT * n5).add(&d_ok, n5).add(&d_T, 5 * tab);
+  sc.slab.add(&d_mx, (size_t)6 * Ne).add(&d_mis, NPh);
+  KLS_CK(c, sc.slab.alloc(&sc.base));
   probe_kernel<<<(NPh + 127) / 128, 128, 0, c->stream>>>(NPh, nwa, c->d_of, c->d_valid, c->d_w1,
                                                          c->d_pha, d_probe);
   KLS_LAUNCHED(c);
@@ -850,7 +849,6 @@ int kls_similar_prepare(kls_ctx* c) {
     rfit[3 * ie + 2] = sq[1] * iv[ie].y;
     for (int q = 0; q < 5; ++q) ok[(size_t)q * Ne + ie] = 1;
   }
-  const size_t n5 = (size_t)5 * Ne;
   std::vector<double> of5((size_t)OF_COUNT * n5, 0.0);
   for (int q = 0; q < 5; ++q)
     for (int ie = 0; ie < Ne; ++ie) {
@@ -867,7 +865,6 @@ int kls_similar_prepare(kls_ctx* c) {
   s->R = c->n_l * Ne;
   s->Nap = (c->Na + PR_T - 1) / PR_T * PR_T;
   s->K2p = ((NR + 1) / 2 + FA_K - 1) / FA_K * FA_K;
-  const size_t fitn = (size_t)Ne * nwa, tab = (size_t)s->R * c->ldv;
   std::vector<int4> tiles;
   s->weight.clear();
   for (int J = 0; 2 * J * PR_T <= c->Na - 1; ++J)
@@ -890,25 +887,12 @@ int kls_similar_prepare(kls_ctx* c) {
     cudaError_t e_ = (call);                                                      \
     if (e_ != cudaSuccess) return bail(kls_cuda_fail(c, e_, #call));              \
   } while (0)
-  if (!s->V) {
-    SIM_CK(cudaMalloc(&s->V, tab * sizeof(double)));
-    SIM_CK(cudaMalloc(&s->Vf, tab * sizeof(float)));
-    SIM_CK(cudaMalloc(&s->D, 2 * tab * sizeof(float)));
-    SIM_CK(cudaMalloc(&s->U, (size_t)3 * NPh * sizeof(double)));
-    SIM_CK(cudaMalloc(&s->Phi, (size_t)2 * s->K2p * s->Nap * sizeof(double)));
-    SIM_CK(cudaMalloc(&s->rot, (size_t)s->Nap * sizeof(double2)));
-    SIM_CK(cudaMalloc(&s->tiles, tiles.size() * sizeof(int4)));
+  if (!s->slab) {
+    KlsSlab b;
+    b.add(&s->V, tab).add(&s->Vf, tab / 2).add(&s->D, tab / 2).add(&s->U, (size_t)3 * NPh);
+    b.add(&s->Phi, (size_t)2 * s->K2p * s->Nap).add(&s->rot, s->Nap).add(&s->tiles, tiles.size());
+    SIM_CK(b.alloc(&s->slab));
   }
-  SIM_CK(sc.get(&d_U, (size_t)2 * NPh));
-  SIM_CK(sc.get(&d_fit, 7 * fitn));
-  SIM_CK(sc.get(&d_rfit, rfit.size()));
-  SIM_CK(sc.get(&d_iv, iv.size()));
-  SIM_CK(sc.get(&d_ref, 3 * n5 * nwa));
-  SIM_CK(sc.get(&d_of5, of5.size()));
-  SIM_CK(sc.get(&d_ok, ok.size()));
-  SIM_CK(sc.get(&d_T, 5 * tab));
-  SIM_CK(sc.get(&d_mx, (size_t)6 * Ne));
-  SIM_CK(sc.get(&d_mis, (size_t)NPh));
   SIM_CK(cudaMemcpyAsync(d_U, U.data(), U.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   SIM_CK(cudaMemcpyAsync(d_rfit, rfit.data(), rfit.size() * sizeof(double), cudaMemcpyHostToDevice,
                          c->stream));
