@@ -16,7 +16,7 @@
 //
 // A training step is 2 L + 1 launches for L layers: the forward layers (the first
 // gathers and converts its rows of X, the last forms the loss and its gradient),
-// a launch per layer for dW, the bias gradient and dH together, and the update.
+// dH of L - 1 layers, dW and the bias gradients of all layers in one, and the update.
 // The steps of an epoch are queued without a wait; the losses are read at its end.
 #include "kls_internal.cuh"
 #include <cuda_bf16.h>
@@ -141,7 +141,7 @@ __device__ void column_sums(const SumArgs& a, int blk, float* sm) {
 // 16 bytes apart modulo 128 (ldmatrix without conflicts).  Every output adds its
 // products over K in order, in steps of 16.
 // Bound: latency - at a batch of 1024 and width 256 a GEMM has 0.13 Gflop and its
-// operands are in L2, 5 to 11 us a launch.  A training step 850 -> 78 us, the
+// operands are in L2, 5 to 11 us a launch.  A training step 850 -> 69 us, the
 // forward pass of 820 rows 139 -> 42 us host to host; before: 2-byte loads, one
 // stage, 64 x 64 tiles (16 blocks for dW), a thread per bias column, the batch
 // gathered on the host and a wait per step.
@@ -305,22 +305,40 @@ __device__ __forceinline__ void gemm_tile(const GemmArgs& g, int blk,
     g.lpart[m0 / BT] = (sloss[0] + sloss[1]) + (sloss[2] + sloss[3]);
 }
 
-// Blocks [0, nb0) compute g0 with EPI; for dW (EPI_STORE) [nb0, nb1) dH in g1, and the
-// others the bias gradient
 template <int BT, int BK, int EPI>
-__global__ void __launch_bounds__(GT_THREADS)
-gemm_kernel(const __grid_constant__ GemmArgs g0, const __grid_constant__ GemmArgs g1,
-            const __grid_constant__ SumArgs cs, int nb0, int nb1) {
+__global__ void __launch_bounds__(GT_THREADS) gemm_kernel(const __grid_constant__ GemmArgs g) {
   __shared__ __align__(16) __nv_bfloat16 sm[GT_STAGES][2][BT * (BK + 8)];
+  __shared__ float sloss[4];
+  after_previous();
+  gemm_tile<BT, BK, EPI>(g, blockIdx.x, sm, sloss);
+}
+
+// dW and the bias gradients of all layers in one launch: the tiles of dW by layer,
+// then the column sums.  Each of these blocks runs through all rows of the batch in
+// order, so in a launch per layer (with dH) they were what it waited for: a step of
+// 1024 rows 81 -> 69 us, of 4096 204 -> 122 (width 256, depth 4).
+constexpr int ML_MAX = 16;                       // layers
+struct GradArgs {
+  int L, tiles[ML_MAX + 1], sums[ML_MAX + 1];
+  GemmArgs w[ML_MAX];
+  SumArgs s[ML_MAX];
+};
+__global__ void __launch_bounds__(GT_THREADS) grad_kernel(const __grid_constant__ GradArgs a) {
+  __shared__ __align__(16) __nv_bfloat16 sm[GT_STAGES][2][GT_S * (GT_SK + 8)];
   __shared__ float sloss[4];
   static_assert(sizeof(sm) >= GT_STAGES * CS_ROWS * CS_COLS * 4, "stages of the sums");
   after_previous();
-  if (EPI == EPI_STORE && (int)blockIdx.x >= nb1)
-    column_sums(cs, blockIdx.x - nb1, reinterpret_cast<float*>(&sm[0][0][0]));
-  else if (EPI == EPI_STORE && (int)blockIdx.x >= nb0)
-    gemm_tile<BT, BK, EPI_GELU_BWD>(g1, blockIdx.x - nb0, sm, sloss);
-  else
-    gemm_tile<BT, BK, EPI>(g0, blockIdx.x, sm, sloss);
+  const int b = blockIdx.x, b2 = b - a.tiles[a.L];
+  int l = 0;
+  if (b2 < 0) {
+    while (b >= a.tiles[l + 1]) ++l;
+    const GemmArgs g = a.w[l];
+    gemm_tile<GT_S, GT_SK, EPI_STORE>(g, b - a.tiles[l], sm, sloss);
+  } else {
+    while (b2 >= a.sums[l + 1]) ++l;
+    const SumArgs s = a.s[l];
+    column_sums(s, b2 - a.sums[l], reinterpret_cast<float*>(&sm[0][0][0]));
+  }
 }
 
 // one layer's view for the update: weights at w, bias behind them
@@ -329,7 +347,6 @@ struct LayerArgs {
   int64_t off;                                   // into the flat parameters
   __nv_bfloat16 *Wb, *Wt;
 };
-constexpr int ML_MAX = 16;                       // layers
 struct UpdateArgs {
   LayerArgs l[ML_MAX];
 };
@@ -429,8 +446,8 @@ struct kls_mlp {
   std::vector<float*> Z;                             // pre-activations [cap][dout_pad]
   std::vector<__nv_bfloat16*> H, Ht;                 // H[l]: input of layer l [cap][din_pad]
   __nv_bfloat16 *dZ[2] = {nullptr, nullptr};         // bf16 [cap][width], by turns
-  __nv_bfloat16 *dZt[2] = {nullptr, nullptr};        // bf16 [width][cap]
-  float* dZf[2] = {nullptr, nullptr};                // fp32 [cap][width]
+  std::vector<__nv_bfloat16*> dZt;                   // bf16 [dout_pad][cap] of every layer
+  std::vector<float*> dZf;                           // fp32 [cap][dout_pad]
   int ltiles = 0;                                    // row tiles of the last batch
   float* lpart = nullptr;                            // squared errors per row tile
   int rows = 0, steps = 0;                           // capacity of the buffers below
@@ -465,22 +482,24 @@ int ensure_cap(kls_mlp* m, int n) {
   for (auto*& z : m->Z) fr(z);
   for (auto*& h : m->H) fr(h);
   for (auto*& h : m->Ht) fr(h);
-  for (int q = 0; q < 2; ++q) { fr(m->dZ[q]); fr(m->dZt[q]); fr(m->dZf[q]); }
+  for (int q = 0; q < 2; ++q) fr(m->dZ[q]);
+  for (auto*& z : m->dZt) fr(z);
+  for (auto*& z : m->dZf) fr(z);
   fr(m->lpart);
   const int L = m->depth;
   m->Z.assign(L, nullptr);             // layers 0 .. L - 2
   m->H.assign(L, nullptr);             // inputs of the layers 1 .. L - 1
   m->Ht.assign(L, nullptr);            // inputs of all layers
+  m->dZt.assign(L, nullptr);
+  m->dZf.assign(L, nullptr);
   for (int l = 0; l < L; ++l) {
     if (l < L - 1) ML_CK(m, cudaMalloc(&m->Z[l], (size_t)cap * m->dout_pad[l] * 4));
     if (l) ML_CK(m, cudaMalloc(&m->H[l], (size_t)cap * m->din_pad[l] * 2));
     ML_CK(m, cudaMalloc(&m->Ht[l], (size_t)cap * m->din_pad[l] * 2));
+    ML_CK(m, cudaMalloc(&m->dZt[l], (size_t)cap * m->dout_pad[l] * 2));
+    ML_CK(m, cudaMalloc(&m->dZf[l], (size_t)cap * m->dout_pad[l] * 4));
   }
-  for (int q = 0; q < 2; ++q) {
-    ML_CK(m, cudaMalloc(&m->dZ[q], (size_t)cap * m->width * 2));
-    ML_CK(m, cudaMalloc(&m->dZt[q], (size_t)cap * m->width * 2));
-    ML_CK(m, cudaMalloc(&m->dZf[q], (size_t)cap * m->width * 4));
-  }
+  for (int q = 0; q < 2; ++q) ML_CK(m, cudaMalloc(&m->dZ[q], (size_t)cap * m->width * 2));
   ML_CK(m, cudaMalloc(&m->lpart, (size_t)(cap / GT_S) * 4));
   m->cap = cap;
   return KLS_OK;
@@ -530,14 +549,15 @@ int tiles(const GemmArgs& g, int t) { return ((g.N + t - 1) / t) * ((g.M + t - 1
 // The large tile from two of its blocks per SM on: there it reads half as much of
 // the operands per product (forward of 32768 rows, width 256, depth 4, host to host:
 // 189 against 222 us); below that the small one has the more SMs at work (a
-// training step of 1024 rows: 78 against 102 us; 8192 rows are alike, 85 us).
+// training step of 1024 rows is a quarter slower in large ones; 8192 rows are alike,
+// 85 us).
 template <int EPI>
-int gemm(kls_mlp* m, const GemmArgs& g, const GemmArgs& h = {}, const SumArgs& s = {}) {
-  const bool large = tiles(g, GT_L) + tiles(h, GT_L) >= 296;
-  const int t = large ? GT_L : GT_S, nb0 = tiles(g, t), nb1 = nb0 + tiles(h, t);
+int gemm(kls_mlp* m, const GemmArgs& g) {
+  const bool large = tiles(g, GT_L) >= 296;
+  const int t = large ? GT_L : GT_S;
   if (EPI == EPI_MSE) m->ltiles = (g.M + t - 1) / t;
   return launch(m, large ? gemm_kernel<GT_L, GT_LK, EPI> : gemm_kernel<GT_S, GT_SK, EPI>,
-                dim3(nb1 + (s.N + CS_COLS - 1) / CS_COLS), GT_THREADS, g, h, s, nb0, nb1);
+                dim3(tiles(g, t)), GT_THREADS, g);
 }
 
 int pack_all(kls_mlp* m) {
@@ -577,9 +597,9 @@ int forward(kls_mlp* m, int n, const int* idx, bool train) {
       r = gemm<EPI_GELU>(m, g);
     } else if (train) {
       g.T = m->Td;
-      g.C = m->dZf[0]; g.ldc = m->dout_pad[l];
+      g.C = m->dZf[l]; g.ldc = m->dout_pad[l];
       g.H = m->dZ[0]; g.ldh = m->dout_pad[l];
-      g.Ht = m->dZt[0];
+      g.Ht = m->dZt[l];
       g.lpart = m->lpart;
       r = gemm<EPI_MSE>(m, g);
     } else {
@@ -594,29 +614,34 @@ int forward(kls_mlp* m, int n, const int* idx, bool train) {
 // backward from the gradient that a training forward leaves in dZ[0]
 int backward(kls_mlp* m, int n) {
   const int L = m->depth;
+  GradArgs a{};
+  a.L = L;
   for (int l = L - 1, q = 0; l >= 0; --l, q ^= 1) {
-    // dW_l [dout][din] = dZ_l^T (dout x n) * H_l (n x din): A = dZt [dout_pad][cap], B = Ht_l
-    GemmArgs w{};
+    // dW_l [dout][din] = dZ_l^T (dout x n) * H_l (n x din): A = dZt_l [dout_pad][cap], B = Ht_l
+    GemmArgs& w = a.w[l];
     w.M = m->dout[l]; w.N = m->din[l]; w.K = n;
-    w.A = m->dZt[q]; w.lda = m->cap;
+    w.A = m->dZt[l]; w.lda = m->cap;
     w.B = m->Ht[l]; w.ldb = m->cap;
     w.C = m->g + m->woff[l]; w.ldc = m->din[l];
+    a.s[l] = {n, m->dout[l], m->dout_pad[l], m->dZf[l], m->g + m->boff[l]};
+    if (l == 0) break;
     // dZ_{l-1} = (dZ_l W_l) * gelu'(Z_{l-1}): A = dZ [n][dout_pad], B = Wt_l [din_pad][dout_pad]
     GemmArgs h{};
-    if (l) {
-      h.M = n; h.N = m->din_pad[l]; h.K = m->dout_pad[l];
-      h.A = m->dZ[q]; h.lda = m->dout_pad[l];
-      h.B = m->Wt[l]; h.ldb = m->dout_pad[l];
-      h.Zin = m->Z[l - 1]; h.ldz = m->dout_pad[l - 1];
-      h.C = m->dZf[q ^ 1]; h.ldc = m->din_pad[l];
-      h.H = m->dZ[q ^ 1]; h.ldh = m->din_pad[l];
-      h.Ht = m->dZt[q ^ 1]; h.ldht = m->cap;
-    }
-    const SumArgs s = {n, m->dout[l], m->dout_pad[l], m->dZf[q], m->g + m->boff[l]};
-    int r = gemm<EPI_STORE>(m, w, h, s);
+    h.M = n; h.N = m->din_pad[l]; h.K = m->dout_pad[l];
+    h.A = m->dZ[q]; h.lda = m->dout_pad[l];
+    h.B = m->Wt[l]; h.ldb = m->dout_pad[l];
+    h.Zin = m->Z[l - 1]; h.ldz = m->dout_pad[l - 1];
+    h.C = m->dZf[l - 1]; h.ldc = m->din_pad[l];
+    h.H = m->dZ[q ^ 1]; h.ldh = m->din_pad[l];
+    h.Ht = m->dZt[l - 1]; h.ldht = m->cap;
+    int r = gemm<EPI_GELU_BWD>(m, h);
     if (r) return r;
   }
-  return KLS_OK;
+  for (int l = 0; l < L; ++l) {
+    a.tiles[l + 1] = a.tiles[l] + tiles(a.w[l], GT_S);
+    a.sums[l + 1] = a.sums[l] + (m->dout[l] + CS_COLS - 1) / CS_COLS;
+  }
+  return launch(m, grad_kernel, dim3(a.tiles[L] + a.sums[L]), GT_THREADS, a);
 }
 
 LossArgs loss_args(const kls_mlp* m, int n, float* loss) {
@@ -695,7 +720,9 @@ int kls_mlp_destroy(kls_mlp* m) {
   for (auto* z : m->Z) fr(z);
   for (auto* x : m->H) fr(x);
   for (auto* x : m->Ht) fr(x);
-  for (int q = 0; q < 2; ++q) { fr(m->dZ[q]); fr(m->dZt[q]); fr(m->dZf[q]); }
+  for (int q = 0; q < 2; ++q) fr(m->dZ[q]);
+  for (auto* z : m->dZt) fr(z);
+  for (auto* z : m->dZf) fr(z);
   fr(m->lpart); fr(m->Xd); fr(m->Td); fr(m->Yd); fr(m->idx);
   cudaStreamDestroy(m->stream);
   delete m;
