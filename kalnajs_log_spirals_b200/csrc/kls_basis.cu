@@ -7,8 +7,8 @@
 //   E = r_k^{-1/2} e^{-i alpha ln r_k}, on the FP64 tensor pipe (DMMA
 //   m8n8k4).  C and E are generated in shared memory per 16-sample chunk:
 //   each thread evaluates one anchor sincos and advances by complex rotation
-//   over a short run (4 harmonics for C, 8 alphas for E), so the
-//   transcendental cost is a small fraction of the contraction.
+//   over a short run (4 harmonics for C, 8 alphas for E); what depends on the
+//   sample alone is computed once per 128 samples, one thread each.
 //   Orbits with non-finite samples are zero rows (BasisFunctions.jl:224-226);
 //   non-finite generated factors are zeroed (BasisFunctions.jl:248).
 // * N_m(alpha) (BasisFunctions.jl:281-304, Eq. 46) through ln|Gamma(z)|:
@@ -48,6 +48,10 @@ struct WlParams {
 #define WL_SMP(t, k) \
   KLS_LD(KLS_IB((int64_t)p * nwa + (k), (int64_t)NPh * nwa, KS_WL_SAMPLES), t[k], 0.0)
 
+// Bound: the FP64 pipe, which DMMA and the generation of C and E share.  255 orbits
+// of the default grid 4.61 -> 3.97 ms, all 25551 456 -> 395 ms: before, each of the 8
+// threads of a sample computed its logarithm, root, two of its four sincos and its
+// weight in every chunk.
 __global__ void __launch_bounds__(WL_THREADS)
 wl_kernel(WlParams P, const double* __restrict__ of, const int* __restrict__ valid,
           const double* __restrict__ w1g, const double* __restrict__ rag,
@@ -56,6 +60,9 @@ wl_kernel(WlParams P, const double* __restrict__ of, const int* __restrict__ val
   __shared__ double sC[WL_LB * WL_SC];
   __shared__ double sEr[WL_BK * WL_SE];
   __shared__ double sEi[WL_BK * WL_SE];
+  // per sample: w1, weight, m phi, cos and sin of w1, ln r, r^-1/2, cos and sin of
+  // the alpha step
+  __shared__ double smp[9][WL_THREADS];
   // one orbit's (l block, alpha block) CTAs are consecutive in launch order,
   // so its w1 / r / theta samples are read from DRAM once and then from L2
   const int nlb = (P.n_l + WL_LB - 1) / WL_LB, nab = (P.np + WL_AB - 1) / WL_AB;
@@ -88,9 +95,8 @@ wl_kernel(WlParams P, const double* __restrict__ of, const int* __restrict__ val
 
   if (ok) {
     for (int k0 = 0; k0 < nwa; k0 += WL_BK) {
-      // ---- generate C and E for samples k0..k0+15
-      const int k = k0 + gk;
-      if (k < nwa) {
+      if (k0 % WL_THREADS == 0 && k0 + tid < nwa) {
+        const int k = k0 + tid;
         double wk = WL_SMP(w1, k), rk = WL_SMP(ra, k);
         double wm = k > 0 ? WL_SMP(w1, k - 1) : 0.0, wp = k < nwa - 1 ? WL_SMP(w1, k + 1) : 0.0;
         double sw;
@@ -99,11 +105,28 @@ wl_kernel(WlParams P, const double* __restrict__ of, const int* __restrict__ val
         else if (k == nwa - 1) sw = (wk - wm) / 2;
         else sw = (wp - wm) / 2;
         double phi = ratio * wk - WL_SMP(pha, k);
+        double lr = log(rk), s, c;
+        smp[0][tid] = wk;
+        smp[1][tid] = sw;
+        smp[2][tid] = (double)P.m * phi;
+        sincos(wk, &s, &c);
+        smp[3][tid] = c;
+        smp[4][tid] = s;
+        smp[5][tid] = lr;
+        smp[6][tid] = 1.0 / sqrt(rk);
+        sincos(-P.astep * lr, &s, &c);
+        smp[7][tid] = c;
+        smp[8][tid] = s;
+      }
+      if (k0 % WL_THREADS == 0) __syncthreads();
+      // ---- generate C and E for samples k0..k0+15
+      const int k = k0 + gk, e = k % WL_THREADS;
+      if (k < nwa) {
         // C: cos(l w1 + m phi), anchor at l_first, rotate by w1
-        double th = (double)(P.l_min + l_first) * wk + (double)P.m * phi;
-        double s, c, ss, cs;
+        const double sw = smp[1][e];
+        double th = (double)(P.l_min + l_first) * smp[0][e] + smp[2][e];
+        double s, c, ss = smp[4][e], cs = smp[3][e];
         sincos(th, &s, &c);
-        sincos(wk, &ss, &cs);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           double v = sw * c;
@@ -114,12 +137,12 @@ wl_kernel(WlParams P, const double* __restrict__ of, const int* __restrict__ val
           c = cn;
         }
         // E: r^{-1/2} e^{-i alpha ln r}, anchor at a_first, rotate by -astep ln r
-        double lr = log(rk);
-        double isq = 1.0 / sqrt(rk);
+        const double lr = smp[5][e], isq = smp[6][e];
         double ta = -KLS_LD(KLS_IB(min(a_first, P.np - 1), P.np, KS_WL_SAMPLES),
                             alpha[min(a_first, P.np - 1)], 0.0) * lr;
         sincos(ta, &s, &c);
-        sincos(-P.astep * lr, &ss, &cs);
+        cs = smp[7][e];
+        ss = smp[8][e];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           double er = c * isq, ei = s * isq;
