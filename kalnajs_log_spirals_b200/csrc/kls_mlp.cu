@@ -30,6 +30,7 @@ struct kls_mlp;
 namespace {
 
 constexpr int ML_IN = 5, ML_OUT = 3;
+constexpr int ML_ROWS = 1 << 22;      // rows of a training set kept on the device (0.15 GB)
 constexpr int ML_PAD = 16;            // input / output dims padded to 16 for the MMA
 constexpr int GT_THREADS = 128;
 // the small and the large tile, rows = columns, with depth and stages of the
@@ -570,9 +571,9 @@ int pack_all(kls_mlp* m) {
   return KLS_OK;
 }
 
-// forward over n rows of X (rows idx, or in order); train: keeps Z and the
+// forward over n rows of X (rows idx, or in order from row0 on); train: keeps Z and the
 // transposes, and ends in the gradient of the loss; else the outputs to m->Yd
-int forward(kls_mlp* m, int n, const int* idx, bool train) {
+int forward(kls_mlp* m, int n, const int* idx, int row0, bool train) {
   const int L = m->depth;
   for (int l = 0; l < L; ++l) {
     GemmArgs g{};
@@ -584,7 +585,7 @@ int forward(kls_mlp* m, int n, const int* idx, bool train) {
     g.ldht = m->cap;
     g.idx = idx;
     if (l == 0) {
-      g.X = m->Xd;
+      g.X = m->Xd + (size_t)row0 * ML_IN;
       g.Xt = train ? m->Ht[0] : nullptr;
     }
     int r;
@@ -596,7 +597,7 @@ int forward(kls_mlp* m, int n, const int* idx, bool train) {
       }
       r = gemm<EPI_GELU>(m, g);
     } else if (train) {
-      g.T = m->Td;
+      g.T = m->Td + (size_t)row0 * ML_OUT;
       g.C = m->dZf[l]; g.ldc = m->dout_pad[l];
       g.H = m->dZ[0]; g.ldh = m->dout_pad[l];
       g.Ht = m->dZt[l];
@@ -649,8 +650,8 @@ LossArgs loss_args(const kls_mlp* m, int n, float* loss) {
 }
 
 // gradients into m->g and the loss by row tiles
-int grad_batch(kls_mlp* m, int n, const int* idx) {
-  int r = forward(m, n, idx, true);
+int grad_batch(kls_mlp* m, int n, const int* idx, int row0) {
+  int r = forward(m, n, idx, row0, true);
   return r ? r : backward(m, n);
 }
 
@@ -763,7 +764,7 @@ int kls_mlp_forward(kls_mlp* m, const float* X, int n, float* Y) {
     if (r || (r = ensure_rows(m, nb, 0))) return r;
     ML_CK(m, cudaMemcpyAsync(m->Xd, X + (size_t)s * ML_IN, (size_t)nb * ML_IN * 4,
                              cudaMemcpyHostToDevice, m->stream));
-    if ((r = forward(m, nb, nullptr, false))) return r;
+    if ((r = forward(m, nb, nullptr, 0, false))) return r;
     ML_CK(m, cudaMemcpyAsync(Y + (size_t)s * ML_OUT, m->Yd, (size_t)nb * ML_OUT * 4,
                              cudaMemcpyDeviceToHost, m->stream));
     ML_CK(m, cudaStreamSynchronize(m->stream));
@@ -779,7 +780,7 @@ int kls_mlp_grad(kls_mlp* m, const float* X, const float* T, int n, float* grads
   if (r || (r = ensure_rows(m, n, 1))) return r;
   ML_CK(m, cudaMemcpyAsync(m->Xd, X, (size_t)n * ML_IN * 4, cudaMemcpyHostToDevice, m->stream));
   ML_CK(m, cudaMemcpyAsync(m->Td, T, (size_t)n * ML_OUT * 4, cudaMemcpyHostToDevice, m->stream));
-  if ((r = grad_batch(m, n, nullptr))) return r;
+  if ((r = grad_batch(m, n, nullptr, 0))) return r;
   if ((r = launch(m, loss_kernel, dim3(1), 32, loss_args(m, n, m->loss)))) return r;
   if (grads) ML_CK(m, cudaMemcpyAsync(grads, m->g, m->nparams * 4, cudaMemcpyDeviceToHost, m->stream));
   if (loss) ML_CK(m, cudaMemcpyAsync(loss, m->loss, 4, cudaMemcpyDeviceToHost, m->stream));
@@ -794,13 +795,22 @@ int kls_mlp_train(kls_mlp* m, const float* X, const float* T, int n, int epochs,
   cudaSetDevice(m->device);
   batch = std::min(batch, n);
   const int steps = n / batch;
+  // up to ML_ROWS rows are on the device for the whole call and gathered there; of
+  // more, a segment of batches at a time in the epoch's order
+  const bool all = n <= ML_ROWS;
+  const int seg = all ? n : std::max(1, ML_ROWS / batch) * batch;
   int r = ensure_cap(m, batch);
-  if (r || (r = ensure_rows(m, n, steps))) return r;
+  if (r || (r = ensure_rows(m, seg, steps))) return r;
   int tiles_w = 1;                                       // blocks of the update, per layer
   for (int l = 0; l < m->depth; ++l)
     tiles_w = std::max(tiles_w, ((m->din[l] + 31) / 32) * ((m->dout[l] + 31) / 32) + 1);
-  ML_CK(m, cudaMemcpyAsync(m->Xd, X, (size_t)n * ML_IN * 4, cudaMemcpyHostToDevice, m->stream));
-  ML_CK(m, cudaMemcpyAsync(m->Td, T, (size_t)n * ML_OUT * 4, cudaMemcpyHostToDevice, m->stream));
+  auto upload = [&](const float* x, const float* t, int rows) -> int {
+    ML_CK(m, cudaMemcpyAsync(m->Xd, x, (size_t)rows * ML_IN * 4, cudaMemcpyHostToDevice, m->stream));
+    ML_CK(m, cudaMemcpyAsync(m->Td, t, (size_t)rows * ML_OUT * 4, cudaMemcpyHostToDevice, m->stream));
+    return KLS_OK;
+  };
+  std::vector<float> xb, tb;
+  if (all && (r = upload(X, T, n))) return r;
   UpdateArgs u{};
   for (int l = 0; l < m->depth; ++l)
     u.l[l] = {m->dout[l], m->din[l], m->dout_pad[l], m->din_pad[l], m->woff[l], m->Wb[l], m->Wt[l]};
@@ -811,9 +821,25 @@ int kls_mlp_train(kls_mlp* m, const float* X, const float* T, int n, int epochs,
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   if (epochs > 0) std::shuffle(idx.begin(), idx.end(), rng);
   for (int ep = 0; ep < epochs; ++ep) {
-    ML_CK(m, cudaMemcpyAsync(m->idx, idx.data(), (size_t)n * 4, cudaMemcpyHostToDevice, m->stream));
+    if (all)
+      ML_CK(m, cudaMemcpyAsync(m->idx, idx.data(), (size_t)n * 4, cudaMemcpyHostToDevice,
+                               m->stream));
     for (int s = 0; s < steps; ++s) {
-      if ((r = grad_batch(m, batch, m->idx + (size_t)s * batch))) return r;
+      const int64_t first = (int64_t)s * batch;
+      if (!all && first % seg == 0) {
+        const int rows = (int)std::min<int64_t>(seg, (int64_t)steps * batch - first);
+        ML_CK(m, cudaStreamSynchronize(m->stream));      // the rows before are used and copied
+        xb.resize((size_t)rows * ML_IN);
+        tb.resize((size_t)rows * ML_OUT);
+        for (int i = 0; i < rows; ++i) {
+          const size_t q = idx[first + i];
+          std::copy_n(X + q * ML_IN, ML_IN, xb.begin() + (size_t)i * ML_IN);
+          std::copy_n(T + q * ML_OUT, ML_OUT, tb.begin() + (size_t)i * ML_OUT);
+        }
+        if ((r = upload(xb.data(), tb.data(), rows))) return r;
+      }
+      if ((r = grad_batch(m, batch, all ? m->idx + first : nullptr, all ? 0 : (int)(first % seg))))
+        return r;
       ++m->step;
       const float c1 = 1.f - std::pow(b1, (float)m->step), c2 = 1.f - std::pow(b2, (float)m->step);
       if ((r = launch(m, adam_kernel, dim3(tiles_w, m->depth), 256,

@@ -66,3 +66,27 @@ def test_mlp_steps_of_an_epoch(lib_path):
     check(a, X, T, 64, 3)
     a.close()
     b.close()
+
+
+def test_mlp_training_set_in_segments(lib_path):
+    """More rows than are kept on the device (2^22): segments in the epoch's order.
+    With lr = 0 the epoch's loss is that of all rows but the one left out (FP32 sums of
+    4e6 terms: 1e-4), and one step over all of the rows is the gradient's."""
+    n = (1 << 22) + 1
+    rng = np.random.default_rng(9)
+    X = rng.normal(size=(n, 5)).astype(np.float32)
+    T = rng.normal(size=(n, 3)).astype(np.float32)
+    mlp = P.MLP(16, 2, seed=4)
+    p = mlp.params()
+    g, loss = mlp.grad(X, T)
+    hist = mlp.train(X, T, epochs=2, batch=1 << 20, lr=0.0, seed=1)
+    assert np.array_equal(mlp.params(), p)
+    assert np.all(np.abs(hist - loss) <= 1e-4 * loss)
+    mlp.close()
+    mlp = P.MLP(16, 2, seed=4)                 # (Adam's moments at zero)
+    mlp.train(X, T, epochs=1, batch=n, lr=1e-3, seed=1)
+    q = mlp.params()
+    big = np.abs(g) > 1e-2 * np.abs(g).max()
+    step = 1e-3 * g / (np.abs(g) + 1e-8)
+    assert np.all(np.abs(q - (p - step))[big] <= 1e-8 + 2e-7 * np.abs(p[big]))
+    mlp.close()
