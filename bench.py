@@ -6,16 +6,17 @@ Workload: Toomre-Zang n_zang=4, q1=7, m=2 disk, NR=501, Ne=51, N_alpha=301 on
 plain FP64 form.  One step = one Newton finite-difference triple
 (omega, omega + m*delta, omega + i*delta) evaluated as one batch.
 
-  value : det evaluations / s with the W table resident in HBM and omegas /
-          dets in device buffers (CUDA events on the launching stream)
+  value : det evaluations / s with the model's tables resident in HBM and
+          omegas / dets in device buffers (CUDA events on the launching stream)
   e2e   : the same through the C ABI with host buffers (kls_det_batch: H2D of
           omegas, D2H of dets and log|det| inside the timed region)
 
-Also reported: roofline of the contraction kernel (algorithmic FLOPs
-8 N_alpha^2 K per determinant against an in-run cuBLAS DGEMM peak, and the
-DMMA work the kernel issues), the split-BF16 form, Newton
+Also reported: roofline of the kernels that form M(omega) (on self-similar
+orbits F and the pair sums, else the contraction over the table) against an
+in-run cuBLAS DGEMM peak, the split-BF16 form, Newton
 time-to-root from the reference start (plain FP64 against the hybrid: split-
-BF16 secant steps, one FP64 anchor, anchored finish), parity against the
+BF16 or, where cheaper, FP64 secant steps, one FP64 anchor, the finish near it),
+parity against the
 default-size oracle fixture, precompute time, the CPU baseline (the oracle's
 BLAS form, one whole determinant on the host cores) and SM clocks sampled
 during the timed region.
@@ -430,9 +431,9 @@ def read_traffic(kernel: str):
         return None, None
 
 
-def precompute_roofline(cfg, dims, pre_ms, peak64: float, peaks: dict):
-    """Orbit integration and W_l quadrature kernels against the FP64 and HBM
-    peaks (CUDA-event times of the precompute in this run)."""
+def precompute_roofline(cfg, dims, pre_ms, peak64: float, peaks: dict, n_wl: int):
+    """Orbit integration and W_l quadrature kernels (n_wl orbits) against the FP64
+    and HBM peaks (CUDA-event times of the precompute in this run)."""
     NPh, Na, n_l, nwa, nw = dims.NPh, dims.N_alpha, dims.n_l, dims.nwa, cfg.grid.nw
     hbm = float(peaks.get("hbm_gbs", 6650.0))
     hbm_note = "of measured (MEASURED_PEAKS.json hbm_gbs)" if "hbm_gbs" in peaks else \
@@ -442,15 +443,15 @@ def precompute_roofline(cfg, dims, pre_ms, peak64: float, peaks: dict):
     if t_orb > 0:
         orb_bytes = 3.0 * nwa * NPh * 8 + 17.0 * NPh * 8 + 2.0 * nw * 8
         out["orbit_kernel"] = {
-            "ms": pre_ms[0], "point_evaluations_per_s": 2.0 * nw * NPh / t_orb,
+            "ms": pre_ms[0], "point_evaluations_per_s": float(nw) * NPh / t_orb,
             "algorithmic_bytes": orb_bytes, "hbm_gbs": orb_bytes / t_orb / 1e9,
             "hbm_frac": orb_bytes / t_orb / 1e9 / hbm, "hbm_peak_note": hbm_note,
-            "bound": "FP64 + transcendentals (2 nw point evaluations per orbit)"}
+            "bound": "instruction issue: FP64 + transcendentals (nw point evaluations per orbit)"}
     if t_wl > 0:
-        wl_bytes = float(NPh) * Na * n_l * 8 + 3.0 * nwa * NPh * 8
-        wl_flops = 2.0 * n_l * nwa * Na * NPh
+        wl_bytes = float(n_wl) * Na * n_l * 8 + 3.0 * nwa * n_wl * 8
+        wl_flops = 2.0 * n_l * nwa * Na * n_wl
         out["wl_kernel"] = {
-            "ms": pre_ms[1], "algorithmic_bytes": wl_bytes, "hbm_gbs": wl_bytes / t_wl / 1e9,
+            "ms": pre_ms[1], "orbits": n_wl, "algorithmic_bytes": wl_bytes, "hbm_gbs": wl_bytes / t_wl / 1e9,
             "hbm_frac": wl_bytes / t_wl / 1e9 / hbm, "hbm_peak_note": hbm_note,
             "algorithmic_flops": wl_flops, "tflops": wl_flops / t_wl / 1e12,
             "fp64_frac": wl_flops / t_wl / 1e12 / peak64,
@@ -921,7 +922,15 @@ def ours(args):
     nb = 3
     # one triangle of a complex symmetric product of real rows; the complex
     # product of the reference takes 8 N_alpha^2 K
+    # A model of self-similar orbits holds no table (8 N_alpha bytes per orbit x l term)
+    # but one row per (l, e).  FP64 work: F, the weights [rows x NR] against the cosines
+    # and sines of the mirrored radii (3 channels x re, im), and 12 FMA per pair of
+    # alphas (a quarter of the matrix) and row.
+    similar = dims.device_bytes < 24 * dims.nwa * dims.NPh + 8 * dims.K_pad * dims.N_alpha
+    rows = dims.n_l * cfg.grid.Ne
     flops_per_det = 2.0 * dims.N_alpha * (dims.N_alpha + 1) * dims.K
+    if similar:
+        flops_per_det = 12.0 * rows * cfg.grid.NR * dims.N_alpha + 6.0 * rows * dims.N_alpha ** 2
     # tensor flops of the 3-product split GEMM per determinant (unpadded)
     mixed_flops_per_det = 3 * 2.0 * (2 * dims.N_alpha) ** 2 * dims.K
     d_det = torch.empty((nb, 2), dtype=torch.float64, device="cuda")
@@ -991,10 +1000,16 @@ def ours(args):
     value = world * nb * args.steps / (ms * 1e-3)
     stage = stage_times(_lib.KLS_MODE_FP64)
     achieved = nb * flops_per_det / (stage[1] * 1e-3) / 1e12
-    # real DMMA flops the kernel issues: the 8 x 8 blocks of one triangle of
-    # T = sum_k w_k V_k^T V_k (V real, w complex: 2 real products)
-    n8 = -(-(-(-dims.N_alpha // 2) * 2) // 8)
-    issued_per_det = 4.0 * 64 * (n8 * (n8 + 1) // 2) * dims.K_pad
+    # real DMMA flops the kernels issue
+    if similar:
+        # F: mirrored radii padded to 8, rows to 16, N_alpha to 32
+        pad = lambda x, k: -(-x // k) * k
+        issued_per_det = 24.0 * pad(rows, 16) * pad((cfg.grid.NR + 1) // 2, 8) * pad(dims.N_alpha, 32)
+    else:
+        # the 8 x 8 blocks of one triangle of T = sum_k w_k V_k^T V_k (V real, w
+        # complex: 2 real products)
+        n8 = -(-(-(-dims.N_alpha // 2) * 2) // 8)
+        issued_per_det = 4.0 * 64 * (n8 * (n8 + 1) // 2) * dims.K_pad
     issued = nb * issued_per_det / (stage[1] * 1e-3) / 1e12
 
     # ---- end to end through the C ABI with host buffers -----------------------
@@ -1171,7 +1186,7 @@ def ours(args):
         dist.destroy_process_group()
     if rank != 0:
         return 0
-    traffic, traffic_scaled = read_traffic("contract_kernel")
+    traffic, traffic_scaled = read_traffic("similar" if similar else "contract_kernel")
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_per_step, "higher_is_better": True,
@@ -1182,17 +1197,24 @@ def ours(args):
                    "NR": cfg.grid.NR, "Ne": cfg.grid.Ne,
                    "N_alpha": cfg.grid.N_alpha, "l": [cfg.grid.l_min, cfg.grid.l_max],
                    "K": dims.K, "omegas_per_step": nb, "parallelism": f"replicas x{world}",
-                   "l2": "inputs larger than L2 (W table %.1f GB in HBM)" % (
-                       8 * dims.K_pad * dims.N_alpha / 1e9)},
+                   "l2": ("inputs larger than L2 (per omega %.0f MB of weights and %.0f MB of F)" % (
+                       16 * dims.K_pad / 1e6, 64e-6 * rows * -(-dims.N_alpha // 32) * 32)
+                       if similar else "inputs larger than L2 (W table %.1f GB in HBM)" % (
+                           8 * dims.K_pad * dims.N_alpha / 1e9))},
         "roofline": {"bound": "tensor",
-                     "kernel": "contract_kernel (FP64 DMMA m8n8k4, one triangle, real table)",
+                     "kernel": ("fourier_kernel (FP64 DMMA m8n8k4) + pair_kernel (FP64 and FP32 "
+                                "FMA)" if similar else
+                                "contract_kernel (FP64 DMMA m8n8k4, one triangle, real table)"),
                      "achieved": achieved, "peak": peak64, "unit": "TFLOP/s",
                      "frac": achieved / peak64,
                      "peak_note": "of measured: cuBLAS DGEMM 8192^3 best-of-5 in this run",
                      "algorithmic_flops_per_launch": nb * flops_per_det,
-                     "algorithmic_note": "2 N_alpha (N_alpha + 1) K per determinant: complex "
-                                         "weights times real rows, one triangle (the "
-                                         "reference's complex product: 8 N_alpha^2 K)",
+                     "algorithmic_note": ("FP64: 12 n_l Ne NR N_alpha (F) + 6 n_l Ne N_alpha^2 "
+                                          "(pairs) per determinant; the pairs' 16 n_l Ne "
+                                          "N_alpha^2 in FP32 are not counted" if similar else
+                                          "2 N_alpha (N_alpha + 1) K per determinant: complex "
+                                          "weights times real rows, one triangle") +
+                                         " (the reference's complex product: 8 N_alpha^2 K)",
                      "dmma_issued_tflops": issued, "dmma_issued_frac": issued / peak64,
                      "traffic": traffic, "traffic_scaled": traffic_scaled, "stage_ms": {"weights": stage[0], "contract": stage[1],
                                                       "reduce": stage[2], "lu": stage[3]}},
@@ -1210,7 +1232,8 @@ def ours(args):
                          "default_ms_per_omega": t.default_ms_per_omega}
                      for k, t in tunes.items()},
         "precompute_s": t_pre,
-        "precompute": precompute_roofline(cfg, dims, pre_ms, peak64, peaks),
+        "precompute": precompute_roofline(cfg, dims, pre_ms, peak64, peaks,
+                                          5 * cfg.grid.Ne if similar else dims.NPh),
         "mixed": mixed,
         "newton": newton,
         "reference_algorithm_gpu": refgpu,

@@ -100,7 +100,7 @@ typedef struct kls_dims {
     int32_t N_alpha;
     int32_t N_alpha_pad;/* N_alpha padded to the split-BF16 table's tiles   */
     int64_t K;          /* NPh * n_l contraction length                     */
-    int64_t K_pad;      /* padded rows of the device W table                */
+    int64_t K_pad;      /* orbit x l terms, padded: rows of the W table     */
     int32_t nwa;
     int64_t device_bytes; /* device memory held by the context             */
 } kls_dims;
@@ -159,13 +159,16 @@ int kls_get_dims(const kls_ctx* ctx, kls_dims* out);
 int kls_set_stream(kls_ctx* ctx, void* cuda_stream);
 
 /* ---- omega-independent stage: precompute_all + to_device ---------------- *
- * Grids, orbit integration, Jacobian + DF, W_l table, N_m(alpha), DJ, F0l,
- * Omega_res; all on the device, table device-resident (BasisFunctions.jl:73). */
+ * Grids, orbit integration, Jacobian + DF, W_l(alpha), N_m(alpha), DJ, F0l,
+ * Omega_res, all device-resident (BasisFunctions.jl:73).  The orbits of one
+ * eccentricity are scaled copies of one another in the logarithmic potential:
+ * where the integrated ones are, to rounding, W_l is kept for one orbit per
+ * eccentricity, else the table of all orbits is built.                      */
 int kls_precompute(kls_ctx* ctx);
 /* Build the split-BF16 copy of the W table used by KLS_MODE_MIXED.         */
 int kls_prepare_mixed(kls_ctx* ctx);
-/* Free the FP64 W table after building the split-BF16 copy (no reference
- * counterpart): a mixed-only context, 13 GB instead of 26 GB at NR=501,
+/* Free the FP64 form (table or common orbits) after building the split-BF16
+ * copy (no reference counterpart): a mixed-only context, 15 GB at NR=501,
  * Ne=51, N_alpha=301, l in [-100, 100], so that many default-size models fit
  * one GPU.  Afterwards KLS_MODE_FP64 calls, kls_export_W and FP64 batches
  * return KLS_ERR_STATE.                                                     */

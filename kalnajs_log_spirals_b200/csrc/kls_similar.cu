@@ -424,9 +424,9 @@ fourier_kernel(int R, int Ne, int NR, int K2p, int Nap, int64_t K_pad,
 // alone take 425 us and the FP32 ones 560, against 200 us each for their pipes
 // and for the shared-memory reads (22 and 26 bytes a pair and row).  Tiles at the
 // edges of the triangle leave out their empty 8 x 8 blocks in code of their own
-// (PairShape) and have the fewer row splits for it.  Default grid: 1542 -> 1030 us
+// (PairShape) and have the fewer row splits for it.  Default grid: 1542 -> 1055 us
 // per omega (before: 4 x 2 pairs with both sums in one thread, 64 bytes a pair, 2.03
-// waves) -> 930 with the edges (run-time branches around the blocks: 1000);
+// waves) -> 965 with the edges (run-time branches around the blocks: 1030);
 // N_alpha = 101, 1071 rows, batch of 16: 22 -> 19.
 constexpr int PR_T = 32, PR_ROWS = 4, PR_STAGES = 3, PR_THREADS = 128;
 constexpr int PR_FA = 0, PR_FB = 1024,                 // bytes in a row: F of 64 d
