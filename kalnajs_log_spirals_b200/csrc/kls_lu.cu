@@ -207,11 +207,13 @@ multi_lu_kernel(const kls_mdesc* __restrict__ md, const int2* __restrict__ pairs
 // column waits for all of them.
 // Waits are bounded (LUP_LIMIT_NS); one that runs out makes the determinant NaN.
 //
-// Measured (1 matrix, B200): N = 101 312 -> 100 us, 201 557 -> 264 us, 301 1022 ->
-// 575 us against one CTA (101) or a cluster with one barrier per column; 16
-// matrices 315 -> 101, 612 -> 374, 2760 -> 1148 us.  A column's chain is about
-// 1000 cycles at 4 rows a lane and 1900 at 10 (update 215 / 385, pivot search
-// 170 / 324, reciprocal 182, multipliers 48 / 111, hand-over 300).
+// Measured (1 matrix, B200): N = 101 312 -> 99 us, 201 557 -> 266 us, 301 1022 ->
+// 558 us against one CTA (101) or a cluster with one barrier per column; 16
+// matrices 315 -> 100, 612 -> 350, 2760 -> 1111 us.  A column's chain is about
+// 1600 cycles at 4 rows a lane and 3300 at 10 (hand-over 160 / 360, update 280 / 540,
+// pivot search with its reciprocal 670 / 1260, broadcast 60 / 80, multipliers and
+// publication 440 / 1100; the marks themselves are some 50 each): about 350
+// instructions that depend on one another.
 constexpr int LUP_WARPS = 8, LUP_THREADS = 32 * LUP_WARPS;
 constexpr unsigned long long LUP_LIMIT_NS = 2000000000ull;
 
@@ -547,13 +549,15 @@ multi_lu_pipe_kernel(const kls_mdesc* __restrict__ md, const int2* __restrict__ 
 // The size classes: rows per lane x columns per warp, CTAs per cluster.  4 columns
 // a warp keep enough matrices on the device at once; a wider form (2 columns) for
 // batches that it holds in one wave.  1 matrix / 16, us:
-//   N =  64  <2,2> x 4   52 /  52   (<2,8> x 1    71 /  71)
-//   N = 101  <4,3> x 6  100 / 101   (<4,4> x 4   105 / 105, <4,2> x 8 128 / 249)
-//   N = 192  <6,4> x 6  276 / 278   (<6,3> x 8   306 / 605), <6,2> x 12 233 / 686
-//   N = 201  <7,5> x 6  372 / 374   (<7,4> x 8   333 / 656), <7,2> x 14 264 / 782
-//   N = 256  <8,4> x 8  462 / 920   (<8,5> x 7   574 / 1140), <8,2> x 16 398 / 1183
-//   N = 301 <10,4> x 10 575 / 1148  (<10,3> x 16 632 / 1887)
-//   N = 400 <13,4> x 13 1513 / 4550 (<16,4> x 16 3277 / 9852)
+//   N =  64  <2,2> x 4   53 /  53   (<2,8> x 1    71 /  71)
+//   N = 101  <4,3> x 6   99 / 100   (<4,4> x 4   105 / 105, <4,2> x 8 128 / 249)
+//   N = 192  <6,4> x 6  276 / 276   (<6,3> x 8   306 / 605), <6,2> x 12 236 / 693
+//   N = 201  <7,5> x 6  350 / 350   (<7,4> x 8   333 / 656), <7,2> x 14 266 / 790
+//   N = 256  <8,4> x 8  455 / 899   (<8,5> x 7   574 / 1140), <8,2> x 16 398 / 1181
+//   N = 301 <10,4> x 10 558 / 1111  (<10,3> x 16 632 / 1887)
+//   N = 400 <13,4> x 13 1250 / 3748 (<16,4> x 16 3277 / 9852)
+//   N = 512 <16,4> x 16 2936 / 8782
+// (in brackets: before the warp whose column is next polled)
 struct LupClass {
   int n_max, C;
   const void *one, *multi;

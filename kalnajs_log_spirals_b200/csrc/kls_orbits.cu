@@ -24,7 +24,7 @@ namespace {
 constexpr int ORB_THREADS = 256;
 
 struct OrbitParams {
-  int NR, Ne, nw, nwa, nwai, Ia_last;
+  int NR, Ne, nw, nwa, nwai;
   double Rc_min, Rc_max, v_min;
   double L0, q1, qz, sigma_r0, DF_const;
   int n_zang;
@@ -343,7 +343,6 @@ int kls_run_orbits(kls_ctx* c) {
   const kls_config& k = c->cfg;
   OrbitParams P{};
   P.NR = c->NR; P.Ne = c->Ne; P.nw = c->nw; P.nwa = c->nwa; P.nwai = c->nwai;
-  P.Ia_last = (c->nwa - 1) * c->nwai;
   P.Rc_min = k.Rc_min; P.Rc_max = k.Rc_max; P.v_min = k.v_min;
   P.L0 = k.L0; P.q1 = k.q1; P.qz = k.q1 - 1.0; P.n_zang = k.n_zang;
   P.sigma_r0 = 1.0 / std::sqrt(k.q1);
