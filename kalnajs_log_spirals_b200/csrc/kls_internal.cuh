@@ -75,7 +75,7 @@ struct alignas(64) kls_tm_model {
   double* part;                // [batch * tiles_a][splits][Npad][128] FP64 partials
   int64_t K_pad;
   unsigned long long wait_ns;
-  int Npad, tiles_a, n_tiles, splits, kb_per_split, nkb_total, chunk, pad;
+  int Npad, tiles_a, n_tiles, splits, kb_per_split, nkb_total, chunk, Nc;
 };
 
 // One work item of the persistent contraction: FP64 form (model, omega z,

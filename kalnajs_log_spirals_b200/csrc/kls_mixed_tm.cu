@@ -78,8 +78,19 @@ size_t tm_smem(int Npad) {
          TM_WSTAGES * TM_WBYTES + 1024;
 }
 
+// Output rows b that are computed: N_alpha rounded up to 32, the step of one MMA's N
+// (M = 256), where one MMA takes them all; two MMAs of equal N leave N_alpha_pad.
+// The rows of the last 64 beyond that are neither loaded nor multiplied; the others'
+// sums are the same bits (contraction of 16 omegas: N_alpha = 90, 96 of 128 rows,
+// 1.02 -> 0.82 ms; 150, 160 of 192, 3.75 -> 3.61; 201, 224 of 256, 17.6 -> 16.5: the
+// wider ones are near the producers' rate as well).
+__host__ __device__ constexpr int tm_cols(int Na, int Npad) {
+  return Npad > 256 || Na <= 64 ? Npad : (Na + 31) / 32 * 32;
+}
+
 struct TmParams {
   int Npad;                 // N_alpha_pad (<= 384, multiple of 64)
+  int Nc;                   // tm_cols
   int tiles_a;              // Npad / 64
   int n_tiles;              // n_omega * tiles_a
   int splits, kb_per_split, nkb_total;
@@ -91,7 +102,7 @@ struct TmParams {
 
 // output row b of the table for accumulator column j (the pair splits each
 // MMA's N columns: the first half from the leader's B rows, the rest from the
-// peer's; CTA c holds table rows [c Npad/2, (c+1) Npad/2))
+// peer's; CTA c holds table rows [c Nc/2, (c+1) Nc/2))
 __device__ __forceinline__ int tm_brow(int j, int Nh, int Nh2) {
   const int nh = j / Nh, jj = j - nh * Nh, h2 = Nh >> 1;
   return jj < h2 ? nh * h2 + jj : Nh2 + nh * h2 + (jj - h2);
@@ -125,12 +136,12 @@ __device__ __forceinline__ void tm_body(const CUtensorMap* tbh, const CUtensorMa
   const int nkb = max(0, min(P.nkb_total, kb0 + P.kb_per_split) - kb0);
   const int CH = P.chunk;
   const int nch = (nkb + CH - 1) / CH;
-  const int Nh2 = P.Npad / 2;                // table rows per CTA
-  const int nmma = P.Npad > 256 ? 2 : 1;     // MMAs along N
+  const int Nh2 = P.Nc / 2;                  // table rows per CTA
+  const int nmma = P.Nc > 256 ? 2 : 1;       // MMAs along N
   const int NA = tm_astages(P.Npad);         // TMEM stages of A
   const uint32_t acol = (uint32_t)(TM_TMEM_COLS - 64 * NA);
-  const int Nh = P.Npad / nmma;              // N of each MMA
-  const int BT = tm_btile(P.Npad), NB = tm_bstages(P.Npad);
+  const int Nh = P.Nc / nmma;                // N of each MMA
+  const int BT = tm_btile(P.Nc), NB = tm_bstages(P.Npad);
   const unsigned long long lim = P.wait_ns;
 
   // B tile (part 0 hi / 1 lo, sub 0 Re rows / 1 Im rows) of B stage s, and
@@ -432,6 +443,7 @@ mixed_tm_multi_kernel(const kls_tm_model* __restrict__ md, const int4* __restric
   tensormap_acquire(&d.ty_l);
   TmParams P;
   P.Npad = d.Npad;
+  P.Nc = d.Nc;
   P.tiles_a = d.tiles_a;
   P.n_tiles = d.n_tiles;
   P.splits = d.splits;
@@ -602,7 +614,7 @@ int kls_tm_create(kls_ctx* c, const void* Xh, const void* Xl, kls_mixed_tm** out
   const cuuint64_t dims[3] = {64, rows, (cuuint64_t)(c->K_pad / 64)};
   const cuuint64_t strides[2] = {64 * sizeof(__nv_bfloat16), rows * 64 * sizeof(__nv_bfloat16)};
   const cuuint32_t estr[3] = {1, 1, 1};
-  const cuuint32_t box_b[3] = {TM_KB, (cuuint32_t)(c->Na_pad / 2), 1};
+  const cuuint32_t box_b[3] = {TM_KB, (cuuint32_t)(tm_cols(c->Na, c->Na_pad) / 2), 1};
   const cuuint32_t box_y[3] = {TM_KB, TM_AB, 1};
   struct { CUtensorMap* m; const void* base; const cuuint32_t* box; } maps[4] = {
       {&t->tb_h, Xh, box_b}, {&t->tb_l, Xl, box_b}, {&t->ty_h, Xh, box_y}, {&t->ty_l, Xl, box_y}};
@@ -670,6 +682,7 @@ int kls_tm_contract(kls_ctx* c, kls_mixed_tm* t, int n, int* d_err, unsigned lon
   KLS_LAUNCHED(c);
   TmParams P{};
   P.Npad = c->Na_pad;
+  P.Nc = tm_cols(c->Na, c->Na_pad);
   P.tiles_a = tiles_a;
   P.n_tiles = n_tiles;
   P.splits = splits;
@@ -694,6 +707,7 @@ void kls_tm_describe(const kls_ctx* c, const kls_mixed_tm* t, unsigned long long
   d->ty_h = t->ty_h;
   d->ty_l = t->ty_l;
   d->Npad = c->Na_pad;
+  d->Nc = tm_cols(c->Na, c->Na_pad);
   d->tiles_a = c->Na_pad / TM_AB;
   d->n_tiles = batch * d->tiles_a;
   d->nkb_total = (int)(c->K_pad / TM_KB);
@@ -704,7 +718,6 @@ void kls_tm_describe(const kls_ctx* c, const kls_mixed_tm* t, unsigned long long
   d->wait_ns = wait_ns;
   d->wt32 = nullptr;
   d->part = nullptr;
-  d->pad = 0;
 }
 
 int kls_tm_multi_launch(cudaStream_t st, const kls_mdesc* d_md, const kls_tm_model* d_tm,
@@ -723,6 +736,7 @@ int kls_tm_multi_launch(cudaStream_t st, const kls_mdesc* d_md, const kls_tm_mod
       const kls_tm_model& d = h_tm[i];
       TmParams P{};
       P.Npad = d.Npad;
+      P.Nc = d.Nc;
       P.tiles_a = d.tiles_a;
       P.n_tiles = d.n_tiles;
       P.splits = d.splits;
