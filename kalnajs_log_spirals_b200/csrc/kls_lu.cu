@@ -685,7 +685,7 @@ int kls_multi_launch_lu(cudaStream_t st, const kls_mdesc* d_md, const int2* d_pa
     int slots = 0;
     size_t smem = 0;
     // one ring size for the class: as many slots as its largest matrix gets
-    slots = lup_slots(max_Na);
+    slots = lup_slots(max_Na, (int64_t)n_pairs * k.C > 148);
     smem = lup_smem(max_Na, slots);
     if ((e = lup_limits(k.multi, k.C)) != cudaSuccess) return (int)e;
     cudaLaunchAttribute at;
