@@ -443,7 +443,9 @@ struct kls_mlp {
   int64_t nparams = 0;
   float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
   std::vector<__nv_bfloat16*> Wb, Wt;
-  // activations for a batch of `cap` rows
+  // activations for a batch of `cap` rows, of a training pass for `tcap`
+  int tcap = 0;
+  void *hslab = nullptr, *tslab = nullptr, *rslab = nullptr;   // their allocations, and X .. idx
   std::vector<float*> Z;                             // pre-activations [cap][dout_pad]
   std::vector<__nv_bfloat16*> H, Ht;                 // H[l]: input of layer l [cap][din_pad]
   __nv_bfloat16 *dZ[2] = {nullptr, nullptr};         // bf16 [cap][width], by turns
@@ -472,58 +474,54 @@ int mfail(kls_mlp* m, const std::string& s) {
     if (e_ != cudaSuccess) return mfail(m, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
-int ensure_cap(kls_mlp* m, int n) {
-  if (n <= m->cap) return KLS_OK;
-  const int cap = ((n + 63) / 64) * 64;
-  m->cap = 0;
-  auto fr = [](auto*& p) {
-    if (p) cudaFree((void*)p);
-    p = nullptr;
-  };
-  for (auto*& z : m->Z) fr(z);
-  for (auto*& h : m->H) fr(h);
-  for (auto*& h : m->Ht) fr(h);
-  for (int q = 0; q < 2; ++q) fr(m->dZ[q]);
-  for (auto*& z : m->dZt) fr(z);
-  for (auto*& z : m->dZf) fr(z);
-  fr(m->lpart);
-  const int L = m->depth;
-  m->Z.assign(L, nullptr);             // layers 0 .. L - 2
-  m->H.assign(L, nullptr);             // inputs of the layers 1 .. L - 1
-  m->Ht.assign(L, nullptr);            // inputs of all layers
-  m->dZt.assign(L, nullptr);
-  m->dZf.assign(L, nullptr);
-  for (int l = 0; l < L; ++l) {
-    if (l < L - 1) ML_CK(m, cudaMalloc(&m->Z[l], (size_t)cap * m->dout_pad[l] * 4));
-    if (l) ML_CK(m, cudaMalloc(&m->H[l], (size_t)cap * m->din_pad[l] * 2));
-    ML_CK(m, cudaMalloc(&m->Ht[l], (size_t)cap * m->din_pad[l] * 2));
-    ML_CK(m, cudaMalloc(&m->dZt[l], (size_t)cap * m->dout_pad[l] * 2));
-    ML_CK(m, cudaMalloc(&m->dZf[l], (size_t)cap * m->dout_pad[l] * 4));
+// activations of n rows; `train`: and all that a training pass leaves
+int ensure_cap(kls_mlp* m, int n, bool train) {
+  const int L = m->depth, cap = ((n + 63) / 64) * 64;
+  if (n > m->cap) {
+    m->cap = 0;
+    cudaFree(m->hslab);
+    KlsSlab b;
+    m->H.assign(L, nullptr);           // inputs of the layers 1 .. L - 1
+    for (int l = 1; l < L; ++l) b.add(&m->H[l], (size_t)cap * m->din_pad[l]);
+    ML_CK(m, b.alloc(&m->hslab));
+    m->cap = cap;
   }
-  for (int q = 0; q < 2; ++q) ML_CK(m, cudaMalloc(&m->dZ[q], (size_t)cap * m->width * 2));
-  ML_CK(m, cudaMalloc(&m->lpart, (size_t)(cap / GT_S) * 4));
-  m->cap = cap;
+  if (train && n > m->tcap) {
+    m->tcap = 0;
+    cudaFree(m->tslab);
+    KlsSlab b;
+    m->Z.assign(L, nullptr);           // layers 0 .. L - 2
+    m->Ht.assign(L, nullptr);          // inputs of all layers
+    m->dZt.assign(L, nullptr);
+    m->dZf.assign(L, nullptr);
+    for (int l = 0; l < L; ++l) {
+      const size_t in = (size_t)cap * m->din_pad[l], out = (size_t)cap * m->dout_pad[l];
+      if (l < L - 1) b.add(&m->Z[l], out);
+      b.add(&m->Ht[l], in).add(&m->dZt[l], out).add(&m->dZf[l], out);
+    }
+    for (int q = 0; q < 2; ++q) b.add(&m->dZ[q], (size_t)cap * m->width);
+    b.add(&m->lpart, (size_t)cap / GT_S);
+    ML_CK(m, b.alloc(&m->tslab));
+    m->tcap = cap;
+  }
   return KLS_OK;
 }
 
 // X, T, Y and the order of n rows; losses of `steps` steps
 int ensure_rows(kls_mlp* m, int n, int steps) {
-  auto fr = [](auto*& p) {
-    if (p) cudaFree((void*)p);
-    p = nullptr;
-  };
   if (n > m->rows) {
     m->rows = 0;
-    fr(m->Xd); fr(m->Td); fr(m->Yd); fr(m->idx);
-    ML_CK(m, cudaMalloc(&m->Xd, (size_t)n * ML_IN * 4));
-    ML_CK(m, cudaMalloc(&m->Td, (size_t)n * ML_OUT * 4));
-    ML_CK(m, cudaMalloc(&m->Yd, (size_t)n * ML_OUT * 4));
-    ML_CK(m, cudaMalloc(&m->idx, (size_t)n * 4));
+    cudaFree(m->rslab);
+    KlsSlab b;
+    b.add(&m->Xd, (size_t)n * ML_IN).add(&m->Td, (size_t)n * ML_OUT);
+    b.add(&m->Yd, (size_t)n * ML_OUT).add(&m->idx, n);
+    ML_CK(m, b.alloc(&m->rslab));
     m->rows = n;
   }
   if (steps > m->steps) {
     m->steps = 0;
-    fr(m->loss);
+    cudaFree(m->loss);
+    m->loss = nullptr;
     ML_CK(m, cudaMalloc(&m->loss, (size_t)steps * 4));
     m->steps = steps;
   }
@@ -582,7 +580,7 @@ int forward(kls_mlp* m, int n, const int* idx, int row0, bool train) {
     g.B = m->Wb[l]; g.ldb = m->din_pad[l];
     // (the last layer's bias covers 3 outputs; the padded ones read zeros behind it)
     g.bias = m->p + m->boff[l];
-    g.ldht = m->cap;
+    g.ldht = m->tcap;
     g.idx = idx;
     if (l == 0) {
       g.X = m->Xd + (size_t)row0 * ML_IN;
@@ -621,8 +619,8 @@ int backward(kls_mlp* m, int n) {
     // dW_l [dout][din] = dZ_l^T (dout x n) * H_l (n x din): A = dZt_l [dout_pad][cap], B = Ht_l
     GemmArgs& w = a.w[l];
     w.M = m->dout[l]; w.N = m->din[l]; w.K = n;
-    w.A = m->dZt[l]; w.lda = m->cap;
-    w.B = m->Ht[l]; w.ldb = m->cap;
+    w.A = m->dZt[l]; w.lda = m->tcap;
+    w.B = m->Ht[l]; w.ldb = m->tcap;
     w.C = m->g + m->woff[l]; w.ldc = m->din[l];
     a.s[l] = {n, m->dout[l], m->dout_pad[l], m->dZf[l], m->g + m->boff[l]};
     if (l == 0) break;
@@ -634,7 +632,7 @@ int backward(kls_mlp* m, int n) {
     h.Zin = m->Z[l - 1]; h.ldz = m->dout_pad[l - 1];
     h.C = m->dZf[l - 1]; h.ldc = m->din_pad[l];
     h.H = m->dZ[q ^ 1]; h.ldh = m->din_pad[l];
-    h.Ht = m->dZt[l - 1]; h.ldht = m->cap;
+    h.Ht = m->dZt[l - 1]; h.ldht = m->tcap;
     int r = gemm<EPI_GELU_BWD>(m, h);
     if (r) return r;
   }
@@ -718,13 +716,7 @@ int kls_mlp_destroy(kls_mlp* m) {
   fr(m->p); fr(m->g); fr(m->m); fr(m->v); fr(m->loss);
   for (auto* x : m->Wb) fr(x);
   for (auto* x : m->Wt) fr(x);
-  for (auto* z : m->Z) fr(z);
-  for (auto* x : m->H) fr(x);
-  for (auto* x : m->Ht) fr(x);
-  for (int q = 0; q < 2; ++q) fr(m->dZ[q]);
-  for (auto* z : m->dZt) fr(z);
-  for (auto* z : m->dZf) fr(z);
-  fr(m->lpart); fr(m->Xd); fr(m->Td); fr(m->Yd); fr(m->idx);
+  fr(m->hslab); fr(m->tslab); fr(m->rslab);
   cudaStreamDestroy(m->stream);
   delete m;
   return KLS_OK;
@@ -760,7 +752,7 @@ int kls_mlp_forward(kls_mlp* m, const float* X, int n, float* Y) {
   const int chunk = 1 << 16;
   for (int s = 0; s < n; s += chunk) {
     int nb = std::min(chunk, n - s);
-    int r = ensure_cap(m, nb);
+    int r = ensure_cap(m, nb, false);
     if (r || (r = ensure_rows(m, nb, 0))) return r;
     ML_CK(m, cudaMemcpyAsync(m->Xd, X + (size_t)s * ML_IN, (size_t)nb * ML_IN * 4,
                              cudaMemcpyHostToDevice, m->stream));
@@ -776,7 +768,7 @@ int kls_mlp_forward(kls_mlp* m, const float* X, int n, float* Y) {
 int kls_mlp_grad(kls_mlp* m, const float* X, const float* T, int n, float* grads, float* loss) {
   if (!m || n < 1 || !X || !T) return KLS_ERR_CONFIG;
   cudaSetDevice(m->device);
-  int r = ensure_cap(m, n);
+  int r = ensure_cap(m, n, true);
   if (r || (r = ensure_rows(m, n, 1))) return r;
   ML_CK(m, cudaMemcpyAsync(m->Xd, X, (size_t)n * ML_IN * 4, cudaMemcpyHostToDevice, m->stream));
   ML_CK(m, cudaMemcpyAsync(m->Td, T, (size_t)n * ML_OUT * 4, cudaMemcpyHostToDevice, m->stream));
@@ -799,7 +791,7 @@ int kls_mlp_train(kls_mlp* m, const float* X, const float* T, int n, int epochs,
   // more, a segment of batches at a time in the epoch's order
   const bool all = n <= ML_ROWS;
   const int seg = all ? n : std::max(1, ML_ROWS / batch) * batch;
-  int r = ensure_cap(m, batch);
+  int r = ensure_cap(m, batch, true);
   if (r || (r = ensure_rows(m, seg, steps))) return r;
   int tiles_w = 1;                                       // blocks of the update, per layer
   for (int l = 0; l < m->depth; ++l)
