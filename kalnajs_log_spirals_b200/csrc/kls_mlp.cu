@@ -441,6 +441,7 @@ struct kls_mlp {
   std::vector<int> din, dout, din_pad, dout_pad;    // per layer
   std::vector<int64_t> woff, boff;                  // offsets into the flat fp32 params
   int64_t nparams = 0;
+  void* pslab = nullptr;                            // the allocation of p .. Wt
   float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
   std::vector<__nv_bfloat16*> Wb, Wt;
   // activations for a batch of `cap` rows, of a training pass for `tcap`
@@ -683,27 +684,30 @@ int kls_mlp_create(int device, int width, int depth, uint64_t seed, kls_mlp** ou
     for (int64_t i = 0; i < (int64_t)m->din[l] * m->dout[l]; ++i) h[m->woff[l] + i] = U(rng);
     for (int i = 0; i < m->dout[l]; ++i) h[m->boff[l] + i] = U(rng);
   }
+  KlsSlab b;
+  b.add(&m->p, alloc).add(&m->g, alloc).add(&m->m, alloc).add(&m->v, alloc);
+  m->Wb.assign(depth, nullptr);
+  m->Wt.assign(depth, nullptr);
+  for (int l = 0; l < depth; ++l) {
+    const size_t n = (size_t)m->dout_pad[l] * m->din_pad[l];
+    b.add(&m->Wb[l], n).add(&m->Wt[l], n);
+  }
   if (cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaMalloc(&m->p, alloc * 4) != cudaSuccess || cudaMalloc(&m->g, alloc * 4) != cudaSuccess ||
-      cudaMalloc(&m->m, alloc * 4) != cudaSuccess || cudaMalloc(&m->v, alloc * 4) != cudaSuccess) {
-    delete m;
+      b.alloc(&m->pslab) != cudaSuccess) {
+    kls_mlp_destroy(m);
     return kls_fail(nullptr, KLS_ERR_OOM, "kls_mlp_create: device allocation failed");
   }
-  cudaMemcpy(m->p, h.data(), alloc * 4, cudaMemcpyHostToDevice);
-  cudaMemset(m->g, 0, alloc * 4);
-  cudaMemset(m->m, 0, alloc * 4);
-  cudaMemset(m->v, 0, alloc * 4);
-  for (int l = 0; l < depth; ++l) {
-    __nv_bfloat16 *a = nullptr, *b = nullptr;
-    size_t n = (size_t)m->dout_pad[l] * m->din_pad[l];
-    if (cudaMalloc(&a, n * 2) != cudaSuccess || cudaMalloc(&b, n * 2) != cudaSuccess)
-      return kls_fail(nullptr, KLS_ERR_OOM, "kls_mlp_create: device allocation failed");
-    m->Wb.push_back(a); m->Wt.push_back(b);
-  }
+  cudaMemcpyAsync(m->p, h.data(), alloc * 4, cudaMemcpyHostToDevice, m->stream);
+  cudaMemsetAsync(m->g, 0, alloc * 4, m->stream);
+  cudaMemsetAsync(m->m, 0, alloc * 4, m->stream);
+  cudaMemsetAsync(m->v, 0, alloc * 4, m->stream);
   int r = pack_all(m);
-  if (r) return r;
-  if (cudaStreamSynchronize(m->stream) != cudaSuccess)
-    return kls_fail(nullptr, KLS_ERR_CUDA, "kls_mlp_create: init failed");
+  if (!r && cudaStreamSynchronize(m->stream) != cudaSuccess)
+    r = kls_fail(nullptr, KLS_ERR_CUDA, "kls_mlp_create: init failed");
+  if (r) {
+    kls_mlp_destroy(m);
+    return r;
+  }
   *out = m;
   return KLS_OK;
 }
@@ -711,13 +715,9 @@ int kls_mlp_create(int device, int width, int depth, uint64_t seed, kls_mlp** ou
 int kls_mlp_destroy(kls_mlp* m) {
   if (!m) return KLS_OK;
   cudaSetDevice(m->device);
-  cudaStreamSynchronize(m->stream);
-  auto fr = [](void* p) { if (p) cudaFree(p); };
-  fr(m->p); fr(m->g); fr(m->m); fr(m->v); fr(m->loss);
-  for (auto* x : m->Wb) fr(x);
-  for (auto* x : m->Wt) fr(x);
-  fr(m->hslab); fr(m->tslab); fr(m->rslab);
-  cudaStreamDestroy(m->stream);
+  if (m->stream) cudaStreamSynchronize(m->stream);
+  for (void* x : {m->pslab, m->hslab, m->tslab, m->rslab, (void*)m->loss}) cudaFree(x);
+  if (m->stream) cudaStreamDestroy(m->stream);
   delete m;
   return KLS_OK;
 }
