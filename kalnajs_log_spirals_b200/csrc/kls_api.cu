@@ -418,6 +418,14 @@ int kls_release_fp64(kls_ctx* c) {
   KLS_CK(c, cudaStreamSynchronize(c->stream));
   kls_drop_table(c);
   kls_similar_free(c);
+  // what only FP64 evaluations use
+  for (void* p : {c->d_F, (void*)c->d_part, (void*)c->d_items, (void*)c->d_tiles}) dfree(p);
+  c->d_F = nullptr;
+  c->d_part = nullptr;
+  c->d_items = nullptr;
+  c->d_tiles = nullptr;
+  c->F_bytes = c->part_elems = 0;
+  c->plan_splits = 0;
   c->fp64_released = true;
   return KLS_OK;
 }

@@ -342,6 +342,12 @@ int replay(kls_multi* m) {
 int run_omegas(kls_multi* m, const std::function<void(int, int, double*)>& fill, int n,
                double* det_ri, double* log_abs) {
   const int B = m->batch;
+  // the graph holds the addresses of the models' FP64 form
+  if (m->mode == KLS_MODE_FP64)
+    for (int i = 0; i < m->n_models; ++i)
+      if (m->ctx[i]->fp64_released)
+        return mfail(m, KLS_ERR_STATE, "model " + std::to_string(i) +
+                                           ": the FP64 table was released (kls_release_fp64)");
   for (int b0 = 0; b0 < n; b0 += B) {
     const int nb = std::min(B, n - b0);
     for (int i = 0; i < m->n_models; ++i) {
