@@ -1176,14 +1176,16 @@ int kls_set_fault_injection(kls_ctx* c, int mode) {
     if (!c->gk0_poisoned) {
       KLS_CK(c, cudaMemcpy(&c->gk0_saved, c->d_Gk, sizeof(double), cudaMemcpyDeviceToHost));
       const double nan = NAN;
-      KLS_CK(c, cudaMemcpy(c->d_Gk, &nan, sizeof(double), cudaMemcpyHostToDevice));
+      KLS_CK(c, cudaMemcpyAsync(c->d_Gk, &nan, sizeof(double), cudaMemcpyHostToDevice, c->stream));
+      KLS_CK(c, cudaStreamSynchronize(c->stream));
       c->gk0_poisoned = true;
     }
     return KLS_OK;
   }
   if (mode == KLS_FAULT_NONE) {
     if (c->gk0_poisoned) {
-      KLS_CK(c, cudaMemcpy(c->d_Gk, &c->gk0_saved, sizeof(double), cudaMemcpyHostToDevice));
+      KLS_CK(c, cudaMemcpyAsync(c->d_Gk, &c->gk0_saved, sizeof(double), cudaMemcpyHostToDevice,
+                                c->stream));
       c->gk0_poisoned = false;
     }
     return c->mixed ? kls_mixed_set_wait(c, 0, KLS_FAULT_NONE) : KLS_OK;

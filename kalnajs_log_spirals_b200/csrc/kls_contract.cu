@@ -584,10 +584,11 @@ int kls_f64_plan(kls_ctx* c) {
   c->plan_splits = 0;
   KLS_CK(c, cudaMalloc(&c->d_items, items.size() * sizeof(int4)));
   KLS_CK(c, cudaMalloc(&c->d_tiles, tiles.size() * sizeof(int2)));
-  KLS_CK(c, cudaMemcpy(c->d_items, items.data(), items.size() * sizeof(int4),
-                       cudaMemcpyHostToDevice));
-  KLS_CK(c, cudaMemcpy(c->d_tiles, tiles.data(), tiles.size() * sizeof(int2),
-                       cudaMemcpyHostToDevice));
+  KLS_CK(c, cudaMemcpyAsync(c->d_items, items.data(), items.size() * sizeof(int4),
+                            cudaMemcpyHostToDevice, c->stream));
+  KLS_CK(c, cudaMemcpyAsync(c->d_tiles, tiles.data(), tiles.size() * sizeof(int2),
+                            cudaMemcpyHostToDevice, c->stream));
+  KLS_CK(c, cudaStreamSynchronize(c->stream));   // an uneven batch copies them on its own stream
   c->items.swap(items);
   c->n_slots = slot;
   c->plan_splits = c->splits;

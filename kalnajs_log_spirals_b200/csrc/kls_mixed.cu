@@ -1336,7 +1336,7 @@ int kls_mixed_check(kls_ctx* c) {
   int h = 0;
   KLS_CK(c, cudaMemcpy(&h, c->mixed->err, sizeof(int), cudaMemcpyDeviceToHost));
   if (h) {
-    cudaMemset(c->mixed->err, 0, sizeof(int));
+    cudaMemsetAsync(c->mixed->err, 0, sizeof(int), c->stream);
     return kls_fail(c, KLS_ERR_TIMEOUT,
                     "mixed contraction pipeline: a bounded wait ran out (code " +
                         std::to_string(h) + "); results of this call are invalid");

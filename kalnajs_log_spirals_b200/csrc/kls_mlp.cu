@@ -738,7 +738,7 @@ int kls_mlp_get_params(kls_mlp* m, float* params) {
 int kls_mlp_set_params(kls_mlp* m, const float* params) {
   if (!m || !params) return KLS_ERR_CONFIG;
   cudaSetDevice(m->device);
-  ML_CK(m, cudaMemcpy(m->p, params, m->nparams * 4, cudaMemcpyHostToDevice));
+  ML_CK(m, cudaMemcpyAsync(m->p, params, m->nparams * 4, cudaMemcpyHostToDevice, m->stream));
   int r = pack_all(m);
   if (r) return r;
   ML_CK(m, cudaStreamSynchronize(m->stream));

@@ -123,6 +123,14 @@ int malloc_buf(kls_multi* m, T** p, size_t count) {
   return KLS_OK;
 }
 
+// The batch's stream does not wait for the default one, on which a synchronous copy
+// from pageable memory (or between device buffers) may still be under way when the
+// call returns: what the batch's kernels read is copied on their stream.
+template <typename T>
+cudaError_t upload(kls_multi* m, T* dst, const std::vector<T>& v) {
+  return cudaMemcpyAsync(dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, m->stream);
+}
+
 // mixed items: effective K splits so that every split owns >= 1 k-block
 constexpr int MIX_BK = 64, MIX_BM = 128, MIX_AB = 64;
 
@@ -222,10 +230,7 @@ int schedule_items(kls_multi* m, int policy) {
     m->grid = std::max(1, n);
   }
   m->schedule = policy;
-  if (cudaMemcpy(m->d_items, m->items.data(), m->items.size() * sizeof(kls_item),
-                 cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(m->d_starts, m->starts.data(), m->starts.size() * sizeof(int),
-                 cudaMemcpyHostToDevice) != cudaSuccess)
+  if (upload(m, m->d_items, m->items) || upload(m, m->d_starts, m->starts))
     return mcuda(m, cudaGetLastError(), "cudaMemcpy (schedule)");
   return KLS_OK;
 }
@@ -439,7 +444,7 @@ int kls_multi_create(kls_ctx* const* models, int n_models, int mode, int batch, 
     return bail(mcuda(m, cudaErrorMemoryAllocation, "cudaMallocHost"));
   *m->h_err = 0;
   std::fill(m->h_omega, m->h_omega + 2 * nz, 0.0);
-  if (cudaMemset(m->d_err, 0, sizeof(int)) != cudaSuccess)
+  if (cudaMemsetAsync(m->d_err, 0, sizeof(int), m->stream) != cudaSuccess)
     return bail(mcuda(m, cudaGetLastError(), "cudaMemset"));
 
   m->md.resize(n_models);
@@ -492,7 +497,8 @@ int kls_multi_create(kls_ctx* const* models, int n_models, int mode, int batch, 
       if ((r = malloc_buf(m, &tiles, nt)) ||
           (r = malloc_buf(m, &d.part, kls_f64_part_elems(c, batch))))
         return bail(r);
-      if (cudaMemcpy(tiles, c->d_tiles, nt * sizeof(int2), cudaMemcpyDeviceToDevice) != cudaSuccess)
+      if (cudaMemcpyAsync(tiles, c->d_tiles, nt * sizeof(int2), cudaMemcpyDeviceToDevice,
+                          m->stream) != cudaSuccess)
         return bail(mcuda(m, cudaGetLastError(), "cudaMemcpy (slot table)"));
       d.tiles = tiles;
       m->max_ldv = std::max(m->max_ldv, c->ldv);
@@ -525,9 +531,10 @@ int kls_multi_create(kls_ctx* const* models, int n_models, int mode, int batch, 
       d.Xh = kls_mixed_tables(c, &xl, &th, &tl);
       d.Xl = xl;
       uint8_t* dm = m->d_tmaps + (size_t)2 * i * sizeof(CUtensorMap);
-      if (cudaMemcpy(dm, th, sizeof(CUtensorMap), cudaMemcpyHostToDevice) != cudaSuccess ||
-          cudaMemcpy(dm + sizeof(CUtensorMap), tl, sizeof(CUtensorMap),
-                     cudaMemcpyHostToDevice) != cudaSuccess)
+      if (cudaMemcpyAsync(dm, th, sizeof(CUtensorMap), cudaMemcpyHostToDevice, m->stream) !=
+              cudaSuccess ||
+          cudaMemcpyAsync(dm + sizeof(CUtensorMap), tl, sizeof(CUtensorMap),
+                          cudaMemcpyHostToDevice, m->stream) != cudaSuccess)
         return bail(mcuda(m, cudaGetLastError(), "cudaMemcpy (tensor maps)"));
       d.tmap_h = dm;
       d.tmap_l = dm + sizeof(CUtensorMap);
@@ -554,10 +561,7 @@ int kls_multi_create(kls_ctx* const* models, int n_models, int mode, int batch, 
     if ((r = malloc_buf(m, &m->d_tm, m->tmd.size())) ||
         (r = malloc_buf(m, &m->d_tm_items, m->tm_items.size())))
       return bail(r);
-    if (cudaMemcpy(m->d_tm, m->tmd.data(), m->tmd.size() * sizeof(kls_tm_model),
-                   cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(m->d_tm_items, m->tm_items.data(), m->tm_items.size() * sizeof(int4),
-                   cudaMemcpyHostToDevice) != cudaSuccess)
+    if (upload(m, m->d_tm, m->tmd) || upload(m, m->d_tm_items, m->tm_items))
       return bail(mcuda(m, cudaGetLastError(), "cudaMemcpy (TMEM-form descriptors)"));
   }
   if (F_bytes) {
@@ -588,22 +592,14 @@ int kls_multi_create(kls_ctx* const* models, int n_models, int mode, int batch, 
       }
     if (g.count) m->lu.push_back(g);
   }
-  if (cudaMemcpy(m->d_pairs_lu, by_class.data(), by_class.size() * sizeof(int2),
-                 cudaMemcpyHostToDevice))
+  if (upload(m, m->d_pairs_lu, by_class))
     return bail(mcuda(m, cudaGetLastError(), "cudaMemcpy (pairs)"));
-  if (cudaMemcpy(m->d_md, m->md.data(), m->md.size() * sizeof(kls_mdesc), cudaMemcpyHostToDevice) ||
-      cudaMemcpy(m->d_pairs, m->pairs.data(), m->pairs.size() * sizeof(int2),
-                 cudaMemcpyHostToDevice) ||
-      cudaMemcpy(m->d_pairs_tab, m->pairs_tab.data(), m->pairs_tab.size() * sizeof(int2),
-                 cudaMemcpyHostToDevice) ||
-      cudaMemcpy(m->d_pairs_tm, m->pairs_tm.data(), m->pairs_tm.size() * sizeof(int2),
-                 cudaMemcpyHostToDevice) ||
-      cudaMemcpy(m->d_pairs_old, m->pairs_old.data(), m->pairs_old.size() * sizeof(int2),
-                 cudaMemcpyHostToDevice))
+  if (upload(m, m->d_md, m->md) || upload(m, m->d_pairs, m->pairs) ||
+      upload(m, m->d_pairs_tab, m->pairs_tab) || upload(m, m->d_pairs_tm, m->pairs_tm) ||
+      upload(m, m->d_pairs_old, m->pairs_old))
     return bail(mcuda(m, cudaGetLastError(), "cudaMemcpy (descriptors)"));
   if (mode == KLS_MODE_FP64) {
-    if (cudaMemcpy(m->d_items, m->items.data(), m->items.size() * sizeof(kls_item),
-                   cudaMemcpyHostToDevice) != cudaSuccess)
+    if (upload(m, m->d_items, m->items))
       return bail(mcuda(m, cudaGetLastError(), "cudaMemcpy (items)"));
     if ((r = eager_pass(m, nullptr))) return bail(r);
   } else {

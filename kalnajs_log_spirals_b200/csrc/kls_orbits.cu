@@ -408,7 +408,10 @@ int kls_upload_alpha(kls_ctx* c) {
       c->cfg.quad_alpha == KLS_QUAD_DEFAULT ? KLS_QUAD_TRAPEZOID : c->cfg.quad_alpha;
   auto x = [&](int i) { return a[i]; };
   for (int i = 0; i < c->Na; ++i) d[i] = quad_w(rule, x, i, c->Na);
-  KLS_CK(c, cudaMemcpy(c->d_alpha, a.data(), c->Na * sizeof(double), cudaMemcpyHostToDevice));
-  KLS_CK(c, cudaMemcpy(c->d_dalpha, d.data(), c->Na * sizeof(double), cudaMemcpyHostToDevice));
+  KLS_CK(c, cudaMemcpyAsync(c->d_alpha, a.data(), c->Na * sizeof(double), cudaMemcpyHostToDevice,
+                            c->stream));
+  KLS_CK(c, cudaMemcpyAsync(c->d_dalpha, d.data(), c->Na * sizeof(double), cudaMemcpyHostToDevice,
+                            c->stream));
+  KLS_CK(c, cudaStreamSynchronize(c->stream));   // (a, d end here)
   return KLS_OK;
 }
