@@ -12,6 +12,7 @@
 // registers, columns passed from warp to warp; lu_det_kernel: one CTA per
 // matrix through L2, any N.  Both return the same bits.
 #include "kls_internal.cuh"
+#include "kls_lu_cols.h"
 #include "kls_tcgen05.cuh"
 #include <algorithm>
 #include <cfloat>
@@ -200,8 +201,8 @@ multi_lu_kernel(const kls_mdesc* __restrict__ md, const int2* __restrict__ pairs
 //    warps run as a pipeline over the columns without a block or cluster
 //    barrier: a column goes to a ring in the shared memory of every CTA of the
 //    cluster and one mbarrier per slot announces it;
-//  * 8 consecutive columns are on one CTA (its warps in turn), so most hand-overs
-//    stay inside an SM.
+//  * 8 consecutive columns are on one CTA (kls_lu_cols.h), so most hand-overs stay
+//    inside an SM.
 // A slot is written again only when every warp has used it: each warp keeps a
 // count of the columns it is done with, and the owner of every (slots / 2)-th
 // column waits for all of them.
@@ -214,7 +215,7 @@ multi_lu_kernel(const kls_mdesc* __restrict__ md, const int2* __restrict__ pairs
 // pivot search with its reciprocal 670 / 1260, broadcast 60 / 80, multipliers and
 // publication 440 / 1100; the marks themselves are some 50 each): about 350
 // instructions that depend on one another.
-constexpr int LUP_WARPS = 8, LUP_THREADS = 32 * LUP_WARPS;
+constexpr int LUP_THREADS = 32 * LUP_WARPS;
 constexpr unsigned long long LUP_LIMIT_NS = 2000000000ull;
 
 struct LupMeta {
@@ -319,10 +320,7 @@ __device__ __forceinline__ void lup_body(int n, int slots, const double2* __rest
   if (tid == 0) { s_abort = 0; s_failed = 0; }
   for (int s = tid; s < slots; s += LUP_THREADS) mbar_init(smem_u32(full + s), 1);
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  // global index of local column lp
-  auto col_of = [&](int lp) {
-    return (lp * (int)C + (int)rank) * LUP_WARPS + warp;
-  };
+  LupCols own(n, (int)C, (int)rank, warp, LP);
   double2 a[LP][RPL];
   int pos[RPL];
 #pragma unroll
@@ -331,7 +329,7 @@ __device__ __forceinline__ void lup_body(int n, int slots, const double2* __rest
     pos[r] = i < n ? i : -1;
 #pragma unroll
     for (int lp = 0; lp < LP; ++lp) {
-      const int g = col_of(lp);
+      const int g = own.col(lp);
       a[lp][r] = make_double2(0.0, 0.0);
       if (i < n && g < n) KLS_IF(LU_IN(i, g)) a[lp][r] = A[(size_t)i * n + g];
     }
@@ -448,29 +446,24 @@ __device__ __forceinline__ void lup_body(int n, int slots, const double2* __rest
 
   const bool keeper = rank == 0 && warp == 0;  // multiplies the pivots up, in order
   LuDet acc;
-  // a[0] is the warp's next column (index `next`), a[1 .. left - 1] those after it
-  int done = 0, left = 0, last = -1, next = col_of(0);
-#pragma unroll
-  for (int lp = 0; lp < LP; ++lp)
-    if (col_of(lp) < n) { last = col_of(lp); ++left; }
+  // a[0] is the warp's next column (index own.next), a[1 .. left - 1] those after it
   auto shift = [&]() {
 #pragma unroll
     for (int lp = 0; lp + 1 < LP; ++lp)
 #pragma unroll
       for (int r = 0; r < RPL; ++r) a[lp][r] = a[lp + 1][r];
-    ++done;
-    --left;
-    next = left ? col_of(done) : n;
+    own.taken();
   };
-  if (next == 0) {
+  if (own.next == 0) {
     factor(a[0], 0, 0);
     shift();
   }
-  const int until = keeper ? n : last;         // columns this warp has to take in
+  const int until = keeper ? n : own.last;     // columns this warp has to take in
   int j = 0, s = 0;                            // column j is in slot s
   uint32_t parity = 0;
   for (; j < until; ++j) {
-    const bool ok = lup_wait(smem_u32(full + s), parity, &s_abort, next == j + 1);
+    const bool ok = lup_wait(smem_u32(full + s), parity, &s_abort,
+                             own.next == j + 1 || j + 1 == until);
     if (!__all_sync(0xffffffffu, ok)) break;
     const LupMeta mt = meta[s];
 #pragma unroll
@@ -479,26 +472,26 @@ __device__ __forceinline__ void lup_body(int n, int slots, const double2* __rest
       pos[r] = here ? j : pos[r] == j ? mt.pos : pos[r];
     }
     const double2* slot = ring + (size_t)s * n;
-    if (next == j + 1) {                       // the chain: this column is wanted next
+    if (own.next == j + 1) {                   // the chain: this column is wanted next
       const double2 u = lup_row<RPL>(a[0], mt.piv);
 #pragma unroll
       for (int r = 0; r < RPL; ++r)
         if (lane + 32 * r < n) a[0][r] = lu_update(a[0][r], slot[lane + 32 * r], u);
-      factor(a[0], next, s + 1 < slots ? s + 1 : 0);
+      factor(a[0], own.next, s + 1 < slots ? s + 1 : 0);
       shift();
     }
-    if (left) {
+    if (own.left) {
       double2 u[LP];
 #pragma unroll
       for (int lp = 0; lp < LP; ++lp)
-        if (lp < left) u[lp] = lup_row<RPL>(a[lp], mt.piv);
+        if (lp < own.left) u[lp] = lup_row<RPL>(a[lp], mt.piv);
 #pragma unroll
       for (int r = 0; r < RPL; ++r) {
         if (lane + 32 * r >= n) continue;
         const double2 l = slot[lane + 32 * r];
 #pragma unroll
         for (int lp = 0; lp < LP; ++lp)
-          if (lp < left) a[lp][r] = lu_update(a[lp][r], l, u[lp]);
+          if (lp < own.left) a[lp][r] = lu_update(a[lp][r], l, u[lp]);
       }
     }
     if (keeper) acc.times(mt.u, mt.pos != j);
