@@ -40,8 +40,9 @@ extern "C" {
 #define KLS_ERR_SINGULAR     6  /* singular 2x2 Newton Jacobian               */
 #define KLS_ERR_UNSUPPORTED  7  /* mode not available on this device          */
 #define KLS_ERR_TIMEOUT      8  /* a bounded device-side wait ran out: the
-                                   contraction pipeline stalled; the call's
-                                   results are invalid, the context stays usable */
+                                   contraction pipeline or the LU stalled; the
+                                   call's results are invalid, the context stays
+                                   usable                                       */
 
 /* ---- precision modes of the contraction -------------------------------- */
 #define KLS_MODE_FP64        0  /* plain FP64 (the oracle form)               */
@@ -425,22 +426,28 @@ int kls_set_mixed_chunk(kls_ctx* ctx, int k_blocks);
 
 /* ---- failure handling of the device pipeline (no reference counterpart) --- *
  * Every wait of the KLS_MIXED_TMEM contraction (on a copy, an MMA or another
- * warp) is bounded by this limit (default 2 s; the older mixed forms keep a
- * fixed 2 s).  A wait that runs out makes the call return KLS_ERR_TIMEOUT
- * instead of hanging the GPU; the context stays usable.                     */
+ * warp) and of the cluster LU (on a column) is bounded by this limit (default
+ * 2 s; the older mixed forms keep a fixed 2 s; an uneven batch takes the longest
+ * of its models' at its creation).  A wait that runs out makes the call return
+ * KLS_ERR_TIMEOUT instead of hanging the GPU; the context stays usable.  The LU
+ * leaves NaN in the determinant; kls_det_batch_device, which does not wait,
+ * reports it in the next determinant call on the context.                    */
 int kls_set_wait_limit(kls_ctx* ctx, double seconds);
 /* Test hooks for the failure paths (no trap, no fault, no unbounded wait):
  * KLS_FAULT_SKIP_ARRIVAL makes the next KLS_MIXED_TMEM contraction skip one
  * producer warp's "operand ready" arrival in its first CTA pair, so the MMA
  * warp's bounded wait runs out and the call returns KLS_ERR_TIMEOUT; it
- * clears itself after that launch.  KLS_FAULT_NAN_ROW writes NaN into the
+ * clears itself after that launch.  KLS_FAULT_LU_COLUMN makes the next cluster LU
+ * (a context's, or that of the first pass of an uneven batch with it) announce one
+ * column to nobody, so its waits run out likewise.  KLS_FAULT_NAN_ROW writes NaN into the
  * device weight numerator G_k = DJ F0l of the first table row, so every
  * determinant is NaN and host-buffer calls (kls_det_batch, kls_scan,
- * kls_newton, ...) return KLS_ERR_NONFINITE.  KLS_FAULT_NONE clears both and
+ * kls_newton, ...) return KLS_ERR_NONFINITE.  KLS_FAULT_NONE clears them and
  * restores the row.                                                        */
 #define KLS_FAULT_NONE          0
 #define KLS_FAULT_SKIP_ARRIVAL  1
 #define KLS_FAULT_NAN_ROW       2
+#define KLS_FAULT_LU_COLUMN     4
 int kls_set_fault_injection(kls_ctx* ctx, int mode);
 
 /* ---- instrumentation ----------------------------------------------------- */

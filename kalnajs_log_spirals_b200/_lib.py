@@ -43,6 +43,7 @@ KLS_MIXED_TMEM = 3
 KLS_FAULT_NONE = 0
 KLS_FAULT_SKIP_ARRIVAL = 1
 KLS_FAULT_NAN_ROW = 2
+KLS_FAULT_LU_COLUMN = 4
 
 KLS_LU_AUTO = 0
 KLS_LU_CTA = 1

@@ -179,8 +179,6 @@ struct kls_ctx {
   double anchor_w[2] = {0.0, 0.0};
   double2* d_det = nullptr;   // [ws_omega]
   double* d_logabs = nullptr; // [ws_omega]
-  double* h_pinned = nullptr; // pinned staging for omegas/dets
-  int h_pinned_cap = 0;
 
   kls_mixed* mixed = nullptr;
 
@@ -193,6 +191,9 @@ struct kls_ctx {
   int lu_mode = 0;
   int lu_class = -2;
   bool lu_wide = false;       // the class's wider form fits as well
+  int* h_lu_err = nullptr;    // pinned: a wait of the pipelined LU ran out
+  unsigned long long lu_wait_ns = 2000000000ull;
+  int lu_skip = -1;           // test hook (one-shot): the column that is not announced
 
   // instrumentation
   int64_t launches = 0;
@@ -234,6 +235,15 @@ __host__ __device__ inline double kls_lin(double a, double b, int n, int i) {
   return a + (double)i * step;
 }
 
+// Waits of the pipelined LU: their bound, where one that ran out is noted, and the test
+// hook's column (-1: none)
+constexpr int KLS_LU_TIMED_OUT = 1000;
+struct KlsLuWait {
+  unsigned long long ns;
+  int* err;
+  int skip;
+};
+
 // ---- stage entry points (host side, launch on ctx->stream) ---------------
 size_t kls_orbit_table(int nw, int nwai);   // entries of d_cs
 int kls_run_orbits(kls_ctx* c);
@@ -273,7 +283,7 @@ int kls_multi_launch_f64(cudaStream_t st, const kls_mdesc* d_md, const int2* d_p
                          const kls_item* d_items, int n_items, int* d_counter, int grid,
                          int max_ldv);
 int kls_multi_launch_lu(cudaStream_t st, const kls_mdesc* d_md, const int2* d_pairs, int n_pairs,
-                        int max_Na, int cls);
+                        int max_Na, int cls, const KlsLuWait& wait);
 int kls_lu_class(int device, int n);
 int kls_lu_classes();
 int kls_multi_launch_f64_weights(cudaStream_t st, const kls_mdesc* d_md, const int2* d_pairs,

@@ -206,7 +206,8 @@ multi_lu_kernel(const kls_mdesc* __restrict__ md, const int2* __restrict__ pairs
 // A slot is written again only when every warp has used it: each warp keeps a
 // count of the columns it is done with, and the owner of every (slots / 2)-th
 // column waits for all of them.
-// Waits are bounded (LUP_LIMIT_NS); one that runs out makes the determinant NaN.
+// Waits are bounded (KlsLuWait); one that runs out makes the determinant NaN and is
+// noted in an error word, which the host turns into KLS_ERR_TIMEOUT.
 //
 // Measured (1 matrix, B200): N = 101 312 -> 99 us, 201 557 -> 266 us, 301 1022 ->
 // 558 us against one CTA (101) or a cluster with one barrier per column; 16
@@ -216,7 +217,6 @@ multi_lu_kernel(const kls_mdesc* __restrict__ md, const int2* __restrict__ pairs
 // publication 440 / 1100; the marks themselves are some 50 each): about 350
 // instructions that depend on one another.
 constexpr int LUP_THREADS = 32 * LUP_WARPS;
-constexpr unsigned long long LUP_LIMIT_NS = 2000000000ull;
 
 struct LupMeta {
   double2 u;                  // pivot
@@ -249,7 +249,7 @@ __device__ __forceinline__ void st_release_cluster(uint32_t addr, int v) {
 // column is next polls for a while, as it wakes up the sooner (N = 301 576 -> 556
 // us, 16 matrices of 201 374 -> 352).
 __device__ __forceinline__ bool lup_wait(uint32_t bar, uint32_t parity, volatile int* abort,
-                                         bool poll) {
+                                         bool poll, unsigned long long limit) {
   for (int it = 0; poll && it < 200; ++it) {
     uint32_t ok;
     asm volatile(
@@ -276,7 +276,7 @@ __device__ __forceinline__ bool lup_wait(uint32_t bar, uint32_t parity, volatile
     if ((it & 15) == 15) {
       const unsigned long long t = kls_tc::globaltimer();
       if (!t0) t0 = t;
-      else if (t - t0 > LUP_LIMIT_NS) {
+      else if (t - t0 > limit) {
         *abort = 1;
         return false;
       }
@@ -304,7 +304,7 @@ __host__ __device__ inline size_t lup_smem(int n, int slots) {
 template <int RPL, int LP>
 __device__ __forceinline__ void lup_body(int n, int slots, const double2* __restrict__ A,
                                          double2* __restrict__ det, double* __restrict__ logabs,
-                                         unsigned char* smem) {
+                                         unsigned char* smem, const KlsLuWait& wait) {
   using namespace kls_tc;
   __shared__ int prog[LUP_WARPS];             // columns each warp is done with
   __shared__ volatile int s_abort;
@@ -409,7 +409,7 @@ __device__ __forceinline__ void lup_body(int n, int slots, const double2* __rest
           if ((it & 63) == 63) {
             const unsigned long long t = globaltimer();
             if (!t0) t0 = t;
-            else if (t - t0 > LUP_LIMIT_NS) { s_abort = 1; break; }
+            else if (t - t0 > wait.ns) { s_abort = 1; break; }
           }
         }
       }
@@ -424,7 +424,7 @@ __device__ __forceinline__ void lup_body(int n, int slots, const double2* __rest
     }
     if (lane == 0) { meta[s].u = u; meta[s].piv = piv; meta[s].pos = q; }
     __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(full + s));
+    if (lane == 0 && g != wait.skip) mbar_arrive(smem_u32(full + s));
     // the other CTAs, the next one first.  One CTA at a time: the release waits
     // for its stores, so the SM's path to the cluster never fills up with
     // stores that the other warps' shared-memory accesses would queue behind.
@@ -440,7 +440,7 @@ __device__ __forceinline__ void lup_body(int n, int slots, const double2* __rest
         st_cluster_v2i(mb + 16, piv, q);
       }
       __syncwarp();
-      if (lane == 0) arrive_cluster(mapa_u32(smem_u32(full + s), to));
+      if (lane == 0 && g != wait.skip) arrive_cluster(mapa_u32(smem_u32(full + s), to));
     }
   };
 
@@ -463,7 +463,7 @@ __device__ __forceinline__ void lup_body(int n, int slots, const double2* __rest
   uint32_t parity = 0;
   for (; j < until; ++j) {
     const bool ok = lup_wait(smem_u32(full + s), parity, &s_abort,
-                             own.next == j + 1 || j + 1 == until);
+                             own.next == j + 1 || j + 1 == until, wait.ns);
     if (!__all_sync(0xffffffffu, ok)) break;
     const LupMeta mt = meta[s];
 #pragma unroll
@@ -512,7 +512,10 @@ __device__ __forceinline__ void lup_body(int n, int slots, const double2* __rest
   __syncwarp();
   cluster_sync_all();                          // nobody leaves while others write here
   if (keeper && lane == 0) {
-    if (s_failed) acc.mant = make_double2(NAN, NAN);
+    if (s_failed) {
+      acc.mant = make_double2(NAN, NAN);
+      *(volatile int*)wait.err = KLS_LU_TIMED_OUT;
+    }
     acc.store(det, logabs);
   }
 }
@@ -520,23 +523,24 @@ __device__ __forceinline__ void lup_body(int n, int slots, const double2* __rest
 template <int RPL, int LP>
 __global__ void __launch_bounds__(LUP_THREADS)
 lu_pipe_kernel(int n, int slots, int C, const double2* __restrict__ Aall,
-               double2* __restrict__ det_out, double* __restrict__ logabs_out) {
+               double2* __restrict__ det_out, double* __restrict__ logabs_out,
+               const __grid_constant__ KlsLuWait wait) {
   extern __shared__ __align__(16) unsigned char lsm[];
   const int m = blockIdx.x / C;
   lup_body<RPL, LP>(n, slots, Aall + (size_t)m * n * n, det_out + m,
-                        logabs_out ? logabs_out + m : nullptr, lsm);
+                    logabs_out ? logabs_out + m : nullptr, lsm, wait);
 }
 
 // one (model, omega) pair per cluster; the ring holds `smem` bytes
 template <int RPL, int LP>
 __global__ void __launch_bounds__(LUP_THREADS)
 multi_lu_pipe_kernel(const kls_mdesc* __restrict__ md, const int2* __restrict__ pairs, int C,
-                     int max_slots) {
+                     int max_slots, const __grid_constant__ KlsLuWait wait) {
   extern __shared__ __align__(16) unsigned char lsm[];
   const int2 pz = pairs[blockIdx.x / C];
   const kls_mdesc& d = md[pz.x];
   lup_body<RPL, LP>(d.Na, d.Na < max_slots ? d.Na : max_slots, d.A + (size_t)pz.y * d.Na * d.Na,
-                        d.det + pz.y, d.logabs + pz.y, lsm);
+                    d.det + pz.y, d.logabs + pz.y, lsm, wait);
 }
 
 // The size classes: rows per lane x columns per warp, CTAs per cluster.  4 columns
@@ -648,7 +652,9 @@ int kls_run_lu(kls_ctx* c, int n) {
       cudaLaunchAttribute at;
       cudaLaunchConfig_t cfg = lup_config(C, n, lup_smem(c->Na, slots), c->stream, &at);
       const double2* A = c->d_A;
-      void* args[] = {&c->Na, (void*)&slots, (void*)&C, &A, &c->d_det, &c->d_logabs};
+      KlsLuWait wait{c->lu_wait_ns, c->h_lu_err, c->lu_skip};
+      c->lu_skip = -1;
+      void* args[] = {&c->Na, (void*)&slots, (void*)&C, &A, &c->d_det, &c->d_logabs, &wait};
       KLS_CK(c, cudaLaunchKernelExC(&cfg, wide ? k.wide : k.one, args));
       KLS_LAUNCHED(c);
       return KLS_OK;
@@ -671,7 +677,7 @@ int kls_lu_classes() { return LUP_CLASSES; }
 
 // the pairs of one size class (class -1: lu_det_body, max_Na rows)
 int kls_multi_launch_lu(cudaStream_t st, const kls_mdesc* d_md, const int2* d_pairs, int n_pairs,
-                        int max_Na, int cls) {
+                        int max_Na, int cls, const KlsLuWait& wait) {
   cudaError_t e;
   if (cls >= 0) {
     const LupClass& k = lup_classes[cls];
@@ -683,7 +689,7 @@ int kls_multi_launch_lu(cudaStream_t st, const kls_mdesc* d_md, const int2* d_pa
     if ((e = lup_limits(k.multi, k.C)) != cudaSuccess) return (int)e;
     cudaLaunchAttribute at;
     cudaLaunchConfig_t cfg = lup_config(k.C, n_pairs, smem, st, &at);
-    void* args[] = {&d_md, &d_pairs, (void*)&k.C, &slots};
+    void* args[] = {&d_md, &d_pairs, (void*)&k.C, &slots, (void*)&wait};
     return (int)cudaLaunchKernelExC(&cfg, k.multi, args);
   }
   size_t sm = 2 * (size_t)max_Na * sizeof(double2);

@@ -263,12 +263,27 @@ int launch_batch(kls_multi* m) {
                                  m->d_items, m->d_starts, m->grid, m->max_K_pad, m->d_err);
   }
   if (r) return mcuda(m, (cudaError_t)r, "uneven batch launch");
+  KlsLuWait wait{0, m->d_err, -1};
+  for (kls_ctx* c : m->ctx) {
+    wait.ns = std::max(wait.ns, c->lu_wait_ns);
+    wait.skip = std::max(wait.skip, c->lu_skip);
+    c->lu_skip = -1;
+  }
   for (const LuGroup& g : m->lu) {
-    r = kls_multi_launch_lu(m->stream, m->d_md, m->d_pairs_lu + g.first, g.count, g.max_Na, g.cls);
+    r = kls_multi_launch_lu(m->stream, m->d_md, m->d_pairs_lu + g.first, g.count, g.max_Na, g.cls,
+                            wait);
     if (r) return mcuda(m, (cudaError_t)r, "uneven batch LU launch");
     ++m->launches;
   }
   return KLS_OK;
+}
+
+// the error word of a pass
+int pass_error(kls_multi* m, int code) {
+  if (code == KLS_LU_TIMED_OUT)
+    return mfail(m, KLS_ERR_TIMEOUT, "LU: a bounded wait ran out; results of this pass are invalid");
+  return mfail(m, KLS_ERR_CUDA,
+               "mixed contraction pipeline timed out (code " + std::to_string(code) + ")");
 }
 
 // One eager pass (kernel attributes are set outside any capture and the
@@ -288,9 +303,7 @@ int eager_pass(kls_multi* m, float* ms) {
   KM_CK(m, cudaEventRecord(m->ev1, m->stream));
   KM_CK(m, cudaMemcpyAsync(m->h_err, m->d_err, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
   KM_CK(m, cudaStreamSynchronize(m->stream));
-  if (*m->h_err)
-    return mfail(m, KLS_ERR_CUDA,
-                 "mixed contraction pipeline timed out (code " + std::to_string(*m->h_err) + ")");
+  if (*m->h_err) return pass_error(m, *m->h_err);
   if (ms) KM_CK(m, cudaEventElapsedTime(ms, m->ev0, m->ev1));
   return KLS_OK;
 }
@@ -337,8 +350,7 @@ int replay(kls_multi* m) {
     *m->h_err = 0;
     cudaMemsetAsync(m->d_err, 0, sizeof(int), m->stream);
     cudaStreamSynchronize(m->stream);
-    return mfail(m, KLS_ERR_CUDA,
-                 "mixed contraction pipeline timed out (code " + std::to_string(code) + ")");
+    return pass_error(m, code);
   }
   return KLS_OK;
 }
