@@ -761,6 +761,8 @@ int pair_ctas(const kls_similar* s, int k) {
   return n;
 }
 
+constexpr int MAX_GRID_Y = 65535;
+
 size_t f_bytes(const kls_similar* s) { return (size_t)s->R * s->Nap * 64; }
 
 }  // namespace
@@ -780,6 +782,10 @@ int kls_similar_prepare(kls_ctx* c) {
   // fewer radii: the table's work is below this form's (2 N^2 NR against
   // 12 N NR + 22 N^2 per row)
   if (NR < 16 || nwa < 8) return KLS_OK;
+  // beyond the grids of fourier_kernel, phase_kernel and fit_kernel: the table
+  if ((int64_t)c->n_l * Ne > (int64_t)MAX_GRID_Y * FA_R || Ne > MAX_GRID_Y ||
+      (NR + 1) / 2 > MAX_GRID_Y / FA_K * FA_K)
+    return KLS_OK;
   Scratch sc;
   double *d_probe, *d_fit, *d_rfit, *d_ref, *d_of5, *d_T;
   double2* d_iv;
@@ -963,7 +969,9 @@ int kls_similar_prepare(kls_ctx* c) {
 // fixed per context; an FP64 and an FP32 CTA per tile and split, two of them on an
 // SM at a time.  One wave while that leaves a split fewer than 64 rows, else up to 6
 // waves (a last wave that is partly empty costs less of them).
-int kls_similar_max_splits(const kls_ctx* c) { return std::max(1, c->sim->R / 8); }
+int kls_similar_max_splits(const kls_ctx* c) {
+  return std::max(1, std::min(c->sim->R / 8, MAX_GRID_Y / 2));   // (two kinds a split)
+}
 int kls_similar_splits(const kls_ctx* c) {
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
