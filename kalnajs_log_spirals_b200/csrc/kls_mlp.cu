@@ -452,6 +452,7 @@ struct kls_mlp {
   __nv_bfloat16 *dZ[2] = {nullptr, nullptr};         // bf16 [cap][width], by turns
   std::vector<__nv_bfloat16*> dZt;                   // bf16 [dout_pad][cap] of every layer
   std::vector<float*> dZf;                           // fp32 [cap][dout_pad]
+  bool lean = false;                                 // dZt and dZf of one layer only, by turns
   int ltiles = 0;                                    // row tiles of the last batch
   float* lpart = nullptr;                            // squared errors per row tile
   int rows = 0, steps = 0;                           // capacity of the buffers below
@@ -490,19 +491,31 @@ int ensure_cap(kls_mlp* m, int n, bool train) {
   if (train && n > m->tcap) {
     m->tcap = 0;
     cudaFree(m->tslab);
-    KlsSlab b;
     m->Z.assign(L, nullptr);           // layers 0 .. L - 2
     m->Ht.assign(L, nullptr);          // inputs of all layers
     m->dZt.assign(L, nullptr);
     m->dZf.assign(L, nullptr);
-    for (int l = 0; l < L; ++l) {
-      const size_t in = (size_t)cap * m->din_pad[l], out = (size_t)cap * m->dout_pad[l];
-      if (l < L - 1) b.add(&m->Z[l], out);
-      b.add(&m->Ht[l], in).add(&m->dZt[l], out).add(&m->dZf[l], out);
+    // dZt and dZf of every layer let one launch take all of dW; where they do not fit
+    // (14 against 8 bytes a row and hidden unit), those of one layer
+    cudaError_t e = cudaSuccess;
+    for (int lean = 0; lean < 2; ++lean) {
+      KlsSlab b;
+      m->lean = lean;
+      for (int l = 0; l < L; ++l) {
+        const size_t in = (size_t)cap * m->din_pad[l], out = (size_t)cap * m->dout_pad[l];
+        if (l < L - 1) b.add(&m->Z[l], out);
+        b.add(&m->Ht[l], in);
+        if (!lean) b.add(&m->dZt[l], out).add(&m->dZf[l], out);
+      }
+      if (lean) b.add(&m->dZt[0], (size_t)cap * m->width).add(&m->dZf[0], (size_t)cap * m->width);
+      for (int q = 0; q < 2; ++q) b.add(&m->dZ[q], (size_t)cap * m->width);
+      b.add(&m->lpart, (size_t)cap / GT_S);
+      e = b.alloc(&m->tslab);
+      if (e != cudaErrorMemoryAllocation) break;
+      cudaGetLastError();
     }
-    for (int q = 0; q < 2; ++q) b.add(&m->dZ[q], (size_t)cap * m->width);
-    b.add(&m->lpart, (size_t)cap / GT_S);
-    ML_CK(m, b.alloc(&m->tslab));
+    ML_CK(m, e);
+    for (int l = 1; m->lean && l < L; ++l) { m->dZt[l] = m->dZt[0]; m->dZf[l] = m->dZf[0]; }
     m->tcap = cap;
   }
   return KLS_OK;
@@ -615,15 +628,27 @@ int forward(kls_mlp* m, int n, const int* idx, int row0, bool train) {
 int backward(kls_mlp* m, int n) {
   const int L = m->depth;
   GradArgs a{};
-  a.L = L;
+  // dW and bias gradients of the layers collected in a
+  auto grads = [&]() {
+    for (int i = 0; i < a.L; ++i) {
+      a.tiles[i + 1] = a.tiles[i] + tiles(a.w[i], GT_S);
+      a.sums[i + 1] = a.sums[i] + (a.s[i].N + CS_COLS - 1) / CS_COLS;
+    }
+    return launch(m, grad_kernel, dim3(a.tiles[a.L] + a.sums[a.L]), GT_THREADS, a);
+  };
   for (int l = L - 1, q = 0; l >= 0; --l, q ^= 1) {
     // dW_l [dout][din] = dZ_l^T (dout x n) * H_l (n x din): A = dZt_l [dout_pad][cap], B = Ht_l
-    GemmArgs& w = a.w[l];
+    GemmArgs& w = a.w[a.L];
     w.M = m->dout[l]; w.N = m->din[l]; w.K = n;
     w.A = m->dZt[l]; w.lda = m->tcap;
     w.B = m->Ht[l]; w.ldb = m->tcap;
     w.C = m->g + m->woff[l]; w.ldc = m->din[l];
-    a.s[l] = {n, m->dout[l], m->dout_pad[l], m->dZf[l], m->g + m->boff[l]};
+    a.s[a.L++] = {n, m->dout[l], m->dout_pad[l], m->dZf[l], m->g + m->boff[l]};
+    int r;
+    if (m->lean) {                     // before the next layer takes their place
+      if ((r = grads())) return r;
+      a.L = 0;
+    }
     if (l == 0) break;
     // dZ_{l-1} = (dZ_l W_l) * gelu'(Z_{l-1}): A = dZ [n][dout_pad], B = Wt_l [din_pad][dout_pad]
     GemmArgs h{};
@@ -634,14 +659,9 @@ int backward(kls_mlp* m, int n) {
     h.C = m->dZf[l - 1]; h.ldc = m->din_pad[l];
     h.H = m->dZ[q ^ 1]; h.ldh = m->din_pad[l];
     h.Ht = m->dZt[l - 1]; h.ldht = m->tcap;
-    int r = gemm<EPI_GELU_BWD>(m, h);
-    if (r) return r;
+    if ((r = gemm<EPI_GELU_BWD>(m, h))) return r;
   }
-  for (int l = 0; l < L; ++l) {
-    a.tiles[l + 1] = a.tiles[l] + tiles(a.w[l], GT_S);
-    a.sums[l + 1] = a.sums[l] + (m->dout[l] + CS_COLS - 1) / CS_COLS;
-  }
-  return launch(m, grad_kernel, dim3(a.tiles[L] + a.sums[L]), GT_THREADS, a);
+  return m->lean ? KLS_OK : grads();
 }
 
 LossArgs loss_args(const kls_mlp* m, int n, float* loss) {
