@@ -249,7 +249,15 @@ int ws_chunk(const kls_ctx* c, int n, int mode) {
   const size_t one = kls_similar_part_elems(c, 1) * sizeof(double2) +
                      ((size_t)c->K_pad + (size_t)c->Na * c->Na) * sizeof(double2);
   const size_t fit = ((size_t)1 << 30) / one;
-  return std::min(n, std::max(WS_CHUNK, (int)std::min<size_t>(fit, WS_CHUNK_MAX)));
+  const int chunk = std::min(n, std::max(WS_CHUNK, (int)std::min<size_t>(fit, WS_CHUNK_MAX)));
+  // a stream capture cannot grow the buffers, which a call of fewer omegas has made
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (chunk > WS_CHUNK && cudaStreamIsCapturing(c->stream, &cap) == cudaSuccess &&
+      cap != cudaStreamCaptureStatusNone &&
+      (c->ws_omega < chunk || c->part_elems < kls_similar_part_elems(c, chunk) ||
+       c->F_bytes < kls_similar_f_bytes(c, chunk)))
+    return WS_CHUNK;
+  return chunk;
 }
 
 // Host-buffer batch: omegas in, dets out, chunked by the workspace size.
