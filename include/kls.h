@@ -360,8 +360,8 @@ int kls_multi_get_info(const kls_multi* mm, kls_multi_info* out);
  * with each candidate K split count (the occupancy-derived default, half,
  * twice and three times it) and, for the split-BF16 form, each kernel (one
  * CTA or a CTA pair per tile), and keeps the fastest for the context.  Results
- * are cached per (device name, mode, N_alpha_pad, K_pad, batch) for the
- * process, and in the text file named by the environment variable
+ * are cached per (device name, mode, FP64 form, NR, Ne, number of l, N_alpha,
+ * batch) for the process, and in the text file named by the environment variable
  * KLS_TUNE_CACHE when it is set.                                            */
 typedef struct kls_tune_result {
     int32_t mode;

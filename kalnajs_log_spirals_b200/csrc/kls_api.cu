@@ -966,8 +966,12 @@ std::string tune_key(const kls_ctx* c, int mode, int batch) {
   if (cudaGetDeviceProperties(&p, c->device) == cudaSuccess) dev = p.name;
   for (char& ch : dev)
     if (ch == ' ') ch = '_';
+  // what a split count means, and how many there can be, follows from the form (an FP64
+  // count is of row splits of the pair sum on self-similar orbits, of K splits over the
+  // table) and from all of the model's sizes; "v2": of the kernels as they are now
   std::ostringstream o;
-  o << dev << "|" << mode << "|" << c->Na_pad << "|" << c->K_pad << "|" << batch;
+  o << dev << "|v2|" << mode << (mode == KLS_MODE_FP64 && c->sim ? "|similar|" : "|table|") << c->NR
+    << "|" << c->Ne << "|" << c->n_l << "|" << c->Na << "|" << batch;
   return o.str();
 }
 
