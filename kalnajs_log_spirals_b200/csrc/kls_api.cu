@@ -130,6 +130,20 @@ void dfree(void* p) {
   if (p) cudaFree(p);
 }
 
+// the buffers that FP64 evaluations alone use
+void free_part(kls_ctx* c) {
+  dfree(c->d_part);
+  c->device_bytes -= (int64_t)(c->part_elems * sizeof(double2));
+  c->d_part = nullptr;
+  c->part_elems = 0;
+}
+void free_F(kls_ctx* c) {
+  dfree(c->d_F);
+  c->device_bytes -= (int64_t)c->F_bytes;
+  c->d_F = nullptr;
+  c->F_bytes = 0;
+}
+
 // the FP64 contraction's work items and partials (self-similar form: F) for n omegas
 int ensure_f64(kls_ctx* c, int n) {
   int r;
@@ -138,9 +152,7 @@ int ensure_f64(kls_ctx* c, int n) {
   if (!c->sim && (r = kls_f64_plan(c))) return r;
   const size_t need = c->sim ? kls_similar_part_elems(c, n) : kls_f64_part_elems(c, n);
   if (c->sim && kls_similar_f_bytes(c, n) > c->F_bytes) {
-    dfree(c->d_F);
-    c->d_F = nullptr;
-    c->F_bytes = 0;
+    free_F(c);
     const size_t fb = kls_similar_f_bytes(c, n);
     char* p = nullptr;
     if ((r = dalloc(c, &p, fb))) return r;
@@ -148,9 +160,7 @@ int ensure_f64(kls_ctx* c, int n) {
     c->F_bytes = fb;
   }
   if (need <= c->part_elems) return KLS_OK;
-  dfree(c->d_part);
-  c->d_part = nullptr;
-  c->part_elems = 0;
+  free_part(c);
   if ((r = dalloc(c, &c->d_part, need))) return r;
   c->part_elems = need;
   return KLS_OK;
@@ -163,7 +173,9 @@ int ensure_ws(kls_ctx* c, int n, int mode) {
   if (n <= c->ws_omega) return KLS_OK;
   int cap = n;
   dfree(c->ws);
+  c->device_bytes -= (int64_t)c->ws_bytes;
   c->ws = nullptr;
+  c->ws_bytes = 0;
   c->d_omega = nullptr; c->d_wt = nullptr; c->d_A = nullptr;
   c->d_det = nullptr; c->d_logabs = nullptr;
   c->ws_omega = 0;
@@ -171,6 +183,7 @@ int ensure_ws(kls_ctx* c, int n, int mode) {
   s.add(&c->d_omega, (size_t)2 * cap).add(&c->d_wt, (size_t)cap * c->K_pad);
   s.add(&c->d_A, (size_t)cap * c->Na * c->Na).add(&c->d_det, cap).add(&c->d_logabs, cap);
   if ((r = dslab(c, &c->ws, s))) return r;
+  c->ws_bytes = s.bytes();
   c->ws_omega = cap;
   return KLS_OK;
 }
@@ -444,13 +457,12 @@ int kls_release_fp64(kls_ctx* c) {
   KLS_CK(c, cudaStreamSynchronize(c->stream));
   kls_drop_table(c);
   kls_similar_free(c);
-  // what only FP64 evaluations use
-  for (void* p : {c->d_F, (void*)c->d_part, (void*)c->d_items, (void*)c->d_tiles}) dfree(p);
-  c->d_F = nullptr;
-  c->d_part = nullptr;
+  free_F(c);
+  free_part(c);
+  dfree(c->d_items);
+  dfree(c->d_tiles);
   c->d_items = nullptr;
   c->d_tiles = nullptr;
-  c->F_bytes = c->part_elems = 0;
   c->plan_splits = 0;
   c->fp64_released = true;
   return KLS_OK;

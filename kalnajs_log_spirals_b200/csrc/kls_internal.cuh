@@ -133,7 +133,8 @@ struct kls_ctx {
 
   // omega-independent device data
   void* base = nullptr;       // the arrays up to d_M, one allocation
-  void* ws = nullptr;         // d_omega, d_wt, d_A, d_det, d_logabs
+  void* ws = nullptr;         // d_omega, d_wt, d_A, d_det, d_logabs: ws_bytes
+  size_t ws_bytes = 0;
   double* d_cosw = nullptr;   // [nw]
   double* d_sinw = nullptr;   // [nw]
   double2* d_cs = nullptr;    // both in the orbit kernel's order

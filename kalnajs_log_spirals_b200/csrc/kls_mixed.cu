@@ -1218,6 +1218,7 @@ int kls_mixed_prepare(kls_ctx* c) {
   c->mixed = m;
   int r = c->d_V ? KLS_OK : kls_build_table(c);
   if (r) {
+    c->device_bytes -= (int64_t)(2 * n * sizeof(__nv_bfloat16));
     kls_mixed_free(c);
     return r;
   }

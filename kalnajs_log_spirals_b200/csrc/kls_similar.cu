@@ -38,7 +38,8 @@
 #include <vector>
 
 struct kls_similar {
-  void* slab = nullptr;       // the arrays below
+  void* slab = nullptr;       // the arrays below, slab_bytes in all
+  size_t slab_bytes = 0;
   int R = 0;                  // rows (l, e): il * Ne + ie
   int Nap = 0;                // N_alpha padded to the pair tiles
   int K2p = 0;                // mirrored pairs of radii, padded to the slabs of fourier_kernel
@@ -771,6 +772,7 @@ void kls_similar_free(kls_ctx* c) {
   kls_similar* s = c->sim;
   if (!s) return;
   cudaFree(s->slab);
+  c->device_bytes -= (int64_t)s->slab_bytes;
   delete s;
   c->sim = nullptr;
 }
@@ -898,6 +900,8 @@ int kls_similar_prepare(kls_ctx* c) {
     b.add(&s->V, tab).add(&s->Vf, tab / 2).add(&s->D, tab / 2).add(&s->U, (size_t)3 * NPh);
     b.add(&s->Phi, (size_t)2 * s->K2p * s->Nap).add(&s->rot, s->Nap).add(&s->tiles, tiles.size());
     SIM_CK(b.alloc(&s->slab));
+    s->slab_bytes = b.bytes();
+    c->device_bytes += (int64_t)s->slab_bytes;
   }
   SIM_CK(cudaMemcpyAsync(d_U, U.data(), U.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   SIM_CK(cudaMemcpyAsync(d_rfit, rfit.data(), rfit.size() * sizeof(double), cudaMemcpyHostToDevice,
