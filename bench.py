@@ -922,11 +922,10 @@ def ours(args):
     nb = 3
     # one triangle of a complex symmetric product of real rows; the complex
     # product of the reference takes 8 N_alpha^2 K
-    # A model of self-similar orbits holds no table (8 N_alpha bytes per orbit x l term)
-    # but one row per (l, e).  FP64 work: F, the weights [rows x NR] against the cosines
+    # A model of self-similar orbits holds no table but one row per (l, e).  FP64 work: F, the weights [rows x NR] against the cosines
     # and sines of the mirrored radii (3 channels x re, im), and 12 FMA per pair of
     # alphas (a quarter of the matrix) and row.
-    similar = dims.device_bytes < 24 * dims.nwa * dims.NPh + 8 * dims.K_pad * dims.N_alpha
+    similar = pc.self_similar
     rows = dims.n_l * cfg.grid.Ne
     flops_per_det = 2.0 * dims.N_alpha * (dims.N_alpha + 1) * dims.K
     if similar:

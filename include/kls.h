@@ -377,6 +377,19 @@ int kls_autotune(kls_ctx* ctx, int mode, int batch, kls_tune_result* out);
 /* Set the K split count of `mode` by hand (clamped to what the table
  * allows); determinants stay batch-independent for a fixed count.         */
 int kls_set_splits(kls_ctx* ctx, int mode, int splits);
+/* Which form FP64 evaluations take (no reference counterpart): 1 over the common
+ * orbits of kls_precompute, 0 over the table of all orbits; -1 before
+ * kls_precompute or after kls_release_fp64.  M(omega) over the common orbits is
+ * the table's up to the rounding of the orbits themselves, whose last bits decide
+ * it either way: an orbit may miss its common form by 1e-10 of max |W| (1e-11 on
+ * average over an eccentricity's; 2e-13 on the default grid), and the first-order
+ * terms, at most 1e-6 of the others, are summed in FP32.                      */
+int kls_get_f64_similar(const kls_ctx* ctx);
+/* on != 0: FP64 evaluations run over the table of all orbits (built if it is not
+ * there), the sum itself to FP64 rounding; on = 0: back to the common orbits where
+ * the model has them, and the table is freed.  Resets the FP64 split count.  A batch
+ * (kls_multi_create) whose model's form was dropped since returns KLS_ERR_STATE. */
+int kls_set_f64_table(kls_ctx* ctx, int on);
 /* FP64 contraction form (no reference counterpart): KLS_F64_4M (default) or
  * KLS_F64_3M; a change resets the K split count to the default.  Both run the
  * same kernel.  An uneven batch (kls_multi_create) needs every FP64 model in

@@ -139,6 +139,8 @@ SIGNATURES = {
     "kls_set_anchor": (C.c_int, [_P, C.c_double, C.c_double, _D]),
     "kls_det": (C.c_int, [_P, C.c_double, C.c_double, C.c_int, _D, _D, _D]),
     "kls_set_f64_form": (C.c_int, [_P, C.c_int]),
+    "kls_get_f64_similar": (C.c_int, [_P]),
+    "kls_set_f64_table": (C.c_int, [_P, C.c_int]),
     "kls_scan": (C.c_int, [_P, C.POINTER(kls_scan_cfg), _D, _D, _D, _D]),
     "kls_newton": (C.c_int, [_P, C.c_double, C.c_double, C.POINTER(kls_newton_cfg),
                              C.POINTER(kls_newton_result), _D]),

@@ -196,6 +196,17 @@ class PrecomputedData:
     def close(self):
         self.ctx.close()
 
+    # -- FP64 form (no reference counterpart) ---------------------------------
+    @property
+    def self_similar(self) -> bool:
+        """FP64 evaluations run over the common orbits (kls_get_f64_similar)."""
+        return self.ctx.lib.kls_get_f64_similar(self.ctx.h) == 1
+
+    def use_table(self, on: bool = True) -> None:
+        """FP64 evaluations over the table of all orbits, whatever the orbits are; off:
+        over the common ones where the model has them (kls_set_f64_table)."""
+        self.ctx.call("kls_set_f64_table", int(bool(on)))
+
     # -- lazy exports --------------------------------------------------------
     def _alpha(self):
         if "alpha" not in self._cache:

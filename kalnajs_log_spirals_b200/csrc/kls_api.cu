@@ -431,7 +431,7 @@ int kls_precompute(kls_ctx* c) {
   if ((r = kls_run_basis(c))) return r;
   // the FP64 form: self-similar where the orbits are, else over the table
   if (!c->fp64_released) {
-    if ((r = kls_similar_prepare(c))) return r;
+    if (!c->sim_off && (r = kls_similar_prepare(c))) return r;
     if (!c->sim && (r = kls_build_table(c))) return r;
     if (!c->precomputed) c->splits = kls_choose_splits(c);
   }
@@ -1253,6 +1253,23 @@ int kls_set_f64_form(kls_ctx* c, int form) {
     return apply_splits(c, KLS_MODE_FP64, kls_choose_splits(c));
   }
   return KLS_OK;
+}
+
+int kls_get_f64_similar(const kls_ctx* c) {
+  return !c || !c->precomputed || c->fp64_released ? -1 : c->sim ? 1 : 0;
+}
+
+int kls_set_f64_table(kls_ctx* c, int on) {
+  int r = check_ready(c);
+  if (r) return r;
+  if (c->fp64_released)
+    return kls_fail(c, KLS_ERR_STATE, "the FP64 table was released (kls_release_fp64)");
+  if (on ? !c->sim : !c->sim_off) return KLS_OK;
+  if (on && (r = kls_build_table(c))) return r;
+  KLS_CK(c, cudaStreamSynchronize(c->stream));
+  std::swap(c->sim, c->sim_off);
+  if (!on) kls_drop_table(c);
+  return apply_splits(c, KLS_MODE_FP64, kls_choose_splits(c));
 }
 
 int kls_set_lu_mode(kls_ctx* c, int mode) {

@@ -154,6 +154,7 @@ struct kls_ctx {
   int ldv = 0;                // row length of the FP64 table (kls_ldv)
   double* d_V = nullptr;      // [K_pad][ldv] FP64 table (null while nothing needs it)
   kls_similar* sim = nullptr; // set when the orbits are self-similar
+  kls_similar* sim_off = nullptr;   // it, while kls_set_f64_table has the table in its place
   bool fp64_released = false; // kls_release_fp64: no FP64 evaluations any more
 
   // per-batch workspace (grown on demand)

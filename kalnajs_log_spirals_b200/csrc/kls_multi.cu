@@ -48,6 +48,7 @@ struct kls_multi {
                                     // item, 2 (TMEM form) one launch per model
   bool tm = false;                  // mixed: some model in the TMEM-operand form
   bool old = false;                 // mixed: some model in the one-CTA / pair forms
+  std::vector<const kls_similar*> sim;   // FP64: the form that each model had (null: the table)
   std::vector<char> use_tm;         // per model: TMEM-operand form
   std::vector<int2> pairs_tm, pairs_old;   // (model, omega) pairs of each form
   int2 *d_pairs_tm = nullptr, *d_pairs_old = nullptr;
@@ -361,10 +362,13 @@ int run_omegas(kls_multi* m, const std::function<void(int, int, double*)>& fill,
   const int B = m->batch;
   // the graph holds the addresses of the models' FP64 form
   if (m->mode == KLS_MODE_FP64)
-    for (int i = 0; i < m->n_models; ++i)
-      if (m->ctx[i]->fp64_released)
-        return mfail(m, KLS_ERR_STATE, "model " + std::to_string(i) +
-                                           ": the FP64 table was released (kls_release_fp64)");
+    for (int i = 0; i < m->n_models; ++i) {
+      const kls_ctx* c = m->ctx[i];
+      const kls_similar* s = m->sim[i];
+      if (s ? s != c->sim && s != c->sim_off : m->md[i].V != c->d_V)
+        return mfail(m, KLS_ERR_STATE, "model " + std::to_string(i) + ": its FP64 form was freed "
+                                       "(kls_release_fp64, kls_set_f64_table)");
+    }
   for (int b0 = 0; b0 < n; b0 += B) {
     const int nb = std::min(B, n - b0);
     for (int i = 0; i < m->n_models; ++i) {
@@ -476,6 +480,7 @@ int kls_multi_create(kls_ctx* const* models, int n_models, int mode, int batch, 
   size_t F_bytes = 0;
   for (int i = 0; i < n_models; ++i) {
     kls_ctx* c = models[i];
+    m->sim.push_back(c->sim);
     kls_mdesc d{};
     d.V = c->d_V;
     d.ldv = c->ldv;

@@ -769,6 +769,7 @@ size_t f_bytes(const kls_similar* s) { return (size_t)s->R * s->Nap * 64; }
 }  // namespace
 
 void kls_similar_free(kls_ctx* c) {
+  if (!c->sim) std::swap(c->sim, c->sim_off);
   kls_similar* s = c->sim;
   if (!s) return;
   cudaFree(s->slab);
