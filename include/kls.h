@@ -476,8 +476,8 @@ int64_t kls_launch_count(const kls_ctx* ctx);
 
 /* ---- bounds-checked build (no reference counterpart) ---------------------- *
  * libkls_checked.so, built from the same sources with KLS_CHECKED, guards
- * the global accesses of the FP64 determinant path (orbits, W_l, rows,
- * weights, contraction, reduction, LU, the allocation-free LU): an index
+ * the global accesses of the FP64 determinant path (orbits, W_l, rows, weights,
+ * the self-similar form, contraction, reduction, LU, the allocation-free LU): an index
  * outside its buffer's extent is skipped and logged instead of read or
  * written.  kls_bounds_report returns, for the current device, the number
  * of skipped accesses since the last reset and the site code (KlsSite in

@@ -62,7 +62,9 @@ __global__ void transpose_kernel(int n, const double2* __restrict__ in, double2*
     if (r0 + y < n && c0 + x < n) t[y][x] = in[(size_t)(r0 + y) * n + c0 + x];
   __syncthreads();
   for (int y = threadIdx.y; y < 32; y += 8)
-    if (c0 + y < n && r0 + x < n) out[(size_t)(c0 + y) * n + r0 + x] = t[x][y];
+    if (c0 + y < n && r0 + x < n)
+      KLS_IF(KLS_IB((int64_t)(c0 + y) * n + r0 + x, (int64_t)n * n, KS_REDUCE))
+      out[(size_t)(c0 + y) * n + r0 + x] = t[x][y];
 }
 
 int validate(const kls_config* k, std::string& msg) {

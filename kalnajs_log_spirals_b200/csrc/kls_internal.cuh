@@ -340,8 +340,8 @@ struct KlsRange {
 
 // ---- bounds-checked build (KLS_CHECKED) ------------------------------------
 // libkls_checked.so is the same sources compiled with -DKLS_CHECKED: every
-// guarded global access of the FP64 determinant path (orbit, W_l, row,
-// weight, contraction, reduction and LU kernels) first tests its element
+// guarded global access of the FP64 determinant path (orbit, W_l, row, weight,
+// self-similar, contraction, reduction and LU kernels) first tests its element
 // index against the extent of the buffer it touches, as the launch's own
 // parameters size it.  An access outside is skipped (a load reads 0) and
 // counted in this translation unit's device log, with the site code, index
@@ -364,6 +364,8 @@ enum KlsSite {
   KS_REDUCE,            // partials summed, I - M and M written
   KS_LU,                // LU matrices, determinants
   KS_LU_STATIC,         // allocation-free LU: input, scratch, determinants
+  KS_SIMILAR_PREP,      // self-similar form: samples, fits, common orbits, phases
+  KS_SIMILAR,           // self-similar form: weights, F, pair partials, I - M and M
 };
 #ifdef KLS_CHECKED
 struct KlsBoundsLog {

@@ -152,6 +152,9 @@ __global__ void order_kernel(int nw, int chunk, const double* __restrict__ cosw,
 
 // table read, guarded in the bounds-checked build (plain t[i] otherwise)
 #define ORB_TAB(t, i) KLS_LD(KLS_IB((i), P.nw, KS_ORBIT_TABLE), t[i], 0.0)
+#define ORB_CS(p)                                                                       \
+  KLS_LD(KLS_IB((p) - cs, (int64_t)(chunk + 1) * ORB_THREADS, KS_ORBIT_TABLE), *p,       \
+         make_double2(0.0, 0.0))
 
 // Bound: instruction issue (a logarithm and a reciprocal square root per point,
 // about 190 instructions, 73 of them FP64).  80 registers and 24 warps per SM: 512
@@ -252,11 +255,11 @@ orbit_kernel(OrbitParams P, int chunk, const double* __restrict__ cosw, const do
       if (i0 > 0) vals_at(i0 - 1, ORB_TAB(cosw, i0 - 1), ORB_TAB(sinw, i0 - 1), x, prev_t, prev_p);
       int j = j0, next = j0 * nwai;
       const double2* src = cs + tid;
-      double2 ahead = *src;                              // cs ends in a spare row
+      double2 ahead = ORB_CS(src);                       // cs ends in a spare row
       for (int i = i0; i < i1; ++i) {
         const double2 q = ahead;
         src += ORB_THREADS;
-        ahead = *src;
+        ahead = ORB_CS(src);
         vals_at(i, q.x, q.y, x, dt1, dt3);
         if (i > 0) { st += (prev_t + dt1) / 2; sp += (prev_p + dt3) / 2; }
         prev_t = dt1; prev_p = dt3;

@@ -56,6 +56,11 @@ struct kls_similar {
 
 namespace {
 
+// element i of an array of n, guarded in the bounds-checked build: arrays of the
+// preparation, and of the evaluation
+#define SIM_IN(i, n) KLS_IB((int64_t)(i), (int64_t)(n), KS_SIMILAR_PREP)
+#define SIM_AT(i, n) KLS_IB((int64_t)(i), (int64_t)(n), KS_SIMILAR)
+
 __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
   asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
       : "+d"(d0), "+d"(d1)
@@ -98,6 +103,7 @@ __global__ void probe_kernel(int NPh, int nwa, const double* __restrict__ of,
                              const double* __restrict__ pha, double* __restrict__ out) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= NPh) return;
+  KLS_UNLESS(SIM_IN((int64_t)OF_DJ * NPh + p, (int64_t)OF_COUNT * NPh), return)
   const double FE = of[(size_t)OF_FE * NPh + p], FL = of[(size_t)OF_FL * NPh + p];
   const double DJ = of[(size_t)OF_DJ * NPh + p];
   double* o = out + (size_t)p * (SIM_PROBES + 2);
@@ -105,6 +111,7 @@ __global__ void probe_kernel(int NPh, int nwa, const double* __restrict__ of,
   o[1] = of[(size_t)OF_OM2 * NPh + p] / of[(size_t)OF_OM1 * NPh + p];
   for (int q = 0; q < 3; ++q) {
     const size_t k = (size_t)p * nwa + probe_at(nwa, q);
+    KLS_UNLESS(SIM_IN(k, (int64_t)NPh * nwa), continue)
     o[2 + q] = w1[k];
     o[5 + q] = pha[k];
   }
@@ -125,6 +132,7 @@ __global__ void fit_kernel(int NR, int Ne, int nwa, const double* __restrict__ p
     const int p = iR + NR * ie;
     if (probes[(size_t)p * (SIM_PROBES + 2)] == 0.0) continue;
     const size_t e = (size_t)p * nwa + k;
+    KLS_UNLESS(SIM_IN(e, (int64_t)NR * Ne * nwa), continue)
     const double w = w1[e], t = pha[e], u = U[p], v = U[(size_t)NR * Ne + p];
     if (n == 0.0) { w0 = w; p0 = t; }
     const double dw = w - w0, dp = t - p0;       // differences of near equals: exact
@@ -134,6 +142,7 @@ __global__ void fit_kernel(int NR, int Ne, int nwa, const double* __restrict__ p
   const double2 iv = inv_var[ie];
   const size_t pl = (size_t)Ne * nwa, o = (size_t)ie * nwa + k;
   const double d = n > 0.0 ? 1.0 / n : 0.0;
+  KLS_UNLESS(SIM_IN(6 * pl + o, 7 * pl), return)
   fit[o] = w0 + sw * d;
   fit[pl + o] = wu * iv.x;
   fit[2 * pl + o] = wv * iv.y;
@@ -152,6 +161,7 @@ __global__ void misfit_kernel(int NR, int Ne, int nwa, double m, double amax,
                               const double* __restrict__ pha, const double* __restrict__ fit,
                               double2* __restrict__ out) {
   const int p = blockIdx.x, ie = p / NR, iR = p % NR;
+  KLS_UNLESS(SIM_IN(p, NR * Ne), return)
   const double* pr = probes + (size_t)p * (SIM_PROBES + 2);
   if (pr[0] == 0.0) {
     if (threadIdx.x == 0) out[p] = make_double2(0.0, 0.0);
@@ -165,6 +175,7 @@ __global__ void misfit_kernel(int NR, int Ne, int nwa, double m, double amax,
   double a = 0.0, b = 0.0;
   for (int k = threadIdx.x; k < nwa; k += blockDim.x) {
     const size_t e = (size_t)p * nwa + k;
+    KLS_UNLESS(SIM_IN(e, (int64_t)NR * pl), continue)
     const double sw = 0.5 * (f[k < nwa - 1 ? k + 1 : k] - f[k > 0 ? k - 1 : k]);
     const double dw = fabs(w1[e] - (f[k] + u * f[pl + k] + v * f[2 * pl + k]));
     const double dp = fabs(pha[e] - (f[3 * pl + k] + u * f[4 * pl + k] + v * f[5 * pl + k]));
@@ -195,6 +206,7 @@ __global__ void reference_kernel(int Ne, int nwa, const double* __restrict__ fit
   const double hu = q == 1 ? SIM_H : q == 2 ? -SIM_H : 0.0;
   const double hv = q == 3 ? SIM_H : q == 4 ? -SIM_H : 0.0;
   const size_t e = ((size_t)q * Ne + ie) * nwa + k;
+  KLS_UNLESS(SIM_IN(e, 5 * pl) && SIM_IN(6 * pl + o, 7 * pl), return)
   w1[e] = fit[o] + hu * fit[pl + o] + hv * fit[2 * pl + o];
   pha[e] = fit[3 * pl + o] + hu * fit[4 * pl + o] + hv * fit[5 * pl + o];
   ra[e] = fit[6 * pl + o];
@@ -211,6 +223,8 @@ __global__ void combine_kernel(int n_l, int Ne, int ldv, int l_min, const double
   const double l = fabs((double)(l_min + il));
   for (int c = threadIdx.x; c < ldv; c += blockDim.x) {
     const size_t p = ((size_t)r * ldv + c) / 2;
+    KLS_UNLESS(SIM_IN(((int64_t)il * 5 * Ne + 4 * Ne + ie) * ldv + c, (int64_t)n_l * 5 * Ne * ldv) &&
+                   SIM_IN((int64_t)r * ldv + c, (int64_t)n_l * Ne * ldv), continue)
     double x[5];
     for (int q = 0; q < 5; ++q) x[q] = T[((size_t)il * 5 * Ne + q * Ne + ie) * ldv + c];
     const double du = (x[1] - x[2]) * (0.5 / SIM_H), dv = (x[3] - x[4]) * (0.5 / SIM_H);
@@ -250,6 +264,7 @@ __global__ void phase_kernel(int NR, int K2p, int Na, int Nap, double da,
   double s = 0.0, c = 0.0;
   if (d < Na && k < (NR + 1) / 2)
     phase(((NR & 1) ? (double)k : k + 0.5) * ((lb - la) / (double)(NR - 1)) * da, &s, &c);
+  KLS_UNLESS(SIM_IN(((int64_t)K2p + k) * Nap + d, 2 * (int64_t)K2p * Nap), return)
   Phi[(size_t)k * Nap + d] = c;
   Phi[((size_t)K2p + k) * Nap + d] = s;
   if (k == 0) {
@@ -263,6 +278,7 @@ __global__ void channel_kernel(int NR, int NPh, const double* __restrict__ rc,
                                const double* __restrict__ uv, double* __restrict__ U) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= NPh) return;
+  KLS_UNLESS(SIM_IN(2 * (int64_t)NPh + p, 3 * (int64_t)NPh), return)
   const double r = 1.0 / rc[p % NR];
   U[p] = r;
   U[NPh + p] = r * uv[p];
@@ -318,14 +334,18 @@ fourier_kernel(int R, int Ne, int NR, int K2p, int Nap, int64_t K_pad,
       // (the centre of an odd grid is its own mirror: counted once)
       const bool u_in = k_in && !(sd && up == dn && k == 0);
       const int at = k_in ? iR : 0;
+      KLS_IF(SIM_AT(wrow + at - w, K_pad))
       cp16z(st + FA_W + 2 * ((sd * FA_R + lr) * FA_S + lk), wrow + at, k_in && row_in ? 16 : 0);
 #pragma unroll
       for (int ch = 0; ch < 3; ++ch)
+        KLS_IF(SIM_AT(urow + ch * uch + at - U, 3 * uch))
         cp8z(st + FA_U + ((ch * 2 + sd) * FA_R + lr) * FA_S + lk, urow + ch * uch + at,
              u_in && row_in ? 8 : 0);
     }
 #pragma unroll
     for (int h = 0; h < 2; ++h)
+      KLS_IF(SIM_AT(prow + ((size_t)h * K2p + (size_t)kt * FA_K) * Nap + 1 - Phi,
+                    2 * (int64_t)K2p * Nap))
       cp16z(st + FA_P + (h * FA_K + pk) * FA_PS + 2 * pc,
             prow + ((size_t)h * K2p + (size_t)kt * FA_K) * Nap, 16);
   };
@@ -388,6 +408,7 @@ fourier_kernel(int R, int Ne, int NR, int K2p, int Nap, int64_t K_pad,
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
       const int d = d0 + wc + 8 * j + 2 * t + x;
+      KLS_UNLESS(SIM_AT(d, Nap), continue)
       const double2 q = rot[d];
       double a[3][4];                                    // A re, im, B re, im
 #pragma unroll
@@ -400,6 +421,7 @@ fourier_kernel(int R, int Ne, int NR, int K2p, int Nap, int64_t K_pad,
         a[h][3] = q.y * ci + q.x * si;
       }
       const size_t o = ((size_t)z * R + r) * Nap + d;
+      KLS_UNLESS(SIM_AT(o, (int64_t)gridDim.z * R * Nap), continue)
       F0[o] = make_double4(a[0][0], a[0][1], a[0][2], a[0][3]);
       Fc[2 * o] = make_float4((float)a[1][0], (float)a[2][0], (float)a[1][1], (float)a[2][1]);
       Fc[2 * o + 1] = make_float4((float)a[1][2], (float)a[2][2], (float)a[1][3], (float)a[2][3]);
@@ -463,6 +485,7 @@ pair_kernel(int R, int Na, int Nap, int ldv, int splits, int n_tiles,
             double4* __restrict__ part) {
   extern __shared__ __align__(16) unsigned char psm[];
   const int tid = threadIdx.x;
+  KLS_UNLESS(SIM_AT(blockIdx.x, n_tiles), return)
   const int4 tl = tiles[blockIdx.x];
   const bool fp64 = !(blockIdx.y & 1);                   // the kinds alternate over the SMs
   const int split = blockIdx.y >> 1, z = blockIdx.z, ns = tile_splits(splits, tl.z);
@@ -480,6 +503,7 @@ pair_kernel(int R, int Na, int Nap, int ldv, int splits, int n_tiles,
     for (int q = 0; q < PR_ROWS; ++q) {                  // F of 64 d, its two halves apart
       const int r = rb + it * PR_ROWS + q, w = tid >> 1, x = tid & 1, d = dlo + w;
       const bool in = r < re && d >= 0;
+      KLS_IF(SIM_AT(in ? 2 * ((int64_t)r * Nap + d) + x : 0, 2 * (int64_t)R * Nap))
       cp16z(st + q * PR_ROW + (x ? PR_FB : PR_FA) + w * 16,
             f + (in ? 2 * ((size_t)r * Nap + d) + x : 0), in ? 16 : 0);
     }
@@ -490,6 +514,7 @@ pair_kernel(int R, int Na, int Nap, int ldv, int splits, int n_tiles,
       const bool in = r < re && al < Na;
       const size_t o = in ? (size_t)r * (ldv >> 1) + pair_index(Na, al) : 0;
       unsigned char* dst = st + row * PR_ROW + PR_W + a * 16;
+      KLS_UNLESS(SIM_AT(o, (int64_t)R * (ldv >> 1)), continue)
       if (fp64) {
         cp16z(dst, V + 2 * o, in ? 16 : 0);
       } else {
@@ -557,6 +582,7 @@ pair_kernel(int R, int Na, int Nap, int ldv, int splits, int n_tiles,
       for (int p = 0; p < 4; ++p) {
         const int e = (tj + 8 * p) * PR_T + ti + 8 * q;
         const double4 o = sh[e], v = value(q, p);
+        KLS_UNLESS(SIM_AT(out + e - part, (int64_t)gridDim.z * n_tiles * 2 * splits * PR_SLOT), continue)
         out[e] = make_double4(v.x + o.x, v.y + o.y, v.z + o.z, v.w + o.w);
       }
   };
@@ -679,6 +705,8 @@ pair_reduce_kernel(int Na, int splits, int n_tiles, double G, const double* __re
   double4 s = make_double4(0, 0, 0, 0);
 #pragma unroll 4
   for (int k = sg; k < slots; k += 4) {
+    KLS_UNLESS(SIM_AT(src + (size_t)k * PR_SLOT - part,
+                      (int64_t)gridDim.z * n_tiles * 2 * splits * PR_SLOT), continue)
     const double4 v = src[(size_t)k * PR_SLOT];
     s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
   }
@@ -700,6 +728,7 @@ pair_reduce_kernel(int Na, int splits, int n_tiles, double G, const double* __re
   const double n = Nk[col];
   const double mr = __dmul_rn(__dmul_rn(sr, G), n), mi = __dmul_rn(__dmul_rn(si, G), n);
   const size_t q = (size_t)row * Na + col;
+  KLS_UNLESS(SIM_AT(q, (int64_t)Na * Na), return)
   Aall[(size_t)z * Na * Na + q] = make_double2((row == col ? 1.0 : 0.0) - mr, -mi);
   if (Mall && z == 0) Mall[q] = make_double2(mr, mi);
 }
