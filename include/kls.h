@@ -400,8 +400,10 @@ int kls_set_f64_form(kls_ctx* ctx, int form);
  * KLS_LU_CLUSTER factors each I - M(omega) on one thread-block cluster of 1 to
  * 16 CTAs with the matrix held in their registers (latency: one matrix per
  * cluster, N_alpha <= 512); KLS_LU_CTA uses one CTA per matrix through L2.
- * KLS_LU_AUTO (default) takes the cluster form wherever it fits.  Both forms
- * return bitwise the same determinants.  KLS_LU_CLUSTER fails with
+ * KLS_LU_AUTO (default) takes the cluster form where it fits and the batch is not so
+ * large that one CTA per matrix is the faster one (from about 90 matrices at N_alpha =
+ * 100 to 150, 130 at 400; at 300 never).  Both forms return bitwise the same
+ * determinants.  KLS_LU_CLUSTER fails with
  * KLS_ERR_UNSUPPORTED when N_alpha is too large for it.                      */
 #define KLS_LU_AUTO          0
 #define KLS_LU_CTA           1

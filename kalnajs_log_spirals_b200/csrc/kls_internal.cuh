@@ -192,7 +192,8 @@ struct kls_ctx {
   // kernel (-2: not looked up yet, -1: it does not fit)
   int lu_mode = 0;
   int lu_class = -2;
-  bool lu_wide = false;       // the class's wider form fits as well
+  int lu_full = 0, lu_half = 0;  // its clusters that the device holds at once, with half a ring
+  int lu_wide = 0;            // and those of its wider form
   int* h_lu_err = nullptr;    // pinned: a wait of the pipelined LU ran out
   unsigned long long lu_wait_ns = 2000000000ull;
   int lu_skip = -1;           // test hook (one-shot): the column that is not announced
@@ -286,7 +287,7 @@ int kls_multi_launch_f64(cudaStream_t st, const kls_mdesc* d_md, const int2* d_p
                          int max_ldv);
 int kls_multi_launch_lu(cudaStream_t st, const kls_mdesc* d_md, const int2* d_pairs, int n_pairs,
                         int max_Na, int cls, const KlsLuWait& wait);
-int kls_lu_class(int device, int n);
+int kls_lu_class(int n);
 int kls_lu_classes();
 int kls_multi_launch_f64_weights(cudaStream_t st, const kls_mdesc* d_md, const int2* d_pairs,
                                  int n_pairs, int64_t max_K_pad);

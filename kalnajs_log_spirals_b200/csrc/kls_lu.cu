@@ -10,7 +10,8 @@
 //
 // lu_pipe_kernel (N <= 512): one thread-block cluster per matrix, the matrix in
 // registers, columns passed from warp to warp; lu_det_kernel: one CTA per
-// matrix through L2, any N.  Both return the same bits.
+// matrix through L2, any N, and batches of many matrices (lup_wins, kls_lu_cols.h).
+// Both return the same bits.
 #include "kls_internal.cuh"
 #include "kls_lu_cols.h"
 #include "kls_tcgen05.cuh"
@@ -545,7 +546,9 @@ multi_lu_pipe_kernel(const kls_mdesc* __restrict__ md, const int2* __restrict__ 
 
 // The size classes: rows per lane x columns per warp, CTAs per cluster.  4 columns
 // a warp keep enough matrices on the device at once; a wider form (2 columns) for
-// batches that it holds in one wave.  1 matrix / 16, us:
+// batches that it holds in one wave (7 matrices).  From <10,4> on, and a little in
+// others, the registers do not hold all of it (142 bytes spilled a thread, <13,4> 1.0
+// KB, <16,4> 2.2 KB).  1 matrix / 16, us:
 //   N =  64  <2,2> x 4   53 /  53   (<2,8> x 1    71 /  71)
 //   N = 101  <4,3> x 6   99 / 100   (<4,4> x 4   105 / 105, <4,2> x 8 128 / 249)
 //   N = 192  <6,4> x 6  276 / 276   (<6,3> x 8   306 / 605), <6,2> x 12 236 / 693
@@ -558,20 +561,21 @@ multi_lu_pipe_kernel(const kls_mdesc* __restrict__ md, const int2* __restrict__ 
 struct LupClass {
   int n_max, C;
   const void *one, *multi;
+  double us;                  // a wave of matrices, per column (lup_wins)
   int Cw;
   const void* wide;
 };
 #define LUP_CLASS(n, c, rpl, lp)                                                     \
   n, c, (const void*)lu_pipe_kernel<rpl, lp>, (const void*)multi_lu_pipe_kernel<rpl, lp>
 const LupClass lup_classes[] = {
-    {LUP_CLASS(64, 4, 2, 2), 0, nullptr},
-    {LUP_CLASS(128, 6, 4, 3), 0, nullptr},
-    {LUP_CLASS(192, 6, 6, 4), 12, (const void*)lu_pipe_kernel<6, 2>},
-    {LUP_CLASS(224, 6, 7, 5), 14, (const void*)lu_pipe_kernel<7, 2>},
-    {LUP_CLASS(256, 8, 8, 4), 16, (const void*)lu_pipe_kernel<8, 2>},
-    {LUP_CLASS(320, 10, 10, 4), 0, nullptr},
-    {LUP_CLASS(416, 13, 13, 4), 0, nullptr},
-    {LUP_CLASS(512, 16, 16, 4), 0, nullptr},
+    {LUP_CLASS(64, 4, 2, 2), 0.84, 0, nullptr},
+    {LUP_CLASS(128, 6, 4, 3), 1.08, 0, nullptr},
+    {LUP_CLASS(192, 6, 6, 4), 1.41, 12, (const void*)lu_pipe_kernel<6, 2>},
+    {LUP_CLASS(224, 6, 7, 5), 1.71, 14, (const void*)lu_pipe_kernel<7, 2>},
+    {LUP_CLASS(256, 8, 8, 4), 1.77, 16, (const void*)lu_pipe_kernel<8, 2>},
+    {LUP_CLASS(320, 10, 10, 4), 1.80, 0, nullptr},
+    {LUP_CLASS(416, 13, 13, 4), 2.90, 0, nullptr},
+    {LUP_CLASS(512, 16, 16, 4), 4.00, 0, nullptr},
 };
 #undef LUP_CLASS
 constexpr int LUP_CLASSES = (int)(sizeof(lup_classes) / sizeof(lup_classes[0]));
@@ -612,43 +616,52 @@ cudaError_t lup_limits(const void* fn, int C) {
 
 }  // namespace
 
-// can the device hold a cluster of C CTAs of fn?
-static bool lup_fits(const void* fn, int C, int n) {
+// clusters of C CTAs of fn that the device holds at once (0: none), with the whole ring
+// or half of it
+static int lup_clusters(const void* fn, int C, int n, bool half) {
   cudaLaunchAttribute at;
-  cudaLaunchConfig_t cfg = lup_config(C, 1, lup_smem(n, lup_slots(n)), nullptr, &at);
+  cudaLaunchConfig_t cfg = lup_config(C, 1, lup_smem(n, lup_slots(n, half)), nullptr, &at);
   int clusters = 0;
-  const bool ok = lup_limits(fn, C) == cudaSuccess &&
-                  cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess &&
-                  clusters > 0;
-  if (!ok) cudaGetLastError();
-  return ok;
+  if (lup_limits(fn, C) == cudaSuccess &&
+      cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess)
+    return clusters;
+  cudaGetLastError();
+  return 0;
 }
 
-// Size class of an n x n factorisation on the current device, -1 where it does not fit
-static int lup_class(int device, int n) {
-  (void)device;
-  for (int k = 0; k < LUP_CLASSES; ++k) {
-    if (n > lup_classes[k].n_max) continue;
-    const LupClass& c = lup_classes[k];
-    return lup_fits(c.one, c.C, n) && lup_fits(c.multi, c.C, n) ? k : -1;
-  }
+// Size class of an n x n factorisation, -1 where there is none
+static int lup_class(int n) {
+  for (int k = 0; k < LUP_CLASSES; ++k)
+    if (n <= lup_classes[k].n_max) return k;
   return -1;
+}
+
+static int lup_sms(int device) {
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  return sms;
 }
 
 int kls_run_lu(kls_ctx* c, int n) {
   if (c->lu_mode != KLS_LU_CTA) {
     if (c->lu_class == -2) {
-      c->lu_class = lup_class(c->device, c->Na);
-      const LupClass* k = c->lu_class >= 0 ? lup_classes + c->lu_class : nullptr;
-      c->lu_wide = k && k->wide && lup_fits(k->wide, k->Cw, c->Na);
+      c->lu_class = lup_class(c->Na);
+      if (c->lu_class >= 0) {
+        const LupClass& k = lup_classes[c->lu_class];
+        c->lu_full = lup_clusters(k.one, k.C, c->Na, false);
+        c->lu_half = lup_clusters(k.one, k.C, c->Na, true);
+        c->lu_wide = k.wide ? lup_clusters(k.wide, k.Cw, c->Na, false) : 0;
+        if (!c->lu_full) c->lu_class = -1;
+      }
     }
-    if (c->lu_class >= 0) {
+    if (c->lu_class >= 0 &&
+        (c->lu_mode == KLS_LU_CLUSTER ||
+         lup_wins(n, c->Na, n <= c->lu_full ? c->lu_full : c->lu_half,
+                  lup_classes[c->lu_class].us, lup_sms(c->device)))) {
       const LupClass& k = lup_classes[c->lu_class];
-      int sms = 148;
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-      const bool wide = c->lu_wide && (int64_t)n * k.Cw <= sms;
+      const bool wide = n <= c->lu_wide;
       const int C = wide ? k.Cw : k.C;
-      const int slots = lup_slots(c->Na, (int64_t)n * C > sms);
+      const int slots = lup_slots(c->Na, n > c->lu_full);
       cudaLaunchAttribute at;
       cudaLaunchConfig_t cfg = lup_config(C, n, lup_smem(c->Na, slots), c->stream, &at);
       const double2* A = c->d_A;
@@ -659,7 +672,7 @@ int kls_run_lu(kls_ctx* c, int n) {
       KLS_LAUNCHED(c);
       return KLS_OK;
     }
-    if (c->lu_mode == KLS_LU_CLUSTER)
+    if (c->lu_class < 0 && c->lu_mode == KLS_LU_CLUSTER)
       return kls_fail(c, KLS_ERR_UNSUPPORTED, "cluster LU does not fit this N_alpha");
   }
   size_t sm = 2 * (size_t)c->Na * sizeof(double2);
@@ -671,24 +684,33 @@ int kls_run_lu(kls_ctx* c, int n) {
   return KLS_OK;
 }
 
-// size class of a model's matrices for kls_multi_launch_lu (-1: one CTA each)
-int kls_lu_class(int device, int n) { return lup_class(device, n); }
+// size class of a model's matrices for kls_multi_launch_lu (-1: one CTA each), on the
+// current device
+int kls_lu_class(int n) {
+  const int k = lup_class(n);
+  return k >= 0 && lup_clusters(lup_classes[k].multi, lup_classes[k].C, n, false) ? k : -1;
+}
 int kls_lu_classes() { return LUP_CLASSES; }
 
-// the pairs of one size class (class -1: lu_det_body, max_Na rows)
+// the pairs of one size class (class -1, or where it is the slower one: lu_det_body,
+// max_Na rows)
 int kls_multi_launch_lu(cudaStream_t st, const kls_mdesc* d_md, const int2* d_pairs, int n_pairs,
                         int max_Na, int cls, const KlsLuWait& wait) {
   cudaError_t e;
-  if (cls >= 0) {
+  int device = 0;
+  if ((e = cudaGetDevice(&device)) != cudaSuccess) return (int)e;
+  // (its limits are those that kls_lu_class set)
+  const int full = cls >= 0 ? lup_clusters(lup_classes[cls].multi, lup_classes[cls].C, max_Na, false)
+                            : 0;
+  const bool half = n_pairs > full;
+  const int clusters =
+      full && half ? lup_clusters(lup_classes[cls].multi, lup_classes[cls].C, max_Na, true) : full;
+  if (full && lup_wins(n_pairs, max_Na, clusters, lup_classes[cls].us, lup_sms(device))) {
     const LupClass& k = lup_classes[cls];
-    int slots = 0;
-    size_t smem = 0;
     // one ring size for the class: as many slots as its largest matrix gets
-    slots = lup_slots(max_Na, (int64_t)n_pairs * k.C > 148);
-    smem = lup_smem(max_Na, slots);
-    if ((e = lup_limits(k.multi, k.C)) != cudaSuccess) return (int)e;
+    int slots = lup_slots(max_Na, half);
     cudaLaunchAttribute at;
-    cudaLaunchConfig_t cfg = lup_config(k.C, n_pairs, smem, st, &at);
+    cudaLaunchConfig_t cfg = lup_config(k.C, n_pairs, lup_smem(max_Na, slots), st, &at);
     void* args[] = {&d_md, &d_pairs, (void*)&k.C, &slots, (void*)&wait};
     return (int)cudaLaunchKernelExC(&cfg, k.multi, args);
   }

@@ -598,7 +598,7 @@ int kls_multi_create(kls_ctx* const* models, int n_models, int mode, int batch, 
     return bail(r);
   std::vector<int2> by_class;
   std::vector<int> lu_class;
-  for (kls_ctx* c : m->ctx) lu_class.push_back(kls_lu_class(m->device, c->Na));
+  for (kls_ctx* c : m->ctx) lu_class.push_back(kls_lu_class(c->Na));
   for (int cls = -1; cls < kls_lu_classes(); ++cls) {
     LuGroup g{cls, (int)by_class.size(), 0, 0};
     for (const int2& p : m->pairs)
