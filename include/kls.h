@@ -211,8 +211,9 @@ int kls_build_M(kls_ctx* ctx, double omega_re, double omega_im, int mode, double
 /* Anchor of KLS_MODE_ANCHORED (no reference counterpart): one FP64
  * evaluation at omega_a that keeps M(omega_a) on the device (N_alpha^2
  * complex) and returns det(I - M(omega_a)) in det_ri (may be NULL).  Needs
- * the FP64 table (KLS_ERR_STATE after kls_release_fp64) and builds the
- * split-BF16 table if it is missing.  A later call moves the anchor.       */
+ * the FP64 form (KLS_ERR_STATE after kls_release_fp64).  The split-BF16 table is
+ * built if it is missing: here over the table, by the first anchored evaluation
+ * over common orbits.  A later call moves the anchor.                       */
 int kls_set_anchor(kls_ctx* ctx, double omega_re, double omega_im, double* det_ri);
 
 /* grid_scan (GridScan.jl:25-88): det_grid [n_gamma, n_Op] column-major

@@ -689,7 +689,8 @@ def newton_search_hybrid(config: KalnajsConfig, precomputed: PrecomputedData,
         Omega_p_init = config.reference.Omega_p
     if gamma_init is None:
         gamma_init = config.reference.gamma
-    precomputed.ctx.call("kls_prepare_mixed")
+    if not precomputed.self_similar:
+        precomputed.ctx.call("kls_prepare_mixed")
     nc = _lib.kls_newton_cfg(int(n.max_iter), float(n.tol), float(n.delta),
                              int(bool(n.use_line_search)), int(n.max_line_search), KLS_MODE_FP64)
     h = _lib.kls_hybrid_cfg(float(hc.mixed_delta), float(hc.mixed_step_tol),

@@ -640,7 +640,9 @@ int kls_set_anchor(kls_ctx* c, double wr, double wi, double* det_ri) {
     return kls_fail(c, KLS_ERR_NONFINITE, "non-finite anchor omega");
   if (c->fp64_released)
     return kls_fail(c, KLS_ERR_STATE, "the FP64 table was released (kls_release_fp64)");
-  if (!c->mixed && (r = kls_mixed_prepare(c))) return r;
+  // (self-similar: the first anchored evaluation builds the split table; a search over FP64
+  // determinants never reads it)
+  if (!c->mixed && !c->sim && (r = kls_mixed_prepare(c))) return r;
   if (!c->d_anchorM && (r = dalloc(c, &c->d_anchorM, (size_t)c->Na * c->Na))) return r;
   if ((r = ensure_ws(c, 1, KLS_MODE_FP64))) return r;
   c->anchor_set = false;

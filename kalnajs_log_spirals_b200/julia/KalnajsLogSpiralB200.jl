@@ -181,7 +181,9 @@ function newton_search_hybrid(config, precomp::PrecomputedData, Omega_p_init::Re
                               fp64_max_iter::Integer=50, anchor_radius::Real=1e-5,
                               final_fp64::Bool=false, far_step::Real=2e-2)
     n = config.newton
-    check(precomp.handle, ccall((:kls_prepare_mixed, LIBKLS), Cint, (Ptr{Cvoid},), precomp.handle))
+    if ccall((:kls_get_f64_similar, LIBKLS), Cint, (Ptr{Cvoid},), precomp.handle) != 1
+        check(precomp.handle, ccall((:kls_prepare_mixed, LIBKLS), Cint, (Ptr{Cvoid},), precomp.handle))
+    end
     nc = Ref(KlsNewtonCfg(n.max_iter, n.tol, n.delta, n.use_line_search, n.max_line_search,
                           KLS_MODE_FP64))
     hc = Ref(KlsHybridCfg(mixed_delta, mixed_step_tol, mixed_max_iter, fp64_max_iter,
