@@ -446,8 +446,9 @@ int kls_set_mixed_chunk(kls_ctx* ctx, int k_blocks);
  * 2 s; the older mixed forms keep a fixed 2 s; an uneven batch takes the longest
  * of its models' at its creation).  A wait that runs out makes the call return
  * KLS_ERR_TIMEOUT instead of hanging the GPU; the context stays usable.  The LU
- * leaves NaN in the determinant; kls_det_batch_device, which does not wait,
- * reports it in the next determinant call on the context.                    */
+ * leaves NaN of the bits KLS_NAN_LU_TIMEOUT in the determinant (both parts) and
+ * log |det|, which is what kls_det_batch_device, which does not wait, reports. */
+#define KLS_NAN_LU_TIMEOUT 0x7ff8004b4c535455ULL
 int kls_set_wait_limit(kls_ctx* ctx, double seconds);
 /* Test hooks for the failure paths (no trap, no fault, no unbounded wait):
  * KLS_FAULT_SKIP_ARRIVAL makes the next KLS_MIXED_TMEM contraction skip one

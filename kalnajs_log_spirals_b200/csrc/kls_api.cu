@@ -247,15 +247,9 @@ int check_ready(kls_ctx* c) {
   return KLS_OK;
 }
 
-// the pipelined LU's error word (pinned: read without a copy), once the stream is idle
-// or for the calls before
-int lu_check(kls_ctx* c) {
-  volatile int* err = c->h_lu_err;
-  if (!*err) return KLS_OK;
-  *err = 0;
-  return kls_fail(c, KLS_ERR_TIMEOUT,
-                  "LU: a bounded wait ran out, in this call or in a kls_det_batch_device before "
-                  "it; the results are invalid");
+int lu_check(kls_ctx* c, const double* det_ri) {
+  if (!kls_lu_timed_out(det_ri)) return KLS_OK;
+  return kls_fail(c, KLS_ERR_TIMEOUT, "LU: a bounded wait ran out; results of this call are invalid");
 }
 
 // omegas of one launch sequence in a batch of n
@@ -297,8 +291,9 @@ int det_batch_host(kls_ctx* c, const double* omega_ri, int n, int mode, double* 
                                 cudaMemcpyDeviceToHost, c->stream));
     KLS_CK(c, cudaStreamSynchronize(c->stream));
     if (mode != KLS_MODE_FP64 && (r = kls_mixed_check(c))) return r;
-    if ((r = lu_check(c)) || (r = collect_timing(c))) return r;
-    for (int i = 0; i < nb; ++i)
+    if ((r = collect_timing(c))) return r;
+    for (int i = 0; i < nb; ++i) {
+      if ((r = lu_check(c, det_ri + 2 * (b + i)))) return r;
       if (std::isnan(det_ri[2 * (b + i)]) || std::isnan(det_ri[2 * (b + i) + 1])) {
         char buf[200];
         snprintf(buf, sizeof buf,
@@ -306,6 +301,7 @@ int det_batch_host(kls_ctx* c, const double* omega_ri, int n, int mode, double* 
                  "or model value)", omega_ri[2 * (b + i)], omega_ri[2 * (b + i) + 1]);
         return kls_fail(c, KLS_ERR_NONFINITE, buf);
       }
+    }
   }
   return KLS_OK;
 }
@@ -385,12 +381,6 @@ int kls_create(const kls_config* cfg, int device, kls_ctx** out) {
     kls_destroy(c);
     return kls_fail(nullptr, r, m);
   }
-  if ((e = cudaMallocHost(&c->h_lu_err, sizeof(int))) != cudaSuccess) {
-    c->h_lu_err = nullptr;
-    kls_destroy(c);
-    return kls_fail(nullptr, KLS_ERR_OOM, std::string("pinned memory: ") + cudaGetErrorString(e));
-  }
-  *c->h_lu_err = 0;
   *out = c;
   return KLS_OK;
 }
@@ -403,7 +393,6 @@ int kls_destroy(kls_ctx* c) {
   kls_similar_free(c);
   void* ptrs[] = {c->base, c->ws, c->d_V, c->d_items, c->d_tiles, c->d_F, c->d_part, c->d_anchorM};
   for (void* p : ptrs) dfree(p);
-  if (c->h_lu_err) cudaFreeHost(c->h_lu_err);
   for (auto& ev : c->ev) if (ev) cudaEventDestroy(ev);
   for (auto& ev : c->pev) if (ev) cudaEventDestroy(ev);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
@@ -590,7 +579,6 @@ int kls_det_batch_device(kls_ctx* c, const double* d_omega, int n, int mode, dou
   if (r) return r;
   if (n < 0 || (n > 0 && (!d_omega || !d_det)))
     return kls_fail(c, KLS_ERR_CONFIG, "bad arguments to kls_det_batch_device");
-  if ((r = lu_check(c))) return r;
   if (c->timing) std::fill(c->stage_ms, c->stage_ms + 4, 0.f);
   const int chunk = ws_chunk(c, n, mode);
   for (int b = 0; b < n; b += chunk) {
@@ -654,7 +642,7 @@ int kls_set_anchor(kls_ctx* c, double wr, double wi, double* det_ri) {
   double2 d;
   KLS_CK(c, cudaMemcpyAsync(&d, c->d_det, sizeof d, cudaMemcpyDeviceToHost, c->stream));
   KLS_CK(c, cudaStreamSynchronize(c->stream));
-  if ((r = lu_check(c)) || (r = collect_timing(c))) return r;
+  if ((r = lu_check(c, &d.x)) || (r = collect_timing(c))) return r;
   if (std::isnan(d.x) || std::isnan(d.y))
     return kls_fail(c, KLS_ERR_NONFINITE, "NaN determinant at the anchor");
   c->anchor_w[0] = wr;

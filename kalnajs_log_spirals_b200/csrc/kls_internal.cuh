@@ -5,6 +5,7 @@
 #include <nvtx3/nvToolsExt.h>
 #include <climits>
 #include <cstdint>
+#include <cstring>
 #include <string>
 #include <vector>
 #include "kls.h"
@@ -194,7 +195,6 @@ struct kls_ctx {
   int lu_class = -2;
   int lu_full = 0, lu_half = 0;  // its clusters that the device holds at once, with half a ring
   int lu_wide = 0;            // and those of its wider form
-  int* h_lu_err = nullptr;    // pinned: a wait of the pipelined LU ran out
   unsigned long long lu_wait_ns = 2000000000ull;
   int lu_skip = -1;           // test hook (one-shot): the column that is not announced
 
@@ -238,14 +238,18 @@ __host__ __device__ inline double kls_lin(double a, double b, int n, int i) {
   return a + (double)i * step;
 }
 
-// Waits of the pipelined LU: their bound, where one that ran out is noted, and the test
-// hook's column (-1: none)
-constexpr int KLS_LU_TIMED_OUT = 1000;
+// Waits of the pipelined LU: their bound, and the test hook's column (-1: none).  One
+// that ran out is told by the determinant itself (KLS_NAN_LU_TIMEOUT): no error word to
+// copy, to keep apart from the next call's or to allocate (4 pinned bytes took 1.3 ms of
+// a small model's 2.1).
 struct KlsLuWait {
   unsigned long long ns;
-  int* err;
   int skip;
 };
+inline bool kls_lu_timed_out(const double* det_ri) {
+  const unsigned long long bits = KLS_NAN_LU_TIMEOUT;
+  return std::memcmp(det_ri, &bits, sizeof bits) == 0;
+}
 
 // ---- stage entry points (host side, launch on ctx->stream) ---------------
 size_t kls_orbit_table(int nw, int nwai);   // entries of d_cs

@@ -207,8 +207,8 @@ multi_lu_kernel(const kls_mdesc* __restrict__ md, const int2* __restrict__ pairs
 // A slot is written again only when every warp has used it: each warp keeps a
 // count of the columns it is done with, and the owner of every (slots / 2)-th
 // column waits for all of them.
-// Waits are bounded (KlsLuWait); one that runs out makes the determinant NaN and is
-// noted in an error word, which the host turns into KLS_ERR_TIMEOUT.
+// Waits are bounded (KlsLuWait); one that runs out makes the determinant a NaN of its
+// own, which the host turns into KLS_ERR_TIMEOUT.
 //
 // Measured (1 matrix, B200): N = 101 312 -> 99 us, 201 557 -> 266 us, 301 1022 ->
 // 558 us against one CTA (101) or a cluster with one barrier per column; 16
@@ -514,10 +514,12 @@ __device__ __forceinline__ void lup_body(int n, int slots, const double2* __rest
   cluster_sync_all();                          // nobody leaves while others write here
   if (keeper && lane == 0) {
     if (s_failed) {
-      acc.mant = make_double2(NAN, NAN);
-      *(volatile int*)wait.err = KLS_LU_TIMED_OUT;
+      const double x = __longlong_as_double((long long)KLS_NAN_LU_TIMEOUT);
+      *det = make_double2(x, x);
+      if (logabs) *logabs = x;
+    } else {
+      acc.store(det, logabs);
     }
-    acc.store(det, logabs);
   }
 }
 
@@ -665,7 +667,7 @@ int kls_run_lu(kls_ctx* c, int n) {
       cudaLaunchAttribute at;
       cudaLaunchConfig_t cfg = lup_config(C, n, lup_smem(c->Na, slots), c->stream, &at);
       const double2* A = c->d_A;
-      KlsLuWait wait{c->lu_wait_ns, c->h_lu_err, c->lu_skip};
+      KlsLuWait wait{c->lu_wait_ns, c->lu_skip};
       c->lu_skip = -1;
       void* args[] = {&c->Na, (void*)&slots, (void*)&C, &A, &c->d_det, &c->d_logabs, &wait};
       KLS_CK(c, cudaLaunchKernelExC(&cfg, wide ? k.wide : k.one, args));

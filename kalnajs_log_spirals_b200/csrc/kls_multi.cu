@@ -264,7 +264,7 @@ int launch_batch(kls_multi* m) {
                                  m->d_items, m->d_starts, m->grid, m->max_K_pad, m->d_err);
   }
   if (r) return mcuda(m, (cudaError_t)r, "uneven batch launch");
-  KlsLuWait wait{0, m->d_err, -1};
+  KlsLuWait wait{0, -1};
   for (kls_ctx* c : m->ctx) {
     wait.ns = std::max(wait.ns, c->lu_wait_ns);
     wait.skip = std::max(wait.skip, c->lu_skip);
@@ -279,12 +279,12 @@ int launch_batch(kls_multi* m) {
   return KLS_OK;
 }
 
-// the error word of a pass
-int pass_error(kls_multi* m, int code) {
-  if (code == KLS_LU_TIMED_OUT)
-    return mfail(m, KLS_ERR_TIMEOUT, "LU: a bounded wait ran out; results of this pass are invalid");
-  return mfail(m, KLS_ERR_CUDA,
-               "mixed contraction pipeline timed out (code " + std::to_string(code) + ")");
+// the determinants of a pass
+int lu_check(kls_multi* m) {
+  for (size_t z = 0; z < (size_t)m->n_models * m->batch; ++z)
+    if (kls_lu_timed_out(m->h_det + 2 * z))
+      return mfail(m, KLS_ERR_TIMEOUT, "LU: a bounded wait ran out; results of this pass are invalid");
+  return KLS_OK;
 }
 
 // One eager pass (kernel attributes are set outside any capture and the
@@ -303,8 +303,13 @@ int eager_pass(kls_multi* m, float* ms) {
   if (r) return r;
   KM_CK(m, cudaEventRecord(m->ev1, m->stream));
   KM_CK(m, cudaMemcpyAsync(m->h_err, m->d_err, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
+  KM_CK(m, cudaMemcpyAsync(m->h_det, m->d_det, nz * sizeof(double2), cudaMemcpyDeviceToHost,
+                           m->stream));
   KM_CK(m, cudaStreamSynchronize(m->stream));
-  if (*m->h_err) return pass_error(m, *m->h_err);
+  if (*m->h_err)
+    return mfail(m, KLS_ERR_CUDA,
+                 "mixed contraction pipeline timed out (code " + std::to_string(*m->h_err) + ")");
+  if ((r = lu_check(m))) return r;
   if (ms) KM_CK(m, cudaEventElapsedTime(ms, m->ev0, m->ev1));
   return KLS_OK;
 }
@@ -351,9 +356,10 @@ int replay(kls_multi* m) {
     *m->h_err = 0;
     cudaMemsetAsync(m->d_err, 0, sizeof(int), m->stream);
     cudaStreamSynchronize(m->stream);
-    return pass_error(m, code);
+    return mfail(m, KLS_ERR_CUDA,
+                 "mixed contraction pipeline timed out (code " + std::to_string(code) + ")");
   }
-  return KLS_OK;
+  return lu_check(m);
 }
 
 // omegas for model i (n of them, interleaved) -> results, chunked by batch
