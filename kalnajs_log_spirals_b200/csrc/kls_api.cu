@@ -67,6 +67,31 @@ __global__ void transpose_kernel(int n, const double2* __restrict__ in, double2*
       out[(size_t)(c0 + y) * n + r0 + x] = t[x][y];
 }
 
+constexpr size_t EXPORT_KEEP = (size_t)64 << 20;
+
+// rows of V (pairs Re, Im at the alphas >= 0) to columns of W: pairs p0 .. p0 + n - 1 to
+// pos[pair - p0][row], their conjugates to neg[alpha - lo][row], alpha = np - 1 - pair,
+// where that alpha is one of the n_neg below 0
+__global__ void __launch_bounds__(256)
+export_kernel(int rows, int ld, int p0, int n, int np, int lo, int n_neg,
+              const double* __restrict__ V, double2* __restrict__ pos, double2* __restrict__ neg) {
+  __shared__ double2 t[32][17];
+  const int r0 = blockIdx.x * 32, q0 = blockIdx.y * 16;
+  for (int e = threadIdx.x; e < 32 * 16; e += 256) {
+    const int r = e >> 4, q = e & 15;
+    if (r0 + r < rows && q0 + q < n)
+      t[r][q] = *reinterpret_cast<const double2*>(V + (size_t)(r0 + r) * ld + 2 * (p0 + q0 + q));
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < 32 * 16; e += 256) {
+    const int r = e & 31, q = e >> 5, a = np - 1 - (p0 + q0 + q);
+    if (r0 + r >= rows || q0 + q >= n) continue;
+    const double2 w = t[r][q];
+    pos[(size_t)(q0 + q) * rows + r0 + r] = w;
+    if (a < n_neg) neg[(size_t)(a - lo) * rows + r0 + r] = make_double2(w.x, -w.y);
+  }
+}
+
 int validate(const kls_config* k, std::string& msg) {
   char buf[256];
   auto bad = [&](const char* m) { msg = m; return KLS_ERR_CONFIG; };
@@ -144,6 +169,13 @@ void free_F(kls_ctx* c) {
   c->device_bytes -= (int64_t)c->F_bytes;
   c->d_F = nullptr;
   c->F_bytes = 0;
+}
+
+void free_export(kls_ctx* c) {
+  dfree(c->d_export);
+  c->device_bytes -= (int64_t)c->export_bytes;
+  c->d_export = nullptr;
+  c->export_bytes = 0;
 }
 
 // the FP64 contraction's work items and partials (self-similar form: F) for n omegas
@@ -391,7 +423,7 @@ int kls_destroy(kls_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   kls_mixed_free(c);
   kls_similar_free(c);
-  void* ptrs[] = {c->base, c->ws, c->d_V, c->d_items, c->d_tiles, c->d_F, c->d_part, c->d_anchorM};
+  void* ptrs[] = {c->base, c->ws, c->d_export, c->d_V, c->d_items, c->d_tiles, c->d_F, c->d_part, c->d_anchorM};
   for (void* p : ptrs) dfree(p);
   for (auto& ev : c->ev) if (ev) cudaEventDestroy(ev);
   for (auto& ev : c->pev) if (ev) cudaEventDestroy(ev);
@@ -514,40 +546,55 @@ int kls_export_W(kls_ctx* c, int il0, int nl, double* W) {
   if (r) return r;
   if (il0 < 0 || nl < 0 || il0 + nl > c->n_l || !W)
     return kls_fail(c, KLS_ERR_CONFIG, "bad harmonic range for kls_export_W");
+  if (nl == 0) return KLS_OK;
+  // Blocks of harmonics; without the table their rows are formed first.  A harmonic is
+  // transposed on the device, a range of pairs (alpha, -alpha) at a time, each range to
+  // its place in W: two copies of whole columns (through host loops one harmonic of 2121
+  // orbits took 1.5 to 2.3 ms).
   const size_t rows = c->NPh, ld = c->ldv;
-  const int np = (c->Na + 1) / 2;
-  std::vector<double> v(rows * ld);
-  // without the table its rows are formed for 32 harmonics at a time
-  constexpr int NB = 32;
-  double* tmp = nullptr;
-  if (!c->d_V && nl > 0)
-    KLS_CK(c, cudaMalloc(&tmp, (size_t)std::min(nl, NB) * rows * ld * sizeof(double)));
-  struct Free { double* p; ~Free() { cudaFree(p); } } guard{tmp};
-  for (int q = 0; q < nl; ++q) {
+  const int np = (c->Na + 1) / 2, n_neg = c->Na - np;
+  const size_t vblk = rows * ld * sizeof(double), pair = 2 * rows * sizeof(double2);
+  const int nb = c->d_V ? 0 : (int)std::min<size_t>(std::min(nl, 32), std::max<size_t>(1, EXPORT_KEEP / vblk));
+  const int np_at = (int)std::min<size_t>(np, std::max<size_t>(1, EXPORT_KEEP / 2 / pair));
+  const size_t need = nb * vblk + np_at * pair;
+  if (need > c->export_bytes) {
+    free_export(c);
+    char* p = nullptr;
+    if ((r = dalloc(c, &p, need))) return r;
+    c->d_export = p;
+    c->export_bytes = need;
+  }
+  double* tmp = (double*)c->d_export;
+  double2* pos = (double2*)((char*)c->d_export + nb * vblk);
+  double2* neg = pos + (size_t)np_at * rows;
+  for (int q = 0; q < nl && !r; ++q) {
     const double* src = c->d_V + (size_t)(il0 + q) * rows * ld;
-    if (!c->d_V) {
-      if (q % NB == 0) {
-        if ((r = kls_run_wl(c, c->NPh, c->cfg.l_min + il0 + q, std::min(NB, nl - q), c->d_of,
-                            c->d_valid, c->d_w1, c->d_ra, c->d_pha, tmp)))
-          return r;
-        KLS_CK(c, cudaStreamSynchronize(c->stream));
-      }
-      src = tmp + (size_t)(q % NB) * rows * ld;
+    if (nb) {
+      if (q % nb == 0)
+        r = kls_run_wl(c, c->NPh, il0 + q, std::min(nb, nl - q), c->d_of, c->d_valid, c->d_w1, c->d_ra,
+                       c->d_pha, tmp);
+      src = tmp + (size_t)(q % nb) * rows * ld;
     }
-    KLS_CK(c, cudaMemcpy(v.data(), src, rows * ld * sizeof(double), cudaMemcpyDeviceToHost));
     // reference layout [NPh, N_alpha, n_l], column-major, interleaved complex;
     // W(-alpha) = conj W(alpha)
     double* blk = W + (size_t)2 * q * rows * c->Na;
-    for (int a = 0; a < c->Na; ++a) {
-      const bool neg = a < c->Na - np;
-      const size_t pair = neg ? np - 1 - a : a - (c->Na - np);
-      for (size_t p = 0; p < rows; ++p) {
-        blk[2 * (p + rows * a)] = v[p * ld + 2 * pair];
-        const double im = v[p * ld + 2 * pair + 1];
-        blk[2 * (p + rows * a) + 1] = neg ? -im : im;
-      }
+    for (int p0 = 0; p0 < np && !r; p0 += np_at) {
+      const int n = std::min(np_at, np - p0);
+      // pairs p0 .. p0 + n - 1: alphas n_neg + p0 .. and, downwards, np - 1 - p0 ..
+      const int lo = std::max(0, np - p0 - n), n_lo = std::min(np - p0, n_neg) - lo;
+      export_kernel<<<dim3((unsigned)((rows + 31) / 32), (n + 15) / 16), 256, 0, c->stream>>>(
+          (int)rows, (int)ld, p0, n, np, lo, n_neg, src, pos, neg);
+      KLS_LAUNCHED(c);
+      KLS_CK(c, cudaMemcpyAsync(blk + 2 * rows * (n_neg + p0), pos, n * rows * sizeof(double2),
+                                cudaMemcpyDeviceToHost, c->stream));
+      if (n_lo > 0)
+        KLS_CK(c, cudaMemcpyAsync(blk + 2 * rows * lo, neg, n_lo * rows * sizeof(double2),
+                                  cudaMemcpyDeviceToHost, c->stream));
     }
   }
+  if (r) return r;
+  KLS_CK(c, cudaStreamSynchronize(c->stream));
+  if (c->export_bytes > EXPORT_KEEP) free_export(c);
   return KLS_OK;
 }
 

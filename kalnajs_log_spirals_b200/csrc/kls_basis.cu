@@ -32,7 +32,6 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
 }
 
 // ---- W table kernel --------------------------------------------------------
-constexpr int WL_LB = 32;      // harmonics per CTA
 constexpr int WL_AB = 64;      // alphas per CTA
 constexpr int WL_BK = 16;      // samples per chunk
 constexpr int WL_SC = WL_BK + 4;   // smem row stride of C [l][k] (== 4 mod 16)
@@ -41,6 +40,7 @@ constexpr int WL_THREADS = 128;
 
 struct WlParams {
   int NPh, nwa, np, ldv, n_l, l_min, m;   // np alphas >= 0
+  int skip;              // first harmonics that are formed for their anchor's sake only
   double astep;          // alpha grid step
 };
 
@@ -51,12 +51,16 @@ struct WlParams {
 // Bound: the FP64 pipe, which DMMA and the generation of C and E share.  255 orbits
 // of the default grid 4.61 -> 3.97 ms, all 25551 456 -> 395 ms: before, each of the 8
 // threads of a sample computed its logarithm, root, two of its four sincos and its
-// weight in every chunk.
+// weight in every chunk.  MT tiles of 8 harmonics a CTA: 4, or 1 for up to 8 harmonics
+// (one exported harmonic of 2121 orbits); a harmonic's bits are the same, as it is
+// rotated from the same multiple of 4.
+template <int MT>
 __global__ void __launch_bounds__(WL_THREADS)
 wl_kernel(WlParams P, const double* __restrict__ of, const int* __restrict__ valid,
           const double* __restrict__ w1g, const double* __restrict__ rag,
           const double* __restrict__ phag, const double* __restrict__ alpha,
           double* __restrict__ V) {
+  constexpr int WL_LB = 8 * MT;   // harmonics per CTA
   __shared__ double sC[WL_LB * WL_SC];
   __shared__ double sEr[WL_BK * WL_SE];
   __shared__ double sEi[WL_BK * WL_SE];
@@ -78,10 +82,10 @@ wl_kernel(WlParams P, const double* __restrict__ of, const int* __restrict__ val
   const double ratio = KLS_LD(KLS_IB(p, NPh, KS_WL_SAMPLES),
                               of[(size_t)OF_OM2 * NPh + p] / of[(size_t)OF_OM1 * NPh + p], 0.0);
 
-  // accumulators: warp covers all 32 harmonics (4 m-tiles) x 16 alphas (2 n-tiles)
-  double accR[4][2][2], accI[4][2][2];
+  // accumulators: warp covers all harmonics (MT m-tiles) x 16 alphas (2 n-tiles)
+  double accR[MT][2][2], accI[MT][2][2];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < MT; ++i)
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       accR[i][j][0] = accR[i][j][1] = 0.0;
@@ -90,7 +94,7 @@ wl_kernel(WlParams P, const double* __restrict__ of, const int* __restrict__ val
 
   // generator assignment: 16 samples x 8 sub-runs
   const int gk = tid & 15, gsub = tid >> 4;       // gsub 0..7
-  const int l_first = lb * WL_LB + gsub * 4;       // C: 4 harmonics
+  const int l_first = lb * WL_LB + gsub * 4;       // C: 4 harmonics (2 MT sub-runs)
   const int a_first = ab * WL_AB + gsub * 8;       // E: 8 alphas
 
   if (ok) {
@@ -123,18 +127,22 @@ wl_kernel(WlParams P, const double* __restrict__ of, const int* __restrict__ val
       const int k = k0 + gk, e = k % WL_THREADS;
       if (k < nwa) {
         // C: cos(l w1 + m phi), anchor at l_first, rotate by w1
-        const double sw = smp[1][e];
-        double th = (double)(P.l_min + l_first) * smp[0][e] + smp[2][e];
-        double s, c, ss = smp[4][e], cs = smp[3][e];
-        sincos(th, &s, &c);
+        double s, c, cs, ss;
+        if (MT == 4 || gsub < 2 * MT) {
+          const double sw = smp[1][e];
+          double th = (double)(P.l_min + l_first) * smp[0][e] + smp[2][e];
+          ss = smp[4][e];
+          cs = smp[3][e];
+          sincos(th, &s, &c);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          double v = sw * c;
-          if (!isfinite(v)) v = 0.0;
-          sC[(gsub * 4 + j) * WL_SC + gk] = (l_first + j < P.n_l) ? v : 0.0;
-          double cn = c * cs - s * ss;
-          s = s * cs + c * ss;
-          c = cn;
+          for (int j = 0; j < 4; ++j) {
+            double v = sw * c;
+            if (!isfinite(v)) v = 0.0;
+            sC[(gsub * 4 + j) * WL_SC + gk] = (l_first + j < P.n_l) ? v : 0.0;
+            double cn = c * cs - s * ss;
+            s = s * cs + c * ss;
+            c = cn;
+          }
         }
         // E: r^{-1/2} e^{-i alpha ln r}, anchor at a_first, rotate by -astep ln r
         const double lr = smp[5][e], isq = smp[6][e];
@@ -155,8 +163,9 @@ wl_kernel(WlParams P, const double* __restrict__ of, const int* __restrict__ val
           c = cn;
         }
       } else {
+        if (MT == 4 || gsub < 2 * MT)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) sC[(gsub * 4 + j) * WL_SC + gk] = 0.0;
+          for (int j = 0; j < 4; ++j) sC[(gsub * 4 + j) * WL_SC + gk] = 0.0;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           sEr[gk * WL_SE + gsub * 8 + j] = 0.0;
@@ -167,9 +176,9 @@ wl_kernel(WlParams P, const double* __restrict__ of, const int* __restrict__ val
       // ---- 4 k-steps of m8n8k4
 #pragma unroll
       for (int kk = 0; kk < WL_BK; kk += 4) {
-        double a[4], br[2], bi[2];
+        double a[MT], br[2], bi[2];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = sC[(i * 8 + (lane >> 2)) * WL_SC + kk + (lane & 3)];
+        for (int i = 0; i < MT; ++i) a[i] = sC[(i * 8 + (lane >> 2)) * WL_SC + kk + (lane & 3)];
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           int col = warp * 16 + j * 8 + (lane >> 2);
@@ -177,7 +186,7 @@ wl_kernel(WlParams P, const double* __restrict__ of, const int* __restrict__ val
           bi[j] = sEi[(kk + (lane & 3)) * WL_SE + col];
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < MT; ++i)
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
             dmma(accR[i][j][0], accR[i][j][1], a[i], br[j]);
@@ -189,10 +198,10 @@ wl_kernel(WlParams P, const double* __restrict__ of, const int* __restrict__ val
   }
   // ---- epilogue: W / pi into rows il*NPh + p
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < MT; ++i) {
     int il = lb * WL_LB + i * 8 + (lane >> 2);
-    if (il >= P.n_l) continue;
-    size_t row = ((size_t)il * NPh + p) * P.ldv;
+    if (il < P.skip || il >= P.n_l) continue;
+    size_t row = ((size_t)(il - P.skip) * NPh + p) * P.ldv;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       int a0 = ab * WL_AB + warp * 16 + j * 8 + 2 * (lane & 3);
@@ -292,17 +301,20 @@ int kls_run_basis(kls_ctx* c) {
   return KLS_OK;
 }
 
-int kls_run_wl(kls_ctx* c, int n_orb, int l_min, int n_l, const double* of, const int* valid,
+int kls_run_wl(kls_ctx* c, int n_orb, int il0, int n_l, const double* of, const int* valid,
                const double* w1, const double* ra, const double* pha, double* V) {
   WlParams P{};
-  P.NPh = n_orb; P.nwa = c->nwa; P.np = (c->Na + 1) / 2; P.ldv = c->ldv; P.n_l = n_l;
-  P.l_min = l_min; P.m = c->cfg.m;
+  // harmonics are rotated from every 4th of the model's
+  P.skip = il0 % 4;
+  P.NPh = n_orb; P.nwa = c->nwa; P.np = (c->Na + 1) / 2; P.ldv = c->ldv; P.n_l = n_l + P.skip;
+  P.l_min = c->cfg.l_min + il0 - P.skip; P.m = c->cfg.m;
   P.astep = c->Na > 1 ? (2.0 * c->cfg.alpha_max) / (double)(c->Na - 1) : 0.0;
-  dim3 grid((unsigned)n_orb * ((n_l + WL_LB - 1) / WL_LB) * ((P.np + WL_AB - 1) / WL_AB));
+  const int lb = P.n_l <= 8 ? 8 : 32;
+  dim3 grid((unsigned)n_orb * ((P.n_l + lb - 1) / lb) * ((P.np + WL_AB - 1) / WL_AB));
   kls_pre_mark(c, 2);
   // the alphas >= 0 are the last np of the grid
-  wl_kernel<<<grid, WL_THREADS, 0, c->stream>>>(P, of, valid, w1, ra, pha,
-                                                c->d_alpha + (c->Na - P.np), V);
+  (lb == 8 ? wl_kernel<1> : wl_kernel<4>)<<<grid, WL_THREADS, 0, c->stream>>>(
+      P, of, valid, w1, ra, pha, c->d_alpha + (c->Na - P.np), V);
   KLS_LAUNCHED(c);
   kls_pre_mark(c, 3);
   return KLS_OK;
@@ -326,7 +338,7 @@ int kls_build_table(kls_ctx* c) {
   if (c->K_pad > c->K)
     KLS_CK(c, cudaMemsetAsync(c->d_V + (size_t)c->K * c->ldv, 0,
                               (size_t)(c->K_pad - c->K) * c->ldv * sizeof(double), c->stream));
-  return kls_run_wl(c, c->NPh, c->cfg.l_min, c->n_l, c->d_of, c->d_valid, c->d_w1, c->d_ra,
+  return kls_run_wl(c, c->NPh, 0, c->n_l, c->d_of, c->d_valid, c->d_w1, c->d_ra,
                     c->d_pha, c->d_V);
 }
 

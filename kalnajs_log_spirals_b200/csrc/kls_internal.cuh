@@ -175,6 +175,8 @@ struct kls_ctx {
   void* d_F = nullptr;        // self-similar form: F of a chunk of omegas
   size_t F_bytes = 0;
   double2* d_A = nullptr;     // [ws_omega][Na][Na]  I - M (row-major), overwritten by LU
+  void* d_export = nullptr;   // kls_export_W: rows and their transpose, kept up to 64 MB
+  size_t export_bytes = 0;
   double2* d_M = nullptr;     // [Na][Na] optional M export (row-major beta, alpha)
   // KLS_MODE_ANCHORED: FP64 M at the anchor omega (row-major beta, alpha)
   double2* d_anchorM = nullptr;
@@ -256,8 +258,9 @@ size_t kls_orbit_table(int nw, int nwai);   // entries of d_cs
 int kls_run_orbits(kls_ctx* c);
 int kls_upload_alpha(kls_ctx* c);
 int kls_run_basis(kls_ctx* c);
-// W rows of n_orb orbits and n_l harmonics from l_min: V[il * n_orb + p][ldv]
-int kls_run_wl(kls_ctx* c, int n_orb, int l_min, int n_l, const double* of, const int* valid,
+// W rows of n_orb orbits and the model's harmonics il0 .. il0 + n_l - 1:
+// V[(il - il0) * n_orb + p][ldv]
+int kls_run_wl(kls_ctx* c, int n_orb, int il0, int n_l, const double* of, const int* valid,
                const double* w1, const double* ra, const double* pha, double* V);
 int kls_build_table(kls_ctx* c);     // the whole FP64 table into c->d_V
 void kls_drop_table(kls_ctx* c);

@@ -954,7 +954,7 @@ int kls_similar_prepare(kls_ctx* c) {
   reference_kernel<<<dim3((nwa + 127) / 128, Ne, 5), 128, 0, c->stream>>>(Ne, nwa, d_fit, rw, rr,
                                                                           rp);
   c->launches += 3;
-  int r = kls_run_wl(c, (int)n5, c->cfg.l_min, c->n_l, d_of5, d_ok, rw, rr, rp, d_T);
+  int r = kls_run_wl(c, (int)n5, 0, c->n_l, d_of5, d_ok, rw, rr, rp, d_T);
   if (r) return bail(r);
   combine_kernel<<<s->R, 128, 0, c->stream>>>(c->n_l, Ne, c->ldv, c->cfg.l_min, d_T, s->V, s->Vf,
                                                 s->D, d_mx);
