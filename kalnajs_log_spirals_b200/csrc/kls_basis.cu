@@ -19,7 +19,13 @@
 // * Per-row resonant data, row k = il*NPh + p (BasisFunctions.jl:127-153):
 //   G_k = DJ_p * F0l[p,l], F0l = (l Om1 + m Om2) FE + m FL,
 //   Omega_res = l Om1 + m Om2.
+// * Resonant weights w_k(omega) = G_k / den for a batch of omegas, den = omega -
+//   Omega_res, den := 1e-12 + 1e-12 i when |den| < 1e-12 (MatrixBuilder.jl:27-69).
+//   Here and not with a contraction: every form takes them, and a module is loaded at
+//   the first call that needs a kernel of it (this one by the precompute; the table
+//   contraction's 3 MB took the first determinant of a process 1.5 ms).
 #include "kls_internal.cuh"
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 
@@ -285,6 +291,76 @@ __global__ void rows_kernel(int NPh, int n_l, int l_min, int m, int64_t K, int64
   F0l[k] = f0l;
 }
 
+// ---- weights ---------------------------------------------------------------
+// 1/z by Smith's algorithm (R. L. Smith, CACM 5(8), 1962), then a * (1/z):
+// the same evaluation order as Julia's a / z for a real a.
+__device__ __forceinline__ double2 real_over_complex(double a, double c, double d) {
+  double p, q;
+  if (fabs(d) <= fabs(c)) {
+    double r = d / c;
+    double t = 1.0 / (c + d * r);
+    p = t;
+    q = -r * t;
+  } else {
+    double r = c / d;
+    double t = 1.0 / (d + c * r);
+    p = r * t;
+    q = -t;
+  }
+  return make_double2(a * p, a * q);
+}
+
+__device__ __forceinline__ double2 weight_at(double g, double ok, double wr, double wi) {
+  double dr = wr - ok, di = wi;
+  if (hypot(dr, di) < 1e-12) { dr = 1e-12; di = 1e-12; }
+  return real_over_complex(g, dr, di);
+}
+
+__device__ __forceinline__ void weights_body(int64_t K_pad, double wr, double wi,
+                                             const double* __restrict__ Gk,
+                                             const double* __restrict__ Ok,
+                                             double2* __restrict__ out) {
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < K_pad;
+       k += (int64_t)gridDim.x * blockDim.x)
+    KLS_IF(KLS_IB(k, K_pad, KS_WEIGHTS)) out[k] = weight_at(Gk[k], Ok[k], wr, wi);
+}
+
+// anchored: w_k(omega) - w_k(omega_a), each with the denominator clamp; the
+// FP64 difference loses ~|w| / |dw| ulps, far below the FP32 rounding the
+// split-BF16 contraction applies next
+__global__ void weights_kernel(int64_t K_pad, const double* __restrict__ omega,
+                               const double* __restrict__ Gk, const double* __restrict__ Ok,
+                               double2* __restrict__ wt, int anchored, double ar, double ai) {
+  const int z = blockIdx.y;
+  const double wr = omega[2 * z], wi = omega[2 * z + 1];
+  double2* out = wt + (size_t)z * K_pad;
+  if (!anchored) {
+    weights_body(K_pad, wr, wi, Gk, Ok, out);
+    return;
+  }
+  if (wr == ar && wi == ai) {                // at the anchor dM is exactly zero
+    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < K_pad;
+         k += (int64_t)gridDim.x * blockDim.x)
+      KLS_IF(KLS_IB(k, K_pad, KS_WEIGHTS)) out[k] = make_double2(0.0, 0.0);
+    return;
+  }
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < K_pad;
+       k += (int64_t)gridDim.x * blockDim.x) {
+    KLS_UNLESS(KLS_IB(k, K_pad, KS_WEIGHTS), continue)
+    const double2 a = weight_at(Gk[k], Ok[k], wr, wi), b = weight_at(Gk[k], Ok[k], ar, ai);
+    out[k] = make_double2(a.x - b.x, a.y - b.y);
+  }
+}
+
+// one (model, omega) pair per grid row
+__global__ void multi_weights_kernel(const kls_mdesc* __restrict__ md,
+                                     const int2* __restrict__ pairs) {
+  const int2 pz = pairs[blockIdx.y];
+  const kls_mdesc& d = md[pz.x];
+  const double* om = d.omega + 2 * pz.y;
+  weights_body(d.K_pad, om[0], om[1], d.Gk, d.Ok, d.wt + (size_t)pz.y * d.K_pad);
+}
+
 }  // namespace
 
 int kls_run_basis(kls_ctx* c) {
@@ -347,4 +423,20 @@ void kls_drop_table(kls_ctx* c) {
   cudaFree(c->d_V);
   c->d_V = nullptr;
   c->device_bytes -= (int64_t)((size_t)c->K_pad * c->ldv * sizeof(double));
+}
+
+int kls_run_weights(kls_ctx* c, int n, const double* anchor) {
+  int blocks = (int)std::min<int64_t>((c->K_pad + 255) / 256, 2048);
+  weights_kernel<<<dim3(blocks, n), 256, 0, c->stream>>>(
+      c->K_pad, c->d_omega, c->d_Gk, c->d_Ok, c->d_wt, anchor ? 1 : 0, anchor ? anchor[0] : 0.0,
+      anchor ? anchor[1] : 0.0);
+  KLS_LAUNCHED(c);
+  return KLS_OK;
+}
+
+int kls_multi_launch_f64_weights(cudaStream_t st, const kls_mdesc* d_md, const int2* d_pairs,
+                                 int n_pairs, int64_t max_K_pad) {
+  int wblocks = (int)std::min<int64_t>((max_K_pad + 255) / 256, 1024);
+  multi_weights_kernel<<<dim3(wblocks, n_pairs), 256, 0, st>>>(d_md, d_pairs);
+  return (int)cudaGetLastError();
 }

@@ -11,7 +11,7 @@
 // pipe (DMMA m8n8k4) and the resonant weight is applied to the A fragment
 // while it is loaded from shared memory, so the weighted copy never exists.
 //
-//   weights_kernel : w_k(omega) for a batch of omegas (FP64, Smith division)
+//   weights_kernel : w_k(omega) for a batch of omegas (kls_basis.cu)
 //   contract_kernel: one triangle of T = sum_k w_k V_k^T V_k, 64 x 64 parts,
 //                    cp.async 4-stage pipeline over 16-row slabs of the
 //                    table, partial parts per K split written to a workspace
@@ -38,76 +38,6 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
-}
-
-// ---- weights ---------------------------------------------------------------
-// 1/z by Smith's algorithm (R. L. Smith, CACM 5(8), 1962), then a * (1/z):
-// the same evaluation order as Julia's a / z for a real a.
-__device__ __forceinline__ double2 real_over_complex(double a, double c, double d) {
-  double p, q;
-  if (fabs(d) <= fabs(c)) {
-    double r = d / c;
-    double t = 1.0 / (c + d * r);
-    p = t;
-    q = -r * t;
-  } else {
-    double r = c / d;
-    double t = 1.0 / (d + c * r);
-    p = r * t;
-    q = -t;
-  }
-  return make_double2(a * p, a * q);
-}
-
-__device__ __forceinline__ double2 weight_at(double g, double ok, double wr, double wi) {
-  double dr = wr - ok, di = wi;
-  if (hypot(dr, di) < 1e-12) { dr = 1e-12; di = 1e-12; }
-  return real_over_complex(g, dr, di);
-}
-
-__device__ __forceinline__ void weights_body(int64_t K_pad, double wr, double wi,
-                                             const double* __restrict__ Gk,
-                                             const double* __restrict__ Ok,
-                                             double2* __restrict__ out) {
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < K_pad;
-       k += (int64_t)gridDim.x * blockDim.x)
-    KLS_IF(KLS_IB(k, K_pad, KS_WEIGHTS)) out[k] = weight_at(Gk[k], Ok[k], wr, wi);
-}
-
-// anchored: w_k(omega) - w_k(omega_a), each with the denominator clamp; the
-// FP64 difference loses ~|w| / |dw| ulps, far below the FP32 rounding the
-// split-BF16 contraction applies next
-__global__ void weights_kernel(int64_t K_pad, const double* __restrict__ omega,
-                               const double* __restrict__ Gk, const double* __restrict__ Ok,
-                               double2* __restrict__ wt, int anchored, double ar, double ai) {
-  const int z = blockIdx.y;
-  const double wr = omega[2 * z], wi = omega[2 * z + 1];
-  double2* out = wt + (size_t)z * K_pad;
-  if (!anchored) {
-    weights_body(K_pad, wr, wi, Gk, Ok, out);
-    return;
-  }
-  if (wr == ar && wi == ai) {                // at the anchor dM is exactly zero
-    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < K_pad;
-         k += (int64_t)gridDim.x * blockDim.x)
-      KLS_IF(KLS_IB(k, K_pad, KS_WEIGHTS)) out[k] = make_double2(0.0, 0.0);
-    return;
-  }
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < K_pad;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    KLS_UNLESS(KLS_IB(k, K_pad, KS_WEIGHTS), continue)
-    const double2 a = weight_at(Gk[k], Ok[k], wr, wi), b = weight_at(Gk[k], Ok[k], ar, ai);
-    out[k] = make_double2(a.x - b.x, a.y - b.y);
-  }
-}
-
-// one (model, omega) pair per grid row
-__global__ void multi_weights_kernel(const kls_mdesc* __restrict__ md,
-                                     const int2* __restrict__ pairs) {
-  const int2 pz = pairs[blockIdx.y];
-  const kls_mdesc& d = md[pz.x];
-  const double* om = d.omega + 2 * pz.y;
-  weights_body(d.K_pad, om[0], om[1], d.Gk, d.Ok, d.wt + (size_t)pz.y * d.K_pad);
 }
 
 // ---- contraction -----------------------------------------------------------
@@ -597,15 +527,6 @@ int kls_f64_plan(kls_ctx* c) {
 
 size_t kls_f64_part_elems(const kls_ctx* c, int n) { return (size_t)n * c->n_slots * CT_SLOT; }
 
-int kls_run_weights(kls_ctx* c, int n, const double* anchor) {
-  int blocks = (int)std::min<int64_t>((c->K_pad + 255) / 256, 2048);
-  weights_kernel<<<dim3(blocks, n), 256, 0, c->stream>>>(
-      c->K_pad, c->d_omega, c->d_Gk, c->d_Ok, c->d_wt, anchor ? 1 : 0, anchor ? anchor[0] : 0.0,
-      anchor ? anchor[1] : 0.0);
-  KLS_LAUNCHED(c);
-  return KLS_OK;
-}
-
 int kls_run_contract_f64(kls_ctx* c, int n) {
   KLS_CK(c, cudaFuncSetAttribute(contract_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)CT_SMEM));
@@ -637,13 +558,6 @@ int kls_multi_launch_f64(cudaStream_t st, const kls_mdesc* d_md, const int2* d_p
   if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
   const int n8 = max_ldv / 8;
   multi_reduce_kernel<<<dim3(n8 * (n8 + 1) / 2, n_pairs), RD_THREADS, 0, st>>>(d_md, d_pairs);
-  return (int)cudaGetLastError();
-}
-
-int kls_multi_launch_f64_weights(cudaStream_t st, const kls_mdesc* d_md, const int2* d_pairs,
-                                 int n_pairs, int64_t max_K_pad) {
-  int wblocks = (int)std::min<int64_t>((max_K_pad + 255) / 256, 1024);
-  multi_weights_kernel<<<dim3(wblocks, n_pairs), 256, 0, st>>>(d_md, d_pairs);
   return (int)cudaGetLastError();
 }
 

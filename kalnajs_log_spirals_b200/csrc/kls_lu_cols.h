@@ -1,4 +1,4 @@
-// The columns that one warp of the pipelined LU (kls_lu.cu) owns, and the one that
+// The columns that one warp of the pipelined LU (kls_lu_pipe.cuh) owns, and the one that
 // it factors next; and the batches that the pipelined form is the faster one for.  Plain
 // C++ as well, so that both can be run on the host.
 #pragma once
