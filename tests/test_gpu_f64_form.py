@@ -67,6 +67,33 @@ def test_self_similar_and_by_choice_the_table(lib_path, Na, NR, Ne, l):
     pc.close()
 
 
+BASE = dict(GRID, **SIMILAR, N_alpha=65, NR=40, Ne=9, l_min=-6, l_max=7)
+
+
+@pytest.mark.parametrize("options", [
+    dict(m=0), dict(m=-2), dict(m=5), dict(n_zang=0), dict(q1=1.2), dict(q1=40),
+    dict(v_min=-1.0), dict(v_min=-0.9, Ne=7), dict(v_min=0.995, Ne=5), dict(Ne=1),
+    dict(Rc_min=1.0, Rc_max=1.0), dict(Rc_min=1e-4, Rc_max=1e4, NR=101), dict(alpha_max=0.0),
+    dict(alpha_max=300.0, N_alpha=129), dict(L0=1e-3), dict(G=1e6), dict(l_min=5, l_max=9),
+    dict(l_min=0, l_max=0), dict(nw=401, nwa=9), dict(nw=101, nwa=101),
+    dict(quadrature="sss"), dict(quadrature="bbb", NR=41), dict(quadrature="tst", NR=41)])
+def test_forms_agree_over_the_options(lib_path, options):
+    """Harmonic number, disk, retrograde and radial orbits, equal radii, a single alpha or
+    eccentricity, quadratures: where the model is self-similar, M as over the table."""
+    o = dict(BASE, **options)
+    quadrature = o.pop("quadrature", "tts")
+    c = kconfig(**o)
+    c.grid.quadrature = quadrature
+    pc = K.precompute_all(c)
+    assert pc.self_similar
+    with np.errstate(all="ignore"):
+        M = K.build_M_matrix(OM[0], pc)
+        tol = tolerance(pc, M)
+        pc.use_table()
+        assert np.all(np.abs(M - K.build_M_matrix(OM[0], pc)) <= tol)
+    pc.close()
+
+
 @pytest.mark.parametrize("grid,NR", [(SIMILAR, 15), (OTHER, 24)])
 def test_models_over_the_table(lib_path, grid, NR):
     """Fewer than 16 radii, or orbits of another form."""
