@@ -20,7 +20,8 @@ GPUBackend.jl:27-31, 50-72     GPUType, detect_gpu_type
 
 Differences a caller can observe, all deliberate:
 
-* ``precompute_all`` runs on the device and leaves the W_l table there; the
+* ``precompute_all`` runs on the device and leaves the FP64 form of M there (W_l of
+  one orbit per eccentricity where the orbits are self-similar, else the table); the
   reference's host arrays (``orbit_data``, ``W_l_mat``, ...) are exported
   lazily on first attribute access.
 * There is no CPU path: ``devprecomp=None`` or ``gpu_type=GPUType.NONE``
@@ -317,7 +318,8 @@ def _mode_for(Tgpu) -> int:
 
 def to_device(precomp: PrecomputedData, gpu_type: GPUType = GPUType.NVIDIA,
               Tgpu="Float64") -> DevicePrecomputed:
-    """BasisFunctions.jl:397-437; the table already lives on the device."""
+    """BasisFunctions.jl:397-437.  The FP64 form already lives on the device; "Float32"
+    builds the split-BF16 table (on self-similar models from the orbits' samples)."""
     mode = _mode_for(Tgpu)
     if mode == KLS_MODE_MIXED:
         precomp.ctx.call("kls_prepare_mixed")
@@ -510,7 +512,7 @@ def harmonic_ranges(l_min: int, l_max: int, n_ranks: int) -> List[Tuple[int, int
 
 def precompute_ksharded(config: KalnajsConfig, group=None, device: Optional[int] = None
                         ) -> PrecomputedData:
-    """This rank's slice of the W table: the harmonics harmonic_ranges(...)[rank]
+    """This rank's slice of the sum over the harmonics: harmonic_ranges(...)[rank]
     (K sharding: the contraction over k = (orbit, l) is a sum, so the slices'
     partial M(omega) add up to M(omega))."""
     import torch

@@ -30,7 +30,7 @@ struct kls_mlp;
 namespace {
 
 constexpr int ML_IN = 5, ML_OUT = 3;
-constexpr int ML_ROWS = 1 << 22;      // rows of a training set kept on the device (0.15 GB)
+constexpr int ML_ROWS = 1 << 22;      // rows of a training set kept on the device (48 B each)
 constexpr int ML_PAD = 16;            // input / output dims padded to 16 for the MMA
 constexpr int GT_THREADS = 128;
 // the small and the large tile, rows = columns, with depth and stages of the
