@@ -804,6 +804,7 @@ int kls_mlp_grad(kls_mlp* m, const float* X, const float* T, int n, float* grads
 int kls_mlp_train(kls_mlp* m, const float* X, const float* T, int n, int epochs, int batch,
                   float lr, uint64_t seed, float* loss_hist) {
   if (!m || n < 1 || batch < 1 || epochs < 0 || !X || !T) return KLS_ERR_CONFIG;
+  if (epochs == 0) return KLS_OK;      // (X and T are the caller's again: no copy of them)
   cudaSetDevice(m->device);
   batch = std::min(batch, n);
   const int steps = n / batch;
@@ -831,7 +832,7 @@ int kls_mlp_train(kls_mlp* m, const float* X, const float* T, int n, int epochs,
   std::mt19937_64 rng(seed);
   std::vector<float> ls(steps);
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-  if (epochs > 0) std::shuffle(idx.begin(), idx.end(), rng);
+  std::shuffle(idx.begin(), idx.end(), rng);
   for (int ep = 0; ep < epochs; ++ep) {
     if (all)
       ML_CK(m, cudaMemcpyAsync(m->idx, idx.data(), (size_t)n * 4, cudaMemcpyHostToDevice,

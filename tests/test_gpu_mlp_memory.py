@@ -34,3 +34,16 @@ def test_gradients_with_little_memory(lib_path):
         torch.cuda.empty_cache()
     assert l0 == l1 and np.array_equal(g0, g1)
     assert np.array_equal(h0, h1) and np.array_equal(p0, p1)
+
+
+def test_no_epochs_touch_nothing(lib_path):
+    """No copy of X and T is under way when a call of no epochs returns: none is made."""
+    n = 1 << 20
+    X, T = np.ones((n, 5), np.float32), np.ones((n, 3), np.float32)
+    mlp = P.MLP(64, 3, seed=2)
+    p = mlp.params()
+    free = torch.cuda.mem_get_info()[0]
+    assert len(mlp.train(X, T, epochs=0, batch=n, lr=1e-3, seed=1)) == 0
+    assert torch.cuda.mem_get_info()[0] == free
+    assert np.array_equal(mlp.params(), p)
+    mlp.close()
