@@ -41,6 +41,7 @@ int kls_fail(kls_ctx* c, int code, const std::string& msg) {
 }
 
 int kls_cuda_fail(kls_ctx* c, cudaError_t e, const char* what) {
+  cudaGetLastError();      // reported here: the next call's launch check must not find it
   std::string m = std::string("CUDA error in ") + what + ": " + cudaGetErrorString(e);
   int code = (e == cudaErrorMemoryAllocation) ? KLS_ERR_OOM : KLS_ERR_CUDA;
   return kls_fail(c, code, m);
@@ -130,6 +131,7 @@ template <typename T>
 int dalloc(kls_ctx* c, T** p, size_t count) {
   cudaError_t e = cudaMalloc((void**)p, count * sizeof(T) + 16);
   if (e != cudaSuccess) {
+    cudaGetLastError();
     *p = nullptr;
     char buf[160];
     snprintf(buf, sizeof buf, "cudaMalloc of %.3f GB failed: %s", count * sizeof(T) / 1e9,

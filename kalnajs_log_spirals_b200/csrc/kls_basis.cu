@@ -401,6 +401,7 @@ int kls_build_table(kls_ctx* c) {
   const bool had = c->d_V != nullptr;
   cudaError_t e = c->d_V ? cudaSuccess : cudaMalloc(&c->d_V, n * sizeof(double));
   if (e != cudaSuccess) {
+    cudaGetLastError();
     c->d_V = nullptr;
     size_t fr = 0, tot = 0;
     cudaMemGetInfo(&fr, &tot);

@@ -107,6 +107,7 @@ struct KlsSlab {
   cudaError_t alloc(void** base) {
     const cudaError_t e = cudaMalloc(base, bytes());
     if (e != cudaSuccess) {
+      cudaGetLastError();    // (the caller reports it)
       *base = nullptr;
       return e;
     }

@@ -473,7 +473,10 @@ int mfail(kls_mlp* m, const std::string& s) {
 #define ML_CK(m, call)                                                            \
   do {                                                                            \
     cudaError_t e_ = (call);                                                      \
-    if (e_ != cudaSuccess) return mfail(m, std::string(#call) + ": " + cudaGetErrorString(e_)); \
+    if (e_ != cudaSuccess) {                                                      \
+      cudaGetLastError();    /* reported here */                                  \
+      return mfail(m, std::string(#call) + ": " + cudaGetErrorString(e_));        \
+    }                                                                             \
   } while (0)
 
 // activations of n rows; `train`: and all that a training pass leaves
@@ -512,7 +515,6 @@ int ensure_cap(kls_mlp* m, int n, bool train) {
       b.add(&m->lpart, (size_t)cap / GT_S);
       e = b.alloc(&m->tslab);
       if (e != cudaErrorMemoryAllocation) break;
-      cudaGetLastError();
     }
     ML_CK(m, e);
     for (int l = 1; m->lean && l < L; ++l) { m->dZt[l] = m->dZt[0]; m->dZf[l] = m->dZf[0]; }

@@ -104,6 +104,7 @@ int mfail(kls_multi* m, int code, const std::string& msg) {
   return code;
 }
 int mcuda(kls_multi* m, cudaError_t e, const char* what) {
+  cudaGetLastError();      // reported here
   return mfail(m, e == cudaErrorMemoryAllocation ? KLS_ERR_OOM : KLS_ERR_CUDA,
                std::string(what) + ": " + cudaGetErrorString(e));
 }
