@@ -314,21 +314,24 @@ int kls_mlp_train(kls_mlp* mlp, const float* X, const float* T, int n, int epoch
  * multi-GPU form GridScan.jl:125-197 splits one model's omega columns over
  * devices).  A kls_multi evaluates `batch` omegas for each of n_models
  * precomputed contexts (any mix of NR, Ne, N_alpha and l range, one device)
- * per pass: the contraction of every model is one persistent launch, and the
- * whole pass (omega upload, weights, contraction, split reduction, LU,
- * result download) is one CUDA graph replay.  Each model keeps its
- * context's K split count (tune with kls_autotune before creating the
- * batch), so every determinant is bitwise what kls_det_batch returns for
- * that context: the batch runs the KLS_MIXED_TMEM kernel body (one CTA pair
- * per model, tile pair and K split, from per-model descriptors) when that is
- * every model's split-BF16 form, else the KLS_MIXED_ONE_CTA body.  The contexts must outlive the batch and are not modified;
- * a batch is not re-entrant.  Errors: kls_multi_last_error (NULL handle:
- * errors of kls_multi_create).                                              */
+ * per pass, and the whole pass (omega upload, weights, M(omega), LU, result
+ * download) is one CUDA graph replay.  In FP64 a self-similar model has its own
+ * launches in the graph and the models over the table share one persistent
+ * contraction; in split BF16 the models of the KLS_MIXED_TMEM form share one
+ * contraction (one CTA pair per model, tile pair and K split) and those of the
+ * other forms one of the KLS_MIXED_ONE_CTA body.  The LU is one launch per size
+ * class.  Each model keeps its context's split count (tune with kls_autotune
+ * before creating the batch), so every determinant is bitwise what kls_det_batch
+ * returns for that context.  The contexts must outlive the batch and are not
+ * modified; an FP64 batch returns KLS_ERR_STATE once a model's FP64 form has been
+ * freed (kls_release_fp64, kls_set_f64_table).  A batch is not re-entrant.  Errors:
+ * kls_multi_last_error (NULL handle: errors of kls_multi_create).           */
 typedef struct kls_multi kls_multi;
 typedef struct kls_multi_info {
     int32_t n_models, batch, mode;
-    int32_t n_items;              /* work items of the persistent contraction */
-    int32_t grid;                 /* CTAs of the persistent contraction       */
+    int32_t n_items;              /* work items of the contractions (a
+                                     self-similar model's: CTAs of its pair sum) */
+    int32_t grid;                 /* CTAs of the contractions                 */
     int32_t graph;                /* 1: passes replay a captured CUDA graph    */
     int32_t launches_per_replay;  /* kernels in one pass                      */
     int64_t replays;              /* passes so far                            */

@@ -736,8 +736,8 @@ def autotune(precomputed: PrecomputedData, Tgpu="Float64", batch: int = 2) -> Tu
 class ModelBatch:
     """Many precomputed models of any sizes evaluated together (kls_multi).
 
-    Each pass evaluates `batch` omegas per model: one persistent contraction
-    launch for all models, replayed from a captured CUDA graph.  Results are
+    Each pass evaluates `batch` omegas per model, replayed from a captured CUDA graph:
+    shared launches, and for self-similar models in FP64 each model's own.  Results are
     bitwise those of compute_determinant_batched on each model's own context.
     """
 

@@ -124,14 +124,14 @@ multi_lu_kernel(const kls_mdesc* __restrict__ md, const int2* __restrict__ pairs
 // batches that it holds in one wave (7 matrices).  From <10,4> on, and a little in
 // others, the registers do not hold all of it (142 bytes spilled a thread, <13,4> 1.0
 // KB, <16,4> 2.2 KB).  1 matrix / 16, us:
-//   N =  64  <2,2> x 4   53 /  53   (<2,8> x 1    71 /  71)
-//   N = 101  <4,3> x 6   99 / 100   (<4,4> x 4   105 / 105, <4,2> x 8 128 / 249)
-//   N = 192  <6,4> x 6  276 / 276   (<6,3> x 8   306 / 605), <6,2> x 12 236 / 693
-//   N = 201  <7,5> x 6  350 / 350   (<7,4> x 8   333 / 656), <7,2> x 14 266 / 790
-//   N = 256  <8,4> x 8  455 / 899   (<8,5> x 7   574 / 1140), <8,2> x 16 398 / 1181
-//   N = 301 <10,4> x 10 558 / 1111  (<10,3> x 16 632 / 1887)
-//   N = 400 <13,4> x 13 1250 / 3748 (<16,4> x 16 3277 / 9852)
-//   N = 512 <16,4> x 16 2936 / 8782
+//   N =  64  <2,2> x 4   51 /  52   (<2,8> x 1    71 /  71)
+//   N = 101  <4,3> x 6   97 /  99   (<4,4> x 4   105 / 105, <4,2> x 8 128 / 249)
+//   N = 192  <6,4> x 6  273 / 275   (<6,3> x 8   306 / 605), <6,2> x 12 236 / 700
+//   N = 201  <7,5> x 6  344 / 348   (<7,4> x 8   333 / 656), <7,2> x 14 267 / 790
+//   N = 256  <8,4> x 8  449 / 892   (<8,5> x 7   574 / 1140), <8,2> x 16 399 / 1185
+//   N = 301 <10,4> x 10 550 / 1097  (<10,3> x 16 632 / 1887)
+//   N = 400 <13,4> x 13 1249 / 3658 (<16,4> x 16 3277 / 9852)
+//   N = 512 <16,4> x 16 2937 / 6513
 // (in brackets: before the warp whose column is next polled)
 struct LupClass {
   int n_max, C;

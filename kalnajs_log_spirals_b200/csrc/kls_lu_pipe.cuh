@@ -1,7 +1,7 @@
 // The pipelined LU, one thread-block cluster per matrix: the kernels of one size class
 // are one translation unit (kls_lu_64.cu and so on).  A module is loaded as a whole at
 // the first call that needs a kernel of it, at about 0.5 ms a megabyte, and all classes
-// together are 6.4 MB.
+// together are 6.4 MB: the first determinant of a process 6.0 -> 1.8 ms.
 #pragma once
 #include "kls_lu_prims.cuh"
 #include "kls_lu_pipe.h"
@@ -28,9 +28,9 @@ namespace {
 // Waits are bounded (KlsLuWait); one that runs out makes the determinant a NaN of its
 // own, which the host turns into KLS_ERR_TIMEOUT.
 //
-// Measured (1 matrix, B200): N = 101 312 -> 99 us, 201 557 -> 266 us, 301 1022 ->
-// 558 us against one CTA (101) or a cluster with one barrier per column; 16
-// matrices 315 -> 100, 612 -> 350, 2760 -> 1111 us.  A column's chain is about
+// Measured (1 matrix, B200): N = 101 312 -> 97 us, 201 557 -> 267 us, 301 1022 ->
+// 550 us against one CTA (101) or a cluster with one barrier per column; 16
+// matrices 315 -> 99, 612 -> 348, 1990 -> 1097 us.  A column's chain is about
 // 1600 cycles at 4 rows a lane and 3300 at 10 (hand-over 160 / 360, update 280 / 540,
 // pivot search with its reciprocal 670 / 1260, broadcast 60 / 80, multipliers and
 // publication 440 / 1100; the marks themselves are some 50 each): about 350

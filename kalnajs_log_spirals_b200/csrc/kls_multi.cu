@@ -8,13 +8,15 @@
 // descriptors (kls_mdesc), and lists the contraction's work items over all
 // models.  One batch is
 //
-//   H2D omegas -> weights (all models) -> persistent contraction (all models)
-//   -> split reduction (all models) -> LU (all models) -> D2H dets
+//   H2D omegas -> weights (all models) -> M(omega) -> LU (a launch per size
+//   class) -> D2H dets
 //
-// captured once into a CUDA graph and replayed for every chunk of omegas.
-// The FP64 contraction takes items from an atomic counter in list order; for
-// the mixed one the batch times one pass with each of two schedules of the
-// same list (a persistent round robin, one CTA per item) and keeps the faster.  Each model's K split count is its context's own
+// captured once into a CUDA graph and replayed for every chunk of omegas.  In FP64 a
+// self-similar model runs its own launches (kls_similar_launch), and the models over
+// the table share a persistent contraction, which takes items from an atomic counter in
+// list order, and a reduction; for the mixed contraction the batch times one pass with
+// each of two schedules of the same list (a persistent round robin, one CTA per item)
+// and keeps the faster.  Each model's split count is its context's own
 // (kls_autotune chooses it), so a determinant from the batch is bitwise the
 // one kls_det_batch returns for the same context.  When every model's
 // split-BF16 form is the TMEM-operand one, the contraction is that form's
