@@ -358,6 +358,8 @@ def cpu_small_size(args, K, local):
 # clocks during the timed region
 # ---------------------------------------------------------------------------
 class ClockSampler:
+    """nvidia-smi every 20 ms; its start takes longer than the timed region may, so the
+    region begins when the first sample is there."""
     FIELDS = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
               "clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
               "clocks_event_reasons.sw_thermal_slowdown,clocks_event_reasons.sw_power_cap")
@@ -367,22 +369,35 @@ class ClockSampler:
         self.f = tempfile.NamedTemporaryFile("w+", suffix=".csv", delete=False)
         try:
             self.p = subprocess.Popen(["nvidia-smi", f"--query-gpu={self.FIELDS}", "--format=csv",
-                                       "-lms", "200", "-i", str(gpu_index)], stdout=self.f,
+                                       "-lms", "20", "-i", str(gpu_index)], stdout=self.f,
                                       stderr=subprocess.DEVNULL)
         except Exception:
             self.p = None
+        self.before = 0
+
+    def _rows(self):
+        with open(self.f.name) as f:
+            text = f.read()
+        return [r.strip() for r in text[:text.rfind("\n") + 1].splitlines()[1:] if r.strip()]
+
+    def ready(self, load, limit: float = 10.0):
+        """Run ``load`` until the first sample is there (at most ``limit`` seconds): the
+        samples from here on are of the timed region."""
+        t0 = time.perf_counter()
+        while self.p is not None and not self._rows() and time.perf_counter() - t0 < limit:
+            load()
+        self.before = len(self._rows())
 
     def stop(self):
         if self.p is None:
             return None
+        rows = self._rows()                # whole lines up to now, the region's end
         self.p.terminate()
         try:
             self.p.wait(timeout=5)
         except Exception:
             self.p.kill()
-        self.f.flush()
-        self.f.seek(0)
-        rows = [r.strip() for r in self.f.read().splitlines()[1:] if r.strip()]
+        rows = rows[self.before:] or rows[-1:]
         sm, mx, reasons = [], None, set()
         names = ["hw_slowdown", "hw_thermal_slowdown", "sw_thermal_slowdown", "sw_power_cap"]
         for r in rows:
@@ -965,6 +980,13 @@ def ours(args):
         barrier()
         torch.cuda.synchronize()
         clocks = ClockSampler(local) if sample_clocks else None
+        if clocks:
+            def load():
+                dev_step(0, mode)
+                torch.cuda.synchronize()
+            clocks.ready(load)
+            barrier()
+            torch.cuda.synchronize()
         l0 = lib.kls_launch_count(h)
         ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         ev0.record(stream)
