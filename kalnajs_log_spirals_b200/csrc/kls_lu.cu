@@ -122,8 +122,8 @@ multi_lu_kernel(const kls_mdesc* __restrict__ md, const int2* __restrict__ pairs
 // The size classes: rows per lane x columns per warp, CTAs per cluster.  4 columns
 // a warp keep enough matrices on the device at once; a wider form (2 columns) for
 // batches that it holds in one wave (7 matrices).  From <10,4> on, and a little in
-// others, the registers do not hold all of it (142 bytes spilled a thread, <13,4> 1.0
-// KB, <16,4> 2.2 KB).  1 matrix / 16, us:
+// others, the registers do not hold all of it (160 bytes spilled a thread, <13,4> 1.0
+// KB, <16,4> 2.1 KB).  1 matrix / 16, us:
 //   N =  64  <2,2> x 4   51 /  52   (<2,8> x 1    71 /  71)
 //   N = 101  <4,3> x 6   97 /  99   (<4,4> x 4   105 / 105, <4,2> x 8 128 / 249)
 //   N = 192  <6,4> x 6  273 / 275   (<6,3> x 8   306 / 605), <6,2> x 12 236 / 700

@@ -64,7 +64,8 @@ struct kls_multi {
   double schedule_ms[2] = {0, 0};   // mixed: eager-pass time of each schedule
   std::vector<int2> pairs;          // (model, omega) pairs
   int grid = 0, max_Na = 0, max_ldv = 0;
-  void* d_F = nullptr;              // FP64: F of the self-similar models, in turn
+  void* d_F = nullptr;              // FP64: F and partials of the self-similar models, in turn
+  double2* d_part = nullptr;
   int similar_ctas = 0, launches = 0;
   std::vector<int2> pairs_tab;      // FP64: (model, omega) pairs over the table
   int2* d_pairs_tab = nullptr;
@@ -254,7 +255,7 @@ int launch_batch(kls_multi* m) {
     for (int i = 0; !r && i < m->n_models; ++i)
       if (m->ctx[i]->sim)
         r = (int)kls_similar_launch(m->ctx[i], m->stream, m->batch, m->md[i].wt, m->d_F,
-                                    m->md[i].part, m->md[i].A, nullptr, &m->launches);
+                                    m->d_part, m->md[i].A, nullptr, &m->launches);
   } else {
     // the mixed weights are converted from the FP64 weights of the same pass
     r = kls_multi_launch_f64_weights(m->stream, m->d_md, m->d_pairs, np, m->max_K_pad);
@@ -486,7 +487,7 @@ int kls_multi_create(kls_ctx* const* models, int n_models, int mode, int batch, 
       else m->old = true;
     }
   }
-  size_t F_bytes = 0;
+  size_t F_bytes = 0, part_elems = 0;
   for (int i = 0; i < n_models; ++i) {
     kls_ctx* c = models[i];
     m->sim.push_back(c->sim);
@@ -507,7 +508,7 @@ int kls_multi_create(kls_ctx* const* models, int n_models, int mode, int batch, 
     if ((r = malloc_buf(m, &d.A, (size_t)batch * c->Na * c->Na))) return bail(r);
     if (mode == KLS_MODE_FP64) {
       if (c->sim) {
-        if ((r = malloc_buf(m, &d.part, kls_similar_part_elems(c, batch)))) return bail(r);
+        part_elems = std::max(part_elems, kls_similar_part_elems(c, batch));
         F_bytes = std::max(F_bytes, kls_similar_f_bytes(c, batch));
         m->similar_ctas += kls_similar_ctas(c) * batch;
         m->md[i] = d;
@@ -592,7 +593,8 @@ int kls_multi_create(kls_ctx* const* models, int n_models, int mode, int batch, 
   }
   if (F_bytes) {
     char* f = nullptr;
-    if ((r = malloc_buf(m, &f, F_bytes))) return bail(r);
+    if ((r = malloc_buf(m, &f, F_bytes)) || (r = malloc_buf(m, &m->d_part, part_elems)))
+      return bail(r);
     m->d_F = f;
   }
   if ((r = build_items(m))) return bail(r);

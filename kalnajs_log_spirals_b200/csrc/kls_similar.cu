@@ -1029,8 +1029,14 @@ int kls_similar_chunk(const kls_ctx* c, int n) {
 size_t kls_similar_f_bytes(const kls_ctx* c, int n) {
   return f_bytes(c->sim) * kls_similar_chunk(c, n);
 }
-size_t kls_similar_part_elems(const kls_ctx* c, int n) {   // double2
-  return (size_t)n * c->sim->n_tiles * 2 * c->splits * PR_SLOT * 2;
+// omegas whose partials are held at once (1 GB, at least one), and their size in double2
+// (a batch of 4096 omegas of N_alpha = 33 and 1071 rows: 71 GB of them)
+int kls_similar_part_chunk(const kls_ctx* c, int n) {
+  const size_t one = (size_t)c->sim->n_tiles * 2 * c->splits * PR_SLOT * sizeof(double4);
+  return (int)std::max<size_t>(1, std::min<size_t>(n, ((size_t)1 << 30) / one));
+}
+size_t kls_similar_part_elems(const kls_ctx* c, int n) {
+  return (size_t)kls_similar_part_chunk(c, n) * c->sim->n_tiles * 2 * c->splits * PR_SLOT * 2;
 }
 int kls_similar_ctas(const kls_ctx* c) { return pair_ctas(c->sim, c->splits); }
 
@@ -1045,23 +1051,28 @@ cudaError_t kls_similar_launch(const kls_ctx* c, cudaStream_t st, int n, const d
       (e = cudaFuncSetAttribute(pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)PR_SMEM)) != cudaSuccess)
     return e;
-  const int nf = kls_similar_chunk(c, n);
+  const int nf = kls_similar_chunk(c, n), np = kls_similar_part_chunk(c, n);
   double4* F0 = reinterpret_cast<double4*>(F);
   float4* Fc = reinterpret_cast<float4*>(F0 + (size_t)nf * s->R * s->Nap);
   double4* p4 = reinterpret_cast<double4*>(part);
   const size_t slots = (size_t)s->n_tiles * 2 * c->splits * PR_SLOT;
-  for (int b = 0; b < n; b += nf) {
-    const int m = std::min(nf, n - b);
-    fourier_kernel<<<dim3(s->Nap / FA_D, (s->R + FA_R - 1) / FA_R, m), FA_THREADS, FA_SMEM, st>>>(
-        s->R, c->Ne, c->NR, s->K2p, s->Nap, c->K_pad, wt + (size_t)b * c->K_pad, s->U, s->Phi,
-        s->rot, F0, Fc);
-    pair_kernel<<<dim3(s->n_tiles, 2 * c->splits, m), PR_THREADS, PR_SMEM, st>>>(
-        s->R, c->Na, s->Nap, c->ldv, c->splits, s->n_tiles, s->tiles, s->V, s->Vf, s->D, F0, Fc,
-        p4 + b * slots);
-    *launches += 2;
+  // ranges of omegas p0 .. p1 - 1 whose partials are reduced together
+  for (int p0 = 0, p1; p0 < n; p0 = p1) {
+    p1 = std::min(n, p0 + np);
+    for (int b = p0; b < p1; b += nf) {
+      const int m = std::min(nf, p1 - b);
+      fourier_kernel<<<dim3(s->Nap / FA_D, (s->R + FA_R - 1) / FA_R, m), FA_THREADS, FA_SMEM, st>>>(
+          s->R, c->Ne, c->NR, s->K2p, s->Nap, c->K_pad, wt + (size_t)b * c->K_pad, s->U, s->Phi,
+          s->rot, F0, Fc);
+      pair_kernel<<<dim3(s->n_tiles, 2 * c->splits, m), PR_THREADS, PR_SMEM, st>>>(
+          s->R, c->Na, s->Nap, c->ldv, c->splits, s->n_tiles, s->tiles, s->V, s->Vf, s->D, F0, Fc,
+          p4 + (b - p0) * slots);
+      *launches += 2;
+    }
+    pair_reduce_kernel<<<dim3(s->n_tiles, PR_SLOT / 64, p1 - p0), 256, 0, st>>>(
+        c->Na, c->splits, s->n_tiles, c->cfg.G, c->d_N, s->tiles, p4,
+        A + (size_t)p0 * c->Na * c->Na, p0 ? nullptr : M);
+    *launches += 1;
   }
-  pair_reduce_kernel<<<dim3(s->n_tiles, PR_SLOT / 64, n), 256, 0, st>>>(
-      c->Na, c->splits, s->n_tiles, c->cfg.G, c->d_N, s->tiles, p4, A, M);
-  *launches += 1;
   return cudaGetLastError();
 }
